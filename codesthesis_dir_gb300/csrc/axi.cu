@@ -9,24 +9,30 @@
 //
 // Layout: each field is a column-major (0:ld-1, 0:nz) array with ld = nr+1,
 // the ten fields of an instance in one allocation.  The multigrid keeps the
-// full-size psif and rc arrays, per level the packed v / f slots, the
-// factored r-line matrix (one per level: its coefficients vary with r only)
-// and one factored z-line matrix per r-row (its diagonal holds -1/r^2).
+// packed v / f slots per level, one residual array, the factored r-line
+// matrix (one per level: its coefficients vary with r only) and one factored
+// z-line matrix per r-row (its diagonal holds -1/r^2).
 //
-// The multigrid solve is one persistent block: the sweep loop, every level
-// and the convergence test run in one launch.  LEX orders the lines as the
-// reference does (rows j = 1..n2-1, then columns i = 1..n1-1, rotann2.f:
-// 698-725) and one thread marches them; ZEBRA solves odd lines, then even
-// lines, one thread per line.
+// The multigrid solve is one launch of one cluster of CTAs (cluster.cuh): the
+// sweep loop, every level and the convergence test run in it.  LEX orders the
+// lines as the reference does (rows j = 1..n2-1, then columns i = 1..n1-1,
+// rotann2.f:698-725), one line after the other; ZEBRA solves odd lines, then
+// even lines.  Mixed precision runs its FP32 cycles in the cluster's shared
+// memory where they fit (meridian.cu).
 #include <math.h>
 #include <stdint.h>
 #include <string.h>
 
 #include <vector>
 
+#include <algorithm>
+
 #include "banded.cuh"
+#include "cluster.cuh"
 #include "gbcommon.cuh"
+#include "meridian.cuh"
 #include "str_internal.cuh"
+#include "warpline.cuh"
 
 #define AXI_THREADS 512
 #define AXI_MAXLEV 8
@@ -35,10 +41,11 @@
 struct AxiLevel {
     int n1, n2, lf;           // sizes; lf = 2^l / 2 scales i into rval
     double hr, hz, hhr, hhz;
+    double ihr, ihhr, ihhz;   // their reciprocals (IEEE)
     double *v, *f;            // packed (n1+1)*(n2+1)
-    double *fac_r;            // r-line factors, 3 (n1-1)
-    double *fac_z;            // z-line factors, 3 (n2-1) for each i = 1..n1-1
-    // mixed precision: FP32 correction cycle (pivots stored as reciprocals)
+    double *fac_r;            // r-line factors, tdma_fac_len(n1-1)
+    double *fac_z;            // z-line factors, tdma_fac_len(n2-1) for each i = 1..n1-1
+    // mixed precision: FP32 correction cycle (folded line tables)
     float *v32, *f32, *fac_r32, *fac_z32;
 };
 
@@ -59,8 +66,9 @@ struct AxiDev {
     double cf1, cf2, cf3, cf4, tolcon;
     double *f[GB_A_COUNT];
     double *rval;             // rotann2.f:626: rval(i) = i hr(1) + r0
-    double *psif, *rc;
-    float *psif32, *rc32, *rval32;
+    double *irv, *irq;        // 1/rval and 1/(rval rval) (IEEE)
+    double *rc;               // the residual of the level it was last formed on, pitch n1 + 1
+    float *rc32, *rval32;
     AxiLevel lev[AXI_MAXLEV];
     double *heat;
     unsigned long long *errmax;   // bit patterns of the step's max |x - x_p|, x = omega, v, T
@@ -448,112 +456,195 @@ __global__ void k_axi_record(AxiDev d) { k_axi_record_body(d, blockIdx.x); }
 // ---------------------------------------------------------------------------
 // Streamfunction multigrid (rotann2.f:543-854)
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ double axi_blk_max(double v, double *s_red)
+template <class T> struct AxiView {
+    int n1, n2, ld, lf;
+    T *v;
+    const T *f;
+    T hr, hhr, hhz, ihr, ihhr, ihhz;
+    const T *rval, *irv, *irq;   // float: rval only
+    const T *fac[2];             // r-lines (one table), z-lines
+};
+__device__ __forceinline__ AxiView<double> axi_view(const AxiDev &d, int l, double)
 {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, o));
-    if (lane == 0) s_red[warp] = v;
-    __syncthreads();
-    if (warp == 0) {
-        v = (lane < nw) ? s_red[lane] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, o));
-        if (lane == 0) s_red[32] = v;
+    const AxiLevel &L = d.lev[l];
+    return {L.n1, L.n2, L.n1 + 1, L.lf, L.v, L.f, L.hr, L.hhr, L.hhz, L.ihr, L.ihhr, L.ihhz, d.rval, d.irv, d.irq, {L.fac_r, L.fac_z}};
+}
+__device__ __forceinline__ AxiView<float> axi_view(const AxiDev &d, int l, float)
+{
+    const AxiLevel &L = d.lev[l];
+    return {L.n1, L.n2, L.n1 + 1, L.lf, L.v32, L.f32, (float)L.hr, (float)L.hhr, (float)L.hhz, (float)L.ihr, (float)L.ihhr,
+            (float)L.ihhz, d.rval32, nullptr, nullptr, {L.fac_r32, L.fac_z32}};
+}
+#define V(i, j) L.v[(i) + L.ld * (j)]
+#define F(i, j) L.f[(i) + L.ld * (j)]
+
+// x / h: the IEEE quotient from the stored reciprocal, or a product with it
+__device__ __forceinline__ double axi_over(double x, double h, double ih) { return div_by_rcp(x, h, ih); }
+__device__ __forceinline__ float axi_over(float x, float, float ih) { return x * ih; }
+
+// Right-hand sides of r-line j at row i (rotann2.f:698-710) and of z-line i
+// at row j (rotann2.f:712-725).
+template <class T> __device__ __forceinline__ T axi_rhs(const AxiView<T> &L, int dir, int i, int j)
+{
+    if (dir == 0) return axi_over(-(V(i, j + 1) + V(i, j - 1)), L.hhz, L.ihhz) + F(i, j);
+    const T rv = L.rval[i * L.lf];
+    T irv;
+    if constexpr (sizeof(T) == 8) irv = L.irv[i * L.lf];
+    else irv = 1.0f / rv;
+    const T vp = V(i + 1, j), vm = V(i - 1, j);
+    return axi_over(-(vp + vm), L.hhr, L.ihhr) + F(i, j) - axi_over(axi_over((vp - vm) * T(0.5), rv, irv), L.hr, L.ihr);
+}
+
+// f - A v at (i, j) (relax's residual, rotann2.f:727-741)
+template <class T> __device__ __forceinline__ T axi_resid(const AxiView<T> &L, T drdz, int i, int j)
+{
+    const T rv = L.rval[i * L.lf];
+    T irv, irq;
+    if constexpr (sizeof(T) == 8) {
+        irv = L.irv[i * L.lf];
+        irq = L.irq[i * L.lf];
+    } else {
+        irv = 1.0f / rv;
+        irq = irv * irv;
     }
-    __syncthreads();
-    const double r = s_red[32];
-    __syncthreads();
-    return r;
+    const T vp = V(i + 1, j), vm = V(i - 1, j), vc = V(i, j);
+    const T a = axi_over(vp + vm, L.hhr, L.ihhr) + axi_over(axi_over((vp - vm) * T(0.5), L.hr, L.ihr), rv, irv) -
+                axi_over(vc, rv * rv, irq) + axi_over(V(i, j + 1) + V(i, j - 1), L.hhz, L.ihhz) - vc * drdz;
+    return F(i, j) - a;
 }
 
-// r-line j of relax (rotann2.f:698-710).
-__device__ __forceinline__ void axi_rline(const AxiDev &d, const AxiLevel &L, int j)
-{
-    const int ld = d.ld, n1 = L.n1;
-    double *psif = d.psif;
-    const double *f = L.f;
-    const double hhz = L.hhz;
-    auto rhs = [&](int q) -> double {
-        const int i = q + 1;
-        return -(psif[AX(i, j + 1)] + psif[AX(i, j - 1)]) / hhz + f[(size_t)j * (n1 + 1) + i];
-    };
-    apply_tdma_rhs(L.fac_r, n1 - 1, psif + AX(1, j), 1, rhs);
-}
+// Dynamic shared memory of a solve: per staged line its right-hand sides and
+// its factors.
+#define AXI_SMEM_BYTES (160 * 1024)
 
-// z-line i of relax (rotann2.f:712-725).
-__device__ __forceinline__ void axi_zline(const AxiDev &d, const AxiLevel &L, int i)
+// The nl lines first, first + step, ... of one direction (DIR 0: r-lines j,
+// DIR 1: z-lines i), which read none of one another: a colour, or one line of
+// the reference's order.  Each CTA takes a contiguous share, in batches that
+// fit its shared memory: the lines' factors are copied there while all
+// threads form the right-hand sides, the lines are eliminated (FP64: one
+// thread per line in the reference's order; FP32: up to 32 lanes per line),
+// the solutions go back.
+template <class T, int DIR>
+__device__ __noinline__ void axi_lines(const AxiDev &d, int l, int first, int step, int nl)
 {
-    const int ld = d.ld, n1 = L.n1, n2 = L.n2;
-    double *psif = d.psif;
-    const double *f = L.f;
-    const double hhr = L.hhr, hr = L.hr, rv = d.rval[i * L.lf];
-    auto rhs = [&](int q) -> double {
-        const int j = q + 1;
-        return -(psif[AX(i + 1, j)] + psif[AX(i - 1, j)]) / hhr + f[(size_t)j * (n1 + 1) + i] -
-               (psif[AX(i + 1, j)] - psif[AX(i - 1, j)]) * 0.5 / rv / hr;
-    };
-    apply_tdma_rhs(L.fac_z + (size_t)(i - 1) * tdma_fac_len(n2 - 1), n2 - 1, psif + AX(i, 1), ld, rhs);
-}
-
-// relax (rotann2.f:668-753): psif from v, nrel sweeps of r-lines then
-// z-lines with the residual after each, psif back into v.  Returns the last
-// residual max norm; *nan_out is set (block-uniform) on a NaN residual.
-__device__ double axi_relax(const AxiDev &d, int klev, double *s_red, int *nan_out)
-{
-    const AxiLevel &L = d.lev[klev];
-    const int ld = d.ld, n1 = L.n1, n2 = L.n2;
-    const double hhr = L.hhr, hhz = L.hhz, hr = L.hr;
-    double *psif = d.psif, *rc = d.rc;
-    const int tp = (n1 + 1) * (n2 + 1);
-    for (int idx = threadIdx.x; idx < tp; idx += blockDim.x) {
-        const int j = idx / (n1 + 1), i = idx - j * (n1 + 1);
-        psif[AX(i, j)] = L.v[idx];
+    extern __shared__ __align__(16) unsigned char s_axi[];
+    constexpr bool F64 = sizeof(T) == 8;
+    T *smem = (T *)s_axi;
+    const Cluster cl = Cluster::self();
+    const AxiView<T> L = axi_view(d, l, T(0));
+    const int n = DIR == 0 ? L.n1 - 1 : L.n2 - 1;
+    const int flen = (int)(F64 ? tdma_fac_len(n) : tdma32_len(n));
+    const int fpitch = DIR == 0 ? 0 : F64 ? flen | 1 : flen;   // r-lines share one table
+    const int lpitch = F64 ? 0 : wl_pitch(n), lg = F64 ? 0 : wl_log2m(n);
+    const int share = (nl + cl.size - 1) / cl.size;
+    const int t0 = cl.rank * share, t1 = min(nl, t0 + share);
+    const int words = (int)(AXI_SMEM_BYTES / sizeof(T)) - (DIR == 0 ? (flen + 3) & ~3 : 0);
+    int B = F64 ? (words - n) / (n + fpitch) : words / (lpitch + fpitch);
+    const bool staged = B >= 1;       // a line with its factors fits (n up to 4000 in FP64)
+    if (!staged) B = 1;
+    B = min(B, min(share, (int)blockDim.x));
+    T *sfac = smem, *x = !staged ? smem : smem + (DIR == 0 ? (flen + 3) & ~3 : B * fpitch);
+    auto table = [&](int line) { return L.fac[DIR] + (DIR == 0 ? 0 : (size_t)(line - 1) * flen); };
+    for (int b0 = t0; b0 < t1; b0 += B) {
+        const int nb = min(B, t1 - b0), pitch = nb | 1;
+        // FP64: [row][line], odd pitch; FP32: [line][row], padded per lane
+        auto at = [&](int t, int q) -> T & { return F64 ? x[q * pitch + t] : x[t * lpitch + wl_slot(lg, q)]; };
+        if (staged)
+            for (int t = 0; t < (DIR == 0 ? 1 : nb); ++t)
+                async_copy(sfac + t * fpitch, table(first + step * (b0 + t)), flen, threadIdx.x, blockDim.x);
+        if (DIR == 0) {
+            const RowSplit split(n);
+            for (int idx = threadIdx.x; idx < nb * n; idx += blockDim.x) {
+                int t, q;
+                split(idx, t, q);
+                at(t, q) = axi_rhs<T>(L, 0, q + 1, first + step * (b0 + t));
+            }
+        } else {
+            const RowSplit split(nb);
+            for (int idx = threadIdx.x; idx < nb * n; idx += blockDim.x) {
+                int q, t;
+                split(idx, q, t);
+                at(t, q) = axi_rhs<T>(L, 1, first + step * (b0 + t), q + 1);
+            }
+        }
+        if constexpr (!F64) {   // rows past the line's end
+            const int pad = wl_rows(n) - n;
+            for (int idx = threadIdx.x; idx < nb * pad; idx += blockDim.x) at(idx / pad, n + idx % pad) = T(0);
+        }
+        async_copy_wait();
+        __syncthreads();
+        if constexpr (F64) {
+            if ((int)threadIdx.x < nb) {
+                const int t = threadIdx.x;
+                if (staged) tdma_staged(sfac + t * fpitch, n, x + t, pitch);
+                else tdma_staged(table(first + step * (b0 + t)), n, x + t, pitch);
+            }
+        } else {
+            if (staged) wl_lines<false>(sfac, fpitch, n, x, lpitch, nb);
+            else wl_lines<false>(table(first + step * b0), DIR == 0 ? 0 : (size_t)step * flen, n, x, lpitch, nb);
+        }
+        __syncthreads();
+        if (DIR == 0) {
+            const RowSplit split(n);
+            for (int idx = threadIdx.x; idx < nb * n; idx += blockDim.x) {
+                int t, q;
+                split(idx, t, q);
+                V(q + 1, first + step * (b0 + t)) = at(t, q);
+            }
+        } else {
+            const RowSplit split(nb);
+            for (int idx = threadIdx.x; idx < nb * n; idx += blockDim.x) {
+                int q, t;
+                split(idx, q, t);
+                V(first + step * (b0 + t), q + 1) = at(t, q);
+            }
+        }
+        if (b0 + B < t1) __syncthreads();
     }
-    __syncthreads();
-    const double drdz = 2.0 * (1.0 / hhr + 1.0 / hhz);
-    double m = 0.0;
-    int nan = 0;
+    cl.sync();
+}
+
+// relax's line sweeps (rotann2.f:668-725), nrel of them, in place on v.  The
+// reference also forms the residual after every sweep; only the last one is
+// ever read, and the caller forms that.
+template <class T> __device__ __forceinline__ void axi_sweeps(const AxiDev &d, int l)
+{
+    const int nj = d.lev[l].n2 - 1, ni = d.lev[l].n1 - 1;
     for (int irel = 0; irel < d.nrel; ++irel) {
         if (d.mode == GB_SMOOTHER_LEX) {
-            if (threadIdx.x == 0)
-                for (int j = 1; j <= n2 - 1; ++j) axi_rline(d, L, j);
-            __syncthreads();
-            if (threadIdx.x == 0)
-                for (int i = 1; i <= n1 - 1; ++i) axi_zline(d, L, i);
-            __syncthreads();
+            for (int j = 1; j <= nj; ++j) axi_lines<T, 0>(d, l, j, 1, 1);
+            for (int i = 1; i <= ni; ++i) axi_lines<T, 1>(d, l, i, 1, 1);
         } else {
-            for (int par = 1; par >= 0; --par) {
-                for (int t = threadIdx.x; 2 * t + 2 - par <= n2 - 1; t += blockDim.x) axi_rline(d, L, 2 * t + 2 - par);
-                __syncthreads();
-            }
-            for (int par = 1; par >= 0; --par) {
-                for (int t = threadIdx.x; 2 * t + 2 - par <= n1 - 1; t += blockDim.x) axi_zline(d, L, 2 * t + 2 - par);
-                __syncthreads();
-            }
+            for (int c = 1; c <= 2; ++c)
+                if (c <= nj) axi_lines<T, 0>(d, l, c, 2, (nj - c) / 2 + 1);
+            for (int c = 1; c <= 2; ++c)
+                if (c <= ni) axi_lines<T, 1>(d, l, c, 2, (ni - c) / 2 + 1);
         }
-        m = 0.0;
-        nan = 0;
-        const int ni = n1 - 1, tot = ni * (n2 - 1);
-        for (int idx = threadIdx.x; idx < tot; idx += blockDim.x) {
-            const int j = idx / ni + 1, i = idx - (j - 1) * ni + 1;
-            const double rv = d.rval[i * L.lf];
-            double temp = (psif[AX(i + 1, j)] + psif[AX(i - 1, j)]) / hhr +
-                          (psif[AX(i + 1, j)] - psif[AX(i - 1, j)]) * 0.5 / hr / rv -
-                          psif[AX(i, j)] / (rv * rv) + (psif[AX(i, j + 1)] + psif[AX(i, j - 1)]) / hhz -
-                          psif[AX(i, j)] * drdz;
-            temp = L.f[(size_t)j * (n1 + 1) + i] - temp;
-            rc[AX(i, j)] = temp;
-            temp = fabs(temp);
-            if (temp != temp) nan = 1;
-            if (temp > m) m = temp;
-        }
-        nan = __syncthreads_or(nan);
-        m = axi_blk_max(m, s_red);
     }
-    for (int idx = threadIdx.x; idx < tp; idx += blockDim.x) {
-        const int j = idx / (n1 + 1), i = idx - j * (n1 + 1);
-        L.v[idx] = psif[AX(i, j)];
+}
+
+// The residual of level l into rc (not followed by a barrier): its largest
+// magnitude and whether one is a NaN over the calling thread's points.
+template <class T, class R> __device__ __noinline__ T axi_residual(const AxiDev &d, int l, R *rc, int *nan_out)
+{
+    const Cluster cl = Cluster::self();
+    const AxiView<T> L = axi_view(d, l, T(0));
+    const T drdz = T(2.0) * (T(1.0) / L.hhr + T(1.0) / L.hhz);
+    const int ni = L.n1 - 1, tot = ni * (L.n2 - 1);
+    const RowSplit split(ni);
+    T m = T(0);
+    int nan = 0;
+    for (int idx = cl.tid(); idx < tot; idx += cl.nthr()) {
+        int j, i;
+        split(idx, j, i);
+        ++i;
+        ++j;
+        const T r = axi_resid<T>(L, drdz, i, j);
+        rc[i + L.ld * j] = (R)r;
+        const T a = fabs(r);
+        if (a != a) nan = 1;
+        if (a > m) m = a;
     }
-    __syncthreads();
     *nan_out = nan;
     return m;
 }
@@ -562,409 +653,228 @@ __device__ double axi_relax(const AxiDev &d, int klev, double *s_red, int *nan_o
 // packed coarse right-hand side; the rows and columns the reference clears
 // (i = 0, n1c and j = 0, n1c: n1 of the coarse level in both directions)
 // are zero, and the coarse solution slot is cleared.
-__device__ void axi_corser(const AxiDev &d, int klev)
+template <class T> __device__ __noinline__ void axi_corser(const AxiDev &d, int l, const T *rc)
 {
-    const int ld = d.ld;
-    const int n1c = d.lev[klev + 1].n1, n2c = d.lev[klev + 1].n2;
-    const double *rf = d.rc;
-    double *fc = d.lev[klev + 1].f, *vc = d.lev[klev + 1].v;
+    const Cluster cl = Cluster::self();
+    const AxiView<T> L = axi_view(d, l + 1, T(0));
+    const int ld = 2 * L.n1 + 1;
+    const int n1c = L.n1, n2c = L.n2;
     const int tot = (n1c + 1) * (n2c + 1);
-    for (int idx = threadIdx.x; idx < tot; idx += blockDim.x) {
-        const int j = idx / (n1c + 1), i = idx - j * (n1c + 1);
-        double temp = 0.0;
+    const RowSplit split(n1c + 1);
+    T *fc = const_cast<T *>(L.f);
+    for (int idx = cl.tid(); idx < tot; idx += cl.nthr()) {
+        int j, i;
+        split(idx, j, i);
+        T temp = T(0);
         if (i >= 1 && i <= n1c - 1 && j >= 1 && j <= n2c - 1 && j != n1c) {
-            const int ii = i + i, jj = j + j;
-            temp = rf[AX(ii, jj)];
-            temp = temp * 2.0 + rf[AX(ii + 1, jj)] + rf[AX(ii - 1, jj)];
-            temp = temp + rf[AX(ii, jj + 1)] + rf[AX(ii, jj - 1)];
-            temp = temp * 2.0 + rf[AX(ii + 1, jj + 1)] + rf[AX(ii - 1, jj - 1)];
-            temp = temp + rf[AX(ii + 1, jj - 1)] + rf[AX(ii - 1, jj + 1)];
-            temp = temp / 16.0;
+            const T *q = rc + (i + i) + ld * (j + j);
+            temp = q[0];
+            temp = temp * T(2) + q[1] + q[-1];
+            temp = temp + q[ld] + q[-ld];
+            temp = temp * T(2) + q[1 + ld] + q[-1 - ld];
+            temp = temp + q[1 - ld] + q[-1 + ld];
+            temp = temp * T(0.0625);   // / 16, exactly
         }
         fc[idx] = temp;
-        vc[idx] = 0.0;
+        L.v[idx] = T(0);
     }
-    __syncthreads();
+    cl.sync();
 }
 
-// finer (rotann2.f:803-854): bilinear prolongation of the coarse solution
-// plus the saved fine solution into psif, the coarse slot cleared, psif
-// packed into the fine slot.
-__device__ void axi_finer(const AxiDev &d, int klev)
+// finer (rotann2.f:803-854): bilinear prolongation added to the fine level.
+// The coarse solution slot is cleared by the next corser.
+template <class T> __device__ __noinline__ void axi_finer(const AxiDev &d, int l)
 {
-    const int ld = d.ld;
-    const int n1c = d.lev[klev].n1;
-    const int n1f = d.lev[klev - 1].n1, n2f = d.lev[klev - 1].n2;
-    const double *vc = d.lev[klev].v;
-    double *vf = d.lev[klev - 1].v, *psif = d.psif;
-    const int tot = (n1f + 1) * (n2f + 1);
-#define PC(ii, jj) vc[(size_t)(jj) * (n1c + 1) + (ii)]
-    for (int idx = threadIdx.x; idx < tot; idx += blockDim.x) {
-        const int j = idx / (n1f + 1), i = idx - j * (n1f + 1);
-        const int i1 = i / 2, j1 = j / 2;
-        double p;
-        if (i1 * 2 == i) {
-            if (j1 * 2 == j) p = PC(i1, j1);
-            else p = (PC(i1, j1) + PC(i1, j1 + 1)) * 0.5;
-        } else {
-            if (j1 * 2 == j) {
-                p = (PC(i1, j1) + PC(i1 + 1, j1)) * 0.5;
-            } else {
-                double temp = PC(i1, j1) + PC(i1 + 1, j1 + 1);
-                temp = temp + PC(i1, j1 + 1) + PC(i1 + 1, j1);
-                p = temp * 0.25;
-            }
-        }
-        psif[AX(i, j)] = p + vf[idx];
+    const Cluster cl = Cluster::self();
+    const AxiView<T> Cc = axi_view(d, l, T(0)), L = axi_view(d, l - 1, T(0));
+    const int tot = L.ld * (L.n2 + 1);
+    const RowSplit split(L.ld);
+    for (int idx = cl.tid(); idx < tot; idx += cl.nthr()) {
+        int j, i;
+        split(idx, j, i);
+        const T *q = Cc.v + (i >> 1) + Cc.ld * (j >> 1);
+        T p;
+        if (!(i & 1)) p = !(j & 1) ? q[0] : (q[0] + q[Cc.ld]) * T(0.5);
+        else if (!(j & 1)) p = (q[0] + q[1]) * T(0.5);
+        else p = (q[0] + q[Cc.ld + 1] + q[Cc.ld] + q[1]) * T(0.25);
+        L.v[idx] = p + L.v[idx];
     }
-#undef PC
-    __syncthreads();
-    const int tc = (n1c + 1) * (d.lev[klev].n2 + 1);
-    for (int idx = threadIdx.x; idx < tc; idx += blockDim.x) d.lev[klev].v[idx] = 0.0;
-    for (int idx = threadIdx.x; idx < tot; idx += blockDim.x) {
-        const int j = idx / (n1f + 1), i = idx - j * (n1f + 1);
-        vf[idx] = psif[AX(i, j)];
-    }
-    __syncthreads();
+    cl.sync();
 }
 
 // poisson (rotann2.f:598-666): phi from omegn.
-__device__ __forceinline__ void k_axi_mg_solve_body(const AxiDev &d, int bidx)
+__device__ __forceinline__ void k_axi_mg_solve_body(const AxiDev &d)
 {
-    __shared__ double s_red[33];
-    if (*d.abort) return;
-    const int ld = d.ld, nlev = d.nlev;
-    const AxiLevel &L1 = d.lev[1];
-    const int n1 = L1.n1, n2 = L1.n2;
+    __shared__ ClMaxState s_max;
+    const Cluster cl = Cluster::self();
+    if (*d.abort) return;   // the same for every CTA: nothing sets it while the solve runs
+    int turn = 0;
+    const int nlev = d.nlev;
+    const AxiView<double> L = axi_view(d, 1, 0.0);
+    const int tp = L.ld * (L.n2 + 1);
     double *psi = d.f[GB_A_phi];
     const double *rhs = d.f[GB_A_omegn];
-    const int tp = (n1 + 1) * (n2 + 1);
-    for (int idx = threadIdx.x; idx < tp; idx += blockDim.x) {
-        const int j = idx / (n1 + 1), i = idx - j * (n1 + 1);
-        L1.f[idx] = rhs[AX(i, j)];
-        L1.v[idx] = psi[AX(i, j)];
-        d.rc[AX(i, j)] = 0.0;
+    for (int idx = cl.tid(); idx < tp; idx += cl.nthr()) {
+        const_cast<double *>(L.f)[idx] = rhs[idx];
+        L.v[idx] = psi[idx];
     }
-    __syncthreads();
-    int status = GB_MAXSWEEPS, sweeps = d.maxsweeps, nan1 = 0, nn = 0;
+    cl.sync();
     double res1 = 0.0;
+    int status = GB_MAXSWEEPS, sweeps = d.maxsweeps, nan1 = 0;
+    // relax on level l and the residual for the restriction or the test that
+    // follows; the norm matters on level 1 only
+    auto relax = [&](int l, bool restricted) {
+        axi_sweeps<double>(d, l);
+        if (l != 1 && !restricted) return;
+        int nan;
+        const double m = axi_residual<double>(d, l, d.rc, &nan);
+        if (l == 1) {
+            res1 = cl_max(cl, s_max, turn, m, nan);
+            nan1 = nan;
+        } else {
+            cl.sync();
+        }
+    };
     for (int sweep = 1; sweep <= d.maxsweeps; ++sweep) {
-        if (sweep == 1 || nlev == 1) res1 = axi_relax(d, 1, s_red, &nan1);
-        if (nlev > 1) {
-            for (int l = 1; l <= nlev - 1; ++l) {
-                axi_corser(d, l);
-                axi_relax(d, l + 1, s_red, &nn);
-            }
-            for (int l = nlev; l >= 2; --l) {
-                axi_finer(d, l);
-                const double r = axi_relax(d, l - 1, s_red, &nn);
-                if (l - 1 == 1) { res1 = r; nan1 = nn; }
-            }
+        if (sweep == 1 || nlev == 1) relax(1, true);
+        for (int l = 1; l <= nlev - 1; ++l) {
+            axi_corser<double>(d, l, d.rc);
+            relax(l + 1, l + 1 < nlev);
+        }
+        for (int l = nlev; l >= 2; --l) {
+            axi_finer<double>(d, l);
+            relax(l - 1, false);
         }
         if (nan1) { status = GB_NAN; sweeps = sweep; break; }
         if (res1 < d.tolcon) {
-            for (int idx = threadIdx.x; idx < tp; idx += blockDim.x) {
-                const int j = idx / (n1 + 1), i = idx - j * (n1 + 1);
-                psi[AX(i, j)] = d.psif[AX(i, j)];
-            }
+            for (int idx = cl.tid(); idx < tp; idx += cl.nthr()) psi[idx] = L.v[idx];
             status = GB_OK;
             sweeps = sweep;
             break;
         }
     }
-    if (threadIdx.x == 0) {
+    if (cl.tid() == 0) {
         d.status[0] = status;
         d.status[1] = sweeps;
         if (status == GB_NAN) *d.abort = 1;
     }
+    cl.sync();   // no CTA leaves while another may still read its reduction slot
 }
 
-__global__ void __maxnreg__(128) k_axi_mg_solve(AxiDev d) { k_axi_mg_solve_body(d, blockIdx.x); }
+__global__ void __maxnreg__(128) k_axi_mg_solve(const __grid_constant__ AxiDev d) { k_axi_mg_solve_body(d); }
 
 // ---------------------------------------------------------------------------
 // Mixed precision: FP64 defect correction around one FP32 V-cycle of the
 // reference's schedule (relax on the finest level, down, up) on A e = r from
-// e = 0; psi += e in FP64 (AXI has no over-relaxation).  Zebra colours stage
-// their lines in shared memory ([row][line], odd pitch) for the elimination.
+// e = 0; psi += e in FP64 (AXI has no over-relaxation).  This form, on global
+// memory, serves the reference's line order and grids whose cycles do not fit
+// a cluster's shared memory; meridian.cu has the other.
 // ---------------------------------------------------------------------------
-#define AX32_LINE_FLOATS 24576
-#define AX32_SMEM_BYTES (AX32_LINE_FLOATS * 4)
-
-__device__ __forceinline__ void tdma32_pitch(const float *fac, int n, float *x, int pitch)
+__device__ __forceinline__ void k_axi_mg_solve_mixed_body(const AxiDev &d)
 {
-    const float *fact = fac, *ibp = fac + n, *c = fac + 2 * n;
-    float prev = x[0];
-#pragma unroll 4
-    for (int j = 1; j < n; ++j) {
-        prev = x[j * pitch] - fact[j] * prev;
-        x[j * pitch] = prev;
-    }
-    float y = prev * ibp[n - 1];
-    x[(n - 1) * pitch] = y;
-#pragma unroll 4
-    for (int j = n - 2; j >= 0; --j) {
-        y = (x[j * pitch] - c[j] * y) * ibp[j];
-        x[j * pitch] = y;
-    }
-}
-
-// right-hand side of r-line j (dir 0) or z-line i (dir 1) at row q+1
-__device__ __forceinline__ float axi_rhs32(const AxiDev &d, const AxiLevel &L, int dir, int line, int q)
-{
-    const int ld = d.ld, n1 = L.n1;
-    const float *psif = d.psif32;
-    if (dir == 0) {
-        const int i = q + 1, j = line;
-        return -(psif[AX(i, j + 1)] + psif[AX(i, j - 1)]) / (float)L.hhz + L.f32[(size_t)j * (n1 + 1) + i];
-    }
-    const int i = line, j = q + 1;
-    const float rv = d.rval32[i * L.lf];
-    return -(psif[AX(i + 1, j)] + psif[AX(i - 1, j)]) / (float)L.hhr + L.f32[(size_t)j * (n1 + 1) + i] -
-           (psif[AX(i + 1, j)] - psif[AX(i - 1, j)]) * 0.5f / rv / (float)L.hr;
-}
-
-// one colour of zebra lines in direction dir, staged in shared memory
-__device__ void axi_colour32(const AxiDev &d, const AxiLevel &L, int dir, int parity)
-{
-    extern __shared__ float s_ax32[];
-    const int ld = d.ld;
-    const int nlen = dir == 0 ? L.n1 - 1 : L.n2 - 1;       // rows of a line
-    const int nl_all = dir == 0 ? L.n2 - 1 : L.n1 - 1;     // lines 1..nl_all
-    const int nlines = (nl_all + parity) / 2;              // lines 2t + 2 - parity
-    int B = AX32_LINE_FLOATS / nlen - 1;
-    if (B > nlines) B = nlines;
-    for (int b0 = 0; b0 < nlines; b0 += B) {
-        const int nb = (nlines - b0 < B) ? nlines - b0 : B;
-        const int pitch = nb | 1;
-        for (int t = threadIdx.x >> 5; t < nb; t += blockDim.x >> 5) {
-            const int line = 2 * (b0 + t) + 2 - parity;
-            for (int q = threadIdx.x & 31; q < nlen; q += 32) s_ax32[q * pitch + t] = axi_rhs32(d, L, dir, line, q);
-        }
-        __syncthreads();
-        for (int t = threadIdx.x; t < nb; t += blockDim.x) {
-            const int line = 2 * (b0 + t) + 2 - parity;
-            const float *fac = dir == 0 ? L.fac_r32 : L.fac_z32 + (size_t)(line - 1) * 3 * nlen;
-            tdma32_pitch(fac, nlen, s_ax32 + t, pitch);
-        }
-        __syncthreads();
-        for (int t = threadIdx.x >> 5; t < nb; t += blockDim.x >> 5) {
-            const int line = 2 * (b0 + t) + 2 - parity;
-            for (int q = threadIdx.x & 31; q < nlen; q += 32) {
-                const float v = s_ax32[q * pitch + t];
-                if (dir == 0) d.psif32[AX(q + 1, line)] = v;
-                else d.psif32[AX(line, q + 1)] = v;
-            }
-        }
-        __syncthreads();
-    }
-}
-
-// one line of the lexicographic order, marched by one thread
-__device__ void axi_line32_lex(const AxiDev &d, const AxiLevel &L, int dir, int line)
-{
-    const int ld = d.ld;
-    const int nlen = dir == 0 ? L.n1 - 1 : L.n2 - 1;
-    const float *fac = dir == 0 ? L.fac_r32 : L.fac_z32 + (size_t)(line - 1) * 3 * nlen;
-    float *x = dir == 0 ? d.psif32 + AX(1, line) : d.psif32 + AX(line, 1);
-    const int stride = dir == 0 ? 1 : ld;
-    const float *fact = fac, *ibp = fac + nlen, *c = fac + 2 * nlen;
-    float prev = axi_rhs32(d, L, dir, line, 0);
-    x[0] = prev;
-    for (int q = 1; q < nlen; ++q) {
-        prev = axi_rhs32(d, L, dir, line, q) - fact[q] * prev;
-        x[(size_t)q * stride] = prev;
-    }
-    float y = prev * ibp[nlen - 1];
-    x[(size_t)(nlen - 1) * stride] = y;
-    for (int q = nlen - 2; q >= 0; --q) {
-        y = (x[(size_t)q * stride] - c[q] * y) * ibp[q];
-        x[(size_t)q * stride] = y;
-    }
-}
-
-__device__ void axi_relax32(const AxiDev &d, int klev)
-{
-    const AxiLevel &L = d.lev[klev];
-    const int ld = d.ld, n1 = L.n1, n2 = L.n2;
-    for (int j = threadIdx.x >> 5; j <= n2; j += blockDim.x >> 5)
-        for (int i = threadIdx.x & 31; i <= n1; i += 32) d.psif32[AX(i, j)] = L.v32[(size_t)j * (n1 + 1) + i];
-    __syncthreads();
-    const float hhr = (float)L.hhr, hhz = (float)L.hhz, hr = (float)L.hr;
-    const float drdz = 2.0f * (1.0f / hhr + 1.0f / hhz);
-    for (int irel = 0; irel < d.nrel; ++irel) {
-        if (d.mode == GB_SMOOTHER_LEX) {
-            if (threadIdx.x == 0)
-                for (int j = 1; j <= n2 - 1; ++j) axi_line32_lex(d, L, 0, j);
-            __syncthreads();
-            if (threadIdx.x == 0)
-                for (int i = 1; i <= n1 - 1; ++i) axi_line32_lex(d, L, 1, i);
-            __syncthreads();
-        } else {
-            for (int par = 1; par >= 0; --par) axi_colour32(d, L, 0, par);
-            for (int par = 1; par >= 0; --par) axi_colour32(d, L, 1, par);
-        }
-    }
-    const float *psif = d.psif32;
-    for (int j = 1 + (threadIdx.x >> 5); j <= n2 - 1; j += blockDim.x >> 5)
-        for (int i = 1 + (threadIdx.x & 31); i <= n1 - 1; i += 32) {
-            const float rv = d.rval32[i * L.lf];
-            const float a = (psif[AX(i + 1, j)] + psif[AX(i - 1, j)]) / hhr +
-                            (psif[AX(i + 1, j)] - psif[AX(i - 1, j)]) * 0.5f / hr / rv - psif[AX(i, j)] / (rv * rv) +
-                            (psif[AX(i, j + 1)] + psif[AX(i, j - 1)]) / hhz - psif[AX(i, j)] * drdz;
-            d.rc32[AX(i, j)] = L.f32[(size_t)j * (n1 + 1) + i] - a;
-        }
-    for (int j = threadIdx.x >> 5; j <= n2; j += blockDim.x >> 5)
-        for (int i = threadIdx.x & 31; i <= n1; i += 32) L.v32[(size_t)j * (n1 + 1) + i] = psif[AX(i, j)];
-    __syncthreads();
-}
-
-__device__ void axi_corser32(const AxiDev &d, int klev)
-{
-    const int ld = d.ld;
-    const int n1c = d.lev[klev + 1].n1, n2c = d.lev[klev + 1].n2;
-    const float *rf = d.rc32;
-    float *fc = d.lev[klev + 1].f32, *vc = d.lev[klev + 1].v32;
-    for (int j = threadIdx.x >> 5; j <= n2c; j += blockDim.x >> 5)
-        for (int i = threadIdx.x & 31; i <= n1c; i += 32) {
-            float t = 0.f;
-            if (i >= 1 && i <= n1c - 1 && j >= 1 && j <= n2c - 1 && j != n1c) {
-                const int ii = i + i, jj = j + j;
-                t = 0.25f * rf[AX(ii, jj)] +
-                    0.125f * (rf[AX(ii + 1, jj)] + rf[AX(ii - 1, jj)] + rf[AX(ii, jj + 1)] + rf[AX(ii, jj - 1)]) +
-                    0.0625f * (rf[AX(ii + 1, jj + 1)] + rf[AX(ii - 1, jj - 1)] + rf[AX(ii + 1, jj - 1)] +
-                               rf[AX(ii - 1, jj + 1)]);
-            }
-            fc[(size_t)j * (n1c + 1) + i] = t;
-            vc[(size_t)j * (n1c + 1) + i] = 0.f;
-        }
-    __syncthreads();
-}
-
-__device__ void axi_finer32(const AxiDev &d, int klev)
-{
-    const int ld = d.ld;
-    const int n1c = d.lev[klev].n1, n2c = d.lev[klev].n2;
-    const int n1f = d.lev[klev - 1].n1, n2f = d.lev[klev - 1].n2;
-    const float *vc = d.lev[klev].v32;
-    float *vf = d.lev[klev - 1].v32, *psif = d.psif32;
-#define PC32(ii, jj) vc[(size_t)(jj) * (n1c + 1) + (ii)]
-    for (int j = threadIdx.x >> 5; j <= n2f; j += blockDim.x >> 5)
-        for (int i = threadIdx.x & 31; i <= n1f; i += 32) {
-            const int i1 = i / 2, j1 = j / 2;
-            float p;
-            if (i1 * 2 == i) p = (j1 * 2 == j) ? PC32(i1, j1) : (PC32(i1, j1) + PC32(i1, j1 + 1)) * 0.5f;
-            else if (j1 * 2 == j) p = (PC32(i1, j1) + PC32(i1 + 1, j1)) * 0.5f;
-            else p = (PC32(i1, j1) + PC32(i1 + 1, j1 + 1) + PC32(i1, j1 + 1) + PC32(i1 + 1, j1)) * 0.25f;
-            psif[AX(i, j)] = p + vf[(size_t)j * (n1f + 1) + i];
-        }
-#undef PC32
-    __syncthreads();
-    for (int q = threadIdx.x; q < (n1c + 1) * (n2c + 1); q += blockDim.x) d.lev[klev].v32[q] = 0.f;
-    for (int j = threadIdx.x >> 5; j <= n2f; j += blockDim.x >> 5)
-        for (int i = threadIdx.x & 31; i <= n1f; i += 32) vf[(size_t)j * (n1f + 1) + i] = psif[AX(i, j)];
-    __syncthreads();
-}
-
-__device__ __forceinline__ void k_axi_mg_solve_mixed_body(const AxiDev &d, int bidx)
-{
-    __shared__ double s_red[33];
+    __shared__ ClMaxState s_max;
+    const Cluster cl = Cluster::self();
     if (*d.abort) return;
-    const int ld = d.ld, nlev = d.nlev;
-    const AxiLevel &L1 = d.lev[1];
-    const int n1 = L1.n1, n2 = L1.n2;
-    double *psi = d.f[GB_A_phi], *psif = d.psif;
+    int turn = 0;
+    const int nlev = d.nlev;
+    const AxiView<double> L = axi_view(d, 1, 0.0);
+    const AxiView<float> L32 = axi_view(d, 1, 0.f);
+    const int tp = L.ld * (L.n2 + 1);
+    double *psi = d.f[GB_A_phi];
     const double *rhs = d.f[GB_A_omegn];
-    for (int idx = threadIdx.x; idx < (n1 + 1) * (n2 + 1); idx += blockDim.x) {
-        const int j = idx / (n1 + 1), i = idx - j * (n1 + 1);
-        L1.f[idx] = rhs[AX(i, j)];
-        psif[AX(i, j)] = psi[AX(i, j)];
+    for (int idx = cl.tid(); idx < tp; idx += cl.nthr()) {
+        const_cast<double *>(L.f)[idx] = rhs[idx];
+        L.v[idx] = psi[idx];
+        L32.v[idx] = 0.f;
     }
-    __syncthreads();
-    const double hhr = L1.hhr, hhz = L1.hhz, hr = L1.hr;
-    const double drdz = 2.0 * (1.0 / hhr + 1.0 / hhz);
-    const int ni = n1 - 1, tot = ni * (n2 - 1);
+    cl.sync();
+    auto relax = [&](int l, bool restricted) {
+        axi_sweeps<float>(d, l);
+        if (!restricted) return;
+        int nan;
+        axi_residual<float>(d, l, d.rc32, &nan);
+        cl.sync();
+    };
     int status = GB_MAXSWEEPS, cycles = 0;
     for (int it = 0;; ++it) {
-        // FP64 residual of the iterate (the relax residual, rotann2.f:727-741)
-        double m = 0.0;
-        int nan = 0;
-        for (int idx = threadIdx.x; idx < tot; idx += blockDim.x) {
-            const int j = idx / ni + 1, i = idx - (j - 1) * ni + 1;
-            const double rv = d.rval[i];
-            double temp = (psif[AX(i + 1, j)] + psif[AX(i - 1, j)]) / hhr +
-                          (psif[AX(i + 1, j)] - psif[AX(i - 1, j)]) * 0.5 / hr / rv - psif[AX(i, j)] / (rv * rv) +
-                          (psif[AX(i, j + 1)] + psif[AX(i, j - 1)]) / hhz - psif[AX(i, j)] * drdz;
-            temp = L1.f[(size_t)j * (n1 + 1) + i] - temp;
-            L1.f32[(size_t)j * (n1 + 1) + i] = (float)temp;
-            temp = fabs(temp);
-            if (temp != temp) nan = 1;
-            if (temp > m) m = temp;
-        }
-        nan = __syncthreads_or(nan);
-        const double res = axi_blk_max(m, s_red);
+        int nan;
+        const double m = axi_residual<double>(d, 1, const_cast<float *>(L32.f), &nan);
+        const double res = cl_max(cl, s_max, turn, m, nan);
         if (nan) { status = GB_NAN; break; }
         if (res < d.tolcon) { status = GB_OK; break; }
         if (it == d.maxsweeps) break;
-        for (int q = threadIdx.x; q < (n1 + 1) * (n2 + 1); q += blockDim.x) L1.v32[q] = 0.f;
-        __syncthreads();
-        axi_relax32(d, 1);
-        if (nlev > 1) {
-            for (int l = 1; l <= nlev - 1; ++l) {
-                axi_corser32(d, l);
-                axi_relax32(d, l + 1);
-            }
-            for (int l = nlev; l >= 2; --l) {
-                axi_finer32(d, l);
-                axi_relax32(d, l - 1);
-            }
+        relax(1, nlev > 1);
+        for (int l = 1; l <= nlev - 1; ++l) {
+            axi_corser<float>(d, l, d.rc32);
+            relax(l + 1, l + 1 < nlev);
         }
-        for (int idx = threadIdx.x; idx < tot; idx += blockDim.x) {
-            const int j = idx / ni + 1, i = idx - (j - 1) * ni + 1;
-            psif[AX(i, j)] += (double)L1.v32[(size_t)j * (n1 + 1) + i];
+        for (int l = nlev; l >= 2; --l) {
+            axi_finer<float>(d, l);
+            relax(l - 1, false);
         }
-        __syncthreads();
+        // psi += e, and e = 0 for the next cycle
+        for (int idx = cl.tid(); idx < tp; idx += cl.nthr()) {
+            L.v[idx] += (double)L32.v[idx];
+            L32.v[idx] = 0.f;
+        }
+        cl.sync();
         cycles = it + 1;
     }
     if (status == GB_OK)
-        for (int idx = threadIdx.x; idx < (n1 + 1) * (n2 + 1); idx += blockDim.x) {
-            const int j = idx / (n1 + 1), i = idx - j * (n1 + 1);
-            psi[AX(i, j)] = psif[AX(i, j)];
-        }
-    if (threadIdx.x == 0) {
+        for (int idx = cl.tid(); idx < tp; idx += cl.nthr()) psi[idx] = L.v[idx];
+    if (cl.tid() == 0) {
         d.status[0] = status;
         d.status[1] = cycles;
         if (status == GB_NAN) *d.abort = 1;
     }
+    cl.sync();
 }
+#undef V
+#undef F
 
-__global__ void __maxnreg__(128) k_axi_mg_solve_mixed(AxiDev d) { k_axi_mg_solve_mixed_body(d, blockIdx.x); }
+__global__ void __maxnreg__(128) k_axi_mg_solve_mixed(const __grid_constant__ AxiDev d) { k_axi_mg_solve_mixed_body(d); }
 
-// FP32 copies of rval and the factors (pivots as reciprocals).
-// FP32 copies of the factors (pivots as reciprocals): block l - 1 converts
-// level l, its threads the level's lines (thread 0 also the r-line table).
+// FP32 copies of rval and the folded factors: block l - 1 takes level l, its
+// threads the level's lines (thread 0 also the r-line table).
 __global__ void k_axi_factors32(AxiDev d)
 {
     const int l = 1 + blockIdx.x;
     if (l == 1)
         for (int i = threadIdx.x; i <= d.lev[1].n1; i += blockDim.x) d.rval32[i] = (float)d.rval[i];
     const AxiLevel &L = d.lev[l];
-    auto conv = [](const double *f, float *g, int n) {
-        for (int j = 0; j < n; ++j) {
-            g[j] = (float)f[j];
-            g[n + j] = (float)(1.0 / f[n + j]);
-            g[2 * n + j] = (float)f[2 * n + j];
-        }
-    };
-    if (threadIdx.x == 0 && L.n1 - 1 >= 1) conv(L.fac_r, L.fac_r32, L.n1 - 1);
-    if (L.n2 - 1 >= 1)
+    if (threadIdx.x == 0 && L.n1 - 1 >= 1) tdma32_fold(L.fac_r, L.n1 - 1, L.fac_r32);
+    if (L.n2 - 1 >= 1) {
+        const int n = L.n2 - 1;
         for (int i = 1 + threadIdx.x; i <= L.n1 - 1; i += blockDim.x)
-            conv(L.fac_z + (size_t)(i - 1) * tdma_fac_len(L.n2 - 1), L.fac_z32 + (size_t)(i - 1) * 3 * (L.n2 - 1),
-                 L.n2 - 1);
+            tdma32_fold(L.fac_z + (size_t)(i - 1) * tdma_fac_len(n), n, L.fac_z32 + (size_t)(i - 1) * tdma32_len(n));
+        wl_common_steps(L.fac_z32, tdma32_len(n), L.n1 - 1);
+    }
+}
+
+// The resident solve's weights (meridian.cu) from relax's operator.
+__global__ void k_axi_weights(const __grid_constant__ AxiDev d, const __grid_constant__ MerDev m)
+{
+    const int l = 1 + blockIdx.y, t = blockIdx.x * blockDim.x + threadIdx.x;
+    const AxiLevel &L = d.lev[l];
+    auto put = [&](const float4 *c4, const MerW *d4, int q, double cm, double cp, double cd) {
+        const_cast<float4 *>(c4)[q] = make_float4((float)cm, (float)cp, 0.f, (float)cd);
+        if (l == 1) const_cast<MerW *>(d4)[q] = MerW{cm, cp, 0.0, cd};
+    };
+    if (t >= 1 && t < L.n1) {
+        const double rv = d.rval[t * L.lf];
+        put(m.lev[l].c4i, m.d4i, t, 1.0 / L.hhr - 0.5 / L.hr / rv, 1.0 / L.hhr + 0.5 / L.hr / rv, -2.0 / L.hhr - 1.0 / (rv * rv));
+    }
+    if (t >= 1 && t < L.n2) put(m.lev[l].c4j, m.d4j, t, 1.0 / L.hhz, 1.0 / L.hhz, -2.0 / L.hhz);
 }
 
 __global__ void k_axi_rval(AxiDev d)
 {
-    for (int i = threadIdx.x; i <= d.lev[1].n1; i += blockDim.x) d.rval[i] = (double)i * d.lev[1].hr + d.r0;
+    for (int i = threadIdx.x; i <= d.lev[1].n1; i += blockDim.x) {
+        const double rv = (double)i * d.lev[1].hr + d.r0;
+        d.rval[i] = rv;
+        d.irv[i] = 1.0 / rv;
+        d.irq[i] = 1.0 / (rv * rv);
+    }
 }
 
 // The factored line matrices of every level, with the coefficients relax
@@ -1023,6 +933,10 @@ struct gb_axi {
     cudaGraphExec_t graph = nullptr;
     gb_axi_params graph_params;
     double dr_set = 0.0, dz_set = 0.0;   // a Fortran caller's /num/ spacings, 0 = derived
+    int ctas = 1;                        // CTAs per ZEBRA solve on global memory
+    MerDev mer;                          // the resident mixed solve, where its plan fits
+    int mer_ctas = 0;                    // its CTAs; 0: k_axi_mg_solve_mixed
+    void *mer_mem = nullptr;
 };
 
 static int axi_levels(int nr, int nz)
@@ -1098,9 +1012,40 @@ extern "C" int gb_axi_destroy(gb_axi *h)
     cudaFree(h->pool);
     cudaFree(h->small);
     cudaFree(h->hist);
+    cudaFree(h->mer_mem);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
     return GB_OK;
+}
+
+// Prepares the resident mixed solve; a grid it cannot hold leaves mer_ctas 0.
+static cudaError_t axi_mer_create(gb_axi *h)
+{
+    const AxiDev &d = h->dev;
+    MerDev &m = h->mer;
+    memset(&m, 0, sizeof(m));
+    m.nlev = d.nlev;
+    for (int l = 1; l <= d.nlev; ++l) {
+        MerLevel &L = m.lev[l];
+        L.n1 = d.lev[l].n1;
+        L.n2 = d.lev[l].n2;
+        L.fac_r = d.lev[l].fac_r32;
+        L.fac_z = d.lev[l].fac_z32;
+        L.fac_r_step = 0;
+        L.fac_z_step = (int)tdma32_len(L.n2 - 1);
+    }
+    m.v = d.lev[1].v;
+    m.psi = d.f[GB_A_phi];
+    m.rhs = d.f[GB_A_omegn];
+    m.status = d.status;
+    m.abort = d.abort;
+    h->mer_ctas = mer_fit(m, CL_MAX_CTAS);
+    if (!h->mer_ctas) return cudaSuccess;
+    cudaError_t e = cudaMalloc(&h->mer_mem, mer_weight_bytes(m));
+    if (e != cudaSuccess) return e;
+    mer_weight_layout(m, h->mer_mem);
+    k_axi_weights<<<dim3(gb_ceil_div((size_t)std::max(m.lev[1].n1, m.lev[1].n2), 128), m.nlev), 128>>>(d, m);
+    return cudaGetLastError();
 }
 
 static int axi_create(const gb_axi_params *p, double dr, double dz, gb_axi **out, int *nlev_out);
@@ -1136,10 +1081,6 @@ static int axi_create(const gb_axi_params *p, double dr, double dz, gb_axi **out
         gb_set_error("gb_axi_create: unknown precision %d", p->precision);
         return GB_ERR_INVALID;
     }
-    if (2 * (nr > nz ? nr : nz) > AX32_LINE_FLOATS) {
-        gb_set_error("gb_axi_create: nr=%d nz=%d exceed the shared-memory line buffer", nr, nz);
-        return GB_ERR_INVALID;
-    }
     gb_axi *h = new gb_axi();
     h->p = *p;
     h->dr_set = dr;
@@ -1156,12 +1097,12 @@ static int axi_create(const gb_axi_params *p, double dr, double dz, gb_axi **out
     if (e != cudaSuccess) { gb_set_error("gb_axi_create: %s", cudaGetErrorString(e)); delete h; return GB_ERR_ALLOC; }
     cudaMemset(h->fields, 0, sizeof(double) * fsz * GB_A_COUNT);
     for (int q = 0; q < GB_A_COUNT; ++q) d.f[q] = h->fields + (size_t)q * fsz;
-    // pool: rval, psif, rc, then per level v, f, fac_r, fac_z; work for the factors
-    size_t need = (size_t)(nr + 2) + 2 * fsz + fsz + (size_t)(nr + 2) / 2 + 8;   // + psif32, rc32, rval32
+    // pool: rval and its reciprocals, rc, rc32, rval32, then per level v, f, fac_r, fac_z and their FP32 forms
+    size_t need = 3 * (size_t)(nr + 2) + fsz + fsz / 2 + (size_t)(nr + 2) / 2 + 8;
     for (int l = 1; l <= nlev; ++l) {
         const size_t n1 = (size_t)nr * 2 / ((size_t)1 << l), n2 = (size_t)nz * 2 / ((size_t)1 << l);
-        const size_t lv = 2 * (n1 + 1) * (n2 + 1) + 4 * n1 + n1 * 4 * (n2 + 1);
-        need += lv + (lv + 1) / 2 + 4;   // FP64 slots, then their FP32 copies
+        need += 2 * (n1 + 1) * (n2 + 1) + 4 * n1 + n1 * 4 * (n2 + 1);
+        need += ((n1 + 1) * (n2 + 1) * 2 + tdma32_len((int)n1) + n1 * tdma32_len((int)n2)) / 2 + 8;
     }
     const size_t work = 3 * (size_t)((nr > nz ? nr : nz) + 2) * (size_t)nlev;   // r-line coefficients, per level
     e = cudaMalloc(&h->pool, sizeof(double) * (need + work));
@@ -1169,11 +1110,11 @@ static int axi_create(const gb_axi_params *p, double dr, double dz, gb_axi **out
     cudaMemset(h->pool, 0, sizeof(double) * (need + work));
     double *b = h->pool;
     d.rval = b; b += nr + 2;
-    d.psif = b; b += fsz;
+    d.irv = b; b += nr + 2;
+    d.irq = b; b += nr + 2;
     d.rc = b; b += fsz;
     {
         float *fb = (float *)b;
-        d.psif32 = fb; fb += fsz;
         d.rc32 = fb; fb += fsz;
         d.rval32 = fb; fb += nr + 2;
         b = (double *)(((uintptr_t)fb + 15) & ~(uintptr_t)15);
@@ -1187,6 +1128,9 @@ static int axi_create(const gb_axi_params *p, double dr, double dz, gb_axi **out
         L.hz = d.dz * (double)(1 << l) / 2.0;
         L.hhr = L.hr * L.hr;
         L.hhz = L.hz * L.hz;
+        L.ihr = 1.0 / L.hr;
+        L.ihhr = 1.0 / L.hhr;
+        L.ihhz = 1.0 / L.hhz;
         const size_t sz = (size_t)(L.n1 + 1) * (L.n2 + 1);
         L.v = b; b += sz;
         L.f = b; b += sz;
@@ -1195,8 +1139,9 @@ static int axi_create(const gb_axi_params *p, double dr, double dz, gb_axi **out
         float *fb = (float *)b;
         L.v32 = fb; fb += sz;
         L.f32 = fb; fb += sz;
-        L.fac_r32 = fb; fb += 3 * (size_t)L.n1;
-        L.fac_z32 = fb; fb += (size_t)L.n1 * 3 * (size_t)(L.n2 + 1);
+        fb = (float *)(((uintptr_t)fb + 15) & ~(uintptr_t)15);   // the tables are copied 16 bytes at a time
+        L.fac_r32 = fb; fb += tdma32_len(std::max(L.n1 - 1, 1));
+        L.fac_z32 = fb; fb += (size_t)(L.n1 - 1) * tdma32_len(std::max(L.n2 - 1, 1));
         b = (double *)(((uintptr_t)fb + 15) & ~(uintptr_t)15);
     }
     if ((size_t)(b - h->pool) > need) {
@@ -1217,7 +1162,12 @@ static int axi_create(const gb_axi_params *p, double dr, double dz, gb_axi **out
     k_axi_rval<<<1, 256>>>(d);
     k_axi_factors<<<d.nlev, 128>>>(d, wk);
     k_axi_factors32<<<d.nlev, 128>>>(d);
-    e = cudaFuncSetAttribute(k_axi_mg_solve_mixed, cudaFuncAttributeMaxDynamicSharedMemorySize, AX32_SMEM_BYTES);
+    e = cl_prepare(k_axi_mg_solve, AXI_SMEM_BYTES);
+    if (e == cudaSuccess) e = cl_prepare(k_axi_mg_solve_mixed, AXI_SMEM_BYTES);
+    if (e == cudaSuccess) {
+        h->ctas = cl_fit(k_axi_mg_solve, CL_MAX_CTAS, AXI_THREADS, AXI_SMEM_BYTES);
+        if (p->precision == GB_PRB_MIXED) e = axi_mer_create(h);
+    }
     if (e != cudaSuccess) { gb_axi_destroy(h); gb_set_error("gb_axi_create: %s", cudaGetErrorString(e)); return GB_ERR_CUDA; }
     e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) { gb_axi_destroy(h); gb_set_error("gb_axi_create: stream"); return GB_ERR_CUDA; }
@@ -1352,6 +1302,16 @@ static void axi_launch_heat(gb_axi *h, cudaStream_t s)
     else k_axi_heat<false><<<1, 256, sizeof(double) * (h->dev.nz + 1), s>>>(h->dev);
 }
 
+// The resident solve with the parameters a caller may have changed.
+static MerDev axi_mer(const gb_axi *h)
+{
+    MerDev m = h->mer;
+    m.tolcon = h->dev.tolcon;
+    m.maxcycles = h->dev.maxsweeps;
+    m.nrel = h->dev.nrel;
+    return m;
+}
+
 static void axi_launch_mg(gb_axi *h, cudaStream_t s)
 {
     const AxiDev &d = h->dev;
@@ -1360,8 +1320,15 @@ static void axi_launch_mg(gb_axi *h, cudaStream_t s)
                              h->p.precision == GB_PRB_MIXED, d.tolcon, d.maxsweeps, d.nrel, d.mode, s);
         return;
     }
-    if (h->p.precision == GB_PRB_MIXED) k_axi_mg_solve_mixed<<<1, AXI_THREADS, AX32_SMEM_BYTES, s>>>(h->dev);
-    else k_axi_mg_solve<<<1, AXI_THREADS, 0, s>>>(h->dev);
+    // the reference's line order is one chain of lines: one CTA
+    const int ctas = d.mode == GB_SMOOTHER_LEX ? 1 : h->ctas;
+    if (h->p.precision != GB_PRB_MIXED) {
+        cl_launch(k_axi_mg_solve, 1, ctas, AXI_THREADS, AXI_SMEM_BYTES, s, d);
+    } else if (d.mode == GB_SMOOTHER_ZEBRA && h->mer_ctas) {
+        mer_launch(axi_mer(h), h->mer_ctas, s);
+    } else {
+        cl_launch(k_axi_mg_solve_mixed, 1, ctas, AXI_THREADS, AXI_SMEM_BYTES, s, d);
+    }
 }
 
 static int axi_sync(gb_axi *h, const char *what)
@@ -1543,7 +1510,7 @@ extern "C" int gb_axi_step(gb_axi *h, int nsteps, double *nu, int *sweeps, int *
 // bit-identical to stepping it alone.  A member whose step index reaches
 // its step count sets its abort flag to GB_RUN_DONE.
 // ---------------------------------------------------------------------------
-enum AxiGangPhase { AG_VV, AG_T, AG_MG, AG_UPD, AG_HEAT, AG_REC, AG_COUNT };
+enum AxiGangPhase { AG_VV, AG_T, AG_UPD, AG_HEAT, AG_REC, AG_COUNT };
 
 struct AxiGangTab {
     const AxiDev *dev;    // [n]
@@ -1583,20 +1550,30 @@ __global__ void k_axi_gang(AxiGangTab g)
     }
 }
 
-// Launched with AXI_THREADS (512) threads; 128 registers keep the solve
-// free of spills (a launch bound of 512 threads left it at 40-64 with spills).
+// The solves of the members listed in `who`, a cluster each.  128 registers
+// keep the solve free of spills (a launch bound of 512 threads left it at
+// 40-64 with spills).
 template <bool MIXED>
-__global__ void __maxnreg__(128) k_axi_gang_mg(AxiGangTab g)
+__global__ void __maxnreg__(128) k_axi_gang_mg(AxiGangTab g, const int *who)
 {
-    const AxiDev &d = g.dev[blockIdx.x];
-    if (MIXED) k_axi_mg_solve_mixed_body(d, 0);
-    else k_axi_mg_solve_body(d, 0);
+    const AxiDev &d = g.dev[who[blockIdx.x / cooperative_groups::this_cluster().num_blocks()]];
+    if (MIXED) k_axi_mg_solve_mixed_body(d);
+    else k_axi_mg_solve_body(d);
 }
 
+// The streamfunction solves of a gang step: every member's as one cluster,
+// the resident ones of a mixed gang in one launch, the others in another per
+// line order (the reference's order takes one CTA).  A cluster holds as many
+// CTAs as leave every member its own SMs, at least what the largest resident
+// member's arrays need; the results do not depend on it.
 struct gb_axi_gang {
     int n = 0, mixed = 0;
     AxiDev *d_dev = nullptr;
-    int *d_off = nullptr, *d_limit = nullptr;
+    int *d_off = nullptr, *d_limit = nullptr, *d_who = nullptr;
+    MerDev *d_mer = nullptr;
+    int nmer = 0, mer_ctas = 0;
+    size_t mer_smem = 0;
+    int nz = 0, nlex = 0, z_ctas = 1;   // members on global memory: zebra, reference order (d_who in this order)
     int blocks[AG_COUNT], threads[AG_COUNT];
     size_t heat_smem = 0;
     cudaStream_t stream = nullptr;
@@ -1610,6 +1587,8 @@ extern "C" int gb_axi_gang_destroy(gb_axi_gang *g)
     cudaFree(g->d_dev);
     cudaFree(g->d_off);
     cudaFree(g->d_limit);
+    cudaFree(g->d_who);
+    cudaFree(g->d_mer);
     if (g->stream) cudaStreamDestroy(g->stream);
     delete g;
     return GB_OK;
@@ -1635,7 +1614,7 @@ extern "C" int gb_axi_gang_create(gb_axi *const *members, const int *nsteps_tota
     gb_axi_gang *g = new gb_axi_gang();
     g->n = n;
     g->mixed = mixed;
-    const int tpb[AG_COUNT] = {AXI_TPB, AXI_TPB, AXI_THREADS, AXI_TPB, 256, 32};
+    const int tpb[AG_COUNT] = {AXI_TPB, AXI_TPB, AXI_TPB, 256, 32};
     std::vector<int> off((size_t)AG_COUNT * (n + 1));
     std::vector<AxiDev> devs(n);
     for (int ph = 0; ph < AG_COUNT; ++ph) {
@@ -1648,7 +1627,7 @@ extern "C" int gb_axi_gang_create(gb_axi *const *members, const int *nsteps_tota
         devs[q] = h->dev;
         const size_t nr = h->dev.nr, nz = h->dev.nz;
         const int nb[AG_COUNT] = {(int)gb_ceil_div((nr - 1) * (nz - 1), AXI_TPB), (int)gb_ceil_div((nr - 1) * (nz + 1), AXI_TPB),
-                                  1, (int)gb_ceil_div((nr + 1) * (nz + 1), AXI_TPB), 1, 1};
+                                  (int)gb_ceil_div((nr + 1) * (nz + 1), AXI_TPB), 1, 1};
         for (int ph = 0; ph < AG_COUNT; ++ph) {
             off[(size_t)ph * (n + 1) + q] = g->blocks[ph];
             g->blocks[ph] += nb[ph];
@@ -1656,6 +1635,39 @@ extern "C" int gb_axi_gang_create(gb_axi *const *members, const int *nsteps_tota
         g->heat_smem = std::max(g->heat_smem, sizeof(double) * (nz + 1));
     }
     for (int ph = 0; ph < AG_COUNT; ++ph) off[(size_t)ph * (n + 1) + n] = g->blocks[ph];
+    std::vector<MerDev> mers;
+    std::vector<int> who, lex;
+    int sms = 0;
+    for (int q = 0; q < n; ++q) {
+        if (mixed && members[q]->p.smoother == GB_SMOOTHER_ZEBRA && members[q]->mer_ctas) mers.push_back(axi_mer(members[q]));
+        else if (members[q]->p.smoother == GB_SMOOTHER_LEX) lex.push_back(q);
+        else who.push_back(q);
+    }
+    g->nz = (int)who.size();
+    g->nlex = (int)lex.size();
+    g->nmer = (int)mers.size();
+    who.insert(who.end(), lex.begin(), lex.end());
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
+    auto per_member = [&](int members_) {
+        int c = CL_MAX_CTAS;
+        while (c > 1 && c * members_ > sms) c >>= 1;
+        return c;
+    };
+    if (g->nmer) {
+        int most = CL_MAX_CTAS;
+        for (int q = 0; q < n; ++q)
+            if (members[q]->mer_ctas) most = std::min(most, members[q]->mer_ctas);
+        for (g->mer_ctas = std::min(most, per_member(g->nmer));; g->mer_ctas <<= 1) {
+            bool fits = true;
+            g->mer_smem = 0;
+            for (MerDev &m : mers) {
+                fits = mer_plan(m, g->mer_ctas) && fits;
+                g->mer_smem = std::max(g->mer_smem, sizeof(float) * (size_t)m.smem_floats);
+            }
+            if (fits || g->mer_ctas >= most) break;
+        }
+    }
+    if (g->nz) g->z_ctas = std::min(members[who[0]]->ctas, per_member(g->nz));
 #define GTRY(x)                                                                   \
     do {                                                                          \
         cudaError_t _e = (x);                                                     \
@@ -1671,9 +1683,17 @@ extern "C" int gb_axi_gang_create(gb_axi *const *members, const int *nsteps_tota
     GTRY(cudaMemcpy(g->d_dev, devs.data(), sizeof(AxiDev) * n, cudaMemcpyHostToDevice));
     GTRY(cudaMemcpy(g->d_off, off.data(), sizeof(int) * off.size(), cudaMemcpyHostToDevice));
     GTRY(cudaMemcpy(g->d_limit, nsteps_total, sizeof(int) * n, cudaMemcpyHostToDevice));
+    if (!who.empty()) {
+        GTRY(cudaMalloc(&g->d_who, sizeof(int) * who.size()));
+        GTRY(cudaMemcpy(g->d_who, who.data(), sizeof(int) * who.size(), cudaMemcpyHostToDevice));
+        GTRY(mixed ? cl_prepare(k_axi_gang_mg<true>, AXI_SMEM_BYTES) : cl_prepare(k_axi_gang_mg<false>, AXI_SMEM_BYTES));
+    }
+    if (g->nmer) {
+        GTRY(cudaMalloc(&g->d_mer, sizeof(MerDev) * mers.size()));
+        GTRY(cudaMemcpy(g->d_mer, mers.data(), sizeof(MerDev) * mers.size(), cudaMemcpyHostToDevice));
+    }
     for (int q = 0; q < n; ++q) GTRY(cudaStreamSynchronize(members[q]->stream));
     GTRY(cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking));
-    GTRY(cudaFuncSetAttribute(k_axi_gang_mg<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, AX32_SMEM_BYTES));
     if (g->heat_smem > 48 * 1024)
         GTRY(cudaFuncSetAttribute(k_axi_gang<AG_HEAT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)g->heat_smem));
 #undef GTRY
@@ -1694,8 +1714,14 @@ extern "C" int gb_axi_gang_enqueue(gb_axi_gang *g, int nsteps, void *stream)
         GB_CUDA_TRY(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
         k_axi_gang<AG_VV><<<g->blocks[AG_VV], g->threads[AG_VV], 0, cs>>>(t);
         k_axi_gang<AG_T><<<g->blocks[AG_T], g->threads[AG_T], 0, cs>>>(t);
-        if (g->mixed) k_axi_gang_mg<true><<<g->n, AXI_THREADS, AX32_SMEM_BYTES, cs>>>(t);
-        else k_axi_gang_mg<false><<<g->n, AXI_THREADS, 0, cs>>>(t);
+        if (g->nmer) mer_launch_many(g->d_mer, g->nmer, 0, g->mer_ctas, g->mer_smem, cs);
+        auto solves = [&](int count, int ctas, const int *who) {
+            if (!count) return;
+            if (g->mixed) cl_launch(k_axi_gang_mg<true>, count, ctas, AXI_THREADS, AXI_SMEM_BYTES, cs, t, who);
+            else cl_launch(k_axi_gang_mg<false>, count, ctas, AXI_THREADS, AXI_SMEM_BYTES, cs, t, who);
+        };
+        solves(g->nz, g->z_ctas, g->d_who);
+        solves(g->nlex, 1, g->d_who + g->nz);
         k_axi_gang<AG_UPD><<<g->blocks[AG_UPD], g->threads[AG_UPD], 0, cs>>>(t);
         k_axi_gang<AG_HEAT><<<g->blocks[AG_HEAT], g->threads[AG_HEAT], g->heat_smem, cs>>>(t);
         k_axi_gang<AG_REC><<<g->blocks[AG_REC], g->threads[AG_REC], 0, cs>>>(t);

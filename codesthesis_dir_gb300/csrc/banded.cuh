@@ -282,3 +282,158 @@ __device__ __forceinline__ void tdma32_smem(const float *fac, int n, float *x, i
         x[j * pitch] = y;
     }
 }
+
+// ---------------------------------------------------------------------------
+// Eliminations in place on a staged line, x[k * pitch] and the line's factors
+// both in shared memory.  A line is one thread's dependent chain, so nothing
+// else may sit on it: each block of rows has its factors and right-hand sides
+// loaded into registers while the block before it is eliminated (the compiler
+// cannot move those loads above the stores to x itself).
+// ---------------------------------------------------------------------------
+
+// Pentadiagonal in FP64, factor_pdma's layout: apply_pdma_rhs's operations in
+// its order.
+template <int U = 2> __device__ __forceinline__ void pdma_staged(const double *fac, int n, double *x, int pitch)
+{
+    const double *cdiv = fac, *bk1 = fac + n, *aa = fac + 2 * n, *dn = fac + 3 * n, *en = fac + 4 * n;
+    const double *icdiv = fac + 5 * n + 1;
+    double rk = x[0], rk1 = x[pitch];
+    double c[U], ic[U], b[U], a[U], r[U];
+    const int reg = n - 2;   // rows with a row two below
+    auto fetch = [&](int k0) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int k = min(k0 + u, reg - 1);
+            c[u] = cdiv[k];
+            ic[u] = icdiv[k];
+            b[u] = bk1[k];
+            a[u] = aa[k + 2];
+            r[u] = x[(k + 2) * pitch];
+        }
+    };
+    if (reg > 0) fetch(0);
+    for (int k0 = 0; k0 < reg; k0 += U) {
+        double c0[U], ic0[U], b0[U], a0[U], r0[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            c0[u] = c[u];
+            ic0[u] = ic[u];
+            b0[u] = b[u];
+            a0[u] = a[u];
+            r0[u] = r[u];
+        }
+        if (k0 + U < reg) fetch(k0 + U);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (k0 + u < reg) {
+                const double q = div_by_rcp(rk, c0[u], ic0[u]);
+                x[(k0 + u) * pitch] = q;
+                rk = rk1 - b0[u] * q;
+                rk1 = r0[u] - a0[u] * q;
+            }
+        }
+    }
+    {   // row n - 2
+        const double q = div_by_rcp(rk, cdiv[n - 2], icdiv[n - 2]);
+        x[(n - 2) * pitch] = q;
+        rk1 = rk1 - bk1[n - 2] * q;
+    }
+    double x1 = div_by_rcp(rk1, fac[5 * n], fac[6 * n + 1]);
+    x[(n - 1) * pitch] = x1;
+    double x0 = x[(n - 2) * pitch] - dn[n - 2] * x1;
+    x[(n - 2) * pitch] = x0;
+    auto fetch_back = [&](int j0) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int j = max(j0 - u, 0);
+            c[u] = dn[j];
+            b[u] = en[j];
+            r[u] = x[j * pitch];
+        }
+    };
+    if (n >= 3) fetch_back(n - 3);
+    for (int j0 = n - 3; j0 >= 0; j0 -= U) {
+        double d0[U], e0[U], r0[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            d0[u] = c[u];
+            e0[u] = b[u];
+            r0[u] = r[u];
+        }
+        if (j0 - U >= 0) fetch_back(j0 - U);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (j0 - u >= 0) {
+                const double xj = r0[u] - d0[u] * x0 - e0[u] * x1;
+                x[(j0 - u) * pitch] = xj;
+                x1 = x0;
+                x0 = xj;
+            }
+        }
+    }
+}
+
+// Tridiagonal in FP64, factor_tdma's layout: apply_tdma_rhs's operations in
+// its order.
+template <int U = 2> __device__ __forceinline__ void tdma_staged(const double *fac, int n, double *x, int pitch)
+{
+    const double *fact = fac, *bp = fac + n, *cc = fac + 2 * n, *ibp = fac + 3 * n;
+    double prev = x[0];
+    double f[U], r[U], b[U], ib[U];
+    auto fetch = [&](int j0) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int j = min(j0 + u, n - 1);
+            f[u] = fact[j];
+            r[u] = x[j * pitch];
+        }
+    };
+    fetch(1);
+    for (int j0 = 1; j0 < n; j0 += U) {
+        double f0[U], r0[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            f0[u] = f[u];
+            r0[u] = r[u];
+        }
+        if (j0 + U < n) fetch(j0 + U);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (j0 + u < n) {
+                prev = r0[u] - f0[u] * prev;
+                x[(j0 + u) * pitch] = prev;
+            }
+        }
+    }
+    double y = div_by_rcp(prev, bp[n - 1], ibp[n - 1]);
+    x[(n - 1) * pitch] = y;
+    auto fetch_back = [&](int j0) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int j = max(j0 - u, 0);
+            f[u] = cc[j];
+            b[u] = bp[j];
+            ib[u] = ibp[j];
+            r[u] = x[j * pitch];
+        }
+    };
+    if (n >= 2) fetch_back(n - 2);
+    for (int j0 = n - 2; j0 >= 0; j0 -= U) {
+        double f0[U], b0[U], ib0[U], r0[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            f0[u] = f[u];
+            b0[u] = b[u];
+            ib0[u] = ib[u];
+            r0[u] = r[u];
+        }
+        if (j0 - U >= 0) fetch_back(j0 - U);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (j0 - u >= 0) {
+                y = div_by_rcp(r0[u] - f0[u] * y, b0[u], ib0[u]);
+                x[(j0 - u) * pitch] = y;
+            }
+        }
+    }
+}

@@ -17,7 +17,10 @@
 // parallel.
 #include "gbcommon.cuh"
 #include "banded.cuh"
+#include "cluster.cuh"
+#include "meridian.cuh"
 #include "str_internal.cuh"
+#include "warpline.cuh"
 
 #include <stdlib.h>
 #include <string.h>
@@ -39,10 +42,10 @@ struct StrLevel {
 };
 
 struct StrDev {
-    int nlev, ld, nrel, maxsweeps, mode;
+    int nlev, nrel, maxsweeps, mode;
     double tolcon;
-    double *psif, *rc;        // ld x ld, ld = max(n1, n2) + 1
-    float *psif32, *rc32;     // the same for the FP32 correction cycles
+    double *rc;               // the residual of the level it was last formed on, pitch n1 + 1
+    float *rc32;              // the same for the FP32 correction cycles
     double *io_psi, *io_rhs;  // level-1 (n1+1) x (n2+1) staging of the caller's arrays
     StrLevel lev[STR_MAXLEV];
     int *status;              // [0] status, [1] sweeps
@@ -50,7 +53,6 @@ struct StrDev {
                               // sets it to 1 when the residual is a NaN
 };
 
-#define PS(i, j) d.psif[(size_t)(i) + (size_t)d.ld * (size_t)(j)]
 #define CR(i, k) L.cr[3 * ((i) - 1) + (k) - 1]
 #define CRR(i, k) L.crr[4 * ((i) - 1) + (k) - 1]
 #define CZZ(j, k) L.czz[4 * ((j) - 1) + (k) - 1]
@@ -123,306 +125,307 @@ __global__ void k_str_factors(const __grid_constant__ StrDev d, const StrJob *jo
     factor_pdma(a, b, c, dd, e, n, fac, scratch);
 }
 
-// r-line j: right-hand side of row i (rcsc.f:1246-1252)
-__device__ __forceinline__ void str_rline(const StrDev &d, const StrLevel &L, int j)
+// ---------------------------------------------------------------------------
+// The solve.  One cluster of CTAs per solve (cluster.cuh); level l's
+// correction v and right-hand side f are (0:n1, 0:n2) arrays of pitch n1 + 1,
+// the residual rc the same with the pitch of the level it was formed on.
+// T is double for the reference's arithmetic and float for the correction
+// cycles of the mixed solve.
+// ---------------------------------------------------------------------------
+template <class T> struct StrView {
+    int n1, n2, ld;
+    T *v;
+    const T *f;
+    const T *cr, *crr, *czz;
+    const T *r, *ir, *irr;    // double: r, 1/r, 1/(r r); float: r only
+    const T *fac[2];          // r-lines, z-lines
+};
+__device__ __forceinline__ StrView<double> str_view(const StrLevel &L, double)
 {
-    const int n1 = L.n1, n2 = L.n2;
-    const double *f = L.f;
-    auto rhs = [&](int q) -> double {
-        const int i = q + 1;
-        if (j <= n2 / 2)
-            return -(CZZ(j, 1) * PS(i, j - 1) + CZZ(j, 3) * PS(i, j + 1) + CZZ(j, 4) * PS(i, j + 2)) +
-                   f[(size_t)i + (size_t)(n1 + 1) * j];
-        return -(CZZ(j, 1) * PS(i, j - 2) + CZZ(j, 2) * PS(i, j - 1) + CZZ(j, 4) * PS(i, j + 1)) +
-               f[(size_t)i + (size_t)(n1 + 1) * j];
-    };
-    const int n = n1 - 1;
-    apply_pdma_rhs(L.fac_r + (size_t)(j - 1) * pdma_fac_len(n), n, &PS(1, j), 1, rhs);
+    return {L.n1, L.n2, L.n1 + 1, L.v, L.f, L.cr, L.crr, L.czz, L.r, L.ir, L.irr, {L.fac_r, L.fac_z}};
 }
-
-// z-line i: right-hand side of row j (rcsc.f:1279-1290)
-__device__ __forceinline__ void str_zline(const StrDev &d, const StrLevel &L, int i)
+__device__ __forceinline__ StrView<float> str_view(const StrLevel &L, float)
 {
-    const int n1 = L.n1, n2 = L.n2;
-    const double *f = L.f;
+    return {L.n1, L.n2, L.n1 + 1, L.v32, L.f32, L.cr32, L.crr32, L.czz32, L.r32, nullptr, nullptr, {L.fac_r32, L.fac_z32}};
+}
+#define V(i, j) L.v[(i) + L.ld * (j)]
+#define F(i, j) L.f[(i) + L.ld * (j)]
+
+// x / r(i): the IEEE quotient, or a product with the rounded reciprocal
+__device__ __forceinline__ double str_over_r(const StrView<double> &L, int i, double x) { return div_by_rcp(x, L.r[i], L.ir[i]); }
+__device__ __forceinline__ float str_over_r(const StrView<float> &L, int i, float x) { return x * (1.0f / L.r[i]); }
+__device__ __forceinline__ double str_over_rr(const StrView<double> &L, int i, double x)
+{
     const double r = L.r[i];
-    auto rhs = [&](int q) -> double {
-        const int j = q + 1;
-        if (i <= n1 / 2)
-            return -(CRR(i, 1) * PS(i - 1, j) + CRR(i, 3) * PS(i + 1, j) + CRR(i, 4) * PS(i + 2, j) +
-                     div_by_rcp(CR(i, 1) * PS(i - 1, j) + CR(i, 3) * PS(i + 1, j), r, L.ir[i])) +
-                   f[(size_t)i + (size_t)(n1 + 1) * j];
-        return -(CRR(i, 1) * PS(i - 2, j) + CRR(i, 2) * PS(i - 1, j) + CRR(i, 4) * PS(i + 1, j) +
-                 div_by_rcp(CR(i, 1) * PS(i - 1, j) + CR(i, 3) * PS(i + 1, j), r, L.ir[i])) +
-               f[(size_t)i + (size_t)(n1 + 1) * j];
-    };
-    const int n = n2 - 1;
-    apply_pdma_rhs(L.fac_z + (size_t)(i - 1) * pdma_fac_len(n), n, &PS(i, 1), d.ld, rhs);
+    return div_by_rcp(x, r * r, L.irr[i]);
+}
+__device__ __forceinline__ float str_over_rr(const StrView<float> &L, int i, float x)
+{
+    const float ir = 1.0f / L.r[i];
+    return x * (ir * ir);
 }
 
-// Shared memory of a solve: the line buffer of the staged two-direction
-// sweeps (96 KB: 12288 doubles or 24576 floats).
-#define STR_LINE_BYTES (96 * 1024)
-
-// Right-hand sides of r-line j at row i and of z-line i at row j, as
-// str_rline and str_zline form them.
-__device__ __forceinline__ double str_rhs_r(const StrDev &d, const StrLevel &L, int j, int i)
+// Right-hand sides of r-line j at row i (rcsc.f:1246-1252) and of z-line i at
+// row j (rcsc.f:1279-1290).
+template <class T> __device__ __forceinline__ T str_rhs(const StrView<T> &L, int dir, int i, int j)
 {
-    const int n1 = L.n1, n2 = L.n2;
-    const double *f = L.f;
-    if (j <= n2 / 2)
-        return -(CZZ(j, 1) * PS(i, j - 1) + CZZ(j, 3) * PS(i, j + 1) + CZZ(j, 4) * PS(i, j + 2)) +
-               f[(size_t)i + (size_t)(n1 + 1) * j];
-    return -(CZZ(j, 1) * PS(i, j - 2) + CZZ(j, 2) * PS(i, j - 1) + CZZ(j, 4) * PS(i, j + 1)) +
-           f[(size_t)i + (size_t)(n1 + 1) * j];
-}
-
-__device__ __forceinline__ double str_rhs_z(const StrDev &d, const StrLevel &L, int i, int j)
-{
-    const int n1 = L.n1;
-    const double *f = L.f;
-    const double r = L.r[i];
-    if (i <= n1 / 2)
-        return -(CRR(i, 1) * PS(i - 1, j) + CRR(i, 3) * PS(i + 1, j) + CRR(i, 4) * PS(i + 2, j) +
-                 div_by_rcp(CR(i, 1) * PS(i - 1, j) + CR(i, 3) * PS(i + 1, j), r, L.ir[i])) +
-               f[(size_t)i + (size_t)(n1 + 1) * j];
-    return -(CRR(i, 1) * PS(i - 2, j) + CRR(i, 2) * PS(i - 1, j) + CRR(i, 4) * PS(i + 1, j) +
-             div_by_rcp(CR(i, 1) * PS(i - 1, j) + CR(i, 3) * PS(i + 1, j), r, L.ir[i])) +
-           f[(size_t)i + (size_t)(n1 + 1) * j];
-}
-
-// One colour (every fourth line from `first`) of one direction (DIR 0:
-// r-lines j, DIR 1: z-lines i) in batches staged in shared memory: the
-// right-hand sides go in as [row][line] with an odd pitch (coalesced along
-// the grid's rows, conflict-free for the per-line elimination), one thread
-// per line eliminates in place, the solutions go back.  The lines of a
-// colour read only lines of the other colours, so staging changes no value.
-template <int DIR>
-__device__ void str_colour_smem(const StrDev &d, const StrLevel &L, int first, double *sline)
-{
-    const int n1 = L.n1, n2 = L.n2;
-    const int lines = DIR == 0 ? n2 - 1 : n1 - 1, n = DIR == 0 ? n1 - 1 : n2 - 1;
-    if (first > lines) return;
-    const int nl = (lines - first) / 4 + 1;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    int B = (int)(STR_LINE_BYTES / sizeof(double)) / n - 1;
-    if (B < 1) {   // lines too long to stage: one thread per line on the level's arrays
-        for (int t = threadIdx.x; t < nl; t += blockDim.x) {
-            if (DIR == 0) str_rline(d, L, first + 4 * t);
-            else str_zline(d, L, first + 4 * t);
-        }
-        __syncthreads();
-        return;
+    const T *crr = L.crr + 4 * (i - 1), *cr = L.cr + 3 * (i - 1), *czz = L.czz + 4 * (j - 1);
+    if (dir == 0) {
+        if (j <= L.n2 / 2) return -(czz[0] * V(i, j - 1) + czz[2] * V(i, j + 1) + czz[3] * V(i, j + 2)) + F(i, j);
+        return -(czz[0] * V(i, j - 2) + czz[1] * V(i, j - 1) + czz[3] * V(i, j + 1)) + F(i, j);
     }
-    if (B > nl) B = nl;
-    for (int b0 = 0; b0 < nl; b0 += B) {
-        const int nb = min(B, nl - b0), pitch = nb | 1;
+    const T over = str_over_r(L, i, cr[0] * V(i - 1, j) + cr[2] * V(i + 1, j));
+    if (i <= L.n1 / 2) return -(crr[0] * V(i - 1, j) + crr[2] * V(i + 1, j) + crr[3] * V(i + 2, j) + over) + F(i, j);
+    return -(crr[0] * V(i - 2, j) + crr[1] * V(i - 1, j) + crr[3] * V(i + 1, j) + over) + F(i, j);
+}
+
+// f - L v at (i, j) (relax's residual, rcsc.f:1300-1330)
+template <class T> __device__ __forceinline__ T str_resid(const StrView<T> &L, int i, int j)
+{
+    const T *crr = L.crr + 4 * (i - 1), *cr = L.cr + 3 * (i - 1), *czz = L.czz + 4 * (j - 1);
+    const T vc = V(i, j), vm = V(i - 1, j), vp = V(i + 1, j), vd = V(i, j - 1), vu = V(i, j + 1);
+    const T over = str_over_r(L, i, cr[0] * vm + cr[1] * vc + cr[2] * vp);
+    const T overq = str_over_rr(L, i, vc);
+    T t;
+    if (i <= L.n1 / 2) t = crr[0] * vm + crr[1] * vc + crr[2] * vp + crr[3] * V(i + 2, j) + over - overq;
+    else t = crr[0] * V(i - 2, j) + crr[1] * vm + crr[2] * vc + crr[3] * vp + over - overq;
+    if (j <= L.n2 / 2) t = t + czz[0] * vd + czz[1] * vc + czz[2] * vu + czz[3] * V(i, j + 2);
+    else t = t + czz[0] * V(i, j - 2) + czz[1] * vd + czz[2] * vc + czz[3] * vu;
+    return F(i, j) - t;
+}
+
+// Dynamic shared memory of a solve: per staged line its n right-hand sides
+// and its factors.
+#define STR_SMEM_BYTES (160 * 1024)
+
+// The nl lines first, first + step, ... of one direction (DIR 0: r-lines j,
+// DIR 1: z-lines i), which read none of one another: the four-colour order's
+// colours, or one line of the reference's order.  Each CTA takes a contiguous
+// share, in batches that fit its shared memory: the lines' factors are copied
+// there asynchronously (read once, coalesced: fetched from L2 inside an
+// elimination they cost each row more than its arithmetic) while all threads
+// form the right-hand sides, the lines are eliminated (FP64: one thread per
+// line in the reference's order; FP32: one warp per line), the solutions go
+// back.  (Not inlined: one copy per type and direction keeps the
+// eliminations' register blocks free of spills.)
+template <class T, int DIR>
+__device__ __noinline__ void str_lines(const StrLevel &lev, int first, int step, int nl)
+{
+    extern __shared__ __align__(16) unsigned char s_str[];
+    constexpr bool F64 = sizeof(T) == 8;
+    T *smem = (T *)s_str;
+    const Cluster cl = Cluster::self();
+    const StrView<T> L = str_view(lev, T(0));
+    const int n = DIR == 0 ? L.n1 - 1 : L.n2 - 1;
+    const int flen = (int)(F64 ? pdma_fac_len(n) : pdma32_len(n));
+    const int fpitch = F64 ? flen | 1 : flen;
+    const int lpitch = F64 ? 0 : wl_pitch(n), lg = F64 ? 0 : wl_log2m(n);
+    const int share = (nl + cl.size - 1) / cl.size;
+    const int t0 = cl.rank * share, t1 = min(nl, t0 + share);
+    const int words = (int)(STR_SMEM_BYTES / sizeof(T));
+    int B = F64 ? (words - n) / (n + fpitch) : words / (lpitch + fpitch);
+    const bool staged = B >= 1;       // a line with its factors fits (n up to 2900 in FP64)
+    if (!staged) B = 1;
+    B = min(B, min(share, (int)blockDim.x));
+    T *sfac = smem, *x = staged ? smem + B * fpitch : smem;
+    for (int b0 = t0; b0 < t1; b0 += B) {
+        const int nb = min(B, t1 - b0), pitch = nb | 1;
+        // FP64: [row][line], odd pitch; FP32: [line][row], padded per lane
+        auto at = [&](int t, int q) -> T & { return F64 ? x[q * pitch + t] : x[t * lpitch + wl_slot(lg, q)]; };
+        if (staged)
+            for (int t = 0; t < nb; ++t)
+                async_copy(sfac + t * fpitch, L.fac[DIR] + (size_t)(first + step * (b0 + t) - 1) * flen, flen, threadIdx.x,
+                           blockDim.x);
         if (DIR == 0) {
-            for (int t = warp; t < nb; t += nw)
-                for (int q = lane; q < n; q += 32) sline[q * pitch + t] = str_rhs_r(d, L, first + 4 * (b0 + t), q + 1);
+            const RowSplit split(n);
+            for (int idx = threadIdx.x; idx < nb * n; idx += blockDim.x) {
+                int t, q;
+                split(idx, t, q);
+                at(t, q) = str_rhs<T>(L, 0, q + 1, first + step * (b0 + t));
+            }
         } else {
-            for (int q = warp; q < n; q += nw)
-                for (int t = lane; t < nb; t += 32) sline[q * pitch + t] = str_rhs_z(d, L, first + 4 * (b0 + t), q + 1);
+            const RowSplit split(nb);
+            for (int idx = threadIdx.x; idx < nb * n; idx += blockDim.x) {
+                int q, t;
+                split(idx, q, t);
+                at(t, q) = str_rhs<T>(L, 1, first + step * (b0 + t), q + 1);
+            }
         }
+        if constexpr (!F64) {   // rows past the line's end
+            const int pad = wl_rows(n) - n;
+            for (int idx = threadIdx.x; idx < nb * pad; idx += blockDim.x) at(idx / pad, n + idx % pad) = T(0);
+        }
+        async_copy_wait();
         __syncthreads();
-        for (int t = threadIdx.x; t < nb; t += blockDim.x) {
-            const int line = first + 4 * (b0 + t);
-            double *x = sline + t;
-            const double *fac = (DIR == 0 ? L.fac_r : L.fac_z) + (size_t)(line - 1) * pdma_fac_len(n);
-            apply_pdma_rhs(fac, n, x, pitch, [&](int q) -> double { return x[q * pitch]; });
+        if constexpr (F64) {
+            if ((int)threadIdx.x < nb) {
+                const int t = threadIdx.x;
+                if (staged) pdma_staged(sfac + t * fpitch, n, x + t, pitch);
+                else pdma_staged(L.fac[DIR] + (size_t)(first + step * (b0 + t) - 1) * flen, n, x + t, pitch);
+            }
+        } else {
+            if (staged) wl_lines<true>(sfac, fpitch, n, x, lpitch, nb);
+            else wl_lines<true>(L.fac[DIR] + (size_t)(first + step * b0 - 1) * flen, (size_t)step * flen, n, x, lpitch, nb);
         }
         __syncthreads();
         if (DIR == 0) {
-            for (int t = warp; t < nb; t += nw)
-                for (int q = lane; q < n; q += 32) PS(q + 1, first + 4 * (b0 + t)) = sline[q * pitch + t];
+            const RowSplit split(n);
+            for (int idx = threadIdx.x; idx < nb * n; idx += blockDim.x) {
+                int t, q;
+                split(idx, t, q);
+                V(q + 1, first + step * (b0 + t)) = at(t, q);
+            }
         } else {
-            for (int q = warp; q < n; q += nw)
-                for (int t = lane; t < nb; t += 32) PS(first + 4 * (b0 + t), q + 1) = sline[q * pitch + t];
+            const RowSplit split(nb);
+            for (int idx = threadIdx.x; idx < nb * n; idx += blockDim.x) {
+                int q, t;
+                split(idx, q, t);
+                V(first + step * (b0 + t), q + 1) = at(t, q);
+            }
         }
-        __syncthreads();
+        if (b0 + B < t1) __syncthreads();
     }
+    cl.sync();
 }
 
-__device__ __forceinline__ double str_blk_max(double v, double *s_red)
-{
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, o));
-    if (lane == 0) s_red[warp] = v;
-    __syncthreads();
-    if (warp == 0) {
-        v = (lane < nw) ? s_red[lane] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, o));
-        if (lane == 0) s_red[32] = v;
-    }
-    __syncthreads();
-    const double r = s_red[32];
-    __syncthreads();
-    return r;
-}
-
-// relax (rcsc.f:1197-1341); returns the last residual max norm.
-__device__ double str_relax(const StrDev &d, int klev, double *s_red, int *nan_out)
+// relax's line sweeps (rcsc.f:1197-1299), nrel of them, in place on v.  The
+// reference also forms the residual after every sweep; only the last one is
+// ever read, and the caller forms that.
+template <class T> __device__ __forceinline__ void str_sweeps(const StrDev &d, int klev)
 {
     const StrLevel &L = d.lev[klev];
-    const int n1 = L.n1, n2 = L.n2;
-    const int tp = (n1 + 1) * (n2 + 1);
-    for (int idx = threadIdx.x; idx < tp; idx += blockDim.x) {
-        const int j = idx / (n1 + 1), i = idx - j * (n1 + 1);
-        PS(i, j) = L.v[idx];
-    }
-    __syncthreads();
-    double m = 0.0;
-    int nan = 0;
+    const int nj = L.n2 - 1, ni = L.n1 - 1;
     for (int irel = 0; irel < d.nrel; ++irel) {
         if (d.mode == GB_SMOOTHER_LEX) {
-            if (threadIdx.x == 0) {
-                for (int j = 1; j <= n2 - 1; ++j) str_rline(d, L, j);
-                for (int i = 1; i <= n1 - 1; ++i) str_zline(d, L, i);
-            }
-            __syncthreads();
+            for (int j = 1; j <= nj; ++j) str_lines<T, 0>(L, j, 1, 1);
+            for (int i = 1; i <= ni; ++i) str_lines<T, 1>(L, i, 1, 1);
         } else {
-            extern __shared__ double s_str_line[];
-            for (int c = 1; c <= 4; ++c) str_colour_smem<0>(d, L, (c & 3) == 0 ? 4 : (c & 3), s_str_line);
-            for (int c = 1; c <= 4; ++c) str_colour_smem<1>(d, L, (c & 3) == 0 ? 4 : (c & 3), s_str_line);
+            for (int c = 1; c <= 4; ++c)
+                if (c <= nj) str_lines<T, 0>(L, c, 4, (nj - c) / 4 + 1);
+            for (int c = 1; c <= 4; ++c)
+                if (c <= ni) str_lines<T, 1>(L, c, 4, (ni - c) / 4 + 1);
         }
-        m = 0.0;
-        nan = 0;
-        const int ni = n1 - 1, tot = ni * (n2 - 1);
-        for (int idx = threadIdx.x; idx < tot; idx += blockDim.x) {
-            const int j = idx / ni + 1, i = idx - (j - 1) * ni + 1;
-            const double r = L.r[i];
-            double temp;
-            if (i <= n1 / 2)
-                temp = CRR(i, 1) * PS(i - 1, j) + CRR(i, 2) * PS(i, j) + CRR(i, 3) * PS(i + 1, j) +
-                       CRR(i, 4) * PS(i + 2, j) + div_by_rcp(CR(i, 1) * PS(i - 1, j) + CR(i, 2) * PS(i, j) + CR(i, 3) * PS(i + 1, j), r, L.ir[i]) -
-                       div_by_rcp(PS(i, j), r * r, L.irr[i]);
-            else
-                temp = CRR(i, 1) * PS(i - 2, j) + CRR(i, 2) * PS(i - 1, j) + CRR(i, 3) * PS(i, j) +
-                       CRR(i, 4) * PS(i + 1, j) + div_by_rcp(CR(i, 1) * PS(i - 1, j) + CR(i, 2) * PS(i, j) + CR(i, 3) * PS(i + 1, j), r, L.ir[i]) -
-                       div_by_rcp(PS(i, j), r * r, L.irr[i]);
-            if (j <= n2 / 2)
-                temp = temp + CZZ(j, 1) * PS(i, j - 1) + CZZ(j, 2) * PS(i, j) + CZZ(j, 3) * PS(i, j + 1) +
-                       CZZ(j, 4) * PS(i, j + 2);
-            else
-                temp = temp + CZZ(j, 1) * PS(i, j - 2) + CZZ(j, 2) * PS(i, j - 1) + CZZ(j, 3) * PS(i, j) +
-                       CZZ(j, 4) * PS(i, j + 1);
-            temp = L.f[(size_t)i + (size_t)(n1 + 1) * j] - temp;
-            d.rc[(size_t)i + (size_t)d.ld * j] = temp;
-            temp = fabs(temp);
-            if (temp != temp) nan = 1;
-            if (temp > m) m = temp;
-        }
-        nan = __syncthreads_or(nan);
-        m = str_blk_max(m, s_red);
     }
-    for (int idx = threadIdx.x; idx < tp; idx += blockDim.x) {
-        const int j = idx / (n1 + 1), i = idx - j * (n1 + 1);
-        L.v[idx] = PS(i, j);
+}
+
+// The residual of level klev into rc (not followed by a barrier), its
+// largest magnitude and whether one is a NaN over the calling thread's points.
+template <class T, class R> __device__ __noinline__ T str_residual(const StrLevel &lev, R *rc, int *nan_out)
+{
+    const Cluster cl = Cluster::self();
+    const StrView<T> L = str_view(lev, T(0));
+    const int ni = L.n1 - 1, tot = ni * (L.n2 - 1);
+    const RowSplit split(ni);
+    T m = T(0);
+    int nan = 0;
+    for (int idx = cl.tid(); idx < tot; idx += cl.nthr()) {
+        int j, i;
+        split(idx, j, i);
+        ++i;
+        ++j;
+        const T r = str_resid<T>(L, i, j);
+        rc[i + L.ld * j] = (R)r;
+        const T a = fabs(r);
+        if (a != a) nan = 1;
+        if (a > m) m = a;
     }
-    __syncthreads();
     *nan_out = nan;
     return m;
 }
 
-// corser (rcsc.f:1343-1390): restriction of rc into the packed coarse
-// right-hand side; rows and columns 0 and n1c of the coarse level (n1 for
-// both directions) are zero, as are the boundary rows the restriction does
-// not reach (never read by the coarse relax); the coarse correction is zero.
-__device__ void str_corser(const StrDev &d, int klev)
+// corser (rcsc.f:1343-1390): restriction of rc into the coarse right-hand
+// side; rows and columns 0 and n1c of the coarse level (n1 for both
+// directions) are zero, as are the boundary rows the restriction does not
+// reach (never read by the coarse relax); the coarse correction is zero.
+template <class T> __device__ __noinline__ void str_corser(const StrLevel &coarse, const T *rc)
 {
-    const int ld = d.ld;
-    const int n1c = d.lev[klev + 1].n1, n2c = d.lev[klev + 1].n2;
-    const double *rf = d.rc;
-    double *fc = d.lev[klev + 1].f, *vc = d.lev[klev + 1].v;
+    const Cluster cl = Cluster::self();
+    const StrView<T> L = str_view(coarse, T(0));
+    const int ld = 2 * L.n1 + 1;
+    const int n1c = L.n1, n2c = L.n2;
     const int tot = (n1c + 1) * (n2c + 1);
-    for (int idx = threadIdx.x; idx < tot; idx += blockDim.x) {
-        const int j = idx / (n1c + 1), i = idx - j * (n1c + 1);
-        double temp = 0.0;
+    const RowSplit split(n1c + 1);
+    T *fc = const_cast<T *>(L.f);
+    for (int idx = cl.tid(); idx < tot; idx += cl.nthr()) {
+        int j, i;
+        split(idx, j, i);
+        T temp = T(0);
         if (i >= 1 && i <= n1c - 1 && j >= 1 && j <= n2c - 1 && j != n1c) {
-            const int ii = i + i, jj = j + j;
-            temp = rf[(size_t)ii + (size_t)ld * jj];
-            temp = temp * 2.0 + rf[(size_t)(ii + 1) + (size_t)ld * jj] + rf[(size_t)(ii - 1) + (size_t)ld * jj];
-            temp = temp + rf[(size_t)ii + (size_t)ld * (jj + 1)] + rf[(size_t)ii + (size_t)ld * (jj - 1)];
-            temp = temp * 2.0 + rf[(size_t)(ii + 1) + (size_t)ld * (jj + 1)] + rf[(size_t)(ii - 1) + (size_t)ld * (jj - 1)];
-            temp = temp + rf[(size_t)(ii + 1) + (size_t)ld * (jj - 1)] + rf[(size_t)(ii - 1) + (size_t)ld * (jj + 1)];
-            temp = temp / 16.0;
+            const T *q = rc + (i + i) + ld * (j + j);
+            temp = q[0];
+            temp = temp * T(2) + q[1] + q[-1];
+            temp = temp + q[ld] + q[-ld];
+            temp = temp * T(2) + q[1 + ld] + q[-1 - ld];
+            temp = temp + q[1 - ld] + q[-1 + ld];
+            temp = temp * T(0.0625);   // / 16, exactly
         }
         fc[idx] = temp;
-        vc[idx] = 0.0;
+        L.v[idx] = T(0);
     }
-    __syncthreads();
+    cl.sync();
 }
 
-// finer (rcsc.f:1392-1444)
-__device__ void str_finer(const StrDev &d, int klev)
+// finer (rcsc.f:1392-1444): bilinear prolongation added to the fine level.
+// The coarse correction is cleared by the next corser.
+template <class T> __device__ __noinline__ void str_finer(const StrLevel &coarse, const StrLevel &fine)
 {
-    const int n1c = d.lev[klev].n1;
-    const int n1f = d.lev[klev - 1].n1, n2f = d.lev[klev - 1].n2;
-    const double *vc = d.lev[klev].v;
-    double *vf = d.lev[klev - 1].v;
-    const int tot = (n1f + 1) * (n2f + 1);
-#define PC(ii, jj) vc[(size_t)(jj) * (n1c + 1) + (ii)]
-    for (int idx = threadIdx.x; idx < tot; idx += blockDim.x) {
-        const int j = idx / (n1f + 1), i = idx - j * (n1f + 1);
-        const int i1 = i / 2, j1 = j / 2;
-        double p;
-        if (i1 * 2 == i) {
-            if (j1 * 2 == j) p = PC(i1, j1);
-            else p = (PC(i1, j1) + PC(i1, j1 + 1)) * 0.5;
-        } else {
-            if (j1 * 2 == j) {
-                p = (PC(i1, j1) + PC(i1 + 1, j1)) * 0.5;
-            } else {
-                double temp = PC(i1, j1) + PC(i1 + 1, j1 + 1);
-                temp = temp + PC(i1, j1 + 1) + PC(i1 + 1, j1);
-                p = temp * 0.25;
-            }
-        }
-        PS(i, j) = p + vf[idx];
+    const Cluster cl = Cluster::self();
+    const StrView<T> Cc = str_view(coarse, T(0)), L = str_view(fine, T(0));
+    const int tot = L.ld * (L.n2 + 1);
+    const RowSplit split(L.ld);
+    for (int idx = cl.tid(); idx < tot; idx += cl.nthr()) {
+        int j, i;
+        split(idx, j, i);
+        const T *q = Cc.v + (i >> 1) + Cc.ld * (j >> 1);
+        T p;
+        if (!(i & 1)) p = !(j & 1) ? q[0] : (q[0] + q[Cc.ld]) * T(0.5);
+        else if (!(j & 1)) p = (q[0] + q[1]) * T(0.5);
+        else p = (q[0] + q[Cc.ld + 1] + q[Cc.ld] + q[1]) * T(0.25);
+        L.v[idx] = p + L.v[idx];
     }
-#undef PC
-    __syncthreads();
-    const int tc = (n1c + 1) * (d.lev[klev].n2 + 1);
-    for (int idx = threadIdx.x; idx < tc; idx += blockDim.x) d.lev[klev].v[idx] = 0.0;
-    for (int idx = threadIdx.x; idx < tot; idx += blockDim.x) {
-        const int j = idx / (n1f + 1), i = idx - j * (n1f + 1);
-        vf[idx] = PS(i, j);
-    }
-    __syncthreads();
+    cl.sync();
 }
 
 // poisson(psi, rhs, nlev, vel) (rcsc.f:1118-1195) on the staged arrays.
-__global__ void __launch_bounds__(STR_THREADS) k_str_solve(const __grid_constant__ StrDev d)
+__global__ void __maxnreg__(128) k_str_solve(const __grid_constant__ StrDev d)
 {
-    __shared__ double s_red[33];
-    if (d.abort && *d.abort) return;   // uniform over the block
+    __shared__ ClMaxState s_max;
+    const Cluster cl = Cluster::self();
+    if (d.abort && *d.abort) return;   // the same for every CTA: nothing sets it while the solve runs
+    int turn = 0;
     const int nlev = d.nlev;
-    const StrLevel &L1 = d.lev[1];
-    const int n1 = L1.n1, n2 = L1.n2;
-    const int tp = (n1 + 1) * (n2 + 1);
-    for (int idx = threadIdx.x; idx < tp; idx += blockDim.x) {
-        L1.f[idx] = d.io_rhs[idx];
-        L1.v[idx] = d.io_psi[idx];
+    const StrView<double> L = str_view(d.lev[1], 0.0);
+    const int tp = L.ld * (L.n2 + 1);
+    for (int idx = cl.tid(); idx < tp; idx += cl.nthr()) {
+        const_cast<double *>(L.f)[idx] = d.io_rhs[idx];
+        L.v[idx] = d.io_psi[idx];
     }
-    for (int idx = threadIdx.x; idx < d.ld * d.ld; idx += blockDim.x) d.rc[idx] = 0.0;
-    __syncthreads();
-    int status = GB_MAXSWEEPS, sweeps = d.maxsweeps, nan1 = 0, nn = 0;
+    cl.sync();
+    // relax on level l and the residual for the restriction or the test
+    // that follows; the norm matters on level 1 only (rcsc.f:1180)
     double res1 = 0.0;
+    int status = GB_MAXSWEEPS, sweeps = d.maxsweeps, nan1 = 0;
+    auto relax = [&](int l, bool restricted) {
+        str_sweeps<double>(d, l);
+        if (l != 1 && !restricted) return;
+        int nan;
+        const double m = str_residual<double>(d.lev[l], d.rc, &nan);
+        if (l == 1) {
+            res1 = cl_max(cl, s_max, turn, m, nan);
+            nan1 = nan;
+        } else {
+            cl.sync();
+        }
+    };
     for (int sweep = 1; sweep <= d.maxsweeps; ++sweep) {
-        if (sweep == 1 || nlev == 1) res1 = str_relax(d, 1, s_red, &nan1);
-        if (nlev > 1) {
-            for (int l = 1; l <= nlev - 1; ++l) {
-                str_corser(d, l);
-                str_relax(d, l + 1, s_red, &nn);
-            }
-            for (int l = nlev; l >= 2; --l) {
-                str_finer(d, l);
-                const double r = str_relax(d, l - 1, s_red, &nn);
-                if (l - 1 == 1) {
-                    res1 = r;
-                    nan1 = nn;
-                }
-            }
+        if (sweep == 1 || nlev == 1) relax(1, true);
+        for (int l = 1; l <= nlev - 1; ++l) {
+            str_corser<double>(d.lev[l + 1], d.rc);
+            relax(l + 1, l + 1 < nlev);
+        }
+        for (int l = nlev; l >= 2; --l) {
+            str_finer<double>(d.lev[l], d.lev[l - 1]);
+            relax(l - 1, false);
         }
         if (nan1) {
             status = GB_NAN;
@@ -430,20 +433,18 @@ __global__ void __launch_bounds__(STR_THREADS) k_str_solve(const __grid_constant
             break;
         }
         if (res1 < d.tolcon) {
-            for (int idx = threadIdx.x; idx < tp; idx += blockDim.x) {
-                const int j = idx / (n1 + 1), i = idx - j * (n1 + 1);
-                d.io_psi[idx] = PS(i, j);
-            }
+            for (int idx = cl.tid(); idx < tp; idx += cl.nthr()) d.io_psi[idx] = L.v[idx];
             status = GB_OK;
             sweeps = sweep;
             break;
         }
     }
-    if (threadIdx.x == 0) {
+    if (cl.tid() == 0) {
         d.status[0] = status;
         d.status[1] = sweeps;
         if (status == GB_NAN && d.abort) *d.abort = 1;
     }
+    cl.sync();   // no CTA leaves while another may still read its reduction slot
 }
 
 // ---------------------------------------------------------------------------
@@ -451,378 +452,88 @@ __global__ void __launch_bounds__(STR_THREADS) k_str_solve(const __grid_constant
 // iteration forms the FP64 residual r = f - L psi of the level-1 iterate
 // (relax's own residual expression), stops when max |r| < tolcon, else runs
 // one FP32 V-cycle of the same schedule on L e = r from e = 0 and updates
-// psi += e in FP64 (rcsc.f's solve has no over-relaxation).  The FP32 line
-// eliminations multiply by stored reciprocal pivots.
+// psi += e in FP64 (rcsc.f's solve has no over-relaxation).
 // ---------------------------------------------------------------------------
-#define PS32(i, j) d.psif32[(size_t)(i) + (size_t)d.ld * (size_t)(j)]
-#define CR32(i, k) L.cr32[3 * ((i) - 1) + (k) - 1]
-#define CRR32(i, k) L.crr32[4 * ((i) - 1) + (k) - 1]
-#define CZZ32(j, k) L.czz32[4 * ((j) - 1) + (k) - 1]
-
-template <class Rhs>
-__device__ inline void apply_pdma_rhs32(const float *fac, int n, float *x, int stride, Rhs rhs)
+__global__ void __maxnreg__(128) k_str_solve_mixed(const __grid_constant__ StrDev d)
 {
-    const float *icdiv = fac, *bk1 = fac + n, *aa = fac + 2 * n, *dn = fac + 3 * n, *en = fac + 4 * n;
-    const float icN = fac[5 * n];
-    float rk = rhs(0);
-    float rk1 = rhs(1);
-#pragma unroll 4
-    for (int k = 0; k <= n - 2; ++k) {
-        rk = rk * icdiv[k];
-        x[(size_t)k * stride] = rk;
-        rk1 = rk1 - bk1[k] * rk;
-        float rk2 = 0.f;
-        if (k != n - 2) rk2 = rhs(k + 2) - aa[k + 2] * rk;
-        rk = rk1;
-        rk1 = rk2;
-    }
-    float x1 = rk * icN;
-    x[(size_t)(n - 1) * stride] = x1;
-    float x0 = x[(size_t)(n - 2) * stride] - dn[n - 2] * x1;
-    x[(size_t)(n - 2) * stride] = x0;
-#pragma unroll 4
-    for (int j = n - 3; j >= 0; --j) {
-        const float xj = x[(size_t)j * stride] - dn[j] * x0 - en[j] * x1;
-        x[(size_t)j * stride] = xj;
-        x1 = x0;
-        x0 = xj;
-    }
-}
-
-__device__ __forceinline__ void str_rline32(const StrDev &d, const StrLevel &L, int j)
-{
-    const int n1 = L.n1, n2 = L.n2;
-    const float *f = L.f32;
-    auto rhs = [&](int q) -> float {
-        const int i = q + 1;
-        if (j <= n2 / 2)
-            return -(CZZ32(j, 1) * PS32(i, j - 1) + CZZ32(j, 3) * PS32(i, j + 1) + CZZ32(j, 4) * PS32(i, j + 2)) +
-                   f[(size_t)i + (size_t)(n1 + 1) * j];
-        return -(CZZ32(j, 1) * PS32(i, j - 2) + CZZ32(j, 2) * PS32(i, j - 1) + CZZ32(j, 4) * PS32(i, j + 1)) +
-               f[(size_t)i + (size_t)(n1 + 1) * j];
-    };
-    const int n = n1 - 1;
-    apply_pdma_rhs32(L.fac_r32 + (size_t)(j - 1) * (5 * n + 1), n, &PS32(1, j), 1, rhs);
-}
-
-__device__ __forceinline__ void str_zline32(const StrDev &d, const StrLevel &L, int i)
-{
-    const int n1 = L.n1, n2 = L.n2;
-    const float *f = L.f32;
-    const float ir = 1.0f / L.r32[i];
-    auto rhs = [&](int q) -> float {
-        const int j = q + 1;
-        if (i <= n1 / 2)
-            return -(CRR32(i, 1) * PS32(i - 1, j) + CRR32(i, 3) * PS32(i + 1, j) + CRR32(i, 4) * PS32(i + 2, j) +
-                     (CR32(i, 1) * PS32(i - 1, j) + CR32(i, 3) * PS32(i + 1, j)) * ir) +
-                   f[(size_t)i + (size_t)(n1 + 1) * j];
-        return -(CRR32(i, 1) * PS32(i - 2, j) + CRR32(i, 2) * PS32(i - 1, j) + CRR32(i, 4) * PS32(i + 1, j) +
-                 (CR32(i, 1) * PS32(i - 1, j) + CR32(i, 3) * PS32(i + 1, j)) * ir) +
-               f[(size_t)i + (size_t)(n1 + 1) * j];
-    };
-    const int n = n2 - 1;
-    apply_pdma_rhs32(L.fac_z32 + (size_t)(i - 1) * (5 * n + 1), n, &PS32(i, 1), d.ld, rhs);
-}
-
-__device__ __forceinline__ float str_rhs_r32(const StrDev &d, const StrLevel &L, int j, int i)
-{
-    const int n1 = L.n1, n2 = L.n2;
-    const float *f = L.f32;
-    if (j <= n2 / 2)
-        return -(CZZ32(j, 1) * PS32(i, j - 1) + CZZ32(j, 3) * PS32(i, j + 1) + CZZ32(j, 4) * PS32(i, j + 2)) +
-               f[(size_t)i + (size_t)(n1 + 1) * j];
-    return -(CZZ32(j, 1) * PS32(i, j - 2) + CZZ32(j, 2) * PS32(i, j - 1) + CZZ32(j, 4) * PS32(i, j + 1)) +
-           f[(size_t)i + (size_t)(n1 + 1) * j];
-}
-
-__device__ __forceinline__ float str_rhs_z32(const StrDev &d, const StrLevel &L, int i, int j)
-{
-    const int n1 = L.n1;
-    const float *f = L.f32;
-    const float ir = 1.0f / L.r32[i];
-    if (i <= n1 / 2)
-        return -(CRR32(i, 1) * PS32(i - 1, j) + CRR32(i, 3) * PS32(i + 1, j) + CRR32(i, 4) * PS32(i + 2, j) +
-                 (CR32(i, 1) * PS32(i - 1, j) + CR32(i, 3) * PS32(i + 1, j)) * ir) +
-               f[(size_t)i + (size_t)(n1 + 1) * j];
-    return -(CRR32(i, 1) * PS32(i - 2, j) + CRR32(i, 2) * PS32(i - 1, j) + CRR32(i, 4) * PS32(i + 1, j) +
-             (CR32(i, 1) * PS32(i - 1, j) + CR32(i, 3) * PS32(i + 1, j)) * ir) +
-           f[(size_t)i + (size_t)(n1 + 1) * j];
-}
-
-// str_colour_smem in FP32 (the correction cycle).
-template <int DIR>
-__device__ void str_colour_smem32(const StrDev &d, const StrLevel &L, int first, float *sline)
-{
-    const int n1 = L.n1, n2 = L.n2;
-    const int lines = DIR == 0 ? n2 - 1 : n1 - 1, n = DIR == 0 ? n1 - 1 : n2 - 1;
-    if (first > lines) return;
-    const int nl = (lines - first) / 4 + 1;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    int B = (int)(STR_LINE_BYTES / sizeof(float)) / n - 1;
-    if (B < 1) {
-        for (int t = threadIdx.x; t < nl; t += blockDim.x) {
-            if (DIR == 0) str_rline32(d, L, first + 4 * t);
-            else str_zline32(d, L, first + 4 * t);
-        }
-        __syncthreads();
-        return;
-    }
-    if (B > nl) B = nl;
-    for (int b0 = 0; b0 < nl; b0 += B) {
-        const int nb = min(B, nl - b0), pitch = nb | 1;
-        if (DIR == 0) {
-            for (int t = warp; t < nb; t += nw)
-                for (int q = lane; q < n; q += 32) sline[q * pitch + t] = str_rhs_r32(d, L, first + 4 * (b0 + t), q + 1);
-        } else {
-            for (int q = warp; q < n; q += nw)
-                for (int t = lane; t < nb; t += 32) sline[q * pitch + t] = str_rhs_z32(d, L, first + 4 * (b0 + t), q + 1);
-        }
-        __syncthreads();
-        for (int t = threadIdx.x; t < nb; t += blockDim.x) {
-            const int line = first + 4 * (b0 + t);
-            const float *fac = (DIR == 0 ? L.fac_r32 : L.fac_z32) + (size_t)(line - 1) * (5 * n + 1);
-            pdma32_smem(fac, n, sline + t, pitch);
-        }
-        __syncthreads();
-        if (DIR == 0) {
-            for (int t = warp; t < nb; t += nw)
-                for (int q = lane; q < n; q += 32) PS32(q + 1, first + 4 * (b0 + t)) = sline[q * pitch + t];
-        } else {
-            for (int q = warp; q < n; q += nw)
-                for (int t = lane; t < nb; t += 32) PS32(first + 4 * (b0 + t), q + 1) = sline[q * pitch + t];
-        }
-        __syncthreads();
-    }
-}
-
-// nrel sweeps of both line directions on level klev, then the residual of
-// the correction into rc32 (for the restriction that follows).
-__device__ void str_relax32(const StrDev &d, int klev)
-{
-    const StrLevel &L = d.lev[klev];
-    const int n1 = L.n1, n2 = L.n2;
-    const int tp = (n1 + 1) * (n2 + 1);
-    for (int idx = threadIdx.x; idx < tp; idx += blockDim.x) {
-        const int j = idx / (n1 + 1), i = idx - j * (n1 + 1);
-        PS32(i, j) = L.v32[idx];
-    }
-    __syncthreads();
-    for (int irel = 0; irel < d.nrel; ++irel) {
-        if (d.mode == GB_SMOOTHER_LEX) {
-            if (threadIdx.x == 0) {
-                for (int j = 1; j <= n2 - 1; ++j) str_rline32(d, L, j);
-                for (int i = 1; i <= n1 - 1; ++i) str_zline32(d, L, i);
-            }
-            __syncthreads();
-        } else {
-            extern __shared__ float s_str_line32[];
-            for (int c = 1; c <= 4; ++c) str_colour_smem32<0>(d, L, (c & 3) == 0 ? 4 : (c & 3), s_str_line32);
-            for (int c = 1; c <= 4; ++c) str_colour_smem32<1>(d, L, (c & 3) == 0 ? 4 : (c & 3), s_str_line32);
-        }
-    }
-    const int ni = n1 - 1, tot = ni * (n2 - 1);
-    for (int idx = threadIdx.x; idx < tot; idx += blockDim.x) {
-        const int j = idx / ni + 1, i = idx - (j - 1) * ni + 1;
-        const float ir = 1.0f / L.r32[i];
-        float temp;
-        if (i <= n1 / 2)
-            temp = CRR32(i, 1) * PS32(i - 1, j) + CRR32(i, 2) * PS32(i, j) + CRR32(i, 3) * PS32(i + 1, j) +
-                   CRR32(i, 4) * PS32(i + 2, j) +
-                   (CR32(i, 1) * PS32(i - 1, j) + CR32(i, 2) * PS32(i, j) + CR32(i, 3) * PS32(i + 1, j)) * ir -
-                   PS32(i, j) * (ir * ir);
-        else
-            temp = CRR32(i, 1) * PS32(i - 2, j) + CRR32(i, 2) * PS32(i - 1, j) + CRR32(i, 3) * PS32(i, j) +
-                   CRR32(i, 4) * PS32(i + 1, j) +
-                   (CR32(i, 1) * PS32(i - 1, j) + CR32(i, 2) * PS32(i, j) + CR32(i, 3) * PS32(i + 1, j)) * ir -
-                   PS32(i, j) * (ir * ir);
-        if (j <= n2 / 2)
-            temp = temp + CZZ32(j, 1) * PS32(i, j - 1) + CZZ32(j, 2) * PS32(i, j) + CZZ32(j, 3) * PS32(i, j + 1) +
-                   CZZ32(j, 4) * PS32(i, j + 2);
-        else
-            temp = temp + CZZ32(j, 1) * PS32(i, j - 2) + CZZ32(j, 2) * PS32(i, j - 1) + CZZ32(j, 3) * PS32(i, j) +
-                   CZZ32(j, 4) * PS32(i, j + 1);
-        d.rc32[(size_t)i + (size_t)d.ld * j] = L.f32[(size_t)i + (size_t)(n1 + 1) * j] - temp;
-    }
-    for (int idx = threadIdx.x; idx < tp; idx += blockDim.x) {
-        const int j = idx / (n1 + 1), i = idx - j * (n1 + 1);
-        L.v32[idx] = PS32(i, j);
-    }
-    __syncthreads();
-}
-
-// corser (rcsc.f:1343-1390) in FP32, with its clearing of rows and columns 0
-// and n1c in both directions
-__device__ void str_corser32(const StrDev &d, int klev)
-{
-    const int ld = d.ld;
-    const int n1c = d.lev[klev + 1].n1, n2c = d.lev[klev + 1].n2;
-    const float *rf = d.rc32;
-    float *fc = d.lev[klev + 1].f32, *vc = d.lev[klev + 1].v32;
-    const int tot = (n1c + 1) * (n2c + 1);
-    for (int idx = threadIdx.x; idx < tot; idx += blockDim.x) {
-        const int j = idx / (n1c + 1), i = idx - j * (n1c + 1);
-        float temp = 0.f;
-        if (i >= 1 && i <= n1c - 1 && j >= 1 && j <= n2c - 1 && j != n1c) {
-            const int ii = i + i, jj = j + j;
-            temp = rf[(size_t)ii + (size_t)ld * jj];
-            temp = temp * 2.f + rf[(size_t)(ii + 1) + (size_t)ld * jj] + rf[(size_t)(ii - 1) + (size_t)ld * jj];
-            temp = temp + rf[(size_t)ii + (size_t)ld * (jj + 1)] + rf[(size_t)ii + (size_t)ld * (jj - 1)];
-            temp = temp * 2.f + rf[(size_t)(ii + 1) + (size_t)ld * (jj + 1)] + rf[(size_t)(ii - 1) + (size_t)ld * (jj - 1)];
-            temp = temp + rf[(size_t)(ii + 1) + (size_t)ld * (jj - 1)] + rf[(size_t)(ii - 1) + (size_t)ld * (jj + 1)];
-            temp = temp * 0.0625f;
-        }
-        fc[idx] = temp;
-        vc[idx] = 0.f;
-    }
-    __syncthreads();
-}
-
-// finer (rcsc.f:1392-1444) in FP32
-__device__ void str_finer32(const StrDev &d, int klev)
-{
-    const int n1c = d.lev[klev].n1;
-    const int n1f = d.lev[klev - 1].n1, n2f = d.lev[klev - 1].n2;
-    const float *vc = d.lev[klev].v32;
-    float *vf = d.lev[klev - 1].v32;
-    const int tot = (n1f + 1) * (n2f + 1);
-#define PC32(ii, jj) vc[(size_t)(jj) * (n1c + 1) + (ii)]
-    for (int idx = threadIdx.x; idx < tot; idx += blockDim.x) {
-        const int j = idx / (n1f + 1), i = idx - j * (n1f + 1);
-        const int i1 = i / 2, j1 = j / 2;
-        float p;
-        if (i1 * 2 == i) p = (j1 * 2 == j) ? PC32(i1, j1) : (PC32(i1, j1) + PC32(i1, j1 + 1)) * 0.5f;
-        else if (j1 * 2 == j) p = (PC32(i1, j1) + PC32(i1 + 1, j1)) * 0.5f;
-        else p = (PC32(i1, j1) + PC32(i1 + 1, j1 + 1) + PC32(i1, j1 + 1) + PC32(i1 + 1, j1)) * 0.25f;
-        PS32(i, j) = p + vf[idx];
-    }
-#undef PC32
-    __syncthreads();
-    const int tc = (n1c + 1) * (d.lev[klev].n2 + 1);
-    for (int idx = threadIdx.x; idx < tc; idx += blockDim.x) d.lev[klev].v32[idx] = 0.f;
-    for (int idx = threadIdx.x; idx < tot; idx += blockDim.x) {
-        const int j = idx / (n1f + 1), i = idx - j * (n1f + 1);
-        vf[idx] = PS32(i, j);
-    }
-    __syncthreads();
-}
-
-// FP64 residual of level 1 (relax's expression, rcsc.f:1300-1330)
-__device__ __forceinline__ double str_resid64(const StrDev &d, const StrLevel &L, int i, int j)
-{
-    const int n1 = L.n1, n2 = L.n2;
-    const double r = L.r[i];
-    double temp;
-    if (i <= n1 / 2)
-        temp = CRR(i, 1) * PS(i - 1, j) + CRR(i, 2) * PS(i, j) + CRR(i, 3) * PS(i + 1, j) + CRR(i, 4) * PS(i + 2, j) +
-               div_by_rcp(CR(i, 1) * PS(i - 1, j) + CR(i, 2) * PS(i, j) + CR(i, 3) * PS(i + 1, j), r, L.ir[i]) - div_by_rcp(PS(i, j), r * r, L.irr[i]);
-    else
-        temp = CRR(i, 1) * PS(i - 2, j) + CRR(i, 2) * PS(i - 1, j) + CRR(i, 3) * PS(i, j) + CRR(i, 4) * PS(i + 1, j) +
-               div_by_rcp(CR(i, 1) * PS(i - 1, j) + CR(i, 2) * PS(i, j) + CR(i, 3) * PS(i + 1, j), r, L.ir[i]) - div_by_rcp(PS(i, j), r * r, L.irr[i]);
-    if (j <= n2 / 2)
-        temp = temp + CZZ(j, 1) * PS(i, j - 1) + CZZ(j, 2) * PS(i, j) + CZZ(j, 3) * PS(i, j + 1) + CZZ(j, 4) * PS(i, j + 2);
-    else
-        temp = temp + CZZ(j, 1) * PS(i, j - 2) + CZZ(j, 2) * PS(i, j - 1) + CZZ(j, 3) * PS(i, j) + CZZ(j, 4) * PS(i, j + 1);
-    return L.f[(size_t)i + (size_t)(n1 + 1) * j] - temp;
-}
-
-__global__ void __launch_bounds__(STR_THREADS) k_str_solve_mixed(const __grid_constant__ StrDev d)
-{
-    __shared__ double s_red[33];
+    __shared__ ClMaxState s_max;
+    const Cluster cl = Cluster::self();
     if (d.abort && *d.abort) return;
+    int turn = 0;
     const int nlev = d.nlev;
-    const StrLevel &L1 = d.lev[1];
-    const int n1 = L1.n1, n2 = L1.n2;
-    const int tp = (n1 + 1) * (n2 + 1);
-    for (int idx = threadIdx.x; idx < tp; idx += blockDim.x) {
-        const int j = idx / (n1 + 1), i = idx - j * (n1 + 1);
-        L1.f[idx] = d.io_rhs[idx];
-        PS(i, j) = d.io_psi[idx];
-        L1.f32[idx] = 0.f;
+    const StrView<double> L = str_view(d.lev[1], 0.0);
+    const StrView<float> L32 = str_view(d.lev[1], 0.f);
+    const int tp = L.ld * (L.n2 + 1);
+    for (int idx = cl.tid(); idx < tp; idx += cl.nthr()) {
+        const_cast<double *>(L.f)[idx] = d.io_rhs[idx];
+        L.v[idx] = d.io_psi[idx];
+        L32.v[idx] = 0.f;
+        const_cast<float *>(L32.f)[idx] = 0.f;
     }
-    for (int idx = threadIdx.x; idx < d.ld * d.ld; idx += blockDim.x) d.rc32[idx] = 0.f;
-    __syncthreads();
-    const int ni = n1 - 1, tot = ni * (n2 - 1);
+    cl.sync();
+    auto relax = [&](int l, bool restricted) {
+        str_sweeps<float>(d, l);
+        if (!restricted) return;
+        int nan;
+        str_residual<float>(d.lev[l], d.rc32, &nan);
+        cl.sync();
+    };
     int status = GB_MAXSWEEPS, cycles = 0;
     for (int it = 0;; ++it) {
-        double m = 0.0;
-        int nan = 0;
-        for (int idx = threadIdx.x; idx < tot; idx += blockDim.x) {
-            const int j = idx / ni + 1, i = idx - (j - 1) * ni + 1;
-            const double rr = str_resid64(d, L1, i, j);
-            L1.f32[(size_t)i + (size_t)(n1 + 1) * j] = (float)rr;
-            const double a = fabs(rr);
-            if (a != a) nan = 1;
-            if (a > m) m = a;
-        }
-        nan = __syncthreads_or(nan);
-        const double res = str_blk_max(m, s_red);
+        int nan;
+        const double m = str_residual<double>(d.lev[1], const_cast<float *>(L32.f), &nan);
+        const double res = cl_max(cl, s_max, turn, m, nan);
         if (nan) { status = GB_NAN; break; }
         if (res < d.tolcon) { status = GB_OK; break; }
         if (it == d.maxsweeps) break;
-        for (int q = threadIdx.x; q < tp; q += blockDim.x) L1.v32[q] = 0.f;
-        __syncthreads();
-        str_relax32(d, 1);
-        if (nlev > 1) {
-            for (int l = 1; l <= nlev - 1; ++l) {
-                str_corser32(d, l);
-                str_relax32(d, l + 1);
-            }
-            for (int l = nlev; l >= 2; --l) {
-                str_finer32(d, l);
-                str_relax32(d, l - 1);
-            }
+        relax(1, nlev > 1);
+        for (int l = 1; l <= nlev - 1; ++l) {
+            str_corser<float>(d.lev[l + 1], d.rc32);
+            relax(l + 1, l + 1 < nlev);
         }
-        for (int idx = threadIdx.x; idx < tot; idx += blockDim.x) {
-            const int j = idx / ni + 1, i = idx - (j - 1) * ni + 1;
-            PS(i, j) += (double)L1.v32[(size_t)i + (size_t)(n1 + 1) * j];
+        for (int l = nlev; l >= 2; --l) {
+            str_finer<float>(d.lev[l], d.lev[l - 1]);
+            relax(l - 1, false);
         }
-        __syncthreads();
+        // psi += e, and e = 0 for the next cycle
+        for (int idx = cl.tid(); idx < tp; idx += cl.nthr()) {
+            L.v[idx] += (double)L32.v[idx];
+            L32.v[idx] = 0.f;
+        }
+        cl.sync();
         cycles = it + 1;
     }
     if (status == GB_OK)
-        for (int idx = threadIdx.x; idx < tp; idx += blockDim.x) {
-            const int j = idx / (n1 + 1), i = idx - j * (n1 + 1);
-            d.io_psi[idx] = PS(i, j);
-        }
-    if (threadIdx.x == 0) {
+        for (int idx = cl.tid(); idx < tp; idx += cl.nthr()) d.io_psi[idx] = L.v[idx];
+    if (cl.tid() == 0) {
         d.status[0] = status;
         d.status[1] = cycles;
         if (status == GB_NAN && d.abort) *d.abort = 1;
     }
+    cl.sync();
 }
 
-// FP32 copies of a level's tables and factors (pivots as reciprocals), one
-// thread per level.
+#undef V
+#undef F
+
+// FP32 copies of a level's tables and its folded factors: block row y takes
+// level y + 1, one thread per r-line, then per z-line.
 __global__ void k_str_factors32(const __grid_constant__ StrDev d)
 {
-    const int l = 1 + blockIdx.x;
-    if (threadIdx.x != 0 || l > d.nlev) return;
-    const StrLevel &L = d.lev[l];
+    const StrLevel &L = d.lev[1 + blockIdx.y];
     const int a = L.n1, b = L.n2;
-    for (int i = 0; i <= a; ++i) L.r32[i] = (float)L.r[i];
-    for (int q = 0; q < 3 * (a - 1); ++q) L.cr32[q] = (float)L.cr[q];
-    for (int q = 0; q < 4 * (a - 1); ++q) L.crr32[q] = (float)L.crr[q];
-    for (int q = 0; q < 4 * (b - 1); ++q) L.czz32[q] = (float)L.czz[q];
-    auto conv = [](const double *fac, float *g, int n) {
-        for (int k = 0; k < n; ++k) g[k] = (float)(1.0 / fac[k]);   // cdiv as reciprocals
-        for (int k = n; k < 5 * n; ++k) g[k] = (float)fac[k];
-        g[5 * n] = (float)(1.0 / fac[5 * n]);
-    };
+    if (blockIdx.x == 0) {
+        for (int i = threadIdx.x; i <= a; i += blockDim.x) L.r32[i] = (float)L.r[i];
+        for (int q = threadIdx.x; q < 3 * (a - 1); q += blockDim.x) L.cr32[q] = (float)L.cr[q];
+        for (int q = threadIdx.x; q < 4 * (a - 1); q += blockDim.x) L.crr32[q] = (float)L.crr[q];
+        for (int q = threadIdx.x; q < 4 * (b - 1); q += blockDim.x) L.czz32[q] = (float)L.czz[q];
+    }
     const int nr = a - 1, nz = b - 1;
-    for (int j = 1; j <= b - 1; ++j)
-        conv(L.fac_r + (size_t)(j - 1) * pdma_fac_len(nr), L.fac_r32 + (size_t)(j - 1) * (5 * nr + 1), nr);
-    for (int i = 1; i <= a - 1; ++i)
-        conv(L.fac_z + (size_t)(i - 1) * pdma_fac_len(nz), L.fac_z32 + (size_t)(i - 1) * (5 * nz + 1), nz);
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t < nz) pdma32_fold(L.fac_r + (size_t)t * pdma_fac_len(nr), nr, L.fac_r32 + (size_t)t * pdma32_len(nr));
+    else if (t < nz + nr)
+        pdma32_fold(L.fac_z + (size_t)(t - nz) * pdma_fac_len(nz), nz, L.fac_z32 + (size_t)(t - nz) * pdma32_len(nz));
 }
-
-#undef PS32
-#undef CR32
-#undef CRR32
-#undef CZZ32
-#undef PS
-#undef CR
-#undef CRR
-#undef CZZ
 
 // ---------------------------------------------------------------------------
 // Host side
@@ -832,13 +543,76 @@ struct gb_str {
     double *pool = nullptr;
     int *status = nullptr;
     cudaStream_t stream = nullptr;
+    int ctas = 1;             // CTAs per four-colour FP64 solve
+    MerDev mer;               // the resident mixed solve (meridian.cu), where its plan fits
+    int mer_ctas = 0;         // its CTAs; 0: k_str_solve_mixed
+    void *mer_mem = nullptr;
 };
+
+// One scan-step count per level and direction (block x: direction).
+__global__ void k_str_steps32(const __grid_constant__ StrDev d)
+{
+    const StrLevel &L = d.lev[1 + blockIdx.y];
+    if (blockIdx.x == 0) wl_common_steps(L.fac_r32, pdma32_len(L.n1 - 1), L.n2 - 1);
+    else wl_common_steps(L.fac_z32, pdma32_len(L.n2 - 1), L.n1 - 1);
+}
+
+// The resident solve's weights: grid.f's first and second derivatives of a
+// row combined in FP64 (and rounded once for the correction cycles).
+__global__ void k_str_weights(const __grid_constant__ StrDev d, const __grid_constant__ MerDev m)
+{
+    const int l = 1 + blockIdx.y, t = blockIdx.x * blockDim.x + threadIdx.x;
+    const StrLevel &L = d.lev[l];
+    auto put = [&](const float4 *c4, const MerW *d4, int q, double cm, double cp, double cf, double cd) {
+        const_cast<float4 *>(c4)[q] = make_float4((float)cm, (float)cp, (float)cf, (float)cd);
+        if (l == 1) const_cast<MerW *>(d4)[q] = MerW{cm, cp, cf, cd};
+    };
+    if (t >= 1 && t < L.n1) {
+        const int i = t;
+        const double r = L.r[i], cr1 = CR(i, 1) / r, cr2 = CR(i, 2) / r - 1.0 / (r * r), cr3 = CR(i, 3) / r;
+        if (i <= L.n1 / 2) put(m.lev[l].c4i, m.d4i, i, CRR(i, 1) + cr1, CRR(i, 3) + cr3, CRR(i, 4), CRR(i, 2) + cr2);
+        else put(m.lev[l].c4i, m.d4i, i, CRR(i, 2) + cr1, CRR(i, 4) + cr3, CRR(i, 1), CRR(i, 3) + cr2);
+    }
+    if (t >= 1 && t < L.n2) {
+        const int j = t;
+        if (j <= L.n2 / 2) put(m.lev[l].c4j, m.d4j, j, CZZ(j, 1), CZZ(j, 3), CZZ(j, 4), CZZ(j, 2));
+        else put(m.lev[l].c4j, m.d4j, j, CZZ(j, 2), CZZ(j, 4), CZZ(j, 1), CZZ(j, 3));
+    }
+}
+
+// Prepares the resident mixed solve; a grid it cannot hold leaves mer_ctas 0.
+static cudaError_t str_mer_create(gb_str *h)
+{
+    const StrDev &d = h->dev;
+    MerDev &m = h->mer;
+    memset(&m, 0, sizeof(m));
+    m.nlev = d.nlev;
+    m.penta = 1;
+    for (int l = 1; l <= d.nlev; ++l) {
+        MerLevel &L = m.lev[l];
+        L.n1 = d.lev[l].n1;
+        L.n2 = d.lev[l].n2;
+        L.fac_r = d.lev[l].fac_r32;
+        L.fac_z = d.lev[l].fac_z32;
+        L.fac_r_step = (int)pdma32_len(L.n1 - 1);
+        L.fac_z_step = (int)pdma32_len(L.n2 - 1);
+    }
+    m.v = d.lev[1].v;
+    h->mer_ctas = mer_fit(m, CL_MAX_CTAS);
+    if (!h->mer_ctas) return cudaSuccess;
+    cudaError_t e = cudaMalloc(&h->mer_mem, mer_weight_bytes(m));
+    if (e != cudaSuccess) return e;
+    mer_weight_layout(m, h->mer_mem);
+    k_str_weights<<<dim3(gb_ceil_div((size_t)std::max(m.lev[1].n1, m.lev[1].n2), 128), m.nlev), 128>>>(d, m);
+    return cudaDeviceSynchronize();
+}
 
 extern "C" int gb_str_destroy(gb_str *h)
 {
     if (!h) return GB_OK;
     cudaFree(h->pool);
     cudaFree(h->status);
+    cudaFree(h->mer_mem);
     if (h->stream) cudaStreamDestroy(h->stream);
     delete h;
     return GB_OK;
@@ -870,23 +644,23 @@ extern "C" int gb_str_create(int nlev, const gb_str_level *lv, double tolcon, in
     StrDev &d = h->dev;
     memset(&d, 0, sizeof(d));
     d.nlev = nlev;
-    d.ld = std::max(n1, n2) + 1;
+    const size_t pts1 = (size_t)(n1 + 1) * (n2 + 1);
     d.nrel = nrel;
     d.maxsweeps = maxsweeps;
     d.mode = smoother;
     d.tolcon = tolcon;
-    size_t need = 2 * (size_t)d.ld * d.ld + 2 * (size_t)(n1 + 1) * (n2 + 1);
+    size_t need = 3 * pts1;
     for (int l = 0; l < nlev; ++l) {
         const size_t a = lv[l].n1, b = lv[l].n2;
         need += 3 * (a + 1) + 3 * (a - 1) + 4 * (a - 1) + 4 * (b - 1) + 2 * (a + 1) * (b + 1);
         need += (b - 1) * pdma_fac_len((int)a - 1) + (a - 1) * pdma_fac_len((int)b - 1);
     }
-    // FP32 copies: psif32, rc32 and every level's tables (half a double each, rounded up per array)
-    size_t need32 = 2 * (size_t)d.ld * d.ld + 16;
+    // FP32 copies: rc32 and every level's tables (half a double each, rounded up per array)
+    size_t need32 = pts1 + 16;
     for (int l = 0; l < nlev; ++l) {
         const size_t a = lv[l].n1, b = lv[l].n2;
         need32 += (a + 1) + 3 * (a - 1) + 4 * (a - 1) + 4 * (b - 1) + 2 * (a + 1) * (b + 1);
-        need32 += (b - 1) * (5 * (a - 1) + 1) + (a - 1) * (5 * (b - 1) + 1) + 16;
+        need32 += (b - 1) * pdma32_len((int)a - 1) + (a - 1) * pdma32_len((int)b - 1) + 16;
     }
     const size_t need64 = need;
     need += (need32 + 1) / 2;
@@ -894,10 +668,9 @@ extern "C" int gb_str_create(int nlev, const gb_str_level *lv, double tolcon, in
     if (e != cudaSuccess) { delete h; gb_set_error("gb_str_create: %s", cudaGetErrorString(e)); return GB_ERR_ALLOC; }
     cudaMemset(h->pool, 0, sizeof(double) * need);
     double *b = h->pool;
-    d.psif = b; b += (size_t)d.ld * d.ld;
-    d.rc = b; b += (size_t)d.ld * d.ld;
-    d.io_psi = b; b += (size_t)(n1 + 1) * (n2 + 1);
-    d.io_rhs = b; b += (size_t)(n1 + 1) * (n2 + 1);
+    d.rc = b; b += pts1;
+    d.io_psi = b; b += pts1;
+    d.io_rhs = b; b += pts1;
     std::vector<StrJob> jobs;
     int wmax = 0;
     for (int l = 0; l < nlev; ++l) {
@@ -940,8 +713,7 @@ extern "C" int gb_str_create(int nlev, const gb_str_level *lv, double tolcon, in
     {
         float *fb = (float *)b;
         float *fend = (float *)(h->pool + need);
-        d.psif32 = fb; fb += (size_t)d.ld * d.ld;
-        d.rc32 = fb; fb += (size_t)d.ld * d.ld;
+        d.rc32 = fb; fb += pts1;
         for (int l = 1; l <= nlev; ++l) {
             StrLevel &L = d.lev[l];
             const size_t a = L.n1, bb = L.n2;
@@ -951,8 +723,9 @@ extern "C" int gb_str_create(int nlev, const gb_str_level *lv, double tolcon, in
             L.czz32 = fb; fb += 4 * (bb - 1);
             L.v32 = fb; fb += (a + 1) * (bb + 1);
             L.f32 = fb; fb += (a + 1) * (bb + 1);
-            L.fac_r32 = fb; fb += (bb - 1) * (5 * (a - 1) + 1);
-            L.fac_z32 = fb; fb += (a - 1) * (5 * (bb - 1) + 1);
+            fb = (float *)(((uintptr_t)fb + 15) & ~(uintptr_t)15);   // the tables are copied 16 bytes at a time
+            L.fac_r32 = fb; fb += (bb - 1) * pdma32_len((int)a - 1);
+            L.fac_z32 = fb; fb += (a - 1) * pdma32_len((int)bb - 1);
         }
         if (fb > fend) {
             gb_str_destroy(h);
@@ -977,7 +750,8 @@ extern "C" int gb_str_create(int nlev, const gb_str_level *lv, double tolcon, in
     cudaFree(djobs);
     cudaFree(work);
     if (e == cudaSuccess) {
-        k_str_factors32<<<nlev, 32>>>(d);
+        k_str_factors32<<<dim3(gb_ceil_div((size_t)n1 + n2, 32), nlev), 32>>>(d);
+        k_str_steps32<<<dim3(2, nlev), 256>>>(d);
         e = cudaDeviceSynchronize();
     }
     if (e != cudaSuccess) { gb_set_error("gb_str_create: factors: %s", cudaGetErrorString(e)); gb_str_destroy(h); return GB_ERR_CUDA; }
@@ -986,11 +760,22 @@ extern "C" int gb_str_create(int nlev, const gb_str_level *lv, double tolcon, in
     d.status = h->status;
     e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) { gb_str_destroy(h); gb_set_error("gb_str_create: stream"); return GB_ERR_CUDA; }
-    e = cudaFuncSetAttribute(k_str_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, STR_LINE_BYTES);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_str_solve_mixed, cudaFuncAttributeMaxDynamicSharedMemorySize, STR_LINE_BYTES);
+    e = cl_prepare(k_str_solve, STR_SMEM_BYTES);
+    if (e == cudaSuccess) e = cl_prepare(k_str_solve_mixed, STR_SMEM_BYTES);
     if (e != cudaSuccess) { gb_str_destroy(h); gb_set_error("gb_str_create: shared memory: %s", cudaGetErrorString(e)); return GB_ERR_CUDA; }
+    h->ctas = cl_fit(k_str_solve, CL_MAX_CTAS, STR_THREADS, STR_SMEM_BYTES);
+    e = str_mer_create(h);
+    if (e != cudaSuccess) { gb_set_error("gb_str_create: %s", cudaGetErrorString(e)); gb_str_destroy(h); return GB_ERR_CUDA; }
     *out = h;
     return GB_OK;
+}
+
+// CTAs per solve.  The reference's line order is one chain of lines, so one
+// CTA; otherwise the whole cluster.
+static int str_ctas(const gb_str *h, int mode)
+{
+    if (mode == GB_SMOOTHER_LEX) return 1;
+    return h->ctas;
 }
 
 // The solve on device arrays (0:n1, 0:n2) with leading dimension n1 + 1,
@@ -1010,9 +795,20 @@ cudaError_t gb_str_launch_device(const gb_str *h, double *psi, const double *rhs
     d.io_rhs = const_cast<double *>(rhs);
     d.status = status;
     d.abort = abort;
-    if (mixed) k_str_solve_mixed<<<1, STR_THREADS, STR_LINE_BYTES, s>>>(d);
-    else k_str_solve<<<1, STR_THREADS, STR_LINE_BYTES, s>>>(d);
-    return cudaGetLastError();
+    if (mixed && mode == GB_SMOOTHER_ZEBRA && h->mer_ctas) {
+        MerDev m = h->mer;
+        m.tolcon = tolcon;
+        m.maxcycles = maxsweeps;
+        m.nrel = nrel;
+        m.psi = psi;
+        m.rhs = rhs;
+        m.status = status;
+        m.abort = abort;
+        return mer_launch(m, h->mer_ctas, s);
+    }
+    const int ctas = str_ctas(h, mode);
+    if (mixed) return cl_launch(k_str_solve_mixed, 1, ctas, STR_THREADS, STR_SMEM_BYTES, s, d);
+    return cl_launch(k_str_solve, 1, ctas, STR_THREADS, STR_SMEM_BYTES, s, d);
 }
 
 extern "C" int gb_str_poisson(gb_str *h, double *psi, const double *rhs, int ld, int *sweeps)
@@ -1026,8 +822,7 @@ extern "C" int gb_str_poisson(gb_str *h, double *psi, const double *rhs, int ld,
                                   h->stream));
     GB_CUDA_TRY(cudaMemcpy2DAsync(d.io_rhs, row, rhs, sizeof(double) * (size_t)ld, row, n2 + 1, cudaMemcpyHostToDevice,
                                   h->stream));
-    k_str_solve<<<1, STR_THREADS, STR_LINE_BYTES, h->stream>>>(d);
-    GB_CUDA_TRY(cudaGetLastError());
+    GB_CUDA_TRY(cl_launch(k_str_solve, 1, str_ctas(h, d.mode), STR_THREADS, STR_SMEM_BYTES, h->stream, d));
     int st[2] = {0, 0};
     GB_CUDA_TRY(cudaMemcpyAsync(st, d.status, sizeof(st), cudaMemcpyDeviceToHost, h->stream));
     GB_CUDA_TRY(cudaStreamSynchronize(h->stream));
