@@ -34,7 +34,7 @@
 #include "str_internal.cuh"
 #include "warpline.cuh"
 
-#define AXI_THREADS 512
+#define AXI_THREADS 256
 #define AXI_MAXLEV 8
 #define AX(i, j) ((size_t)(i) + (size_t)ld * (size_t)(j))
 
@@ -761,7 +761,7 @@ __device__ __forceinline__ void k_axi_mg_solve_body(const AxiDev &d)
     cl.sync();   // no CTA leaves while another may still read its reduction slot
 }
 
-__global__ void __maxnreg__(128) k_axi_mg_solve(const __grid_constant__ AxiDev d) { k_axi_mg_solve_body(d); }
+__global__ void __maxnreg__(255) k_axi_mg_solve(const __grid_constant__ AxiDev d) { k_axi_mg_solve_body(d); }
 
 // ---------------------------------------------------------------------------
 // Mixed precision: FP64 defect correction around one FP32 V-cycle of the
@@ -832,7 +832,7 @@ __device__ __forceinline__ void k_axi_mg_solve_mixed_body(const AxiDev &d)
 #undef V
 #undef F
 
-__global__ void __maxnreg__(128) k_axi_mg_solve_mixed(const __grid_constant__ AxiDev d) { k_axi_mg_solve_mixed_body(d); }
+__global__ void __maxnreg__(255) k_axi_mg_solve_mixed(const __grid_constant__ AxiDev d) { k_axi_mg_solve_mixed_body(d); }
 
 // FP32 copies of rval and the folded factors: block l - 1 takes level l, its
 // threads the level's lines (thread 0 also the r-line table).
@@ -1554,7 +1554,7 @@ __global__ void k_axi_gang(AxiGangTab g)
 // keep the solve free of spills (a launch bound of 512 threads left it at
 // 40-64 with spills).
 template <bool MIXED>
-__global__ void __maxnreg__(128) k_axi_gang_mg(AxiGangTab g, const int *who)
+__global__ void __maxnreg__(255) k_axi_gang_mg(AxiGangTab g, const int *who)
 {
     const AxiDev &d = g.dev[who[blockIdx.x / cooperative_groups::this_cluster().num_blocks()]];
     if (MIXED) k_axi_mg_solve_mixed_body(d);

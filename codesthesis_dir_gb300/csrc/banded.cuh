@@ -21,7 +21,7 @@
 // Doubles of each factor layout.
 __host__ __device__ inline size_t tdma_fac_len(int n) { return 4 * (size_t)n; }
 __host__ __device__ inline size_t ptdma_fac_len(int n) { return 6 * (size_t)n + 3; }
-__host__ __device__ inline size_t pdma_fac_len(int n) { return 6 * (size_t)n + 2; }
+__host__ __device__ inline size_t pdma_fac_len(int n) { return 6 * (size_t)n + 4; }
 
 // ---------------------------------------------------------------------------
 // Tridiagonal (tdma, velvor2dperiodicrbconv.f:3046-3064), n unknowns.
@@ -133,8 +133,9 @@ __device__ inline void apply_ptdma(const double *fac, int n, double *x, int stri
 // ---------------------------------------------------------------------------
 // Pentadiagonal (pdma, velvor2dperiodicrbconv.f:3118-3164), n >= 3.
 // a: 2nd sub, b: sub, c: diag, d: super, e: 2nd super.
-// Factor layout (6n + 2 doubles): cdiv[n), bk1[n), a[n), dn[n), en[n), cN,
-// 1/cdiv[n), 1/cN.
+// Factor layout (6n + 4 doubles): cdiv[n), bk1[n), a[n), dn[n), en[n), cN,
+// 1/cdiv[n), 1/cN, then as whole numbers the first k with a[k + 2] != 0 (n - 2
+// if none) and the last j < n - 2 with en[j] != 0 (-1 if none).
 // ---------------------------------------------------------------------------
 __device__ inline void factor_pdma(const double *a0, const double *b0, const double *c0,
                                    const double *d0, const double *e0, int n, double *fac,
@@ -168,6 +169,13 @@ __device__ inline void factor_pdma(const double *a0, const double *b0, const dou
     fac[5 * n] = c[n - 1];
     for (int k = 0; k <= n - 2; ++k) fac[5 * n + 1 + k] = 1.0 / cdiv[k];
     fac[6 * n + 1] = 1.0 / c[n - 1];
+    int ka = n - 2, je = -1;
+    for (int k = n - 3; k >= 0; --k)
+        if (aa[k + 2] != 0.0) ka = k;
+    for (int j = 0; j < n - 2; ++j)
+        if (e[j] != 0.0) je = j;
+    fac[6 * n + 2] = (double)ka;
+    fac[6 * n + 3] = (double)je;
 }
 
 // Solve with the right-hand side produced by rhs(j) (0-based row j), writing
@@ -285,96 +293,126 @@ __device__ __forceinline__ void tdma32_smem(const float *fac, int n, float *x, i
 
 // ---------------------------------------------------------------------------
 // Eliminations in place on a staged line, x[k * pitch] and the line's factors
-// both in shared memory.  A line is one thread's dependent chain, so nothing
-// else may sit on it: each block of rows has its factors and right-hand sides
-// loaded into registers while the block before it is eliminated (the compiler
-// cannot move those loads above the stores to x itself).
+// both in shared memory, one thread per line.  What bounds them is the FP64
+// unit of an SM quarter: it takes one warp instruction every 64 cycles however
+// many lanes are active and whether or not it depends on the last one
+// (measured: 1, 2, 3, 4 independent chains 64.7, 128.5, 192.3, 256.3 cycles a
+// step), so a row costs 64 cycles times its FP64 instructions.  Hence:
+//   - products with a's and e's zeros are left out (only the walls' one-sided
+//     rows, or half of a stretched line, have them; r - 0 q is r for every
+//     finite q, the sign of a zero aside);
+//   - quotients without the selection of div_by_rcp (the pivots of these
+//     diagonally dominant lines are negative);
+//   - factors and right-hand sides of the next rows are loaded into registers
+//     while a row is eliminated (the compiler cannot move those loads above
+//     the stores to x).
+// A row of the layer's pentadiagonal lines: 902 cycles with all products and
+// selections, 470 now (7 FP64 instructions).
 // ---------------------------------------------------------------------------
 
-// Pentadiagonal in FP64, factor_pdma's layout: apply_pdma_rhs's operations in
-// its order.
-template <int U = 2> __device__ __forceinline__ void pdma_staged(const double *fac, int n, double *x, int pitch)
+// Rows k0 .. k1 - 1 of the pentadiagonal forward elimination; A: with the
+// products by a.  (rk, rk1) are the current and the next row's right-hand
+// sides.
+template <int U, bool A>
+__device__ __forceinline__ void pdma_down(const double *fac, int n, double *x, int pitch, int k0, int k1, double &rk, double &rk1)
 {
-    const double *cdiv = fac, *bk1 = fac + n, *aa = fac + 2 * n, *dn = fac + 3 * n, *en = fac + 4 * n;
-    const double *icdiv = fac + 5 * n + 1;
-    double rk = x[0], rk1 = x[pitch];
+    if (k0 >= k1) return;
+    const double *cdiv = fac, *bk1 = fac + n, *aa = fac + 2 * n, *icdiv = fac + 5 * n + 1;
     double c[U], ic[U], b[U], a[U], r[U];
-    const int reg = n - 2;   // rows with a row two below
-    auto fetch = [&](int k0) {
+    auto fetch = [&](int k2) {
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            const int k = min(k0 + u, reg - 1);
+            const int k = min(k2 + u, k1 - 1);
             c[u] = cdiv[k];
             ic[u] = icdiv[k];
             b[u] = bk1[k];
-            a[u] = aa[k + 2];
+            if (A) a[u] = aa[k + 2];
             r[u] = x[(k + 2) * pitch];
         }
     };
-    if (reg > 0) fetch(0);
-    for (int k0 = 0; k0 < reg; k0 += U) {
+    fetch(k0);
+    for (int k = k0; k < k1; k += U) {
         double c0[U], ic0[U], b0[U], a0[U], r0[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             c0[u] = c[u];
             ic0[u] = ic[u];
             b0[u] = b[u];
-            a0[u] = a[u];
+            if (A) a0[u] = a[u];
             r0[u] = r[u];
         }
-        if (k0 + U < reg) fetch(k0 + U);
+        if (k + U < k1) fetch(k + U);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            if (k0 + u < reg) {
-                const double q = div_by_rcp(rk, c0[u], ic0[u]);
-                x[(k0 + u) * pitch] = q;
+            if (k + u < k1) {
+                const double q = div_by_rcp_neg(rk, c0[u], ic0[u]);
+                x[(k + u) * pitch] = q;
                 rk = rk1 - b0[u] * q;
-                rk1 = r0[u] - a0[u] * q;
+                rk1 = A ? r0[u] - a0[u] * q : r0[u];
             }
         }
     }
-    {   // row n - 2
-        const double q = div_by_rcp(rk, cdiv[n - 2], icdiv[n - 2]);
-        x[(n - 2) * pitch] = q;
-        rk1 = rk1 - bk1[n - 2] * q;
-    }
-    double x1 = div_by_rcp(rk1, fac[5 * n], fac[6 * n + 1]);
-    x[(n - 1) * pitch] = x1;
-    double x0 = x[(n - 2) * pitch] - dn[n - 2] * x1;
-    x[(n - 2) * pitch] = x0;
-    auto fetch_back = [&](int j0) {
+}
+// Rows j0 down to j1 of the back substitution; E: with the products by e.
+// (x0, x1) are the two rows above.
+template <int U, bool E>
+__device__ __forceinline__ void pdma_up(const double *fac, int n, double *x, int pitch, int j0, int j1, double &x0, double &x1)
+{
+    if (j0 < j1) return;
+    const double *dn = fac + 3 * n, *en = fac + 4 * n;
+    double d[U], e[U], r[U];
+    auto fetch = [&](int j2) {
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            const int j = max(j0 - u, 0);
-            c[u] = dn[j];
-            b[u] = en[j];
+            const int j = max(j2 - u, j1);
+            d[u] = dn[j];
+            if (E) e[u] = en[j];
             r[u] = x[j * pitch];
         }
     };
-    if (n >= 3) fetch_back(n - 3);
-    for (int j0 = n - 3; j0 >= 0; j0 -= U) {
+    fetch(j0);
+    for (int j = j0; j >= j1; j -= U) {
         double d0[U], e0[U], r0[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            d0[u] = c[u];
-            e0[u] = b[u];
+            d0[u] = d[u];
+            if (E) e0[u] = e[u];
             r0[u] = r[u];
         }
-        if (j0 - U >= 0) fetch_back(j0 - U);
+        if (j - U >= j1) fetch(j - U);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            if (j0 - u >= 0) {
-                const double xj = r0[u] - d0[u] * x0 - e0[u] * x1;
-                x[(j0 - u) * pitch] = xj;
+            if (j - u >= j1) {
+                double xj = r0[u] - d0[u] * x0;
+                if (E) xj = xj - e0[u] * x1;
+                x[(j - u) * pitch] = xj;
                 x1 = x0;
                 x0 = xj;
             }
         }
     }
 }
+// Pentadiagonal, factor_pdma's layout: apply_pdma_rhs's operations in its order.
+template <int U = 2> __device__ __forceinline__ void pdma_staged(const double *fac, int n, double *x, int pitch)
+{
+    const int ka = (int)fac[6 * n + 2], je = (int)fac[6 * n + 3];
+    double rk = x[0], rk1 = x[pitch];
+    pdma_down<U, false>(fac, n, x, pitch, 0, ka, rk, rk1);
+    pdma_down<U, true>(fac, n, x, pitch, ka, n - 2, rk, rk1);
+    {   // row n - 2
+        const double q = div_by_rcp_neg(rk, fac[n - 2], fac[5 * n + 1 + n - 2]);
+        x[(n - 2) * pitch] = q;
+        rk1 = rk1 - fac[n + n - 2] * q;
+    }
+    double x1 = div_by_rcp_neg(rk1, fac[5 * n], fac[6 * n + 1]);
+    x[(n - 1) * pitch] = x1;
+    double x0 = x[(n - 2) * pitch] - fac[3 * n + n - 2] * x1;
+    x[(n - 2) * pitch] = x0;
+    pdma_up<U, false>(fac, n, x, pitch, n - 3, je + 1, x0, x1);
+    pdma_up<U, true>(fac, n, x, pitch, min(je, n - 3), 0, x0, x1);
+}
 
-// Tridiagonal in FP64, factor_tdma's layout: apply_tdma_rhs's operations in
-// its order.
+// Tridiagonal, factor_tdma's layout: apply_tdma_rhs's operations in its order.
 template <int U = 2> __device__ __forceinline__ void tdma_staged(const double *fac, int n, double *x, int pitch)
 {
     const double *fact = fac, *bp = fac + n, *cc = fac + 2 * n, *ibp = fac + 3 * n;
@@ -405,7 +443,7 @@ template <int U = 2> __device__ __forceinline__ void tdma_staged(const double *f
             }
         }
     }
-    double y = div_by_rcp(prev, bp[n - 1], ibp[n - 1]);
+    double y = div_by_rcp_neg(prev, bp[n - 1], ibp[n - 1]);
     x[(n - 1) * pitch] = y;
     auto fetch_back = [&](int j0) {
 #pragma unroll
@@ -431,7 +469,7 @@ template <int U = 2> __device__ __forceinline__ void tdma_staged(const double *f
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             if (j0 - u >= 0) {
-                y = div_by_rcp(r0[u] - f0[u] * y, b0[u], ib0[u]);
+                y = div_by_rcp_neg(r0[u] - f0[u] * y, b0[u], ib0[u]);
                 x[(j0 - u) * pitch] = y;
             }
         }

@@ -1273,8 +1273,11 @@ __global__ void k_prb_gang(GangTab g)
 
 struct gb_prb_gang {
     int n = 0, mixed = 0;
-    int spread = 1;                // CTAs per equation of the batched multigrid (1 or a cluster)
-    size_t mg_smem = 0;            // shared memory of the mixed solves: the largest member's
+    int spread = 1;                // the batched multigrid's equations on one CTA (1) or a cluster each
+    std::vector<MgEq> eqs;         // the members' equations, those in the reference's line order last
+    int nzebra = 0;                // the others
+    int nres = 0, ctas = 1, smem = 0;   // resident ones (first), CTAs per cluster, shared memory
+    int most = 1;                  // the largest cluster the device holds
     PrbDev *d_dev = nullptr;
     int *d_off = nullptr, *d_limit = nullptr;
     GangRec *d_rec = nullptr;
@@ -1286,6 +1289,8 @@ struct gb_prb_gang {
     cudaGraphExec_t graph = nullptr;
     long long launches_per_step = 0;
 };
+
+static cudaError_t prb_gang_plan(gb_prb_gang *g, gb_prb *const *members);
 
 extern "C" int gb_prb_gang_destroy(gb_prb_gang *g)
 {
@@ -1327,14 +1332,13 @@ extern "C" int gb_prb_gang_create(gb_prb *const *members, const int *nsteps_tota
     std::vector<int> off((size_t)GP_COUNT * (n + 1));
     std::vector<PrbDev> devs(n);
     std::vector<GangRec> rec(n);
-    std::vector<MgEq> eqs(2 * (size_t)n);
+    std::vector<MgEq> lex;
     g->blocks.assign(GP_COUNT, 0);
     for (int q = 0; q < n; ++q) {
         gb_prb *h = members[q];
         prb_refresh_scalars(h);
         const PrbDev &d = h->dev;
         devs[q] = d;
-        g->mg_smem = std::max(g->mg_smem, prb_mg_smem(h));
         const size_t nr = d.nr, np = d.np;
         const int nb[GP_COUNT] = {(int)gb_ceil_div(np + 1, 64), (int)gb_ceil_div(nr - 1, 64),
                                   (int)gb_ceil_div((nr - 1) * (np + 1), TPB), (int)gb_ceil_div((nr - 1) * (np + 1), TPB),
@@ -1361,9 +1365,11 @@ extern "C" int gb_prb_gang_create(gb_prb *const *members, const int *nsteps_tota
             E.maxsweeps = h->p.maxsweeps;
             E.tolcon = h->p.tolcon;
             E.sor = h->p.sor;
-            eqs[2 * (size_t)q + e] = E;
+            (E.mode == GB_SMOOTHER_LEX ? lex : g->eqs).push_back(E);
         }
     }
+    g->nzebra = (int)g->eqs.size();
+    g->eqs.insert(g->eqs.end(), lex.begin(), lex.end());
     for (int ph = 0; ph < GP_COUNT; ++ph) off[(size_t)ph * (n + 1) + n] = g->blocks[ph];
 #define GTRY(x)                                                                   \
     do {                                                                          \
@@ -1378,12 +1384,12 @@ extern "C" int gb_prb_gang_create(gb_prb *const *members, const int *nsteps_tota
     GTRY(cudaMalloc(&g->d_off, sizeof(int) * off.size()));
     GTRY(cudaMalloc(&g->d_limit, sizeof(int) * n));
     GTRY(cudaMalloc(&g->d_rec, sizeof(GangRec) * n));
-    GTRY(cudaMalloc(&g->d_eqs, sizeof(MgEq) * eqs.size()));
+    GTRY(cudaMalloc(&g->d_eqs, sizeof(MgEq) * g->eqs.size()));
     GTRY(cudaMemcpy(g->d_dev, devs.data(), sizeof(PrbDev) * n, cudaMemcpyHostToDevice));
     GTRY(cudaMemcpy(g->d_off, off.data(), sizeof(int) * off.size(), cudaMemcpyHostToDevice));
     GTRY(cudaMemcpy(g->d_limit, nsteps_total, sizeof(int) * n, cudaMemcpyHostToDevice));
     GTRY(cudaMemcpy(g->d_rec, rec.data(), sizeof(GangRec) * n, cudaMemcpyHostToDevice));
-    GTRY(cudaMemcpy(g->d_eqs, eqs.data(), sizeof(MgEq) * eqs.size(), cudaMemcpyHostToDevice));
+    GTRY(prb_gang_plan(g, members));
     // the members' own queued work (their first steps) finishes before the gang's
     for (int q = 0; q < n; ++q) GTRY(cudaStreamSynchronize(members[q]->stream));
     GTRY(cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking));
@@ -1408,11 +1414,42 @@ static void prb_gang_enqueue_step(gb_prb_gang *g, cudaStream_t s)
     GL(GP_TROB);
     GL(GP_HEAT);
     GL(GP_RHS);
-    prb_mg_launch_eqs(g->d_eqs, 2 * g->n, g->mixed, g->spread, g->mg_smem, s);
+    prb_mg_launch_eqs(g->d_eqs, 0, g->nres, g->mixed, g->ctas, g->smem, s);
+    prb_mg_launch_eqs(g->d_eqs, g->nres, g->nzebra - g->nres, g->mixed, g->ctas, 0, s);
+    prb_mg_launch_eqs(g->d_eqs, g->nzebra, 2 * g->n - g->nzebra, g->mixed, 1, 0, s);
     GL(GP_UPD);
     GL(GP_REC);
 #undef GL
-    g->launches_per_step = GP_COUNT + 1;
+    g->launches_per_step = GP_COUNT + (g->nres > 0) + (g->nzebra > g->nres) + (2 * g->n > g->nzebra);
+}
+
+// Plans the gang's solves.  A cluster takes as many CTAs as leave every
+// equation its own SMs (a CTA fills one), at least what keeps every member
+// that fits a cluster's shared memory there: a gang step waits for its
+// slowest solve.  The results do not depend on it.
+static cudaError_t prb_gang_plan(gb_prb_gang *g, gb_prb *const *members)
+{
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
+    if (members) g->most = members[0]->mg_ctas;
+    MgEq *e = g->eqs.data();
+    auto resident = [](const MgEq &q) { return q.smem > 0; };
+    if (g->spread == 1) {
+        g->ctas = 1;
+        prb_mg_plan(e, g->nzebra, g->mixed, 1);
+    } else {
+        prb_mg_plan(e, g->nzebra, g->mixed, g->most);
+        const long can = std::count_if(e, e + g->nzebra, resident);
+        for (g->ctas = 1; 2 * g->ctas <= g->most && 2 * g->ctas * g->nzebra <= sms;) g->ctas *= 2;
+        for (;; g->ctas *= 2) {
+            prb_mg_plan(e, g->nzebra, g->mixed, g->ctas);
+            if (std::count_if(e, e + g->nzebra, resident) == can || 2 * g->ctas > g->most) break;
+        }
+    }
+    g->nres = (int)(std::stable_partition(e, e + g->nzebra, resident) - e);
+    g->smem = 0;
+    for (int q = 0; q < g->nres; ++q) g->smem = std::max(g->smem, e[q].smem);
+    return cudaMemcpy(g->d_eqs, e, sizeof(MgEq) * g->eqs.size(), cudaMemcpyHostToDevice);
 }
 
 // Queues nsteps leapfrog steps (not the first step of a run) of every
@@ -1440,7 +1477,9 @@ extern "C" int gb_prb_gang_set_solve_spread(gb_prb_gang *g, int ctas)
         return GB_ERR_INVALID;
     }
     if (g->spread != ctas) {
+        GB_CUDA_TRY(cudaStreamSynchronize(g->stream));   // queued steps use the present plan
         g->spread = ctas;
+        GB_CUDA_TRY(prb_gang_plan(g, nullptr));
         if (g->graph) { cudaGraphExecDestroy(g->graph); g->graph = nullptr; }
     }
     return GB_OK;

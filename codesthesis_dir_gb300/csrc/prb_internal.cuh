@@ -8,6 +8,7 @@
 #include "gbcommon.cuh"
 
 #define PRB_MAXLEV 7
+#define MG_MAX_NR 1638   // longest r-line of a solve
 
 // One multigrid level of one equation (COMMON /step/, /ints/ of
 // velvor2dperiodicrbconv.f:1810-1814, plus the packed v/f slots).
@@ -23,6 +24,10 @@ struct MgLevel {
     float *v32, *f32;    // packed correction / right-hand side
     float *fac32;        // factors with the pivots stored as reciprocals
     float *rvi32, *rvq32;
+    // the resident solve's plan (prb_resident.cu): lines per CTA, row pitch,
+    // byte offsets of v, f, the line factors, 1/r and 1/r^2, and the addresses
+    // of the lines
+    int rp, pitch, o_v, o_f, o_fac, o_rv, o_rows;
 };
 
 // Device description of one Poisson solve (poisson2 or poisson3).
@@ -34,7 +39,6 @@ struct MgEq {
     int seam_keep;       // the annulus's corser keeps the coarse seam residual
     int xwall;           // the tank: side walls in x (velvor2dhorconvtank.f:1032-1303)
     int stop_on_max;     // the sweep limit fails the step (PRB's STOP) or only is reported
-    int smem_fac;        // mixed solve: floats of shared memory before its line buffer (>= the level-1 factors)
     double r0;
     double tolcon, sor;
     MgLevel lev[PRB_MAXLEV];
@@ -45,6 +49,7 @@ struct MgEq {
     int *status;         // [0] status, [1] sweeps
     double *resmax;      // last level-1 residual max norm
     int *abort;          // set on failure: later kernels of a step skip their work
+    int o_rc, o_psip, smem;   // the resident solve's residual, previous iterate and total (bytes; 0: it does not fit)
 };
 
 struct PrbDev {
@@ -102,16 +107,24 @@ struct gb_prb {
     double *diag_buf = nullptr;   // 4 running means + kt + CFL history (hist_cap slots)
     int diag_cap = 0;
     int steps_done = 0;
-    int mg_spread = 1;            // CTAs per zebra solve (gb_prb_set_solve_spread): 1 or 8
+    int mg_ctas = 1;              // the largest cluster the device holds for a solve
+    int mg_spread = 0;            // CTAs per zebra solve a caller asked for (gb_prb_set_solve_spread): 1 or 8; 0: mg_ctas
 };
 
 int prb_mg_levels(int nr, int variant);
 int prb_mg_create(gb_prb *h);
 void prb_mg_destroy(gb_prb *h);
 int prb_launch_mg(gb_prb *h, int do_v, int do_u, cudaStream_t s);
-void prb_mg_launch_eqs(const MgEq *d_eqs, int neq, int mixed, int spread, size_t smem, cudaStream_t s);
-size_t prb_mg_smem(const gb_prb *h);
+bool prb_mg_plan(MgEq *eqs, int n, int mixed, int ctas);
+void prb_mg_launch_eqs(const MgEq *d_eqs, int first, int neq, int mixed, int ctas, int smem, cudaStream_t s);
 int prb_mg_cluster_ctas();
+// The solve in a cluster's shared memory (prb_resident.cu): plans E for
+// clusters of ctas CTAs (E.smem = 0 when it does not fit), prepares the
+// kernels, launches neq of them.
+void prb_resident_plan(MgEq &E, int mixed, int ctas);
+cudaError_t prb_resident_prepare();
+int prb_resident_fit(int mixed, int ctas, int smem);
+void prb_resident_launch(const MgEq *d_eqs, int first, int neq, int mixed, int ctas, int smem, cudaStream_t s);
 int prb_refresh_scalars(gb_prb *h);
 // the tank's transport (tank.cu)
 int tank_launch_cvorticity(gb_prb *h, int first, cudaStream_t s);

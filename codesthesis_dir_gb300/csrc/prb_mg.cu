@@ -1,16 +1,18 @@
 // Velocity-component multigrid solves of the 2D periodic Rayleigh-Benard
 // driver (poisson2/poisson3, relax2/relax3, corser, finer of
-// velvor2dperiodicrbconv.f:1724-2859) as one persistent thread block per
-// equation: the whole outer sweep loop, every level and every convergence
-// test run inside one launch, so a solve costs one kernel launch however many
-// sweeps it takes.  The v and u solves of a step are the two blocks of one
-// launch (the reference runs them as two OpenMP sections, PRB:370-380).
+// velvor2dperiodicrbconv.f:1724-2859): one launch per solve, one CTA or one
+// cluster of CTAs (cluster.cuh) per equation.  The whole outer sweep loop,
+// every level and every convergence test run inside it, so a solve costs one
+// kernel launch however many sweeps it takes.  The v and u solves of a step
+// are two clusters of one launch (the reference runs them as two OpenMP
+// sections, PRB:370-380).
 //
 // Two smoother orderings:
-//   LEX   - lines k = 1..n3 in order, the reference schedule; one thread
-//           marches the lines (the ordering is sequential by definition).
-//   ZEBRA - odd lines, then even lines; every line of a colour is solved by
-//           its own thread.
+//   LEX   - lines k = 1..n3 in order, the reference schedule: each line needs
+//           the one before it, so one CTA (its threads form a line's
+//           right-hand side together, one carries the elimination).
+//   ZEBRA - odd lines, then even lines, the lines of a colour shared out over
+//           the cluster.
 // Either way each line is solved with the reference's banded elimination in
 // the reference's operation order (-fmad=false), so LEX results are
 // bit-identical to the reference algorithm and ZEBRA results to the same
@@ -28,443 +30,331 @@
 // relaxation and seam reset.
 //
 // Storage differs from the reference only in scratch that no output depends
-// on: the right-hand sides are read from the packed per-level arrays instead
-// of being unpacked into rf, and the prolongation reads the coarse solution
-// straight from its packed slot (the reference stages both through psic/rf/
-// tempa).  Every value the solution depends on is formed by the same
-// arithmetic on the same operands.
+// on: each level keeps its solution in place (level 1 in psif, the coarser
+// ones in their packed slots; the reference copies the level at hand through
+// psif), the right-hand sides are read from the packed per-level arrays, and
+// residuals are formed where something reads them.  Every value the solution
+// depends on is formed by the same arithmetic on the same operands.
 #include <stdint.h>
 #include <string.h>
 
-#include <cooperative_groups.h>
+#include <algorithm>
 
 #include "banded.cuh"
+#include "cluster.cuh"
 #include "gbcommon.cuh"
+#include "mg_op.cuh"
 #include "prb_internal.cuh"
+#include "warpline.cuh"
 
-namespace cg = cooperative_groups;
+// FP64: the eliminations want registers.  FP32 on global memory serves the
+// large grids, whose passes want threads (272 x 1200 annulus, a step: 24.2 ms
+// with 256, 20.7 with 512).
+#define MG_THREADS 256
+#define MG_THREADS_MIXED 512
+#define MG_SPREAD 8    // the cluster size a caller may ask for (gb_prb_set_solve_spread)
 
-#define MG_THREADS 512
-#define MG_CLUSTER 8   // CTAs sharing one FP64 zebra solve (gb_prb_step's single-instance path)
-
-__device__ __forceinline__ double blk_max(double v, double *s_red)
-{
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, o));
-    if (lane == 0) s_red[warp] = v;
-    __syncthreads();
-    if (warp == 0) {
-        v = (lane < nw) ? s_red[lane] : 0.0;
-        for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, o));
-        if (lane == 0) s_red[32] = v;
-    }
-    __syncthreads();
-    const double r = s_red[32];
-    __syncthreads();
-    return r;
-}
-
-// The threads that share one equation's solve: one CTA (MgBlock), or the
-// CTAs of a thread-block cluster (MgCluster), which meet at the hardware
-// cluster barrier (arrive with release, wait with acquire at cluster scope:
-// what any CTA of the cluster wrote to global memory before it is seen by
-// every CTA after it) and reduce through distributed shared memory.  A
-// cluster spreads a solve's lines over several SMs' FP64 units; the work of
-// each line is unchanged, so both give the same bits.
-struct MgBlock {
-    static constexpr int C = 1;
-    __device__ static int tid() { return threadIdx.x; }
-    __device__ static int nthr() { return blockDim.x; }
-    __device__ static void sync() { __syncthreads(); }
+// One level of one equation: its solution in place (level 1: psif, else the
+// packed slot), pitch ld.
+template <class T> struct MgView {
+    int which, n1, n3, ld, polar, xwall;
+    T *v;
+    const T *f;
+    T hhri, hhpi, hri;
+    const T *rvi, *rvq, *fac;
+    // unknowns of a line and the last line (the tank's v lines stop short of
+    // its wall k = n3, velvor2dhorconvtank.f:1170, :1216)
+    __device__ __forceinline__ int rows() const { return which == 2 ? n1 : n1 - 1; }
+    __device__ __forceinline__ int lines() const { return xwall && which == 2 ? n3 - 1 : n3; }
+    // the line after k: periodic, or the tank's last u line's zero k = 0 as
+    // its wall (velvor2dhorconvtank.f:1275)
+    __device__ __forceinline__ int after(int k) const { return k == n3 ? (xwall ? 0 : 1) : k + 1; }
 };
-template <int CS> struct MgCluster {
-    static constexpr int C = CS;
-    __device__ static int tid() { return (int)cg::this_cluster().block_rank() * blockDim.x + threadIdx.x; }
-    __device__ static int nthr() { return CS * blockDim.x; }
-    __device__ static void sync() { cg::this_cluster().sync(); }
-};
-
-// Maximum (NaNs ignored, as blk_max) and logical or over the group.
-template <class G> __device__ __forceinline__ double grp_max(double v, double *s_red)
+__device__ __forceinline__ MgView<double> mg_view(const MgEq &E, int l, double)
 {
-    v = blk_max(v, s_red);
-    if constexpr (G::C > 1) {
-        __shared__ double s_pub;
-        if (threadIdx.x == 0) s_pub = v;
-        G::sync();
-        cg::cluster_group cl = cg::this_cluster();
-        double m = 0.0;
-        for (int r = 0; r < G::C; ++r) m = fmax(m, *cl.map_shared_rank(&s_pub, r));
-        G::sync();   // every CTA has read every slot before the next reduction writes it
-        v = m;
-    }
-    return v;
+    const MgLevel &L = E.lev[l];
+    return {E.which, L.n1, L.n3, l == 1 ? E.ld : L.n1 + 1, E.polar, E.xwall, l == 1 ? E.psif : L.v, L.f, L.hhri, L.hhpi, L.hri,
+            L.rvi, L.rvq, L.fac};
 }
-template <class G> __device__ __forceinline__ int grp_or(int x)
+__device__ __forceinline__ MgView<float> mg_view(const MgEq &E, int l, float)
 {
-    x = __syncthreads_or(x);
-    if constexpr (G::C > 1) {
-        __shared__ int s_or;
-        if (threadIdx.x == 0) s_or = x;
-        G::sync();
-        cg::cluster_group cl = cg::this_cluster();
-        int o = 0;
-        for (int r = 0; r < G::C; ++r) o |= *cl.map_shared_rank(&s_or, r);
-        G::sync();
-        x = o;
-    }
-    return x;
+    const MgLevel &L = E.lev[l];
+    return {E.which, L.n1, L.n3, l == 1 ? E.ld : L.n1 + 1, E.polar, E.xwall, l == 1 ? E.psif32 : L.v32, L.f32, (float)L.hhri,
+            (float)L.hhpi, (float)L.hri, L.rvi32, L.rvq32, L.fac32};
 }
 
-// The level operator applied at (i, k) (the part of relax2/relax3's
-// residual before it is subtracted from f): PRB:2306-2357 (v),
-// PRB:2553-2587 (u), and the annulus forms of velvor2dnewsch3.4.f:2300-2346
-// and :2546-2579.  Instantiated for double (bit-identical to the reference)
-// and for float (the mixed-precision correction cycle).
-template <class T>
-__device__ __forceinline__ T mg_apply_op(const T *psif, int ld, int i, int k, int ka, int km, int which, int polar,
-                                         int n1, T hhri, T hhpi, T hri, const T *rvi, const T *rvq)
-{
-    const T two = T(2.0), c53 = T(5.0 / 3.0), c02 = T(0.2), c15 = T(1.5), c43 = T(4.0 / 3.0);
-    T temp;
-    if (polar && which == 2) {
-        temp = (psif[GIX(i, ka, ld)] - two * psif[GIX(i, k, ld)] + psif[GIX(i, km, ld)]) * hhpi * rvq[i] +
-               psif[GIX(i, k, ld)] * rvq[i];
-        if (i == 1)
-            temp = temp + (-two * psif[GIX(i, k, ld)] + c53 * psif[GIX(i + 1, k, ld)] -
-                           c02 * psif[GIX(i + 2, k, ld)]) * hhri +
-                   c43 * psif[GIX(i + 1, k, ld)] * hri * rvi[i];
-        else if (i == n1)
-            temp = temp + (-two * psif[GIX(i, k, ld)] + c53 * psif[GIX(i - 1, k, ld)] -
-                           c02 * psif[GIX(i - 2, k, ld)]) * hhri -
-                   c43 * psif[GIX(i - 1, k, ld)] * hri * rvi[i];
-        else
-            temp = temp + (psif[GIX(i - 1, k, ld)] - two * psif[GIX(i, k, ld)] + psif[GIX(i + 1, k, ld)]) * hhri +
-                   c15 * (psif[GIX(i + 1, k, ld)] - psif[GIX(i - 1, k, ld)]) * hri * rvi[i];
-    } else if (polar) {
-        temp = (psif[GIX(i + 1, k, ld)] + psif[GIX(i - 1, k, ld)]) * hhri +
-               c15 * (psif[GIX(i + 1, k, ld)] - psif[GIX(i - 1, k, ld)]) * hri * rvi[i] +
-               psif[GIX(i, k, ld)] * rvq[i] +
-               (psif[GIX(i, ka, ld)] + psif[GIX(i, km, ld)]) * hhpi * rvq[i] -
-               psif[GIX(i, k, ld)] * (two * hhri + two * hhpi * rvq[i]);
-    } else if (which == 2) {
-        temp = (psif[GIX(i, ka, ld)] - two * psif[GIX(i, k, ld)] + psif[GIX(i, km, ld)]) * hhpi;
-        if (i == 1)
-            temp = temp + (-two * psif[GIX(i, k, ld)] + c53 * psif[GIX(i + 1, k, ld)] -
-                           c02 * psif[GIX(i + 2, k, ld)]) * hhri;
-        else if (i == n1)
-            temp = temp + (-two * psif[GIX(i, k, ld)] + c53 * psif[GIX(i - 1, k, ld)] -
-                           c02 * psif[GIX(i - 2, k, ld)]) * hhri;
-        else
-            temp = temp + (psif[GIX(i - 1, k, ld)] - two * psif[GIX(i, k, ld)] + psif[GIX(i + 1, k, ld)]) * hhri;
-    } else {
-        temp = (psif[GIX(i + 1, k, ld)] + psif[GIX(i - 1, k, ld)]) * hhri +
-               (psif[GIX(i, ka, ld)] + psif[GIX(i, km, ld)]) * hhpi -
-               psif[GIX(i, k, ld)] * (two * hhri + two * hhpi);
-    }
-    return temp;
-}
+// Dynamic shared memory of a solve: the level's line factors and the staged
+// lines' right-hand sides.
+#define MG_SMEM_BYTES (160 * 1024)
 
-// One line k of relax2 (pentadiagonal, rows i = 1..n1, PRB:2113-2191) or
-// relax3 (tridiagonal, rows i = 1..n1-1, PRB:2414-2460).
-__device__ __forceinline__ void mg_line(const MgEq &E, const MgLevel &L, int k)
+// The nl lines first, first + step, ... (relax2 PRB:2113-2191 pentadiagonal,
+// relax3 PRB:2414-2460 tridiagonal), which read none of one another: a
+// colour, or one line of the reference's order.  Each CTA takes a contiguous
+// share, in batches that fit its shared memory: all threads form the
+// right-hand sides, the lines are eliminated (FP64: one thread per line in the
+// reference's order; FP32: up to 32 lanes per line), the solutions go back.
+template <class T> __device__ __noinline__ void mg_lines(const MgEq &E, int l, int first, int step, int nl)
 {
-    const int ld = E.ld, n1 = L.n1, n3 = L.n3;
-    double *psif = E.psif;
-    const double *f = L.f;
-    const double hhpi = L.hhpi;
-    // the tank's last u line takes the zero k = 0 as its wall (velvor2dhorconvtank.f:1275)
-    const int ka = (k == n3) ? (E.xwall ? 0 : 1) : k + 1, km = k - 1;
-    const bool polar = E.polar;
-    const double *rvq = L.rvq;
-    auto rhs = [&](int j) -> double {
-        const int i = j + 1;
-        double t = -(psif[GIX(i, ka, ld)] + psif[GIX(i, km, ld)]) * hhpi;
-        if (polar) t = t * rvq[i];
-        return t + f[(size_t)k * (n1 + 1) + i];
-    };
-    const int nrow = (E.which == 2) ? n1 : n1 - 1;
-    if (E.which == 2) apply_pdma_rhs(L.fac, n1, psif + GIX(1, k, ld), 1, rhs);
-    else apply_tdma_rhs(L.fac, n1 - 1, psif + GIX(1, k, ld), 1, rhs);
-    if (k == n3)
-        for (int i = 1; i <= nrow; ++i) psif[GIX(i, 0, ld)] = E.xwall ? 0.0 : psif[GIX(i, k, ld)];
-}
-
-// Shared memory of the FP64 solves: the line buffer of the staged colour
-// sweeps (96 KB).
-#define MG64_LINE_DOUBLES 12288
-#define MG64_SMEM_BYTES (MG64_LINE_DOUBLES * 8)
-
-// One colour (lines k = 2t + 2 - parity, up to klast) of the zebra sweep, in
-// batches of lines staged in shared memory: the right-hand sides of mg_line
-// go in as [row][line] with an odd pitch (coalesced along rows), one thread
-// per line eliminates in place with the level's factors, the solutions go
-// back (with mg_line's seam copy).  The lines of a colour read only lines of
-// the other colour, so the values are mg_line's.  On a cluster the batches
-// go round the CTAs.
-template <class G>
-__device__ void mg_colour_smem(const MgEq &E, const MgLevel &L, int parity, int klast)
-{
-    extern __shared__ double s_mg64[];
-    const int ld = E.ld, n1 = L.n1, n3 = L.n3;
-    const int nrow = (E.which == 2) ? n1 : n1 - 1;
-    double *psif = E.psif;
-    const double *f = L.f, *rvq = L.rvq;
-    const double hhpi = L.hhpi;
-    const bool polar = E.polar;
-    const int nlines = n3 / 2;
-    int B = MG64_LINE_DOUBLES / nrow - 1;
-    if (B > nlines) B = nlines;
-    int rank = 0;
-    if constexpr (G::C > 1) rank = (int)cg::this_cluster().block_rank();
-    for (int b0 = rank * B; b0 < nlines; b0 += G::C * B) {
-        const int nb = (nlines - b0 < B) ? nlines - b0 : B;
-        const int pitch = nb | 1;
-        for (int j = threadIdx.x >> 5; j < nb; j += blockDim.x >> 5) {
-            const int k = 2 * (b0 + j) + 2 - parity;
-            if (k > klast) continue;
-            const int ka = (k == n3) ? (E.xwall ? 0 : 1) : k + 1, km = k - 1;
-            for (int i = 1 + (threadIdx.x & 31); i <= nrow; i += 32) {
-                double t = -(psif[GIX(i, ka, ld)] + psif[GIX(i, km, ld)]) * hhpi;
-                if (polar) t = t * rvq[i];
-                s_mg64[(i - 1) * pitch + j] = t + f[(size_t)k * (n1 + 1) + i];
+    extern __shared__ __align__(16) unsigned char s_mg[];
+    constexpr bool F64 = sizeof(T) == 8;
+    const Cluster cl = Cluster::self();
+    const MgView<T> L = mg_view(E, l, T(0));
+    const int n = L.rows(), ldf = L.n1 + 1;
+    const int flen = (int)(F64 ? (L.which == 2 ? pdma_fac_len(n) : tdma_fac_len(n)) : (L.which == 2 ? pdma32_len(n) : tdma32_len(n)));
+    const int lpitch = F64 ? 0 : wl_pitch(n), lg = F64 ? 0 : wl_log2m(n);
+    const int share = (nl + cl.size - 1) / cl.size;
+    const int t0 = cl.rank * share, t1 = min(nl, t0 + share);
+    const int words = (int)(MG_SMEM_BYTES / sizeof(T)) - ((flen + 3) & ~3);
+    int B = F64 ? words / n - 1 : words / lpitch;
+    const bool staged = B >= 1;   // the factors and a line fit (rows up to 2900 in FP64)
+    if (!staged) B = 1;
+    B = min(B, min(share, (int)blockDim.x));
+    T *sfac = (T *)s_mg, *x = staged ? sfac + ((flen + 3) & ~3) : sfac;
+    const RowSplit split(n);
+    if (staged && t0 < t1) async_copy(sfac, L.fac, flen, threadIdx.x, blockDim.x);
+    for (int b0 = t0; b0 < t1; b0 += B) {
+        const int nb = min(B, t1 - b0), pitch = nb | 1;
+        // FP64: [row][line], odd pitch; FP32: [line][row], padded per lane
+        auto at = [&](int t, int q) -> T & { return F64 ? x[q * pitch + t] : x[t * lpitch + wl_slot(lg, q)]; };
+        for (int idx = threadIdx.x; idx < nb * n; idx += blockDim.x) {
+            int t, q;
+            split(idx, t, q);
+            const int k = first + step * (b0 + t), i = q + 1;
+            T r = -(L.v[i + L.ld * L.after(k)] + L.v[i + L.ld * (k - 1)]) * L.hhpi;
+            if (L.polar) r = r * L.rvq[i];
+            at(t, q) = r + L.f[i + ldf * k];
+        }
+        if constexpr (!F64) {   // rows past the line's end
+            const int pad = wl_rows(n) - n;
+            for (int idx = threadIdx.x; idx < nb * pad; idx += blockDim.x) at(idx / pad, n + idx % pad) = T(0);
+        }
+        async_copy_wait();
+        __syncthreads();
+        if constexpr (F64) {
+            if ((int)threadIdx.x < nb) {
+                T *y = x + threadIdx.x;
+                if (!staged) {
+                    if (L.which == 2) pdma_staged(L.fac, n, y, pitch);
+                    else tdma_staged(L.fac, n, y, pitch);
+                } else if (L.which == 2) {
+                    pdma_staged(sfac, n, y, pitch);
+                } else {
+                    tdma_staged(sfac, n, y, pitch);
+                }
             }
-        }
-        __syncthreads();
-        for (int j = threadIdx.x; j < nb; j += blockDim.x) {
-            const int k = 2 * (b0 + j) + 2 - parity;
-            if (k > klast) continue;
-            double *x = s_mg64 + j;
-            auto in = [&](int q) -> double { return x[q * pitch]; };
-            if (E.which == 2) apply_pdma_rhs(L.fac, n1, x, pitch, in);
-            else apply_tdma_rhs(L.fac, n1 - 1, x, pitch, in);
-        }
-        __syncthreads();
-        for (int j = threadIdx.x >> 5; j < nb; j += blockDim.x >> 5) {
-            const int k = 2 * (b0 + j) + 2 - parity;
-            if (k > klast) continue;
-            for (int i = 1 + (threadIdx.x & 31); i <= nrow; i += 32) {
-                const double v = s_mg64[(i - 1) * pitch + j];
-                psif[GIX(i, k, ld)] = v;
-                if (k == n3) psif[GIX(i, 0, ld)] = E.xwall ? 0.0 : v;
-            }
-        }
-        __syncthreads();
-    }
-    if constexpr (G::C > 1) G::sync();
-}
-
-// relax2 / relax3: line sweeps (one with nrel = 1; three in the annulus),
-// then the residual into rc, its max norm, and psif packed into v.  Only
-// the last sweep's residual is formed: the reference recomputes rc and
-// resmax after every sweep and keeps the last.  Returns the level's
-// residual max norm (NaNs ignored as in the reference's comparison);
-// *nan_out (uniform over the block) is set when a NaN residual appears.
-template <class G>
-__device__ double mg_relax(const MgEq &E, int klev, double *s_red, int *nan_out)
-{
-    const MgLevel &L = E.lev[klev];
-    const int ld = E.ld, n1 = L.n1, n3 = L.n3;
-    const double hhri = L.hhri, hhpi = L.hhpi, hri = L.hri;
-    const double *rvi = L.rvi, *rvq = L.rvq;
-    double *psif = E.psif, *rc = E.rc;
-    const double *f = L.f;
-    const int nrel = E.nrelax;
-    // the tank's v lines stop short of its wall k = n3 (velvor2dhorconvtank.f:1170, :1216)
-    const int klast = (E.xwall && E.which == 2) ? n3 - 1 : n3;
-    for (int irel = 0; irel < nrel; ++irel) {
-        if (E.mode == GB_SMOOTHER_LEX) {
-            if (G::tid() == 0)
-                for (int k = 1; k <= klast; ++k) mg_line(E, L, k);
-            G::sync();
         } else {
-            for (int parity = 1; parity >= 0; --parity) mg_colour_smem<G>(E, L, parity, klast);
+            const T *tab = staged ? sfac : L.fac;
+            if (L.which == 2) wl_lines<true>(tab, 0, n, x, lpitch, nb);
+            else wl_lines<false>(tab, 0, n, x, lpitch, nb);
+        }
+        __syncthreads();
+        for (int idx = threadIdx.x; idx < nb * n; idx += blockDim.x) {
+            int t, q;
+            split(idx, t, q);
+            const int k = first + step * (b0 + t);
+            const T v = at(t, q);
+            L.v[q + 1 + L.ld * k] = v;
+            if (k == L.n3) L.v[q + 1] = L.xwall ? T(0) : v;   // k = 0 repeats k = n3; the tank's wall is zero
+        }
+        if (b0 + B < t1) __syncthreads();
+    }
+    cl.sync();
+}
+
+// relax2 / relax3's line sweeps (one with nrel = 1; three in the annulus), in
+// place on the level's solution.
+template <class T> __device__ __forceinline__ void mg_sweeps(const MgEq &E, int l)
+{
+    const int n3 = E.lev[l].n3, klast = E.xwall && E.which == 2 ? n3 - 1 : n3;
+    for (int irel = 0; irel < E.nrelax; ++irel) {
+        if (E.mode == GB_SMOOTHER_LEX) {
+            for (int k = 1; k <= klast; ++k) mg_lines<T>(E, l, k, 1, 1);
+        } else {
+            mg_lines<T>(E, l, 1, 2, (klast + 1) / 2);
+            mg_lines<T>(E, l, 2, 2, klast / 2);
         }
     }
-    // residual, PRB:2306-2357 (v) and PRB:2553-2587 (u)
-    double m = 0.0;
+}
+
+// The residual of level l, PRB:2306-2357 (v) and PRB:2553-2587 (u), into rc
+// (pitch ldr; not followed by a barrier): its largest magnitude (NaNs ignored
+// as in the reference's comparison) and whether one is a NaN over the calling
+// thread's points.
+template <class T, class R> __device__ __noinline__ T mg_residual(const MgEq &E, int l, R *rc, int ldr, int *nan_out)
+{
+    const Cluster cl = Cluster::self();
+    const MgView<T> L = mg_view(E, l, T(0));
+    const int n = L.rows(), ldf = L.n1 + 1, tot = n * L.lines();
+    const RowSplit split(n);
+    T m = T(0);
     int nan = 0;
-    const int nrow = (E.which == 2) ? n1 : n1 - 1;
-    const int tot = nrow * klast;
-    for (int idx = G::tid(); idx < tot; idx += G::nthr()) {
-        const int k = idx / nrow + 1, i = idx - (k - 1) * nrow + 1;
-        const int ka = (k == n3) ? (E.xwall ? 0 : 1) : k + 1, km = k - 1;
-        double temp = mg_apply_op<double>(psif, ld, i, k, ka, km, E.which, E.polar, n1, hhri, hhpi, hri, rvi, rvq);
-        temp = f[(size_t)k * (n1 + 1) + i] - temp;
-        rc[GIX(i, k, ld)] = temp;
-        temp = fabs(temp);
-        if (temp != temp) nan = 1;
-        if (temp > m) m = temp;
+    for (int idx = cl.tid(); idx < tot; idx += cl.nthr()) {
+        int k, i;
+        split(idx, k, i);
+        ++i;
+        ++k;
+        const T *row = L.v + L.ld * k;
+        T r = mg_apply_op<T>([&](int q) { return row[q]; }, L.v[i + L.ld * L.after(k)], L.v[i + L.ld * (k - 1)], i, L.which, L.polar,
+                             L.n1, L.hhri, L.hhpi, L.hri, L.rvi, L.rvq);
+        r = L.f[i + ldf * k] - r;
+        rc[i + ldr * k] = (R)r;
+        r = fabs(r);
+        if (r != r) nan = 1;
+        if (r > m) m = r;
     }
-    *nan_out = grp_or<G>(nan);
-    m = grp_max<G>(m, s_red);
-    // trans1(psif -> v)
-    const int tp = (n1 + 1) * (n3 + 1);
-    for (int idx = G::tid(); idx < tp; idx += G::nthr()) {
-        const int k = idx / (n1 + 1), i = idx - k * (n1 + 1);
-        L.v[idx] = psif[GIX(i, k, ld)];
-    }
-    G::sync();
+    *nan_out = nan;
     return m;
 }
 
-// corser (PRB:2603-2718): full weighting of rc onto the packed coarse
-// right-hand side; psif zeroed over the coarse region.
-template <class G>
-__device__ void mg_corser(const MgEq &E, int klev)
+// corser (PRB:2603-2718): full weighting of rc (pitch E.ld on every level:
+// row k = 0 is never written and stays zero) onto the coarse right-hand side;
+// the coarse solution is cleared.  The annulus keeps the residual stored at
+// the seam lines k = 0 and n3c of the coarse level.
+template <class T> __device__ __noinline__ void mg_corser(const MgEq &E, int l)
 {
-    const int ld = E.ld;
-    const int n1c = E.lev[klev + 1].n1, n3c = E.lev[klev + 1].n3;
-    const double *rf = E.rc;
-    double *psif = E.psif, *fc = E.lev[klev + 1].f;
+    const Cluster cl = Cluster::self();
+    const MgView<T> L = mg_view(E, l + 1, T(0));
+    const int ld = E.ld, n1c = L.n1, n3c = L.n3, seam = E.seam_keep;
+    const T *rf = sizeof(T) == 8 ? (const T *)E.rc : (const T *)E.rc32;
+    T *fc = const_cast<T *>(L.f);
     const int tot = (n1c + 1) * (n3c + 1);
-    for (int idx = G::tid(); idx < tot; idx += G::nthr()) {
-        const int k = idx / (n1c + 1), i = idx - k * (n1c + 1);
-        psif[GIX(i, k, ld)] = 0.0;
-        double t = 0.0;
+    const RowSplit split(n1c + 1);
+    for (int idx = cl.tid(); idx < tot; idx += cl.nthr()) {
+        int k, i;
+        split(idx, k, i);
+        T t = T(0);
         if (i >= 1 && i <= n1c - 1 && k >= 1 && k <= n3c - 1) {
-            const int ii = i + i, kk = k + k;
-            const int iip = ii + 1, iim = ii - 1, kkp = kk + 1, kkm = kk - 1;
-            t = rf[GIX(ii, kk, ld)];
-            t = t + t;
-            t = t + rf[GIX(iip, kk, ld)];
-            t = t + rf[GIX(iim, kk, ld)];
-            t = t + rf[GIX(ii, kk, ld)];
-            t = t + rf[GIX(ii, kk, ld)];
-            t = t + rf[GIX(ii, kkp, ld)];
-            t = t + rf[GIX(ii, kkm, ld)];
-            t = t + t;
-            t = t + rf[GIX(iip, kk, ld)];
-            t = t + rf[GIX(iip, kk, ld)];
-            t = t + rf[GIX(iim, kk, ld)];
-            t = t + rf[GIX(iim, kk, ld)];
-            t = t + rf[GIX(iip, kkp, ld)];
-            t = t + rf[GIX(iip, kkm, ld)];
-            t = t + rf[GIX(iim, kkp, ld)];
-            t = t + rf[GIX(iim, kkm, ld)];
-            t = t + rf[GIX(ii, kkp, ld)];
-            t = t + rf[GIX(ii, kkm, ld)];
-            t = t + rf[GIX(ii, kkp, ld)];
-            t = t + rf[GIX(ii, kkm, ld)];
-            t = t + t;
-            t = t + rf[GIX(iip, kkp, ld)];
-            t = t + rf[GIX(iip, kkm, ld)];
-            t = t + rf[GIX(iip, kkp, ld)];
-            t = t + rf[GIX(iip, kkm, ld)];
-            t = t + rf[GIX(iim, kkp, ld)];
-            t = t + rf[GIX(iim, kkm, ld)];
-            t = t + rf[GIX(iim, kkp, ld)];
-            t = t + rf[GIX(iim, kkm, ld)];
-            t = t * 0.015625;
-        } else if (E.seam_keep && i >= 1 && i <= n1c - 1) {
-            t = rf[GIX(i, k, ld)];   // seam lines k = 0, n3c keep rc (k = 0 is never written)
+            const T *q = rf + (i + i) + ld * (k + k);
+            const T c0 = q[0], ip = q[1], im = q[-1], kp = q[ld], km = q[-ld];
+            const T pp = q[1 + ld], pm = q[1 - ld], mp = q[-1 + ld], mm = q[-1 - ld];
+            t = mg_full_weight(c0, ip, im, kp, km, pp, pm, mp, mm);
+        } else if (seam && i >= 1 && i <= n1c - 1) {
+            t = rf[i + ld * k];
         }
         fc[idx] = t;
+        L.v[idx] = T(0);
     }
-    G::sync();
+    cl.sync();
 }
 
-// finer (PRB:2721-2803): bilinear prolongation of the coarse correction plus
-// the saved fine solution.
-template <class G>
-__device__ void mg_finer(const MgEq &E, int klev)
+// finer (PRB:2721-2803): bilinear prolongation of the coarse correction added
+// to the fine solution.
+template <class T> __device__ __noinline__ void mg_finer(const MgEq &E, int l)
 {
-    const int ld = E.ld;
-    const int n1c = E.lev[klev].n1;
-    const int n1f = E.lev[klev - 1].n1, n3f = E.lev[klev - 1].n3;
-    const double *vc = E.lev[klev].v, *vf = E.lev[klev - 1].v;
-    double *psif = E.psif;
-    const int tot = (n1f + 1) * (n3f + 1);
-#define PC(ii, kk) vc[(size_t)(kk) * (n1c + 1) + (ii)]
-    for (int idx = G::tid(); idx < tot; idx += G::nthr()) {
-        const int k = idx / (n1f + 1), i = idx - k * (n1f + 1);
-        const int i1 = i / 2, k1 = k / 2;
-        double p;
-        if (i1 * 2 == i) {
-            if (k1 * 2 == k) p = PC(i1, k1);
-            else p = (PC(i1, k1) + PC(i1, k1 + 1)) * 0.5;
-        } else {
-            if (k1 * 2 == k) p = (PC(i1, k1) + PC(i1 + 1, k1)) * 0.5;
-            else p = (PC(i1, k1) + PC(i1 + 1, k1) + PC(i1, k1 + 1) + PC(i1 + 1, k1 + 1)) * 0.25;
-        }
-        psif[GIX(i, k, ld)] = p + vf[idx];
+    const Cluster cl = Cluster::self();
+    const MgView<T> Cc = mg_view(E, l, T(0)), L = mg_view(E, l - 1, T(0));
+    const int tot = (L.n1 + 1) * (L.n3 + 1);
+    const RowSplit split(L.n1 + 1);
+    for (int idx = cl.tid(); idx < tot; idx += cl.nthr()) {
+        int k, i;
+        split(idx, k, i);
+        const T *q = Cc.v + (i >> 1) + Cc.ld * (k >> 1);
+        const bool io = i & 1, ko = k & 1;
+        const T p = mg_prolong(io, ko, q[0], io ? q[1] : T(0), ko ? q[Cc.ld] : T(0), io && ko ? q[1 + Cc.ld] : T(0));
+        T *v = L.v + i + L.ld * k;
+        *v = p + *v;
     }
-#undef PC
-    G::sync();
+    cl.sync();
+}
+
+// The FMG-flavoured down and up legs of PRB:1869-1893.  relax(l, restricted):
+// a relaxation on level l, with the residual when a restriction follows;
+// level 1 always ends a leg or the cycle and needs it.
+template <class T, class Relax> __device__ __forceinline__ void mg_legs(const MgEq &E, Relax relax)
+{
+    const int nlev = E.nlev;
+    if (nlev < 2) return;
+    for (int l = 1; l <= nlev - 1; ++l) {
+        mg_corser<T>(E, l);
+        relax(l + 1, l + 1 < nlev);
+    }
+    for (int ifmg = 0; ifmg <= nlev - 2; ++ifmg) {
+        for (int l = nlev; l >= nlev - ifmg; --l) {
+            mg_finer<T>(E, l);
+            relax(l - 1, l == nlev - ifmg);
+        }
+        for (int l = nlev - ifmg - 1; l <= nlev - 1; ++l) {
+            mg_corser<T>(E, l);
+            relax(l + 1, l + 1 < nlev);
+        }
+    }
+    for (int l = nlev; l >= 2; --l) {
+        mg_finer<T>(E, l);
+        relax(l - 1, false);
+    }
+}
+
+// The equation's descriptor in shared memory: behind a global pointer every
+// field would come from L2 again after each cluster barrier.
+__device__ __forceinline__ void mg_descriptor(MgEq &dst, const MgEq &src)
+{
+    for (int q = threadIdx.x; q < (int)(sizeof(MgEq) / 4); q += blockDim.x) ((unsigned *)&dst)[q] = ((const unsigned *)&src)[q];
+    __syncthreads();
 }
 
 // poisson2 / poisson3 (PRB:1796-1927 / PRB:1930-2059).
-template <class G>
-__device__ __forceinline__ void mg_solve(const MgEq *eqs, int first_eq)
+// This form, on global memory, serves the reference's line order and the
+// grids whose levels do not fit a cluster's shared memory (prb_resident.cu).
+__global__ void __maxnreg__(255) k_mg_solve(const MgEq *eqs, int first_eq)
 {
-    __shared__ double s_red[33];
-    int nan1 = 0, nan_c = 0;
-    const MgEq &E = eqs[first_eq + blockIdx.x / G::C];
-    if (*E.abort == GB_RUN_DONE) return;   // a gang member past its last step (uniform over the block)
+    __shared__ ClMaxState s_max;
+    __shared__ MgEq E;
+    const Cluster cl = Cluster::self();
+    mg_descriptor(E, eqs[first_eq + blockIdx.x / cl.size]);
+    if (*E.abort == GB_RUN_DONE) return;   // a gang member past its last step (the same for every CTA)
+    int turn = 0;
     const int ld = E.ld, np = E.np, nlev = E.nlev;
     const int imax = (E.which == 2) ? E.nr + 1 : E.nr;
     const int n1 = E.lev[1].n1;
     double *psif = E.psif, *psi = E.psi, *psip = E.psip;
     const int rows = imax + 1, tot = rows * (np + 1);
-    // initial guess 2 psi - psip; level-1 right-hand side and solution packed
-    for (int idx = G::tid(); idx < tot; idx += G::nthr()) {
-        const int k = idx / rows, i = idx - k * rows;
-        const size_t c = GIX(i, k, ld);
-        const double pf = 2.0 * psi[c] - psip[c];
-        psif[c] = pf;
-        if (i <= n1) {
-            E.lev[1].f[(size_t)k * (n1 + 1) + i] = E.rhs[c];
-            E.lev[1].v[(size_t)k * (n1 + 1) + i] = pf;
-        }
+    const RowSplit split(rows);
+    // initial guess 2 psi - psip; level-1 right-hand side packed
+    for (int idx = cl.tid(); idx < tot; idx += cl.nthr()) {
+        int k, i;
+        split(idx, k, i);
+        const int c = i + ld * k;
+        psif[c] = 2.0 * psi[c] - psip[c];
+        if (i <= n1) E.lev[1].f[(size_t)k * (n1 + 1) + i] = E.rhs[c];
     }
-    G::sync();
-    int status = GB_MAXSWEEPS, sweeps = 0;
+    cl.sync();
+    int status = GB_MAXSWEEPS, sweeps = 0, nan1 = 0;
     double res1 = 0.0;
+    auto relax = [&](int l, bool restricted) {
+        mg_sweeps<double>(E, l);
+        if (l != 1 && !restricted) return;
+        int nan;
+        const double m = mg_residual<double>(E, l, E.rc, ld, &nan);
+        if (l == 1) {
+            res1 = cl_max(cl, s_max, turn, m, nan);
+            nan1 = nan;
+        } else {
+            cl.sync();
+        }
+    };
     for (int sweep = 1; sweep <= E.maxsweeps; ++sweep) {
         sweeps = sweep;
         if (sweep != 1) {
-            for (int idx = G::tid(); idx < tot; idx += G::nthr()) {
-                const int k = idx / rows, i = idx - k * rows;
-                const size_t c = GIX(i, k, ld);
+            for (int idx = cl.tid(); idx < tot; idx += cl.nthr()) {
+                int k, i;
+                split(idx, k, i);
+                const int c = i + ld * k;
                 const double pf = psip[c] + E.sor * (psif[c] - psip[c]);
                 psif[c] = pf;
                 psip[c] = pf;
-                if (i <= n1) E.lev[1].v[(size_t)k * (n1 + 1) + i] = pf;
             }
-            G::sync();
+            cl.sync();
         }
         if (sweep == 1 || nlev == 1) {
-            res1 = mg_relax<G>(E, 1, s_red, &nan1);
-            for (int idx = G::tid(); idx < tot; idx += G::nthr()) {
-                const int k = idx / rows, i = idx - k * rows;
-                psip[GIX(i, k, ld)] = psif[GIX(i, k, ld)];
+            relax(1, true);
+            for (int idx = cl.tid(); idx < tot; idx += cl.nthr()) {
+                int k, i;
+                split(idx, k, i);
+                psip[i + ld * k] = psif[i + ld * k];
             }
-            G::sync();
+            cl.sync();
         }
-        if (nlev > 1) {
-            for (int l = 1; l <= nlev - 1; ++l) {
-                mg_corser<G>(E, l);
-                mg_relax<G>(E, l + 1, s_red, &nan_c);
-            }
-            for (int ifmg = 0; ifmg <= nlev - 2; ++ifmg) {
-                for (int l = nlev; l >= nlev - ifmg; --l) {
-                    mg_finer<G>(E, l);
-                    int nn = 0;
-                    double r = mg_relax<G>(E, l - 1, s_red, &nn);
-                    if (l - 1 == 1) { res1 = r; nan1 = nn; }
-                }
-                for (int l = nlev - ifmg - 1; l <= nlev - 1; ++l) {
-                    mg_corser<G>(E, l);
-                    mg_relax<G>(E, l + 1, s_red, &nan_c);
-                }
-            }
-            for (int l = nlev; l >= 2; --l) {
-                mg_finer<G>(E, l);
-                int nn = 0;
-                double r = mg_relax<G>(E, l - 1, s_red, &nn);
-                if (l - 1 == 1) { res1 = r; nan1 = nn; }
-            }
-        }
+        mg_legs<double>(E, relax);
         // The last relax of a sweep is on level 1; its NaN flag decides.
         if (nan1) {
             status = GB_NAN;
@@ -474,434 +364,122 @@ __device__ __forceinline__ void mg_solve(const MgEq *eqs, int first_eq)
             // the tank: v on k = 1..np-1, u on k = 1..np, zero side walls
             // (velvor2dhorconvtank.f:1032-1043, :1129-1140)
             const int kend = (E.which == 2) ? np - 1 : np;
-            for (int idx = G::tid(); idx < tot; idx += G::nthr()) {
-                const int k = idx / rows, i = idx - k * rows;
-                const size_t c = GIX(i, k, ld);
+            for (int idx = cl.tid(); idx < tot; idx += cl.nthr()) {
+                int k, i;
+                split(idx, k, i);
+                const int c = i + ld * k;
                 psip[c] = psi[c];
                 if (i == 0 || i == imax || (E.xwall && (k == 0 || k > kend))) psi[c] = 0.0;
                 else psi[c] = psif[c];
             }
             if (E.xwall && E.which == 3)
-                for (int i = G::tid(); i <= imax; i += G::nthr()) psi[GIX(i, np + 1, ld)] = 0.0;
+                for (int i = cl.tid(); i <= imax; i += cl.nthr()) psi[GIX(i, np + 1, ld)] = 0.0;
             status = GB_OK;
             break;
         }
     }
-    if (G::tid() == 0) {
+    if (cl.tid() == 0) {
         E.status[0] = status;
         E.status[1] = sweeps;
         *E.resmax = res1;
         if (status == GB_NAN || (status == GB_MAXSWEEPS && E.stop_on_max)) *E.abort = 1;
     }
-}
-
-// Launched with MG_THREADS (512) threads per block.  With a launch bound of
-// 512 threads ptxas held the solve to 64 registers and spilled 604 / 1456
-// bytes; allowing 128 (a whole SM's register file per block) removes every
-// spill, and the bound that matters, the SM's FP64 pipe, is the same with
-// one block per SM as with two.
-__global__ void __maxnreg__(128) k_mg_solve(const MgEq *eqs, int first_eq)
-{
-    mg_solve<MgBlock>(eqs, first_eq);
-}
-
-// The same solve with each equation on a cluster of MG_CLUSTER CTAs
-// (launch MG_CLUSTER blocks of MG_THREADS per equation).
-__global__ void __cluster_dims__(MG_CLUSTER, 1, 1) __maxnreg__(128) k_mg_solve_cluster(const MgEq *eqs, int first_eq)
-{
-    mg_solve<MgCluster<MG_CLUSTER>>(eqs, first_eq);
+    cl.sync();   // no CTA leaves while another may still read its reduction slot
 }
 
 // ---------------------------------------------------------------------------
 // Mixed precision (GB_PRB_MIXED): FP64 defect correction around the
 // reference's sweep schedule run in FP32 on the correction equation A e = r.
 // A dependent FP32 operation costs a few cycles where an FP64 one costs tens
-// (and an FP64 division hundreds) on this part, and the line eliminations
-// are dependent chains, so the inner cycle runs an order of magnitude faster.
-// The FP32 line solves multiply by stored reciprocal pivots.
+// (and an FP64 division hundreds) on this part, and the line eliminations are
+// linear recurrences that FP32 may split over a warp's lanes (warpline.cuh).
+// psif holds the FP64 iterate.
 // ---------------------------------------------------------------------------
-template <class Rhs>
-__device__ __forceinline__ void apply_pdma32(const float *fac, int n, float *x, Rhs rhs)
+__global__ void __maxnreg__(128) k_mg_solve_mixed(const MgEq *eqs, int first_eq)
 {
-    const float *icdiv = fac, *bk1 = fac + n, *aa = fac + 2 * n, *dn = fac + 3 * n, *en = fac + 4 * n;
-    const float icN = fac[5 * n];
-    float rk = rhs(0), rk1 = rhs(1);
-#pragma unroll 4
-    for (int k = 0; k <= n - 2; ++k) {
-        rk = rk * icdiv[k];
-        x[k] = rk;
-        rk1 = rk1 - bk1[k] * rk;
-        float rk2 = 0.f;
-        if (k != n - 2) rk2 = rhs(k + 2) - aa[k + 2] * rk;
-        rk = rk1;
-        rk1 = rk2;
-    }
-    float x1 = rk * icN;
-    x[n - 1] = x1;
-    float x0 = x[n - 2] - dn[n - 2] * x1;
-    x[n - 2] = x0;
-#pragma unroll 4
-    for (int j = n - 3; j >= 0; --j) {
-        const float xj = x[j] - dn[j] * x0 - en[j] * x1;
-        x[j] = xj;
-        x1 = x0;
-        x0 = xj;
-    }
-}
-
-template <class Rhs>
-__device__ __forceinline__ void apply_tdma32(const float *fac, int n, float *x, Rhs rhs)
-{
-    const float *fact = fac, *ibp = fac + n, *c = fac + 2 * n;
-    float prev = rhs(0);
-    x[0] = prev;
-#pragma unroll 4
-    for (int j = 1; j < n; ++j) {
-        const float rj = rhs(j) - fact[j] * prev;
-        x[j] = rj;
-        prev = rj;
-    }
-    float y = prev * ibp[n - 1];
-    x[n - 1] = y;
-#pragma unroll 4
-    for (int j = n - 2; j >= 0; --j) {
-        y = (x[j] - c[j] * y) * ibp[j];
-        x[j] = y;
-    }
-}
-
-__device__ __forceinline__ void mg_line32(const MgEq &E, const MgLevel &L, int k)
-{
-    const int ld = E.ld, n1 = L.n1, n3 = L.n3;
-    float *psif = E.psif32;
-    const float *f = L.f32, *rvq = L.rvq32;
-    const float hhpi = (float)L.hhpi;
-    const int ka = (k == n3) ? 1 : k + 1, km = k - 1;
-    const int polar = E.polar;
-    auto rhs = [&](int j) -> float {
-        const int i = j + 1;
-        float t = -(psif[GIX(i, ka, ld)] + psif[GIX(i, km, ld)]) * hhpi;
-        if (polar) t = t * rvq[i];
-        return t + f[(size_t)k * (n1 + 1) + i];
-    };
-    const int nrow = (E.which == 2) ? n1 : n1 - 1;
-    if (E.which == 2) apply_pdma32(L.fac32, n1, psif + GIX(1, k, ld), rhs);
-    else apply_tdma32(L.fac32, n1 - 1, psif + GIX(1, k, ld), rhs);
-    if (k == n3)
-        for (int i = 1; i <= nrow; ++i) psif[GIX(i, 0, ld)] = psif[GIX(i, k, ld)];
-}
-
-// Shared memory of the mixed-precision kernel: the level's FP32 factors,
-// then a buffer of lines stored [row][line] with an odd pitch, so that
-// lanes walking rows (staging) and threads walking their own line
-// (elimination) both hit distinct banks.
-#define MG32_FAC_FLOATS 8192                  // >= 5 n1 + 1 for n1 <= 1600
-#define MG32_LINE_FLOATS 24576                // 96 KB of lines
-#define MG32_SMEM_BYTES ((MG32_FAC_FLOATS + MG32_LINE_FLOATS) * 4)
-
-// One colour (lines k = 2t + 2 - parity) of the zebra line sweep of the
-// correction cycle, in batches of lines staged in shared memory: right-hand
-// sides in (coalesced along rows), one thread per line eliminates, solutions
-// out.
-template <class G>
-__device__ void mg_colour32_smem(const MgEq &E, const MgLevel &L, int parity)
-{
-    extern __shared__ float s_mg32[];
-    float *sfac = s_mg32, *sline = s_mg32 + E.smem_fac;
-    const int ld = E.ld, n1 = L.n1, n3 = L.n3;
-    const int nrow = (E.which == 2) ? n1 : n1 - 1;
-    const int nfac = (E.which == 2) ? 5 * n1 + 1 : 3 * (n1 - 1);
-    for (int j = threadIdx.x; j < nfac; j += blockDim.x) sfac[j] = L.fac32[j];
-    float *psif = E.psif32;
-    const float *f = L.f32, *rvq = L.rvq32;
-    const float hhpi = (float)L.hhpi;
-    const int nlines = n3 / 2;
-    int B = MG32_LINE_FLOATS / nrow - 1;
-    if (B > nlines) B = nlines;
-    // batches of lines in turn over the group's CTAs; within a batch only
-    // this CTA's threads meet
-    int rank = 0;
-    if constexpr (G::C > 1) rank = (int)cg::this_cluster().block_rank();
-    for (int b0 = rank * B; b0 < nlines; b0 += G::C * B) {
-        const int nb = (nlines - b0 < B) ? nlines - b0 : B;
-        const int pitch = nb | 1;
-        for (int j = threadIdx.x >> 5; j < nb; j += blockDim.x >> 5) {
-            const int k = 2 * (b0 + j) + 2 - parity;
-            const int ka = (k == n3) ? 1 : k + 1, km = k - 1;
-            for (int i = 1 + (threadIdx.x & 31); i <= nrow; i += 32) {
-                float r = -(psif[GIX(i, ka, ld)] + psif[GIX(i, km, ld)]) * hhpi;
-                if (E.polar) r = r * rvq[i];
-                sline[(i - 1) * pitch + j] = r + f[(size_t)k * (n1 + 1) + i];
-            }
-        }
-        __syncthreads();
-        for (int j = threadIdx.x; j < nb; j += blockDim.x) {
-            if (E.which == 2) pdma32_smem(sfac, n1, sline + j, pitch);
-            else tdma32_smem(sfac, n1 - 1, sline + j, pitch);
-        }
-        __syncthreads();
-        for (int j = threadIdx.x >> 5; j < nb; j += blockDim.x >> 5) {
-            const int k = 2 * (b0 + j) + 2 - parity;
-            for (int i = 1 + (threadIdx.x & 31); i <= nrow; i += 32) {
-                const float v = sline[(i - 1) * pitch + j];
-                psif[GIX(i, k, ld)] = v;
-                if (k == n3) psif[GIX(i, 0, ld)] = v;
-            }
-        }
-        __syncthreads();
-    }
-    if constexpr (G::C > 1) G::sync();
-}
-
-// relax2/relax3 of the correction cycle: line sweeps, residual into rc32,
-// psif32 packed into v32.
-template <class G>
-__device__ void mg_relax32(const MgEq &E, int klev)
-{
-    const MgLevel &L = E.lev[klev];
-    const int ld = E.ld, n1 = L.n1, n3 = L.n3;
-    const float hhri = (float)L.hhri, hhpi = (float)L.hhpi, hri = (float)L.hri;
-    float *psif = E.psif32, *rc = E.rc32;
-    const int nrel = E.nrelax;
-    for (int irel = 0; irel < nrel; ++irel) {
-        if (E.mode == GB_SMOOTHER_LEX) {
-            if (G::tid() == 0)
-                for (int k = 1; k <= n3; ++k) mg_line32(E, L, k);
-            G::sync();
-        } else {
-            for (int parity = 1; parity >= 0; --parity) mg_colour32_smem<G>(E, L, parity);
-        }
-    }
-    const int nrow = (E.which == 2) ? n1 : n1 - 1;
-    const int tot = nrow * n3;
-    for (int k = 1 + (G::tid() >> 5); k <= n3; k += (G::nthr() >> 5))
-        for (int i = 1 + (threadIdx.x & 31); i <= nrow; i += 32) {
-        const int ka = (k == n3) ? 1 : k + 1, km = k - 1;
-        const float a = mg_apply_op<float>(psif, ld, i, k, ka, km, E.which, E.polar, n1, hhri, hhpi, hri, L.rvi32,
-                                           L.rvq32);
-        rc[GIX(i, k, ld)] = L.f32[(size_t)k * (n1 + 1) + i] - a;
-    }
-    G::sync();
-    const int tp = (n1 + 1) * (n3 + 1);
-    for (int k = (G::tid() >> 5); k < (tp) / ((n1 + 1)); k += (G::nthr() >> 5))
-        for (int i = threadIdx.x & 31; i < (n1 + 1); i += 32) {
-            const int idx = k * (n1 + 1) + i;
-        L.v32[idx] = psif[GIX(i, k, ld)];
-    }
-    G::sync();
-}
-
-template <class G>
-__device__ void mg_corser32(const MgEq &E, int klev)
-{
-    const int ld = E.ld;
-    const int n1c = E.lev[klev + 1].n1, n3c = E.lev[klev + 1].n3;
-    const float *rf = E.rc32;
-    float *psif = E.psif32, *fc = E.lev[klev + 1].f32;
-    const int tot = (n1c + 1) * (n3c + 1);
-    for (int k = (G::tid() >> 5); k < (tot) / ((n1c + 1)); k += (G::nthr() >> 5))
-        for (int i = threadIdx.x & 31; i < (n1c + 1); i += 32) {
-            const int idx = k * (n1c + 1) + i;
-        psif[GIX(i, k, ld)] = 0.f;
-        float t = 0.f;
-        if (i >= 1 && i <= n1c - 1 && k >= 1 && k <= n3c - 1) {
-            const int ii = i + i, kk = k + k;
-            // full weighting: 1/4 centre, 1/8 edges, 1/16 corners
-            t = 0.25f * rf[GIX(ii, kk, ld)] +
-                0.125f * (rf[GIX(ii + 1, kk, ld)] + rf[GIX(ii - 1, kk, ld)] + rf[GIX(ii, kk + 1, ld)] +
-                          rf[GIX(ii, kk - 1, ld)]) +
-                0.0625f * (rf[GIX(ii + 1, kk + 1, ld)] + rf[GIX(ii + 1, kk - 1, ld)] + rf[GIX(ii - 1, kk + 1, ld)] +
-                           rf[GIX(ii - 1, kk - 1, ld)]);
-        } else if (E.seam_keep && i >= 1 && i <= n1c - 1 && k == n3c) {
-            t = rf[GIX(i, k, ld)];
-        }
-        fc[idx] = t;
-    }
-    G::sync();
-}
-
-template <class G>
-__device__ void mg_finer32(const MgEq &E, int klev)
-{
-    const int ld = E.ld;
-    const int n1c = E.lev[klev].n1;
-    const int n1f = E.lev[klev - 1].n1, n3f = E.lev[klev - 1].n3;
-    const float *vc = E.lev[klev].v32, *vf = E.lev[klev - 1].v32;
-    float *psif = E.psif32;
-    const int tot = (n1f + 1) * (n3f + 1);
-#define PC(ii, kk) vc[(size_t)(kk) * (n1c + 1) + (ii)]
-    for (int k = (G::tid() >> 5); k < (tot) / ((n1f + 1)); k += (G::nthr() >> 5))
-        for (int i = threadIdx.x & 31; i < (n1f + 1); i += 32) {
-            const int idx = k * (n1f + 1) + i;
-        const int i1 = i / 2, k1 = k / 2;
-        float p;
-        if (i1 * 2 == i) {
-            if (k1 * 2 == k) p = PC(i1, k1);
-            else p = (PC(i1, k1) + PC(i1, k1 + 1)) * 0.5f;
-        } else {
-            if (k1 * 2 == k) p = (PC(i1, k1) + PC(i1 + 1, k1)) * 0.5f;
-            else p = (PC(i1, k1) + PC(i1 + 1, k1) + PC(i1, k1 + 1) + PC(i1 + 1, k1 + 1)) * 0.25f;
-        }
-        psif[GIX(i, k, ld)] = p + vf[idx];
-    }
-#undef PC
-    G::sync();
-}
-
-// One FP32 cycle of the reference's sweep schedule (relax on the finest
-// level, the FMG-flavoured down and up legs of PRB:1869-1893) on A e = r
-// from e = 0.
-template <class G>
-__device__ void mg_cycle32(const MgEq &E)
-{
-    const int nlev = E.nlev;
-    mg_relax32<G>(E, 1);
-    if (nlev > 1) {
-        for (int l = 1; l <= nlev - 1; ++l) {
-            mg_corser32<G>(E, l);
-            mg_relax32<G>(E, l + 1);
-        }
-        for (int ifmg = 0; ifmg <= nlev - 2; ++ifmg) {
-            for (int l = nlev; l >= nlev - ifmg; --l) {
-                mg_finer32<G>(E, l);
-                mg_relax32<G>(E, l - 1);
-            }
-            for (int l = nlev - ifmg - 1; l <= nlev - 1; ++l) {
-                mg_corser32<G>(E, l);
-                mg_relax32<G>(E, l + 1);
-            }
-        }
-        for (int l = nlev; l >= 2; --l) {
-            mg_finer32<G>(E, l);
-            mg_relax32<G>(E, l - 1);
-        }
-    }
-}
-
-// poisson2 / poisson3 in mixed precision.  psif holds the FP64 iterate.
-template <class G>
-__device__ __forceinline__ void mg_solve_mixed(const MgEq *eqs, int first_eq)
-{
-    __shared__ double s_red[33];
-    const MgEq &E = eqs[first_eq + blockIdx.x / G::C];
-    if (*E.abort == GB_RUN_DONE) return;   // a gang member past its last step (uniform over the block)
-    const MgLevel &L1 = E.lev[1];
+    __shared__ ClMaxState s_max;
+    __shared__ MgEq E;
+    const Cluster cl = Cluster::self();
+    mg_descriptor(E, eqs[first_eq + blockIdx.x / cl.size]);
+    if (*E.abort == GB_RUN_DONE) return;   // a gang member past its last step (the same for every CTA)
+    int turn = 0;
     const int ld = E.ld, np = E.np;
     const int imax = (E.which == 2) ? E.nr + 1 : E.nr;
-    const int n1 = L1.n1, n3 = L1.n3;
+    const int n1 = E.lev[1].n1, n3 = E.lev[1].n3;
     double *psif = E.psif, *psi = E.psi, *psip = E.psip;
     const int rows = imax + 1, tot = rows * (np + 1);
-    for (int k = (G::tid() >> 5); k < (tot) / (rows); k += (G::nthr() >> 5))
-        for (int i = threadIdx.x & 31; i < rows; i += 32) {
-            const int idx = k * rows + i;
-        const size_t c = GIX(i, k, ld);
+    const RowSplit split(rows);
+    for (int idx = cl.tid(); idx < tot; idx += cl.nthr()) {
+        int k, i;
+        split(idx, k, i);
+        const int c = i + ld * k;
         psif[c] = 2.0 * psi[c] - psip[c];
-        if (i <= n1) L1.f[(size_t)k * (n1 + 1) + i] = E.rhs[c];
+        if (i <= n1) E.lev[1].f[(size_t)k * (n1 + 1) + i] = E.rhs[c];
     }
-    G::sync();
+    for (int idx = cl.tid(); idx < ld * (n3 + 1); idx += cl.nthr()) E.psif32[idx] = 0.f;
+    cl.sync();
+    auto relax = [&](int l, bool restricted) {
+        mg_sweeps<float>(E, l);
+        if (!restricted) return;
+        int nan;
+        mg_residual<float>(E, l, E.rc32, ld, &nan);
+        cl.sync();
+    };
     const int nrow = (E.which == 2) ? n1 : n1 - 1;
+    const RowSplit inner(nrow);
     int status = GB_MAXSWEEPS, cycles = 0;
     double res = 0.0;
     for (int it = 0;; ++it) {
         // FP64 residual of the iterate; its FP32 copy is the cycle's right-hand side
-        double m = 0.0;
-        int nan = 0;
-        // packed 1D mapping: partly filled warps cost a full FP64 issue slot
-        for (int idx = G::tid(); idx < nrow * n3; idx += G::nthr()) {
-            const int k = idx / nrow + 1, i = idx - (k - 1) * nrow + 1;
-            const int ka = (k == n3) ? 1 : k + 1, km = k - 1;
-            const double a = mg_apply_op<double>(psif, ld, i, k, ka, km, E.which, E.polar, n1, L1.hhri, L1.hhpi,
-                                                 L1.hri, L1.rvi, L1.rvq);
-            const double r = L1.f[(size_t)k * (n1 + 1) + i] - a;
-            L1.f32[(size_t)k * (n1 + 1) + i] = (float)r;
-            const double ar = fabs(r);
-            if (ar != ar) nan = 1;
-            if (ar > m) m = ar;
-        }
-        nan = grp_or<G>(nan);
-        res = grp_max<G>(m, s_red);
+        int nan;
+        const double m = mg_residual<double>(E, 1, E.lev[1].f32, n1 + 1, &nan);
+        res = cl_max(cl, s_max, turn, m, nan);
         if (nan) { status = GB_NAN; break; }
         if (res < E.tolcon) { status = GB_OK; break; }
         if (it == E.maxsweeps) break;
-        // e = 0 on the finest level, then one FP32 cycle
-        for (int k = (G::tid() >> 5); k < (n3 + 1); k += (G::nthr() >> 5))
-            for (int i = threadIdx.x & 31; i < (n1 + 2); i += 32) {
-                const int idx = k * (n1 + 2) + i;
-            E.psif32[GIX(i, k, ld)] = 0.f;
-        }
-        G::sync();
-        mg_cycle32<G>(E);
+        relax(1, E.nlev > 1);
+        mg_legs<float>(E, relax);
+        // psi += w e, and e = 0 for the next cycle
         const double w = (it == 0) ? 1.0 : E.sor;
-        for (int idx = G::tid(); idx < nrow * (n3 + 1); idx += G::nthr()) {
-            const int k = idx / nrow, i = idx - k * nrow + 1;
-            psif[GIX(i, k, ld)] += w * (double)E.psif32[GIX(i, k, ld)];
+        for (int idx = cl.tid(); idx < nrow * (n3 + 1); idx += cl.nthr()) {
+            int k, i;
+            inner(idx, k, i);
+            const int c = i + 1 + ld * k;
+            psif[c] += w * (double)E.psif32[c];
+            E.psif32[c] = 0.f;
         }
-        G::sync();
+        cl.sync();
         cycles = it + 1;
     }
     if (status == GB_OK) {
-        for (int k = (G::tid() >> 5); k < (tot) / (rows); k += (G::nthr() >> 5))
-            for (int i = threadIdx.x & 31; i < rows; i += 32) {
-                const int idx = k * rows + i;
-            const size_t c = GIX(i, k, ld);
+        for (int idx = cl.tid(); idx < tot; idx += cl.nthr()) {
+            int k, i;
+            split(idx, k, i);
+            const int c = i + ld * k;
             psip[c] = psi[c];
             psi[c] = (i == 0 || i == imax) ? 0.0 : psif[c];
         }
     }
-    if (G::tid() == 0) {
+    if (cl.tid() == 0) {
         E.status[0] = status;
         E.status[1] = cycles;
         *E.resmax = res;
         if (status == GB_NAN || (status == GB_MAXSWEEPS && E.stop_on_max)) *E.abort = 1;
     }
+    cl.sync();
 }
 
-__global__ void __maxnreg__(128) k_mg_solve_mixed(const MgEq *eqs, int first_eq)
-{
-    mg_solve_mixed<MgBlock>(eqs, first_eq);
-}
-
-// The mixed solve with each equation on a cluster of MG_CLUSTER CTAs: the
-// FP64 residual passes, the FP32 residual and transfer passes and the
-// batches of each colour's lines are spread over the cluster's SMs.
-__global__ void __cluster_dims__(MG_CLUSTER, 1, 1) __maxnreg__(128) k_mg_solve_mixed_cluster(const MgEq *eqs,
-                                                                                              int first_eq)
-{
-    mg_solve_mixed<MgCluster<MG_CLUSTER>>(eqs, first_eq);
-}
-
-// FP32 copies of the factors (pivots as reciprocals) and radii.
+// FP32 copies of the radii and the folded factors, a block per level.
 __global__ void k_mg_factors32(MgEq eq)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    for (int l = 1; l <= eq.nlev; ++l) {
-        const MgLevel &L = eq.lev[l];
-        const int n1 = L.n1;
-        float *f32 = L.fac32;
-        const double *f = L.fac;
-        if (eq.which == 2) {
-            const int n = n1;
-            for (int j = 0; j < n; ++j) {
-                f32[j] = (float)(1.0 / f[j]);                     // cdiv
-                f32[n + j] = (float)f[n + j];                     // bk1
-                f32[2 * n + j] = (float)f[2 * n + j];             // a
-                f32[3 * n + j] = (float)f[3 * n + j];             // d
-                f32[4 * n + j] = (float)f[4 * n + j];             // e
-            }
-            f32[5 * n] = (float)(1.0 / f[5 * n]);
-        } else {
-            const int n = n1 - 1;
-            for (int j = 0; j < n; ++j) {
-                f32[j] = (float)f[j];                             // fact
-                f32[n + j] = (float)(1.0 / f[n + j]);             // bp
-                f32[2 * n + j] = (float)f[2 * n + j];             // c
-            }
-        }
-        for (int i = 0; i <= n1 + 1; ++i) {
-            L.rvi32[i] = (float)L.rvi[i];
-            L.rvq32[i] = (float)L.rvq[i];
-        }
+    const MgLevel &L = eq.lev[1 + blockIdx.x];
+    for (int i = threadIdx.x; i <= L.n1 + 1; i += blockDim.x) {
+        L.rvi32[i] = (float)L.rvi[i];
+        L.rvq32[i] = (float)L.rvq[i];
     }
+    if (threadIdx.x != 0) return;
+    if (eq.which == 2) pdma32_fold(L.fac, L.n1, L.fac32);
+    else tdma32_fold(L.fac, L.n1 - 1, L.fac32);
 }
 
 // Factored line matrices of every level (one thread), the coefficients of
@@ -987,8 +565,8 @@ int prb_mg_create(gb_prb *h)
     const int nr = p.nr, np = p.np, nlev = h->nlev;
     const int ld = h->dev.ld;
     const double dr = h->dev.dr, dp = h->dev.dp;
-    if (5 * nr + 1 > MG32_FAC_FLOATS || 2 * nr > MG32_LINE_FLOATS) {
-        gb_set_error("nr=%d exceeds the multigrid kernel's shared-memory line buffers", nr);
+    if (nr > MG_MAX_NR) {
+        gb_set_error("nr=%d exceeds the multigrid kernel's line length", nr);
         return GB_ERR_INVALID;
     }
     if (np % (1 << nlev) != 0) {
@@ -1001,7 +579,7 @@ int prb_mg_create(gb_prb *h)
         const int n1 = nr * 2 / (1 << l), n3 = np * 2 / (1 << l);
         per_eq += 2 * (size_t)(n1 + 1) * (n3 + 1) + pdma_fac_len(n1 + 2) + 2 * (size_t)(n1 + 2);
         // FP32: v32, f32, fac32, rvi32, rvq32 (counted in doubles, rounded up)
-        per_eq += ((2 * (size_t)(n1 + 1) * (n3 + 1) + 5 * (size_t)(n1 + 2) + 1 + 2 * (size_t)(n1 + 2)) + 1) / 2 + 4;
+        per_eq += ((2 * (size_t)(n1 + 1) * (n3 + 1) + pdma32_len(n1) + 2 * (size_t)(n1 + 2)) + 1) / 2 + 8;
     }
     const size_t work = 8 * (size_t)(nr + 2);
     cudaError_t e = cudaMalloc(&h->mg_pool, sizeof(double) * (2 * per_eq + work));
@@ -1020,7 +598,6 @@ int prb_mg_create(gb_prb *h)
         E.xwall = p.variant == GB_PRB_TANK || p.variant == GB_PRB_DVD;
         if (E.xwall && p.precision != GB_PRB_FP64) return GB_ERR_INVALID;
         E.stop_on_max = p.variant != GB_PRB_ANNULUS;
-        E.smem_fac = ((5 * nr + 1 + 31) / 32) * 32;   // the level-1 pentadiagonal factors, rounded to 128 B
         E.r0 = p.r0;
         double *base = h->mg_pool + q * per_eq;
         E.psif = base; base += (size_t)ld * (np + 1);
@@ -1049,7 +626,8 @@ int prb_mg_create(gb_prb *h)
             float *fb = (float *)base;
             L.v32 = fb; fb += sz;
             L.f32 = fb; fb += sz;
-            L.fac32 = fb; fb += 5 * (size_t)(L.n1 + 2) + 1;
+            fb = (float *)(((uintptr_t)fb + 15) & ~(uintptr_t)15);   // copied 16 bytes at a time
+            L.fac32 = fb; fb += pdma32_len(L.n1);                    // >= tdma32_len(n1 - 1)
             L.rvi32 = fb; fb += (size_t)(L.n1 + 2);
             L.rvq32 = fb; fb += (size_t)(L.n1 + 2);
             base = (double *)(((uintptr_t)fb + 15) & ~(uintptr_t)15);
@@ -1061,15 +639,15 @@ int prb_mg_create(gb_prb *h)
         E.resmax = h->dev.mg_resmax + q;
         E.abort = h->dev.abort;
         k_mg_factors<<<1, 1>>>(E, wk);
-        k_mg_factors32<<<1, 1>>>(E);
+        k_mg_factors32<<<nlev, 128>>>(E);
     }
-    e = cudaFuncSetAttribute(k_mg_solve_mixed, cudaFuncAttributeMaxDynamicSharedMemorySize, MG32_SMEM_BYTES);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(k_mg_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, MG64_SMEM_BYTES);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_mg_solve_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, MG64_SMEM_BYTES);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_mg_solve_mixed_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, MG32_SMEM_BYTES);
+    e = cl_prepare(k_mg_solve, MG_SMEM_BYTES);
+    if (e == cudaSuccess) e = cl_prepare(k_mg_solve_mixed, MG_SMEM_BYTES);
     if (e != cudaSuccess) { gb_set_error("multigrid shared memory: %s", cudaGetErrorString(e)); return GB_ERR_CUDA; }
+    h->mg_ctas = cl_fit(k_mg_solve, CL_MAX_CTAS, MG_THREADS, MG_SMEM_BYTES);
+    e = prb_resident_prepare();
+    if (e != cudaSuccess) { gb_set_error("multigrid shared memory: %s", cudaGetErrorString(e)); return GB_ERR_CUDA; }
+    prb_mg_plan(h->eq_host, 2, p.precision == GB_PRB_MIXED, h->mg_ctas);
     e = cudaMalloc(&h->eq_dev, sizeof(MgEq) * 2);
     if (e != cudaSuccess) { gb_set_error("multigrid descriptors: %s", cudaGetErrorString(e)); return GB_ERR_ALLOC; }
     cudaMemcpy(h->eq_dev, h->eq_host, sizeof(MgEq) * 2, cudaMemcpyHostToDevice);
@@ -1084,36 +662,38 @@ void prb_mg_destroy(gb_prb *h)
     h->eq_dev = nullptr;
 }
 
-// Refreshes the solve parameters that a caller may change between calls
-// (tolerance, sweep limit, smoother, SOR factor) and launches the solves.
-// Shared memory of one instance's mixed solve: its factors, then the line
-// buffer.
-size_t prb_mg_smem(const gb_prb *h)
+// Plans n equations for clusters of ctas CTAs: in shared memory
+// (prb_resident.cu) those that fit, E.smem their bytes, else 0.  Returns
+// whether all of them fit.
+bool prb_mg_plan(MgEq *eqs, int n, int mixed, int ctas)
 {
-    return sizeof(float) * ((size_t)h->eq_host[0].smem_fac + MG32_LINE_FLOATS);
+    bool all = true;
+    for (int q = 0; q < n; ++q) {
+        prb_resident_plan(eqs[q], mixed, ctas);
+        if (eqs[q].smem && prb_resident_fit(mixed, ctas, eqs[q].smem) != ctas) eqs[q].smem = 0;
+        all = all && eqs[q].smem;
+    }
+    return all;
 }
 
-// The solves of neq equation descriptors (any instances') in one launch,
-// one block or one cluster of MG_CLUSTER blocks each (the gangs' batched
-// multigrid); smem: the largest member's prb_mg_smem.  A gang step waits
-// for its slowest solve, so the solves keep the single-instance block of
-// MG_THREADS: with half-size blocks, two per SM, the served sweep's mixed
-// arm ran 1.5 instead of 2.25 solves/s.
-void prb_mg_launch_eqs(const MgEq *d_eqs, int neq, int mixed, int spread, size_t smem, cudaStream_t s)
+// The solves of neq equation descriptors (any instances') in one launch, one
+// cluster of ctas CTAs each; smem: the most any of them takes in shared
+// memory, 0: on global memory.
+void prb_mg_launch_eqs(const MgEq *d_eqs, int first, int neq, int mixed, int ctas, int smem, cudaStream_t s)
 {
     if (neq <= 0) return;
-    if (spread > 1) {
-        if (mixed) k_mg_solve_mixed_cluster<<<neq * MG_CLUSTER, MG_THREADS, smem, s>>>(d_eqs, 0);
-        else k_mg_solve_cluster<<<neq * MG_CLUSTER, MG_THREADS, MG64_SMEM_BYTES, s>>>(d_eqs, 0);
-    } else if (mixed) {
-        k_mg_solve_mixed<<<neq, MG_THREADS, smem, s>>>(d_eqs, 0);
-    } else {
-        k_mg_solve<<<neq, MG_THREADS, MG64_SMEM_BYTES, s>>>(d_eqs, 0);
+    if (smem) {
+        prb_resident_launch(d_eqs, first, neq, mixed, ctas, smem, s);
+        return;
     }
+    if (mixed) cl_launch(k_mg_solve_mixed, neq, ctas, MG_THREADS_MIXED, MG_SMEM_BYTES, s, d_eqs, first);
+    else cl_launch(k_mg_solve, neq, ctas, MG_THREADS, MG_SMEM_BYTES, s, d_eqs, first);
 }
 
-int prb_mg_cluster_ctas() { return MG_CLUSTER; }
+int prb_mg_cluster_ctas() { return MG_SPREAD; }
 
+// Refreshes the solve parameters that a caller may change between calls
+// (tolerance, sweep limit, smoother, SOR factor) and launches the solves.
 int prb_launch_mg(gb_prb *h, int do_v, int do_u, cudaStream_t s)
 {
     bool changed = false;
@@ -1128,14 +708,13 @@ int prb_launch_mg(gb_prb *h, int do_v, int do_u, cudaStream_t s)
     const int first = do_v ? 0 : 1;
     const int n = (do_v ? 1 : 0) + (do_u ? 1 : 0);
     if (n == 0) return GB_OK;
-    const bool spread = h->mg_spread > 1 && h->p.smoother == GB_SMOOTHER_ZEBRA;
-    if (h->p.precision == GB_PRB_MIXED) {
-        if (spread) k_mg_solve_mixed_cluster<<<n * MG_CLUSTER, MG_THREADS, prb_mg_smem(h), s>>>(h->eq_dev, first);
-        else k_mg_solve_mixed<<<n, MG_THREADS, prb_mg_smem(h), s>>>(h->eq_dev, first);
-    } else if (spread) {
-        k_mg_solve_cluster<<<n * MG_CLUSTER, MG_THREADS, MG64_SMEM_BYTES, s>>>(h->eq_dev, first);
+    const int mixed = h->p.precision == GB_PRB_MIXED;
+    if (h->p.smoother == GB_SMOOTHER_LEX) {
+        prb_mg_launch_eqs(h->eq_dev, first, n, mixed, 1, 0, s);
     } else {
-        k_mg_solve<<<n, MG_THREADS, MG64_SMEM_BYTES, s>>>(h->eq_dev, first);
+        // v and u in one launch: in shared memory when both fit
+        const int smem = h->eq_host[0].smem && h->eq_host[1].smem ? std::max(h->eq_host[0].smem, h->eq_host[1].smem) : 0;
+        prb_mg_launch_eqs(h->eq_dev, first, n, mixed, h->mg_spread ? std::min(h->mg_spread, h->mg_ctas) : h->mg_ctas, smem, s);
     }
     h->launches += 1;
     return GB_OK;
@@ -1143,12 +722,15 @@ int prb_launch_mg(gb_prb *h, int do_v, int do_u, cudaStream_t s)
 
 extern "C" int gb_prb_set_solve_spread(gb_prb *h, int ctas)
 {
-    if (!h || (ctas != 1 && ctas != MG_CLUSTER)) {
-        gb_set_error("gb_prb_set_solve_spread: ctas must be 1 or %d", MG_CLUSTER);
+    if (!h || (ctas != 1 && ctas != MG_SPREAD)) {
+        gb_set_error("gb_prb_set_solve_spread: ctas must be 1 or %d", MG_SPREAD);
         return GB_ERR_INVALID;
     }
     if (h->mg_spread != ctas) {
+        GB_CUDA_TRY(cudaStreamSynchronize(h->stream));   // queued steps use the present plan
         h->mg_spread = ctas;
+        prb_mg_plan(h->eq_host, 2, h->p.precision == GB_PRB_MIXED, std::min(ctas, h->mg_ctas));
+        GB_CUDA_TRY(cudaMemcpy(h->eq_dev, h->eq_host, sizeof(MgEq) * 2, cudaMemcpyHostToDevice));
         if (h->graph_exec) { cudaGraphExecDestroy(h->graph_exec); h->graph_exec = nullptr; }
         if (h->graph_exec1) { cudaGraphExecDestroy(h->graph_exec1); h->graph_exec1 = nullptr; }
     }

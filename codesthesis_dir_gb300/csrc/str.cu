@@ -28,7 +28,7 @@
 #include <algorithm>
 #include <vector>
 
-#define STR_THREADS 512
+#define STR_THREADS 256
 #define STR_MAXLEV 8
 
 struct StrLevel {
@@ -387,7 +387,7 @@ template <class T> __device__ __noinline__ void str_finer(const StrLevel &coarse
 }
 
 // poisson(psi, rhs, nlev, vel) (rcsc.f:1118-1195) on the staged arrays.
-__global__ void __maxnreg__(128) k_str_solve(const __grid_constant__ StrDev d)
+__global__ void __maxnreg__(255) k_str_solve(const __grid_constant__ StrDev d)
 {
     __shared__ ClMaxState s_max;
     const Cluster cl = Cluster::self();
@@ -454,7 +454,7 @@ __global__ void __maxnreg__(128) k_str_solve(const __grid_constant__ StrDev d)
 // one FP32 V-cycle of the same schedule on L e = r from e = 0 and updates
 // psi += e in FP64 (rcsc.f's solve has no over-relaxation).
 // ---------------------------------------------------------------------------
-__global__ void __maxnreg__(128) k_str_solve_mixed(const __grid_constant__ StrDev d)
+__global__ void __maxnreg__(255) k_str_solve_mixed(const __grid_constant__ StrDev d)
 {
     __shared__ ClMaxState s_max;
     const Cluster cl = Cluster::self();

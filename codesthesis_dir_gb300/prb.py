@@ -127,9 +127,9 @@ class PRB:
         return self._poisson(3)
 
     def set_solve_spread(self, ctas):
-        """CTAs sharing one two-colour solve (FP64 or mixed): 1 (the
-        default, one CTA per equation) or 8 (a cluster).  Both give the same
-        bits."""
+        """CTAs sharing one two-colour solve (FP64 or mixed): 1 (one CTA per
+        equation) or 8 (a cluster); without a call the largest cluster the
+        device holds.  All give the same bits."""
         _L.check(_L.load().gb_prb_set_solve_spread(self._h, ctas), "set_solve_spread")
 
     def update(self):

@@ -208,15 +208,13 @@ int gb_prb_rhsu(gb_prb *h);                         /* PRB:1679-1721 */
  * which = 3: poisson3 on uel/uelp/urh (PRB:1930-2059).
  * Returns GB_OK, GB_MAXSWEEPS or GB_NAN; *sweeps gets the sweep count. */
 int gb_prb_poisson(gb_prb *h, int which, int *sweeps);
-/* CTAs that share one two-colour solve of this instance (FP64 or mixed):
- * 1 (the default: one CTA per equation) or 8 (the lines of a colour, the
- * residuals and the transfers of each level are spread over a cluster of 8
- * CTAs that meet at the hardware cluster barrier and reduce through
- * distributed shared memory).  Both give the same bits; the reference's
- * line order always uses one CTA.  The solve of a line is a dependent
- * chain that a cluster does not shorten: on the 129 x 65 layer the cluster
- * takes 0.95-1.02x the time of one CTA.  No counterpart in the reference
- * (its solves are serial). */
+/* CTAs that share one two-colour solve of this instance (FP64 or mixed): 1
+ * (one CTA per equation) or 8 (the lines of a colour, the residuals and the
+ * transfers of each level are spread over a cluster of 8 CTAs that meet at
+ * the hardware cluster barrier and reduce through distributed shared memory).
+ * Without a call: the largest cluster the device holds (16).  All give the
+ * same bits; the reference's line order always uses one CTA.  No counterpart
+ * in the reference (its solves are serial). */
 int gb_prb_set_solve_spread(gb_prb *h, int ctas);
 /* update (PRB:1557-1626); *clamps (may be NULL) gets the number of
  * temperatures clamped, each of which the reference reports with
@@ -413,9 +411,10 @@ int gb_prb_gang_enqueue(gb_prb_gang *g, int nsteps, void *stream);
 int gb_prb_gang_query(gb_prb_gang *g);
 void *gb_prb_gang_stream(gb_prb_gang *g);
 long long gb_prb_gang_launches_per_step(const gb_prb_gang *g);
-/* CTAs per equation of a PRB gang's batched multigrid: 1 (the default) or
- * 8 (a cluster per equation, as gb_prb_set_solve_spread); the same bits
- * either way.  Takes effect at the next enqueue. */
+/* A PRB gang's batched multigrid: 1 (the default: one CTA per equation) or 8
+ * (a cluster per equation, of as many CTAs as leave every equation its own
+ * SMs, at least what keeps its arrays in shared memory); the same bits either
+ * way.  Takes effect at the next enqueue. */
 int gb_prb_gang_set_solve_spread(gb_prb_gang *g, int ctas);
 int gb_prb_gang_destroy(gb_prb_gang *g);
 typedef struct gb_axi_gang gb_axi_gang;
