@@ -48,12 +48,13 @@ struct Cluster {
     }
 };
 
-// idx / n and idx % n by one high multiplication: magic = 2^32 / n + 1 gives
-// a quotient at most one too large for every 0 <= idx < 2^31.
+// idx / n and idx % n by one high multiplication: magic = (2^32 - 1) / n + 1
+// gives a quotient at most one too large for every 0 <= idx < 2^31 (formed by
+// a 32-bit division; a 64-bit one costs as much as a short phase).
 struct RowSplit {
     int n;
     unsigned magic;
-    __device__ __forceinline__ explicit RowSplit(int n_) : n(n_), magic((unsigned)(0x100000000ull / (unsigned)n_) + 1u)
+    __device__ __forceinline__ explicit RowSplit(int n_) : n(n_), magic(0xffffffffu / (unsigned)n_ + 1u)
     {
         if (n_ == 1) magic = 0;
     }

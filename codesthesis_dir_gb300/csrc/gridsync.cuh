@@ -17,37 +17,52 @@ struct GridSync {
     unsigned long long *tally;   // optional (may be null): barriers passed, counted once per barrier by block 0
 };
 
-// Default wait limit: about 1-2 s of polling at 64 ns per poll.
+// Default wait limit: some seconds of polling at an L2 round trip per poll.
 #define GB_GRID_WAIT_LIMIT_DEFAULT (1LL << 24)
 
-__device__ __forceinline__ bool grid_sync(const GridSync &gs)
+// Arrival and wait of one thread per block.  The arrival count grows from one
+// barrier to the next (gen counts the barriers passed), so that nothing is
+// reset: the last arriver publishes the next generation, and the release and
+// acquire are those of the counter and the generation themselves instead of
+// fences around relaxed accesses.
+__device__ __forceinline__ void grid_barrier(const GridSync &gs)
+{
+    unsigned g, arrived;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(g) : "l"(gs.gen) : "memory");
+    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(arrived) : "l"(gs.count) : "memory");
+    if (arrived + 1u == (g + 1u) * gridDim.x) {
+        asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(gs.gen), "r"(g + 1u) : "memory");
+    } else {
+        unsigned now = g;
+        for (long long it = 0; now == g;) {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(gs.gen) : "memory");
+            if (now != g) break;
+            if (++it > gs.limit || ((it & 15) == 0 && *(volatile int *)gs.err)) {
+                atomicExch(gs.err, 1);
+                break;
+            }
+        }
+    }
+}
+
+// The barrier for the whole grid; false when it gave up.  meanwhile(): what
+// the threads outside the first warp do while its first thread waits (it may
+// touch shared memory and constants only).
+template <class F> __device__ __forceinline__ bool grid_sync(const GridSync &gs, F meanwhile)
 {
     __shared__ int s_grid_ok;
     __syncthreads();
     if (threadIdx.x == 0) {
-        volatile unsigned *vgen = gs.gen;
-        const unsigned g = *vgen;
-        __threadfence();
-        const unsigned arrived = atomicAdd(gs.count, 1u);
-        if (arrived == gridDim.x - 1) {
-            atomicExch(gs.count, 0u);
-            __threadfence();
-            atomicAdd(gs.gen, 1u);
-        } else {
-            long long it = 0;
-            while (*vgen == g) {
-                if (++it > gs.limit || *(volatile int *)gs.err) {
-                    atomicExch(gs.err, 1);
-                    break;
-                }
-                __nanosleep(64);
-            }
-        }
-        __threadfence();
+        grid_barrier(gs);
         s_grid_ok = *(volatile int *)gs.err == 0;
         if (gs.tally && blockIdx.x == 0) atomicAdd(gs.tally, 1ull);
+    } else if (threadIdx.x >= 32) {
+        meanwhile();
     }
     __syncthreads();
     return s_grid_ok != 0;
 }
-
+__device__ __forceinline__ bool grid_sync(const GridSync &gs)
+{
+    return grid_sync(gs, [] {});
+}

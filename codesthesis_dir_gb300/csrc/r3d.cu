@@ -24,8 +24,11 @@
 // a later anti-diagonal), GB_SMOOTHER_ZEBRA the two-colour order with the
 // one-sided boundary rows last.
 #include "gbcommon.cuh"
+#include "banded.cuh"
+#include "cluster.cuh"
+#include "convert.cuh"
 #include "gridsync.cuh"
-#include "divrn.cuh"
+#include "warpline.cuh"
 
 #include <math.h>
 #include <stdlib.h>
@@ -49,15 +52,20 @@ struct R3Work {
 struct R3Lev {
     int n1, n2, n3, L1, L2;
     double hr, hz, hp, hhr, hhz, hhp;
+    double ihr, ihhr, ihhz, ihhp;   // reciprocals (IEEE)
     double *rvc, *rvv;          // r0 + (i - 1/2) hr and i hr + r0, i = 0..n1+1
+    double *dirc, *dirv, *diqc, *diqv;   // 1/r and 1/(r r) of both (IEEE)
     double *fac[4][3];          // [component][direction] factor tables
     int *lines[4][3];           // packed p | q << 16, phase by phase
     int *poff[4][3];            // phase offsets (nphase + 1)
     int nphase[4][3];
     // FP32 inner cycles (GB_PRB_MIXED)
-    float *irc, *irv, *iqc, *iqv;   // 1/r and 1/r^2 at cell centres and faces, i = 0..n1+1
-    float ihr, ihhr, ihhz, ihhp;
-    float *fac32[4][3];         // the factor tables with reciprocal pivots
+    // weights of the FP32 operator, per component: of the rows i (i-1, i+1,
+    // far, diagonal) and (phi neighbours), of the rows j (j-1, j+1, far, diagonal);
+    // far is the one-sided rows' point two over
+    float4 *wi[4], *wj[4];
+    float *wp[4];
+    float *fac32[4][3];         // folded line tables (warpline.cuh); phi-lines: R3Ring per radius
 };
 
 struct R3Dev {
@@ -633,7 +641,11 @@ __host__ __device__ __forceinline__ int r3_len(int comp, int dir, int n1, int n2
 }
 __host__ __device__ __forceinline__ int r3_tabsize(int kind, int n)
 {
-    return kind == 0 ? 6 * n : kind == 1 ? 4 * n : 7 * n;   // the last n: reciprocals of the pivots
+    return kind == 0 ? (int)pdma_fac_len(n) : kind == 1 ? (int)tdma_fac_len(n) : 7 * n;
+}
+__host__ __device__ __forceinline__ int r3_tabsize32(int kind, int n)
+{
+    return kind == 0 ? (int)pdma32_len(n) : kind == 1 ? (int)tdma32_len(n) : 4;
 }
 __host__ __device__ __forceinline__ int r3_imax(int comp, int n1) { return comp == 3 ? n1 - 1 : n1; }
 __host__ __device__ __forceinline__ int r3_jmax(int comp, int n2) { return comp == 1 ? n2 - 1 : n2; }
@@ -782,13 +794,12 @@ struct FacJob {
 };
 
 // Runs the matrix half of the reference's eliminations once per line class
-// and records what the right-hand-side half needs (one thread per class).
-//   pdma  [C | B | A | D | E]: divisor c(k) at step k, b(k) as used at step
-//         k-1, a(k), the normalised d(k), e(k); C(n) is the last divisor.
-//   tdma  [F | B | C]: multipliers a(j)/b(j-1), eliminated diagonal, c.
-//   ptdma [A | B | C | F1 | F2 | F3]: eliminated a (fill-in column), b, c;
-//         multipliers of row j and of row n at step j; the last multiplier.
-__global__ void k_r3d_factors(const __grid_constant__ R3Dev d, const FacJob *jobs, int njobs)
+// and records what the right-hand-side half needs (one thread per class, seven
+// rows of scratch each): pdma and tdma in banded.cuh's layouts,
+//   ptdma [A | B | C | F1 | F2 | F3 | 1/B]: eliminated a (fill-in column), b,
+//         c; multipliers of row j and of row n at step j; the last multiplier;
+//         reciprocals of the pivots.
+__global__ void k_r3d_factors(const __grid_constant__ R3Dev d, const FacJob *jobs, int njobs, double *work, int wstride)
 {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= njobs) return;
@@ -797,32 +808,12 @@ __global__ void k_r3d_factors(const __grid_constant__ R3Dev d, const FacJob *job
     const int kind = r3_kind(J.comp, J.dir);
     const int n = r3_len(J.comp, J.dir, L.n1, L.n2, L.n3);
     double *T = J.tab;
-    if (kind == 0) {
-        double *Cc = T, *Bb = T + n, *Aa = T + 2 * n, *Dd = T + 3 * n, *Ee = T + 4 * n;
-        for (int e = 0; e < n; ++e) r3_coef(L, J.comp, J.dir, J.ti, e, Aa[e], Bb[e], Cc[e], Dd[e], Ee[e]);
-        for (int k = 0; k <= n - 2; ++k) {
-            const double ck = Cc[k];
-            Dd[k] = Dd[k] / ck;
-            Ee[k] = Ee[k] / ck;
-            Cc[k + 1] = Cc[k + 1] - Bb[k + 1] * Dd[k];
-            if (k != n - 2) Dd[k + 1] = Dd[k + 1] - Bb[k + 1] * Ee[k];
-            if (k != n - 2) {
-                Bb[k + 2] = Bb[k + 2] - Aa[k + 2] * Dd[k];
-                Cc[k + 2] = Cc[k + 2] - Aa[k + 2] * Ee[k];
-            }
-        }
-        for (int k = 0; k < n; ++k) T[5 * n + k] = 1.0 / Cc[k];
-    } else if (kind == 1) {
-        double *F = T, *Bb = T + n, *Cc = T + 2 * n;
-        double dummy_d, dummy_e;
-        for (int e = 0; e < n; ++e) r3_coef(L, J.comp, J.dir, J.ti, e, F[e], Bb[e], Cc[e], dummy_d, dummy_e);
-        F[0] = 0.0;
-        for (int j = 1; j < n; ++j) {
-            const double fact = F[j] / Bb[j - 1];
-            Bb[j] = Bb[j] - fact * Cc[j - 1];
-            F[j] = fact;
-        }
-        for (int j = 0; j < n; ++j) T[3 * n + j] = 1.0 / Bb[j];
+    if (kind <= 1) {
+        double *w = work + (size_t)q * wstride;
+        double *a = w, *b = w + n, *c = w + 2 * n, *dd = w + 3 * n, *ee = w + 4 * n;
+        for (int e = 0; e < n; ++e) r3_coef(L, J.comp, J.dir, J.ti, e, a[e], b[e], c[e], dd[e], ee[e]);
+        if (kind == 0) factor_pdma(a, b, c, dd, ee, n, T, w + 5 * n);
+        else factor_tdma(a, b, c, n, T);
     } else {
         double *a = T, *b = T + n, *c = T + 2 * n, *F1 = T + 3 * n, *F2 = T + 4 * n, *F3 = T + 5 * n;
         double dummy_d, dummy_e;
@@ -860,6 +851,20 @@ __global__ void k_r3d_factors(const __grid_constant__ R3Dev d, const FacJob *job
 
 static const double F02 = (double)0.2f;   // REAL*4 literal 0.2 (rot3dmg.f:1626, 1800, 2029, 2106 ...)
 
+// Divisors with their stored reciprocals: x / d is the IEEE quotient (divrn.cuh)
+// up to the sign of a zero, in 3 FP64 instructions where the hardware division
+// takes 9 (562 cycles of an SM quarter's FP64 unit against 192).
+struct Dv {
+    double v, inv;
+};
+struct Rv {   // a radius, with the reciprocal of its square
+    double v, inv, inv2;
+};
+__device__ __forceinline__ double operator/(double a, const Dv &d) { return div_by_rcp_neg(a, d.v, d.inv); }
+__device__ __forceinline__ double operator/(double a, const Rv &r) { return div_by_rcp_neg(a, r.v, r.inv); }
+__device__ __forceinline__ Dv operator*(const Rv &r, const Rv &) { return {r.v * r.v, r.inv2}; }
+#define DV3 (Dv{3.0, 1.0 / 3.0})
+
 #define PV(i, j, k) v[(size_t)(i) + (size_t)L1 * ((size_t)(j) + (size_t)L2 * (size_t)(k))]
 #define RF(i, j, k) f[(size_t)(i) + (size_t)L1 * ((size_t)(j) + (size_t)L2 * (size_t)(k))]
 
@@ -870,18 +875,18 @@ template <int COMP>
 __device__ __forceinline__ double r3_rhs(const R3Lev &L, const R3Work &W, int dir, int p, int q, int e)
 {
     const int n1 = L.n1, n2 = L.n2, n3 = L.n3, L1 = L.L1, L2 = L.L2;
-    const double hr = L.hr, hhr = L.hhr, hhz = L.hhz, hhp = L.hhp;
+    const Dv hr{L.hr, L.ihr}, hhr{L.hhr, L.ihhr}, hhz{L.hhz, L.ihhz}, hhp{L.hhp, L.ihhp};
     const double *v = W.v, *f = W.f;
     if (dir == 0) {
         const int i = e + 1, j = p, k = q;
         const int ka = k == n3 ? 1 : k + 1, km = k - 1;
         if (COMP == 1) {
-            const double rval = L.rvc[i];
+            const Rv rval{L.rvc[i], L.dirc[i], L.diqc[i]};
             return -(PV(i, j + 1, k) + PV(i, j - 1, k)) / hhz - (PV(i, j, ka) + PV(i, j, km)) / hhp / (rval * rval) +
                    RF(i, j, k);
         } else if (COMP == 2) {
-            const double rval = L.rvc[i];
-            const double rq = rval * rval;
+            const Rv rval{L.rvc[i], L.dirc[i], L.diqc[i]};
+            const Dv rq = rval * rval;
             if (j == 1)
                 return -(5.0 / 3.0 * PV(i, j + 1, k) - F02 * PV(i, j + 2, k)) / hhz -
                        (PV(i, j, ka) + PV(i, j, km)) / hhp / rq + RF(i, j, k);
@@ -890,13 +895,13 @@ __device__ __forceinline__ double r3_rhs(const R3Lev &L, const R3Work &W, int di
                        (PV(i, j, ka) + PV(i, j, km)) / hhp / rq + RF(i, j, k);
             return -(PV(i, j - 1, k) + PV(i, j + 1, k)) / hhz - (PV(i, j, ka) + PV(i, j, km)) / hhp / rq + RF(i, j, k);
         } else {
-            const double rval = L.rvv[i];
-            const double rq = rval * rval;
+            const Rv rval{L.rvv[i], L.dirv[i], L.diqv[i]};
+            const Dv rq = rval * rval;
             if (j == 1)
-                return -(5.0 * PV(i, j + 1, k) / 3.0 - F02 * PV(i, j + 2, k)) / hhz -
+                return -(5.0 * PV(i, j + 1, k) / DV3 - F02 * PV(i, j + 2, k)) / hhz -
                        (PV(i, j, ka) + PV(i, j, km)) / hhp / rq + RF(i, j, k);
             if (j == n2)
-                return -(5.0 * PV(i, j - 1, k) / 3.0 - F02 * PV(i, j - 2, k)) / hhz -
+                return -(5.0 * PV(i, j - 1, k) / DV3 - F02 * PV(i, j - 2, k)) / hhz -
                        (PV(i, j, ka) + PV(i, j, km)) / hhp / rq + RF(i, j, k);
             return -(PV(i, j - 1, k) + PV(i, j + 1, k)) / hhz - (PV(i, j, ka) + PV(i, j, km)) / hhp / rq + RF(i, j, k);
         }
@@ -904,18 +909,18 @@ __device__ __forceinline__ double r3_rhs(const R3Lev &L, const R3Work &W, int di
         const int i = p, j = e + 1, k = q;
         const int ka = k == n3 ? 1 : k + 1, km = k - 1;
         if (COMP == 1) {
-            const double rval = L.rvc[i];
+            const Rv rval{L.rvc[i], L.dirc[i], L.diqc[i]};
             if (i == 1)
-                return -(5.0 * PV(i + 1, j, k) / 3.0 - F02 * PV(i + 2, j, k)) / hhr - 1.0 * PV(i + 1, j, k) / hr / rval * 0.5 -
+                return -(5.0 * PV(i + 1, j, k) / DV3 - F02 * PV(i + 2, j, k)) / hhr - 1.0 * PV(i + 1, j, k) / hr / rval * 0.5 -
                        (PV(i, j, ka) + PV(i, j, km)) / hhp / (rval * rval) + RF(i, j, k);
             if (i == n1)
-                return -(5.0 * PV(i - 1, j, k) / 3.0 - F02 * PV(i - 2, j, k)) / hhr + 1.0 * PV(i - 1, j, k) / hr / rval * 0.5 -
+                return -(5.0 * PV(i - 1, j, k) / DV3 - F02 * PV(i - 2, j, k)) / hhr + 1.0 * PV(i - 1, j, k) / hr / rval * 0.5 -
                        (PV(i, j, ka) + PV(i, j, km)) / hhp / (rval * rval) + RF(i, j, k);
             return -(PV(i + 1, j, k) + PV(i - 1, j, k)) / hhr - 0.5 * (PV(i + 1, j, k) - PV(i - 1, j, k)) / hr / rval -
                    (PV(i, j, ka) + PV(i, j, km)) / hhp / (rval * rval) + RF(i, j, k);
         } else if (COMP == 2) {
-            const double rval = L.rvc[i];
-            const double rq = rval * rval;
+            const Rv rval{L.rvc[i], L.dirc[i], L.diqc[i]};
+            const Dv rq = rval * rval;
             if (i == 1)
                 return -(5.0 / 3.0 * PV(i + 1, j, k) - 0.2 * PV(i + 2, j, k)) / hhr - 4.0 / 3.0 * PV(i + 1, j, k) / hr / rval -
                        (PV(i, j, ka) + PV(i, j, km)) / hhp / rq + RF(i, j, k);
@@ -925,25 +930,25 @@ __device__ __forceinline__ double r3_rhs(const R3Lev &L, const R3Work &W, int di
             return -(PV(i + 1, j, k) + PV(i - 1, j, k)) / hhr - 1.5 * (PV(i + 1, j, k) - PV(i - 1, j, k)) / hr / rval -
                    (PV(i, j, ka) + PV(i, j, km)) / hhp / rq + RF(i, j, k);
         } else {
-            const double rval = L.rvv[i];
-            const double rq = rval * rval;
+            const Rv rval{L.rvv[i], L.dirv[i], L.diqv[i]};
+            const Dv rq = rval * rval;
             return -(PV(i + 1, j, k) + PV(i - 1, j, k)) / hhr - 1.5 * (PV(i + 1, j, k) - PV(i - 1, j, k)) / hr / rval -
                    (PV(i, j, ka) + PV(i, j, km)) / hhp / rq + RF(i, j, k);
         }
     } else {
         const int i = p, j = q, k = e + 1;
         if (COMP == 1) {
-            const double rval = L.rvc[i];
+            const Rv rval{L.rvc[i], L.dirc[i], L.diqc[i]};
             if (i == 1)
-                return -(5.0 * PV(i + 1, j, k) / 3.0 - F02 * PV(i + 2, j, k)) / hhr - PV(i + 1, j, k) / hr / rval * 0.5 -
+                return -(5.0 * PV(i + 1, j, k) / DV3 - F02 * PV(i + 2, j, k)) / hhr - PV(i + 1, j, k) / hr / rval * 0.5 -
                        (PV(i, j + 1, k) + PV(i, j - 1, k)) / hhz + RF(i, j, k);
             if (i == n1)
-                return -(5.0 * PV(i - 1, j, k) / 3.0 - F02 * PV(i - 2, j, k)) / hhr + PV(i - 1, j, k) / hr / rval * 0.5 -
+                return -(5.0 * PV(i - 1, j, k) / DV3 - F02 * PV(i - 2, j, k)) / hhr + PV(i - 1, j, k) / hr / rval * 0.5 -
                        (PV(i, j + 1, k) + PV(i, j - 1, k)) / hhz + RF(i, j, k);
             return -(PV(i + 1, j, k) + PV(i - 1, j, k)) / hhr - 0.5 * (PV(i + 1, j, k) - PV(i - 1, j, k)) / hr / rval -
                    (PV(i, j + 1, k) + PV(i, j - 1, k)) / hhz + RF(i, j, k);
         } else if (COMP == 2) {
-            const double rval = L.rvc[i];
+            const Rv rval{L.rvc[i], L.dirc[i], L.diqc[i]};
             double rr;
             if (i == 1)
                 rr = -(5.0 / 3.0 * PV(i + 1, j, k) - 0.2 * PV(i + 2, j, k)) / hhr - 4.0 / 3.0 * PV(i + 1, j, k) / hr / rval;
@@ -955,132 +960,272 @@ __device__ __forceinline__ double r3_rhs(const R3Lev &L, const R3Work &W, int di
             if (j == n2) return rr - (5.0 / 3.0 * PV(i, j - 1, k) - 0.2 * PV(i, j - 2, k)) / hhz + RF(i, j, k);
             return rr - (PV(i, j - 1, k) + PV(i, j + 1, k)) / hhz + RF(i, j, k);
         } else {
-            const double rval = L.rvv[i];
+            const Rv rval{L.rvv[i], L.dirv[i], L.diqv[i]};
             if (j == 1)
                 return -(PV(i + 1, j, k) + PV(i - 1, j, k)) / hhr - 1.5 * (PV(i + 1, j, k) - PV(i - 1, j, k)) / hr / rval -
-                       (5.0 * PV(i, j + 1, k) / 3.0 - F02 * PV(i, j + 2, k)) / hhz + RF(i, j, k);
+                       (5.0 * PV(i, j + 1, k) / DV3 - F02 * PV(i, j + 2, k)) / hhz + RF(i, j, k);
             if (j == n2)
                 return -(PV(i + 1, j, k) + PV(i - 1, j, k)) / hhr - 1.5 * (PV(i + 1, j, k) - PV(i - 1, j, k)) / hr / rval -
-                       (5.0 * PV(i, j - 1, k) / 3.0 - F02 * PV(i, j - 2, k)) / hhz + RF(i, j, k);
+                       (5.0 * PV(i, j - 1, k) / DV3 - F02 * PV(i, j - 2, k)) / hhz + RF(i, j, k);
             return -(PV(i + 1, j, k) + PV(i - 1, j, k)) / hhr - 1.5 * (PV(i + 1, j, k) - PV(i - 1, j, k)) / hr / rval -
                    (PV(i, j + 1, k) + PV(i, j - 1, k)) / hhz + RF(i, j, k);
         }
     }
 }
 
-// Solves line (p, q) of direction dir whose right-hand side s[0..n-1] a
-// block formed beforehand in shared memory: the elimination runs in s and
-// the solution goes to the level's correction v.  Lines along r and z on
-// plane k = n3 also write plane 0; phi-lines write plane 0 from plane n3.
-template <int COMP>
-__device__ void r3_line(const R3Lev &L, const R3Work &W, int dir, int p, int q, double *s)
+// Periodic tridiagonal in place on a staged line: the reference's ptdma in its
+// order, the factors of the next rows loaded while a row is eliminated (see
+// banded.cuh).
+template <int U = 2> __device__ __forceinline__ void ptdma_staged(const double *T, int n, double *x, int pitch)
 {
-    const int n1 = L.n1, n2 = L.n2, n3 = L.n3, L1 = L.L1, L2 = L.L2;
-    const int kind = r3_kind(COMP, dir);
-    const int n = r3_len(COMP, dir, n1, n2, n3);
-    double *v = W.v;
-    size_t base;
-    long long step;
-    if (dir == 0) {
-        base = (size_t)1 + (size_t)L1 * ((size_t)p + (size_t)L2 * (size_t)q);
-        step = 1;
-    } else if (dir == 1) {
-        base = (size_t)p + (size_t)L1 * ((size_t)1 + (size_t)L2 * (size_t)q);
-        step = L1;
-    } else {
-        base = (size_t)p + (size_t)L1 * ((size_t)q + (size_t)L2);
-        step = (long long)L1 * L2;
+    const double *Aa = T, *Bb = T + n, *Cc = T + 2 * n, *F1 = T + 3 * n, *F2 = T + 4 * n, *F3 = T + 5 * n, *iB = T + 6 * n;
+    const int N = n - 1;
+    double rN = x[N * pitch], prev = x[0];
+    double f[U], g[U], r[U], b[U], ib[U];
+    auto fetch = [&](int j0) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int j = min(j0 + u, n - 2);
+            f[u] = F1[j];
+            g[u] = F2[j];
+            r[u] = x[j * pitch];
+        }
+    };
+    fetch(1);
+    for (int j0 = 1; j0 <= n - 2; j0 += U) {
+        double f0[U], g0[U], r0[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            f0[u] = f[u];
+            g0[u] = g[u];
+            r0[u] = r[u];
+        }
+        if (j0 + U <= n - 2) fetch(j0 + U);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (j0 + u <= n - 2) {
+                const double rj = r0[u] - f0[u] * prev;
+                rN = rN - g0[u] * prev;
+                x[(j0 + u) * pitch] = rj;
+                prev = rj;
+            }
+        }
     }
-    const long long plane = (long long)L1 * L2 * n3;
-    const bool seam = dir != 2 && q == n3;
-    const double *T = L.fac[COMP][dir];
-    if (dir != 0) T += (size_t)(p - 1) * r3_tabsize(kind, n);
-#define PUT(e, x)                                                                     \
-    do {                                                                              \
-        const double _x = (x);                                                        \
-        v[base + (size_t)((long long)(e) * step)] = _x;                               \
-        if (seam) v[base + (size_t)((long long)(e) * step) - plane] = _x;             \
-    } while (0)
-    if (kind == 0) {
-        const double *Cc = T, *Bb = T + n, *Aa = T + 2 * n, *Dd = T + 3 * n, *Ee = T + 4 * n, *iC = T + 5 * n;
-        double r0 = s[0], r1 = s[1];
-#pragma unroll 4
-        for (int k = 0; k <= n - 2; ++k) {
-            const double rk = div_by_rcp(r0, Cc[k], iC[k]);
-            s[k] = rk;
-            const double rk1 = r1 - Bb[k + 1] * rk;
-            double rk2 = 0.0;
-            if (k != n - 2) rk2 = s[k + 2] - Aa[k + 2] * rk;
-            r0 = rk1;
-            r1 = rk2;
+    rN = rN - F3[0] * prev;
+    const double yN = div_by_rcp_neg(rN, Bb[N], iB[N]);
+    x[N * pitch] = yN;
+    double y = div_by_rcp_neg(prev - Cc[n - 2] * yN, Bb[n - 2], iB[n - 2]);
+    x[(n - 2) * pitch] = y;
+    auto fetch_back = [&](int j0) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int j = max(j0 - u, 0);
+            f[u] = Cc[j];
+            g[u] = Aa[j];
+            b[u] = Bb[j];
+            ib[u] = iB[j];
+            r[u] = x[j * pitch];
         }
-        double x1 = div_by_rcp(r0, Cc[n - 1], iC[n - 1]);
-        PUT(n - 1, x1);
-        double x0 = s[n - 2] - Dd[n - 2] * x1;
-        PUT(n - 2, x0);
-        double x2 = x1;
-        x1 = x0;
-#pragma unroll 4
-        for (int j = n - 3; j >= 0; --j) {
-            const double x = s[j] - Dd[j] * x1 - Ee[j] * x2;
-            PUT(j, x);
-            x2 = x1;
-            x1 = x;
+    };
+    fetch_back(n - 3);
+    for (int j0 = n - 3; j0 >= 0; j0 -= U) {
+        double f0[U], g0[U], b0[U], ib0[U], r0[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            f0[u] = f[u];
+            g0[u] = g[u];
+            b0[u] = b[u];
+            ib0[u] = ib[u];
+            r0[u] = r[u];
         }
-    } else if (kind == 1) {
-        const double *F = T, *Bb = T + n, *Cc = T + 2 * n, *iB = T + 3 * n;
-        double rprev = s[0];
-#pragma unroll 4
-        for (int j = 1; j < n; ++j) {
-            const double rj = s[j] - F[j] * rprev;
-            s[j] = rj;
-            rprev = rj;
+        if (j0 - U >= 0) fetch_back(j0 - U);
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (j0 - u >= 0) {
+                y = div_by_rcp_neg(r0[u] - f0[u] * y - g0[u] * yN, b0[u], ib0[u]);
+                x[(j0 - u) * pitch] = y;
+            }
         }
-        double y = div_by_rcp(rprev, Bb[n - 1], iB[n - 1]);
-        PUT(n - 1, y);
-#pragma unroll 4
-        for (int j = n - 2; j >= 0; --j) {
-            y = div_by_rcp(s[j] - Cc[j] * y, Bb[j], iB[j]);
-            PUT(j, y);
-        }
-    } else {
-        const double *Aa = T, *Bb = T + n, *Cc = T + 2 * n, *F1 = T + 3 * n, *F2 = T + 4 * n, *F3 = T + 5 * n;
-        const double *iB = T + 6 * n;
-        const int N = n - 1;
-        double rN = s[N];
-        double rprev = s[0];
-#pragma unroll 4
-        for (int j = 1; j <= n - 3; ++j) {
-            const double rj = s[j] - F1[j] * rprev;
-            rN = rN - F2[j] * rprev;
-            s[j] = rj;
-            rprev = rj;
-        }
-        const double rn2 = s[n - 2] - F1[n - 2] * rprev;
-        rN = rN - F2[n - 2] * rprev;
-        rN = rN - F3[0] * rn2;
-        const double yN = div_by_rcp(rN, Bb[N], iB[N]);
-        PUT(N, yN);
-        double y = div_by_rcp(rn2 - Cc[n - 2] * yN, Bb[n - 2], iB[n - 2]);
-        PUT(n - 2, y);
-#pragma unroll 4
-        for (int j = n - 3; j >= 0; --j) {
-            y = div_by_rcp(s[j] - Cc[j] * y - Aa[j] * yN, Bb[j], iB[j]);
-            PUT(j, y);
-        }
-        v[base - (size_t)step] = yN;   // plane 0 = plane n3
     }
-#undef PUT
 }
 
-// Shared memory of a solve block: right-hand sides of up to R3_SMEM_DOUBLES
-// line elements (each line padded to an odd pitch against bank conflicts).
-#define R3_SMEM_DOUBLES 6144
+// A phi-line's matrix is the same in every row, a (x(k-1) + x(k+1)) + b x(k)
+// = r(k) around the ring, and factors into two first-order recurrences with
+// one coefficient: with rho + 1/rho = -b/a, 0 < rho < 1,
+//   z(k) = r(k) / s + rho z(k-1),   x(k) = z(k) + rho x(k+1),   s = -a/rho,
+// each around the ring: run from zero, its value after one turn, divided by
+// 1 - rho^n, is the value it should have entered with.
+struct R3Ring {
+    float rho, scale, turn;   // rho, 1/s, 1/(1 - rho^n)
+    int steps;                // scan steps (warpline.cuh); -1: a ring of the level is not diagonally dominant
+};
 
-// One phase of independent lines [a, b) of the list: each block takes a
-// contiguous share, forms the right-hand sides of a chunk of its lines with
-// all its threads (every element independently, so the loads and divisions
-// overlap), then one thread per line runs the elimination.
+// y(u) = t(u) + rho y(u-1) around the ring of n rows over W = 2^lw lanes (BACK:
+// t(u) + rho y(u+1)), in place; rows past the end are left zero.
+template <int M, bool BACK>
+__device__ __forceinline__ void r3_ring(int lw, int n, const R3Ring &R, float (&t)[M])
+{
+    const unsigned full = 0xffffffffu;
+    const int W = 1 << lw, lane = threadIdx.x & (W - 1), last = (n - 1) / M;   // the last lane with rows
+    const int pos = BACK ? last - lane : lane;
+    float w = 0.f, p = 1.f;
+#pragma unroll
+    for (int s = 0; s < M; ++s) {
+        const int u = BACK ? M - 1 - s : s;
+        if (lane * M + u < n) {
+            w = __fmaf_rn(R.rho, w, t[u]);
+            p *= R.rho;
+        }
+    }
+#pragma unroll 1
+    for (int d = 1; d < 1 << R.steps; d <<= 1) {
+        const int src = BACK ? lane + d : lane - d;
+        const float v = __shfl_sync(full, w, src, W), g = __shfl_sync(full, p, src, W);
+        if (pos >= d) {
+            w = __fmaf_rn(p, v, w);
+            p *= g;
+        }
+    }
+    const float c = __shfl_sync(full, w, BACK ? 0 : last, W) * R.turn;
+    const float s = __fmaf_rn(p, c, w);
+    float y = __shfl_sync(full, s, BACK ? lane + 1 : lane - 1, W);
+    if (pos == 0) y = c;
+#pragma unroll
+    for (int q = 0; q < M; ++q) {
+        const int u = BACK ? M - 1 - q : q;
+        if (lane * M + u < n) {
+            y = __fmaf_rn(R.rho, y, t[u]);
+            t[u] = y;
+        }
+    }
+}
+
+// Rings of n rows, nl of them, in place in shared memory (x: [line][row], a
+// lane's rows padded); rings longer than a warp's 512 rows by one thread each.
+template <int M> __device__ __forceinline__ void r3_rings_m(const R3Ring *tab, const int *lines, int n, float *x, int xpitch, int nl)
+{
+    const int lw = wl_log2w(n), per = 32 >> lw;
+    const int sub = (threadIdx.x & 31) >> lw, lane = threadIdx.x & ((1 << lw) - 1);
+    const int slot = (threadIdx.x >> 5) * per + sub, nslots = ((int)blockDim.x >> 5) * per;
+    for (int t0 = 0; t0 < nl; t0 += nslots) {
+        if (t0 + slot - sub >= nl) continue;   // no line for this warp
+        const bool live = t0 + slot < nl;
+        const int l = live ? t0 + slot : t0 + slot - sub;   // idle groups repeat a line and store nothing
+        const R3Ring R = tab[(lines[l] & 0xffff) - 1];
+        float *xs = x + (size_t)l * xpitch + lane * (M + 1);
+        float t[M];
+#pragma unroll
+        for (int u = 0; u < M; ++u) t[u] = lane * M + u < n ? xs[u] * R.scale : 0.f;
+        r3_ring<M, false>(lw, n, R, t);
+        r3_ring<M, true>(lw, n, R, t);
+        if (live) {
+#pragma unroll
+            for (int u = 0; u < M; ++u) xs[u] = t[u];
+        }
+    }
+}
+// Levels with a ring that is not diagonally dominant (radii below the mesh
+// size) take the FP64 factors, a thread per line.
+__device__ __forceinline__ void r3_rings(const R3Ring *tab, const double *fac, const int *lines, int n, float *x, int xpitch, int nl)
+{
+    if (tab[0].steps < 0) {
+        const int lg = wl_log2m(n), N = n - 1;
+        for (int l = threadIdx.x; l < nl; l += blockDim.x) {
+            const double *T = fac + (size_t)((lines[l] & 0xffff) - 1) * 7 * n;
+            const double *Aa = T, *Bb = T + n, *Cc = T + 2 * n, *F1 = T + 3 * n, *F2 = T + 4 * n, *F3 = T + 5 * n;
+            float *y = x + (size_t)l * xpitch;
+            double rN = y[wl_slot(lg, N)], prev = y[wl_slot(lg, 0)];
+            for (int k = 1; k <= n - 2; ++k) {
+                const double r = y[wl_slot(lg, k)] - F1[k] * prev;
+                rN -= F2[k] * prev;
+                y[wl_slot(lg, k)] = (float)r;
+                prev = r;
+            }
+            rN -= F3[0] * prev;
+            const double yN = rN / Bb[N];
+            double yk = (prev - Cc[n - 2] * yN) / Bb[n - 2];
+            y[wl_slot(lg, N)] = (float)yN;
+            y[wl_slot(lg, n - 2)] = (float)yk;
+            for (int k = n - 3; k >= 0; --k) {
+                yk = (y[wl_slot(lg, k)] - Cc[k] * yk - Aa[k] * yN) / Bb[k];
+                y[wl_slot(lg, k)] = (float)yk;
+            }
+        }
+    } else if (n <= 256) {
+        r3_rings_m<8>(tab, lines, n, x, xpitch, nl);
+    } else if (n <= 512) {
+        r3_rings_m<16>(tab, lines, n, x, xpitch, nl);
+    } else {
+        for (int l = threadIdx.x; l < nl; l += blockDim.x) {
+            const R3Ring R = tab[(lines[l] & 0xffff) - 1];
+            float *y = x + (size_t)l * xpitch;
+            const int lg = wl_log2m(n);
+            float c = 0.f;
+            for (int k = 0; k < n; ++k) c = __fmaf_rn(R.rho, c, y[wl_slot(lg, k)] * R.scale);
+            c *= R.turn;
+            for (int k = 0; k < n; ++k) y[wl_slot(lg, k)] = c = __fmaf_rn(R.rho, c, y[wl_slot(lg, k)] * R.scale);
+            c = 0.f;
+            for (int k = n - 1; k >= 0; --k) c = __fmaf_rn(R.rho, c, y[wl_slot(lg, k)]);
+            c *= R.turn;
+            for (int k = n - 1; k >= 0; --k) y[wl_slot(lg, k)] = c = __fmaf_rn(R.rho, c, y[wl_slot(lg, k)]);
+        }
+    }
+}
+
+// Dynamic shared memory of a solve block (two blocks an SM): the levels'
+// descriptors, the staged lines' right-hand sides (R3_CHUNK_BYTES; a group of
+// lines that must share a chunk fits them, r3_phases) and their factors.
+// Behind the kernel's parameter each descriptor field would be a load of its
+// own ahead of every pass's loads, and after each barrier again.
+#define R3_LEVS 5   // levels 1 .. 4
+#define R3_WEIGHTS 512   // float4: grids up to about 110 x 110 keep all levels' here
+struct R3Shared {
+    R3Lev lev[R3_LEVS];
+    R3Work work[R3_LEVS];
+    int my0, my1;           // the block's share of the phase at hand
+    int p0, staged;         // its first chunk's factors: first radius, whether staged
+    int line[R3_THREADS];   // its first chunk's lines
+    float4 weights[R3_WEIGHTS];   // the FP32 operator's, where they fit
+};
+#define R3_SMEM_BYTES (110 * 1024)
+#define R3_CHUNK_BYTES (44 * 1024)
+#define R3_FAC_BYTES (52 * 1024)
+static_assert(sizeof(R3Shared) + R3_CHUNK_BYTES + R3_FAC_BYTES <= R3_SMEM_BYTES, "shared memory of a solve block");
+__device__ __forceinline__ R3Shared &r3_shared()
+{
+    extern __shared__ __align__(16) unsigned char s_r3[];
+    return *(R3Shared *)s_r3;
+}
+__device__ __forceinline__ void r3_descriptors(const R3Dev &d, int comp, bool mixed)
+{
+    R3Shared &S = r3_shared();
+    for (int q = threadIdx.x; q < (int)(R3_LEVS * sizeof(R3Lev) / 4); q += R3_THREADS) ((unsigned *)S.lev)[q] = ((const unsigned *)d.lev)[q];
+    for (int q = threadIdx.x; q < (int)(R3_LEVS * sizeof(R3Work) / 4); q += R3_THREADS)
+        ((unsigned *)S.work)[q] = ((const unsigned *)d.work[comp])[q];
+    __syncthreads();
+    if (!mixed) return;
+    int at = 0;
+    for (int l = 1; l <= d.nlev; ++l) {
+        const int n1 = S.lev[l].n1, n2 = S.lev[l].n2, need = (n1 + 1) + (n2 + 1) + (n1 + 4) / 4;
+        if (at + need > R3_WEIGHTS) break;
+        float4 *wi = S.weights + at, *wj = wi + n1 + 1;
+        float *wp = (float *)(wj + n2 + 1);
+        for (int i = threadIdx.x; i <= n1; i += R3_THREADS) {
+            wi[i] = S.lev[l].wi[comp][i];
+            wp[i] = S.lev[l].wp[comp][i];
+        }
+        for (int j = threadIdx.x; j <= n2; j += R3_THREADS) wj[j] = S.lev[l].wj[comp][j];
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            S.lev[l].wi[comp] = wi;
+            S.lev[l].wj[comp] = wj;
+            S.lev[l].wp[comp] = wp;
+        }
+        at += need;
+    }
+    __syncthreads();
+}
+
 // A block's share of a phase's entries [a, b) starts at x moved forward
 // past the rest of a group that x would split (entries marked as continued
 // belong with the next one); every block moves its two ends the same way,
@@ -1101,29 +1246,198 @@ __device__ __forceinline__ int r3_chunk_end(const int *lines, int c0, int c1)
     return e;
 }
 
+template <int COMP> struct R3Point;
 template <int COMP>
-__device__ void r3_phase(const R3Lev &L, const R3Work &W, int dir, const int *lines, int a, int b, double *sm)
+__device__ __forceinline__ void r3_rhs32_batch(const R3Lev &L, const R3Work &W, int dir, const int *s_line, int nl, int n, const RowSplit &split,
+                               float *x, int lpitch, int lg);
+
+// Lines a chunk holds, and floats or doubles of factors beside them.
+template <int COMP, class T> __device__ __forceinline__ int r3_chunk(int dir, int n, int len)
 {
-    const int n = r3_len(COMP, dir, L.n1, L.n2, L.n3);
-    const int pitch = n | 1;
+    constexpr bool F64 = sizeof(T) == 8;
+    int chunk = min(R3_THREADS, (int)(R3_CHUNK_BYTES / sizeof(T)) / (F64 ? n | 1 : wl_pitch(n)));
+    if (!F64 && dir == 1) chunk = min(chunk, (int)(R3_FAC_BYTES / sizeof(T)) / len);   // a table per line
+    return max(1, chunk);
+}
+
+// Starts the copy of the factors of nl lines: one table in direction 0, else
+// one per radius p.  FP64 lists keep a radius's lines together, so the tables
+// of a chunk's radii are few and lie in a row (p0 gets the first); FP32 ones
+// take a table per line (a ring's is four words, read where it is used).
+// Returns whether they fit.  line(t): the t-th line.
+template <int COMP, class T, class Line>
+__device__ __forceinline__ bool r3_fetch(const R3Lev &L, int dir, int n, int len, int nl, Line line, int tid, int nthr, int &p0)
+{
+    constexpr bool F64 = sizeof(T) == 8;
+    extern __shared__ __align__(16) unsigned char s_r3[];
+    T *sfac = (T *)(s_r3 + sizeof(R3Shared) + R3_CHUNK_BYTES);
+    const T *fac = F64 ? (const T *)L.fac[COMP][dir] : (const T *)L.fac32[COMP][dir];
+    const int room = (int)(R3_FAC_BYTES / sizeof(T));
+    p0 = 1;
+    if (dir == 0) {
+        if (len > room) return false;
+        async_copy(sfac, fac, len, tid, nthr);
+    } else if constexpr (F64) {
+        int a = line(0) & 0xffff, b = a;
+        for (int t = threadIdx.x & 31; t < nl; t += 32) {
+            a = min(a, line(t) & 0xffff);
+            b = max(b, line(t) & 0xffff);
+        }
+        p0 = __reduce_min_sync(0xffffffffu, a);
+        b = __reduce_max_sync(0xffffffffu, b);
+        if ((b - p0 + 1) * len > room) return false;
+        async_copy(sfac, fac + (size_t)(p0 - 1) * len, (b - p0 + 1) * len, tid, nthr);
+    } else if (dir == 1) {
+        if (nl * len > room) return false;
+        for (int t = 0; t < nl; ++t) async_copy(sfac + t * len, fac + (size_t)((line(t) & 0xffff) - 1) * len, len, tid, nthr);
+    }
+    return true;
+}
+
+// What phase ph of direction dir on level lev reads besides the solution: the
+// block's share of the lines, the first chunk's lines and factors.  None of it
+// changes during a solve, so it is fetched while the block waits at the
+// barrier before the phase (threads 32 .. of the block).
+template <int COMP, class T> __device__ __noinline__ void r3_prepare(int lev, int dir, int ph)
+{
+    R3Shared &S = r3_shared();
+    const R3Lev &L = S.lev[lev];
+    constexpr bool F64 = sizeof(T) == 8;
+    const int tid = (int)threadIdx.x - 32, nthr = R3_THREADS - 32;
+    const int *lines = L.lines[COMP][dir];
+    const int a = L.poff[COMP][dir][ph], b = L.poff[COMP][dir][ph + 1];
+    const int kind = r3_kind(COMP, dir), n = r3_len(COMP, dir, L.n1, L.n2, L.n3);
+    const int len = F64 ? r3_tabsize(kind, n) : r3_tabsize32(kind, n);
     const int per = (b - a + (int)gridDim.x - 1) / (int)gridDim.x;
     const int my0 = r3_group_start(lines, a, b, a + (int)blockIdx.x * per);
     const int my1 = r3_group_start(lines, a, b, a + ((int)blockIdx.x + 1) * per);
-    const int chunk = max(1, min((int)blockDim.x, R3_SMEM_DOUBLES / pitch));
+    int p0 = 1;
+    bool staged = false;
+    if (my0 < my1) {
+        const int c1 = r3_chunk_end(lines, my0, min(my1, my0 + r3_chunk<COMP, T>(dir, n, len)));
+        for (int t = tid; t < c1 - my0; t += nthr) S.line[t] = lines[my0 + t] & 0x7fffffff;
+        staged = r3_fetch<COMP, T>(L, dir, n, len, c1 - my0, [&](int t) { return lines[my0 + t] & 0x7fffffff; }, tid, nthr, p0);
+    }
+    if (tid == 0) {
+        S.my0 = my0;
+        S.my1 = my1;
+        S.p0 = p0;
+        S.staged = staged;
+    }
+}
+
+// One phase of independent lines, prepared by r3_prepare: each block takes a
+// contiguous share, in chunks that fit its shared memory.  All threads form a
+// chunk's right-hand sides (along the line in direction 0, across the lines in
+// the others, whichever runs with memory), the lines are eliminated (FP64: one
+// thread per line in the reference's order; FP32: up to 32 lanes per line),
+// the solutions go to the level's correction v.  Lines along r and z on plane
+// k = n3 also write plane 0; phi-lines write plane 0 from plane n3.
+template <int COMP, class T> __device__ __noinline__ void r3_phase(int lev, int dir)
+{
+    extern __shared__ __align__(16) unsigned char s_r3[];
+    R3Shared &S = r3_shared();
+    const R3Lev &L = S.lev[lev];
+    const R3Work &W = S.work[lev];
+    constexpr bool F64 = sizeof(T) == 8;
+    const int my0 = S.my0, my1 = S.my1;
+    if (my0 >= my1) return;
+    const int n1 = L.n1, n2 = L.n2, n3 = L.n3;
+    const size_t L1 = L.L1, L2 = L.L2;
+    const int kind = r3_kind(COMP, dir), n = r3_len(COMP, dir, n1, n2, n3);
+    const int len = F64 ? r3_tabsize(kind, n) : r3_tabsize32(kind, n);
+    const int lpitch = F64 ? 0 : wl_pitch(n), lg = F64 ? 0 : wl_log2m(n);
+    const int chunk = r3_chunk<COMP, T>(dir, n, len);
+    const int *lines = L.lines[COMP][dir];
+    int *s_line = S.line;
+    T *v = F64 ? (T *)W.v : (T *)W.v32;
+    const T *fac = F64 ? (const T *)L.fac[COMP][dir] : (const T *)L.fac32[COMP][dir];
+    T *x = (T *)(s_r3 + sizeof(R3Shared)), *sfac = (T *)(s_r3 + sizeof(R3Shared) + R3_CHUNK_BYTES);
+    const RowSplit by_line(n);
     for (int c0 = my0; c0 < my1;) {
         const int c1 = r3_chunk_end(lines, c0, min(my1, c0 + chunk));
-        const int nl = c1 - c0;
-        for (int t = threadIdx.x; t < nl * n; t += blockDim.x) {
-            const int li = t / n, e = t - li * n;
-            const int pk = lines[c0 + li] & 0x7fffffff;
-            sm[li * pitch + e] = r3_rhs<COMP>(L, W, dir, pk & 0xffff, pk >> 16, e);
+        const int nl = c1 - c0, pitch = nl | 1;
+        auto at = [&](int t, int e) -> T & { return F64 ? x[e * pitch + t] : x[t * lpitch + wl_slot(lg, e)]; };
+        int p0 = S.p0;
+        bool staged = S.staged;
+        if (c0 != my0) {
+            __syncthreads();   // the chunk before has left s_line, the factors and x
+            for (int t = threadIdx.x; t < nl; t += R3_THREADS) s_line[t] = lines[c0 + t] & 0x7fffffff;
+            __syncthreads();
+            staged = r3_fetch<COMP, T>(L, dir, n, len, nl, [&](int t) { return s_line[t]; }, threadIdx.x, R3_THREADS, p0);
+        }
+        if constexpr (!F64) {
+            r3_rhs32_batch<COMP>(L, W, dir, s_line, nl, n, dir == 0 ? by_line : RowSplit(nl), x, lpitch, lg);
+        } else if (dir == 0) {
+            for (int idx = threadIdx.x; idx < nl * n; idx += R3_THREADS) {
+                int t, e;
+                by_line(idx, t, e);
+                at(t, e) = r3_rhs<COMP>(L, W, 0, s_line[t] & 0xffff, s_line[t] >> 16, e);
+            }
+        } else {
+            const RowSplit by_row(nl);
+            for (int idx = threadIdx.x; idx < nl * n; idx += R3_THREADS) {
+                int e, t;
+                by_row(idx, e, t);
+                at(t, e) = r3_rhs<COMP>(L, W, dir, s_line[t] & 0xffff, s_line[t] >> 16, e);
+            }
+        }
+        if constexpr (!F64) {   // rows past the line's end
+            const int pad = wl_rows(n) - n;
+            for (int idx = threadIdx.x; idx < nl * pad; idx += R3_THREADS) at(idx / pad, n + idx % pad) = T(0);
+        }
+        async_copy_wait();
+        __syncthreads();
+        if constexpr (F64) {
+            const int t = threadIdx.x;
+            if (t < nl) {
+                auto solve = [&](const double *tab) {
+                    if (kind == 0) pdma_staged(tab, n, x + t, pitch);
+                    else if (kind == 1) tdma_staged(tab, n, x + t, pitch);
+                    else ptdma_staged(tab, n, x + t, pitch);
+                };
+                const int p = dir == 0 ? 1 : s_line[t] & 0xffff;
+                if (staged) solve(sfac + (size_t)(p - p0) * len);
+                else solve(fac + (size_t)(p - 1) * len);
+            }
+        } else if (kind == 2) {
+            r3_rings((const R3Ring *)fac, L.fac[COMP][2], s_line, n, x, lpitch, nl);
+        } else if (staged) {
+            if (kind == 0) wl_lines<true>(sfac, dir == 0 ? 0 : len, n, x, lpitch, nl);
+            else wl_lines<false>(sfac, dir == 0 ? 0 : len, n, x, lpitch, nl);
+        } else {   // each line's table from global memory
+            for (int t = 0; t < nl; ++t) {
+                const T *tab = fac + (dir == 0 ? 0 : (size_t)((s_line[t] & 0xffff) - 1) * len);
+                if (threadIdx.x < 32) {
+                    if (kind == 0) wl_lines_m<16, true>(tab, 0, n, x + t * lpitch, lpitch, 1, 0, 1);
+                    else wl_lines_m<16, false>(tab, 0, n, x + t * lpitch, lpitch, 1, 0, 1);
+                }
+            }
         }
         __syncthreads();
-        if ((int)threadIdx.x < nl) {
-            const int pk = lines[c0 + threadIdx.x] & 0x7fffffff;
-            r3_line<COMP>(L, W, dir, pk & 0xffff, pk >> 16, sm + threadIdx.x * pitch);
+        if (dir == 0) {
+            for (int idx = threadIdx.x; idx < nl * n; idx += R3_THREADS) {
+                int t, e;
+                by_line(idx, t, e);
+                const int j = s_line[t] & 0xffff, k = s_line[t] >> 16;
+                const T val = at(t, e);
+                const size_t o = (size_t)(e + 1) + L1 * ((size_t)j + L2 * (size_t)k);
+                v[o] = val;
+                if (k == n3) v[o - L1 * L2 * (size_t)n3] = val;
+            }
+        } else {
+            const RowSplit by_row(nl);
+            for (int idx = threadIdx.x; idx < nl * n; idx += R3_THREADS) {
+                int e, t;
+                by_row(idx, e, t);
+                const int i = s_line[t] & 0xffff, q = s_line[t] >> 16;
+                const int j = dir == 1 ? e + 1 : q, k = dir == 1 ? q : e + 1;
+                const T val = at(t, e);
+                const size_t o = (size_t)i + L1 * ((size_t)j + L2 * (size_t)k);
+                v[o] = val;
+                if (k == n3) v[o - L1 * L2 * (size_t)n3] = val;
+            }
         }
-        __syncthreads();
         c0 = c1;
     }
 }
@@ -1134,26 +1448,26 @@ template <int COMP>
 __device__ __forceinline__ double r3_resid(const R3Lev &L, const R3Work &W, int i, int j, int k)
 {
     const int n1 = L.n1, n2 = L.n2, n3 = L.n3, L1 = L.L1, L2 = L.L2;
-    const double hr = L.hr, hhr = L.hhr, hhz = L.hhz, hhp = L.hhp;
+    const Dv hr{L.hr, L.ihr}, hhr{L.hhr, L.ihhr}, hhz{L.hhz, L.ihhz}, hhp{L.hhp, L.ihhp};
     const double *v = W.v, *f = W.f;
     const int ka = k == n3 ? 1 : k + 1, km = k - 1;
     double temp;
     if (COMP == 1) {
-        const double rval = L.rvc[i];
+        const Rv rval{L.rvc[i], L.dirc[i], L.diqc[i]};
         temp = (PV(i, j + 1, k) + PV(i, j - 1, k)) / hhz + (PV(i, j, ka) + PV(i, j, km)) / hhp / (rval * rval) -
                PV(i, j, k) * (2.0 / hhz + 2.0 / hhp / (rval * rval));
         if (i == 1)
-            temp = temp + (-2.0 * PV(i, j, k) + 5.0 * PV(i + 1, j, k) / 3.0 - 0.2 * PV(i + 2, j, k)) / hhr +
+            temp = temp + (-2.0 * PV(i, j, k) + 5.0 * PV(i + 1, j, k) / DV3 - 0.2 * PV(i + 2, j, k)) / hhr +
                    0.5 * (-PV(i, j, k) + PV(i + 1, j, k)) / hr / rval;
         else if (i == n1)
-            temp = temp + (-2.0 * PV(i, j, k) + 5.0 * PV(i - 1, j, k) / 3.0 - 0.2 * PV(i - 2, j, k)) / hhr +
+            temp = temp + (-2.0 * PV(i, j, k) + 5.0 * PV(i - 1, j, k) / DV3 - 0.2 * PV(i - 2, j, k)) / hhr +
                    0.5 * (PV(i, j, k) - PV(i - 1, j, k)) / hr / rval;
         else
             temp = temp + (PV(i - 1, j, k) - 2.0 * PV(i, j, k) + PV(i + 1, j, k)) / hhr +
                    0.5 * (PV(i + 1, j, k) - PV(i - 1, j, k)) / hr / rval;
     } else if (COMP == 2) {
-        const double rval = L.rvc[i];
-        const double rq = rval * rval;
+        const Rv rval{L.rvc[i], L.dirc[i], L.diqc[i]};
+        const Dv rq = rval * rval;
         temp = (PV(i, j, ka) - 2.0 * PV(i, j, k) + PV(i, j, km)) / hhp / rq + PV(i, j, k) / rq;
         if (i == 1)
             temp = temp + (-2.0 * PV(i, j, k) + 5.0 / 3.0 * PV(i + 1, j, k) - 0.2 * PV(i + 2, j, k)) / hhr +
@@ -1171,14 +1485,14 @@ __device__ __forceinline__ double r3_resid(const R3Lev &L, const R3Work &W, int 
         else
             temp = temp + (PV(i, j + 1, k) - 2.0 * PV(i, j, k) + PV(i, j - 1, k)) / hhz;
     } else {
-        const double rval = L.rvv[i];
-        const double rq = rval * rval;
+        const Rv rval{L.rvv[i], L.dirv[i], L.diqv[i]};
+        const Dv rq = rval * rval;
         temp = (PV(i + 1, j, k) + PV(i - 1, j, k)) / hhr + 1.5 * (PV(i + 1, j, k) - PV(i - 1, j, k)) / hr / rval +
                PV(i, j, k) / rq + (PV(i, j, ka) + PV(i, j, km)) / hhp / rq - PV(i, j, k) * (2.0 / hhr + 2.0 / hhp / rq);
         if (j == 1)
-            temp = temp + (-2.0 * PV(i, j, k) + 5.0 * PV(i, j + 1, k) / 3.0 - 0.2 * PV(i, j + 2, k)) / hhz;
+            temp = temp + (-2.0 * PV(i, j, k) + 5.0 * PV(i, j + 1, k) / DV3 - 0.2 * PV(i, j + 2, k)) / hhz;
         else if (j == n2)
-            temp = temp + (-2.0 * PV(i, j, k) + 5.0 * PV(i, j - 1, k) / 3.0 - 0.2 * PV(i, j - 2, k)) / hhz;
+            temp = temp + (-2.0 * PV(i, j, k) + 5.0 * PV(i, j - 1, k) / DV3 - 0.2 * PV(i, j - 2, k)) / hhz;
         else
             temp = temp + (PV(i, j + 1, k) - 2.0 * PV(i, j, k) + PV(i, j - 1, k)) / hhz;
     }
@@ -1189,83 +1503,105 @@ __device__ __forceinline__ double r3_resid(const R3Lev &L, const R3Work &W, int 
 #undef RF
 
 struct SolveCtx {
-    int m;              // residual evaluations so far (selects the max slot)
+    int m;              // level-1 residual evaluations so far (selects the max slot)
 };
 
-// One relaxation call relax<COMP>(nrel, klev); returns false when a grid
-// barrier timed out.
-template <int COMP>
-__device__ bool r3_relax(const R3Dev &d, int klev, SolveCtx &cx, double *sm)
+// relax's line sweeps on level klev, whose first phase the barrier before has
+// prepared; the barrier after each phase prepares the next.
+template <int COMP, class T> __device__ __noinline__ bool r3_sweeps(const R3Dev &d, int klev)
 {
-    const R3Lev &L = d.lev[klev];
-    const R3Work &W = d.work[COMP][klev];
+    const R3Lev &L = r3_shared().lev[klev];
+    const GridSync gs = d.gs[COMP];
+    const int nrel = d.nrel;
+    for (int irel = 1; irel <= nrel; ++irel)
+        for (int dir = 0; dir < 3; ++dir) {
+            const int nph = L.nphase[COMP][dir];
+            for (int ph = 0; ph < nph; ++ph) {
+                r3_phase<COMP, T>(klev, dir);
+                const int nd = ph + 1 < nph ? dir : dir < 2 ? dir + 1 : 0, np = ph + 1 < nph ? ph + 1 : 0;
+                const bool more = nd > dir || np > 0 || irel < nrel;
+                if (!grid_sync(gs, [&] {
+                        if (more) r3_prepare<COMP, T>(klev, nd, np);
+                    })) {
+                    async_copy_wait();
+                    return false;
+                }
+            }
+        }
+    return true;
+}
+
+// One relaxation call relax<COMP>(nrel, klev); returns false when a grid
+// barrier timed out.  The reference forms the residual after every sweep; it
+// is read where a restriction follows (`residual`) and its norm on level 1.
+template <int COMP>
+__device__ bool r3_relax(const R3Dev &d, int klev, SolveCtx &cx, bool residual)
+{
+    if (!r3_sweeps<COMP, double>(d, klev)) return false;
+    if (!residual && klev != 1) return true;
+    const R3Lev &L = r3_shared().lev[klev];
+    const R3Work &W = r3_shared().work[klev];
     const GridSync &gs = d.gs[COMP];
     unsigned long long *resmax = d.resmax + 2 * COMP;
     int *nanflag = d.nanflag + 2 * COMP;
-    const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long T = (long long)gridDim.x * blockDim.x;
+    const int gt = blockIdx.x * blockDim.x + threadIdx.x, T = gridDim.x * blockDim.x;
     const int im = r3_imax(COMP, L.n1), jm = r3_jmax(COMP, L.n2), n3 = L.n3;
-    for (int irel = 1; irel <= d.nrel; ++irel) {
-        for (int dir = 0; dir < 3; ++dir) {
-            const int *lines = L.lines[COMP][dir];
-            const int *off = L.poff[COMP][dir];
-            for (int ph = 0; ph < L.nphase[COMP][dir]; ++ph) {
-                r3_phase<COMP>(L, W, dir, lines, off[ph], off[ph + 1], sm);
-                if (!grid_sync(gs)) return false;
-            }
-        }
-        // residual and its max norm into slot m & 1; the other slot is
-        // cleared for the next evaluation (nobody reads it before then)
-        const int slot = cx.m & 1;
-        if (gt == 0) {
-            resmax[slot ^ 1] = 0ull;
-            nanflag[slot ^ 1] = 0;
-        }
-        const long long npts = (long long)im * jm * n3;
-        double lmax = 0.0;
-        int lnan = 0;
-        for (long long t = gt; t < npts; t += T) {
-            const int i = 1 + (int)(t % im);
-            const long long rest = t / im;
-            const int j = 1 + (int)(rest % jm);
-            const int k = 1 + (int)(rest / jm);
-            const double r = r3_resid<COMP>(L, W, i, j, k);
-            W.res[(size_t)i + (size_t)L.L1 * ((size_t)j + (size_t)L.L2 * (size_t)k)] = r;
-            const double a = fabs(r);
-            if (a != a) lnan = 1;
-            if (a > lmax) lmax = a;
-        }
+    // its max norm goes into slot m & 1; the other slot is cleared for the
+    // next evaluation (nobody reads it before then)
+    const int slot = cx.m & 1;
+    if (klev == 1 && gt == 0) {
+        resmax[slot ^ 1] = 0ull;
+        nanflag[slot ^ 1] = 0;
+    }
+    const int npts = im * jm * n3;
+    const RowSplit si(im), sj(jm);
+    unsigned long long lmax = 0;   // bit patterns of non-negative doubles are ordered as they are
+    int lnan = 0;
+    for (int t = gt; t < npts; t += T) {
+        int i, j, k, rest;
+        si(t, rest, i);
+        sj(rest, k, j);
+        ++i;
+        ++j;
+        ++k;
+        const double r = r3_resid<COMP>(L, W, i, j, k);
+        W.res[(size_t)i + (size_t)L.L1 * ((size_t)j + (size_t)L.L2 * (size_t)k)] = r;
+        const unsigned long long a = (unsigned long long)__double_as_longlong(r) & 0x7fffffffffffffffull;
+        if (a > 0x7ff0000000000000ull) lnan = 1;
+        else if (a > lmax) lmax = a;
+    }
+    if (klev == 1) {
         for (int o = 16; o > 0; o >>= 1) {
-            lmax = fmax(lmax, __shfl_xor_sync(0xffffffffu, lmax, o));
+            const unsigned long long v = __shfl_xor_sync(0xffffffffu, lmax, o);
+            lmax = v > lmax ? v : lmax;
             lnan |= __shfl_xor_sync(0xffffffffu, lnan, o);
         }
         if ((threadIdx.x & 31) == 0) {
-            if (lmax > 0.0) atomicMax(&resmax[slot], (unsigned long long)__double_as_longlong(lmax));
+            if (lmax) atomicMax(&resmax[slot], lmax);
             if (lnan) atomicOr(&nanflag[slot], 1);
         }
         cx.m++;
-        if (!grid_sync(gs)) return false;
     }
-    return true;
+    return grid_sync(gs);
 }
 
 // corser (rot3dmg.f:2176-2265): coarse right-hand side and zero correction.
 __device__ void r3_corser(const R3Dev &d, int comp, int klev)
 {
-    const R3Lev &F = d.lev[klev], &Cl = d.lev[klev + 1];
-    const R3Work &FW = d.work[comp][klev], &CW = d.work[comp][klev + 1];
+    const R3Lev &F = r3_shared().lev[klev], &Cl = r3_shared().lev[klev + 1];
+    const R3Work &FW = r3_shared().work[klev], &CW = r3_shared().work[klev + 1];
     const int n1c = Cl.n1, n2c = Cl.n2, n3c = Cl.n3;
-    const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long T = (long long)gridDim.x * blockDim.x;
-    const long long npts = (long long)Cl.L1 * Cl.L2 * (n3c + 1);
+    const int gt = blockIdx.x * blockDim.x + threadIdx.x;
+    const int T = gridDim.x * blockDim.x;
+    const int npts = Cl.L1 * Cl.L2 * (n3c + 1);
+    const RowSplit si(Cl.L1), sj(Cl.L2);
     const double *rf = FW.res;
     const size_t F1 = (size_t)F.L1, F2 = (size_t)F.L2;
 #define R(i, j, k) rf[(size_t)(i) + F1 * ((size_t)(j) + F2 * (size_t)(k))]
-    for (long long t = gt; t < npts; t += T) {
-        const int i = (int)(t % Cl.L1);
-        const long long rest = t / Cl.L1;
-        const int j = (int)(rest % Cl.L2);
-        const int k = (int)(rest / Cl.L2);
+    for (int t = gt; t < npts; t += T) {
+        int i, j, k, rest;
+        si(t, rest, i);
+        sj(rest, k, j);
         double val;
         if (i == 0 || i == n1c || j == 0 || j == n2c) {
             val = 0.0;
@@ -1294,19 +1630,19 @@ __device__ void r3_corser(const R3Dev &d, int comp, int klev)
 // level.  The coarse correction is cleared by the next corser.
 __device__ void r3_finer(const R3Dev &d, int comp, int klev)
 {
-    const R3Lev &Cl = d.lev[klev], &F = d.lev[klev - 1];
-    const R3Work &CW = d.work[comp][klev], &FW = d.work[comp][klev - 1];
-    const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long T = (long long)gridDim.x * blockDim.x;
-    const long long npts = (long long)F.L1 * F.L2 * (F.n3 + 1);
+    const R3Lev &Cl = r3_shared().lev[klev], &F = r3_shared().lev[klev - 1];
+    const R3Work &CW = r3_shared().work[klev], &FW = r3_shared().work[klev - 1];
+    const int gt = blockIdx.x * blockDim.x + threadIdx.x;
+    const int T = gridDim.x * blockDim.x;
+    const int npts = F.L1 * F.L2 * (F.n3 + 1);
+    const RowSplit si(F.L1), sj(F.L2);
     const double *pc = CW.v;
     const size_t C1 = (size_t)Cl.L1, C2 = (size_t)Cl.L2;
 #define PC(i, j, k) pc[(size_t)(i) + C1 * ((size_t)(j) + C2 * (size_t)(k))]
-    for (long long t = gt; t < npts; t += T) {
-        const int i = (int)(t % F.L1);
-        const long long rest = t / F.L1;
-        const int j = (int)(rest % F.L2);
-        const int k = (int)(rest / F.L2);
+    for (int t = gt; t < npts; t += T) {
+        int i, j, k, rest;
+        si(t, rest, i);
+        sj(rest, k, j);
         const int i1 = i / 2, j1 = j / 2, k1 = k / 2;
         const bool ie = i1 * 2 == i, je = j1 * 2 == j, ke = k1 * 2 == k;
         double p;
@@ -1341,54 +1677,60 @@ __device__ void r3_finer(const R3Dev &d, int comp, int klev)
 template <int COMP>
 __global__ void __launch_bounds__(R3_THREADS, 2) k_r3d_solve(const __grid_constant__ R3Dev d, int step)
 {
-    __shared__ double sm[R3_SMEM_DOUBLES];
     if (*(volatile int *)d.abort) return;
     const int ni = d.ni, nj = d.nj;
-    const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long T = (long long)gridDim.x * blockDim.x;
+    const int gt = blockIdx.x * blockDim.x + threadIdx.x, T = gridDim.x * blockDim.x;
+    r3_descriptors(d, COMP, false);
     double *psi = d.fld[COMP == 1 ? GB_R_wel : COMP == 2 ? GB_R_vel : GB_R_uel];
     double *psip = d.fld[COMP == 1 ? GB_R_welp : COMP == 2 ? GB_R_velp : GB_R_uelp];
     const double *rhs = d.fld[COMP == 1 ? GB_R_wrh : COMP == 2 ? GB_R_vrh : GB_R_urh];
-    const R3Lev &L = d.lev[1];
-    const R3Work &W = d.work[COMP][1];
-    const GridSync &gs = d.gs[COMP];
-    const long long n1p = L.L1, n2p = L.L2;
-    const long long nlvl = n1p * n2p * (L.n3 + 1);
-    for (long long t = gt; t < nlvl; t += T) {
-        const int i = (int)(t % n1p);
-        const long long rest = t / n1p;
-        const int j = (int)(rest % n2p);
-        const int k = (int)(rest / n2p);
+    const R3Lev &L = r3_shared().lev[1];
+    const R3Work W = r3_shared().work[1];
+    const GridSync gs = d.gs[COMP];
+    const int n1p = L.L1, n2p = L.L2;
+    const int nlvl = n1p * n2p * (L.n3 + 1);
+    const RowSplit si(n1p), sj(n2p);
+    // a barrier that prepares the first line phase of level l
+    auto sync_before = [&](int l) {
+        const bool ok = grid_sync(gs, [&] { r3_prepare<COMP, double>(l, 0, 0); });
+        if (!ok) async_copy_wait();   // no copy in flight outlives the block
+        return ok;
+    };
+    for (int t = gt; t < nlvl; t += T) {
+        int i, j, k, rest;
+        si(t, rest, i);
+        sj(rest, k, j);
         W.f[t] = FX(rhs, i, j, k);
         W.v[t] = 2.0 * FX(psi, i, j, k) - FX(psip, i, j, k);
     }
-    if (!grid_sync(gs)) return;
+    if (!sync_before(1)) return;
     SolveCtx cx;
     cx.m = 0;
     int status = GB_MAXSWEEPS, sweeps = d.maxsweeps;
     const int nlev = d.nlev;
     for (int sweep = 1; sweep <= d.maxsweeps; ++sweep) {
         if (sweep != 1 && !d.horizontal) {
-            for (long long t = gt; t < nlvl; t += T) {
-                const int i = (int)(t % n1p);
-                const long long rest = t / n1p;
-                const int j = (int)(rest % n2p);
-                const int k = (int)(rest / n2p);
+            for (int t = gt; t < nlvl; t += T) {
+                int i, j, k, rest;
+                si(t, rest, i);
+                sj(rest, k, j);
                 const double pp = FX(psip, i, j, k);
                 const double nv = pp + d.sor * (W.v[t] - pp);
                 W.v[t] = nv;
                 FX(psip, i, j, k) = nv;
             }
-            if (!grid_sync(gs)) return;
+            // with one level a relaxation of level 1 follows, else a restriction
+            if (!(nlev == 1 ? sync_before(1) : grid_sync(gs))) return;
+        } else if (sweep != 1 && nlev == 1) {
+            if (!sync_before(1)) return;
         }
         if (sweep == 1 || nlev == 1) {
-            if (!r3_relax<COMP>(d, 1, cx, sm)) return;
+            if (!r3_relax<COMP>(d, 1, cx, true)) return;
             if (!d.horizontal) {
-                for (long long t = gt; t < nlvl; t += T) {
-                    const int i = (int)(t % n1p);
-                    const long long rest = t / n1p;
-                    const int j = (int)(rest % n2p);
-                    const int k = (int)(rest / n2p);
+                for (int t = gt; t < nlvl; t += T) {
+                    int i, j, k, rest;
+                    si(t, rest, i);
+                    sj(rest, k, j);
                     FX(psip, i, j, k) = W.v[t];
                 }
                 if (!grid_sync(gs)) return;
@@ -1397,13 +1739,13 @@ __global__ void __launch_bounds__(R3_THREADS, 2) k_r3d_solve(const __grid_consta
         if (nlev > 1) {
             for (int l = 1; l <= nlev - 1; ++l) {
                 r3_corser(d, COMP, l);
-                if (!grid_sync(gs)) return;
-                if (!r3_relax<COMP>(d, l + 1, cx, sm)) return;
+                if (!sync_before(l + 1)) return;
+                if (!r3_relax<COMP>(d, l + 1, cx, l + 1 < nlev)) return;
             }
             for (int l = nlev; l >= 2; --l) {
                 r3_finer(d, COMP, l);
-                if (!grid_sync(gs)) return;
-                if (!r3_relax<COMP>(d, l - 1, cx, sm)) return;
+                if (!sync_before(l - 1)) return;
+                if (!r3_relax<COMP>(d, l - 1, cx, false)) return;
             }
         }
         const int slot = (cx.m - 1) & 1;
@@ -1425,12 +1767,12 @@ __global__ void __launch_bounds__(R3_THREADS, 2) k_r3d_solve(const __grid_consta
         const int jmax = COMP == 1 ? d.nz : d.nz + 1;
         const int ii1 = COMP == 3 ? d.nr - 1 : d.nr;
         const int jj1 = COMP == 1 ? d.nz - 1 : d.nz;
-        const long long npts = (long long)(imax + 1) * (jmax + 1) * (d.np + 1);
-        for (long long t = gt; t < npts; t += T) {
-            const int i = (int)(t % (imax + 1));
-            const long long rest = t / (imax + 1);
-            const int j = (int)(rest % (jmax + 1));
-            const int k = (int)(rest / (jmax + 1));
+        const int npts = (imax + 1) * (jmax + 1) * (d.np + 1);
+        const RowSplit ti(imax + 1), tj(jmax + 1);
+        for (int t = gt; t < npts; t += T) {
+            int i, j, k, rest;
+            ti(t, rest, i);
+            tj(rest, k, j);
             const double old = FX(psi, i, j, k);
             FX(psip, i, j, k) = old;
             const bool inner = i >= 1 && i <= ii1 && j >= 1 && j <= jj1;
@@ -1453,8 +1795,8 @@ __global__ void __launch_bounds__(R3_THREADS, 2) k_r3d_solve(const __grid_consta
 // stored as reciprocals.
 // ---------------------------------------------------------------------------
 
-// FP32 copies of the factor tables (one thread per line class).
-__global__ void k_r3d_factors32(const __grid_constant__ R3Dev d, const FacJob *jobs, int njobs, float *const *dst)
+// FP32 folded tables (one thread per line class).
+__global__ void k_r3d_factors32(const __grid_constant__ R3Dev d, const FacJob *jobs, int njobs)
 {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= njobs) return;
@@ -1462,293 +1804,211 @@ __global__ void k_r3d_factors32(const __grid_constant__ R3Dev d, const FacJob *j
     const R3Lev &L = d.lev[J.lev];
     const int kind = r3_kind(J.comp, J.dir);
     const int n = r3_len(J.comp, J.dir, L.n1, L.n2, L.n3);
-    const double *T = J.tab;
-    float *o = dst[q];
-    const int m = r3_tabsize(kind, n);
-    for (int t = 0; t < m; ++t) o[t] = (float)T[t];
-    if (kind == 0)
-        for (int t = 0; t < n; ++t) o[t] = (float)(1.0 / T[t]);            // divisors c(k)
-    else
-        for (int t = 0; t < n; ++t) o[n + t] = (float)(1.0 / T[n + t]);    // eliminated diagonal b
-}
-
-#define PV(i, j, k) v[(size_t)(i) + (size_t)L1 * ((size_t)(j) + (size_t)L2 * (size_t)(k))]
-#define RF(i, j, k) f[(size_t)(i) + (size_t)L1 * ((size_t)(j) + (size_t)L2 * (size_t)(k))]
-
-template <int COMP>
-__device__ __forceinline__ float r3_rhs32(const R3Lev &L, const R3Work &W, int dir, int p, int q, int e)
-{
-    const int n1 = L.n1, n2 = L.n2, n3 = L.n3, L1 = L.L1, L2 = L.L2;
-    const float ihr = L.ihr, ihhr = L.ihhr, ihhz = L.ihhz, ihhp = L.ihhp;
-    const float c53 = 5.0f / 3.0f, c43 = 4.0f / 3.0f;
-    const float *v = W.v32, *f = W.f32;
-    if (dir == 0) {
-        const int i = e + 1, j = p, k = q;
-        const int ka = k == n3 ? 1 : k + 1, km = k - 1;
-        const float iq = COMP == 3 ? L.iqv[i] : L.iqc[i];
-        const float ph = (PV(i, j, ka) + PV(i, j, km)) * ihhp * iq;
-        float zz;
-        if (COMP == 1) zz = (PV(i, j + 1, k) + PV(i, j - 1, k)) * ihhz;
-        else if (j == 1) zz = (c53 * PV(i, j + 1, k) - 0.2f * PV(i, j + 2, k)) * ihhz;
-        else if (j == n2) zz = (c53 * PV(i, j - 1, k) - 0.2f * PV(i, j - 2, k)) * ihhz;
-        else zz = (PV(i, j - 1, k) + PV(i, j + 1, k)) * ihhz;
-        return RF(i, j, k) - zz - ph;
-    } else if (dir == 1) {
-        const int i = p, j = e + 1, k = q;
-        const int ka = k == n3 ? 1 : k + 1, km = k - 1;
-        const float iq = COMP == 3 ? L.iqv[i] : L.iqc[i];
-        const float ir = COMP == 3 ? L.irv[i] : L.irc[i];
-        const float ph = (PV(i, j, ka) + PV(i, j, km)) * ihhp * iq;
-        float rr;
-        if (COMP == 1) {
-            if (i == 1) rr = -(c53 * PV(i + 1, j, k) - 0.2f * PV(i + 2, j, k)) * ihhr - 0.5f * PV(i + 1, j, k) * ihr * ir;
-            else if (i == n1) rr = -(c53 * PV(i - 1, j, k) - 0.2f * PV(i - 2, j, k)) * ihhr + 0.5f * PV(i - 1, j, k) * ihr * ir;
-            else rr = -(PV(i + 1, j, k) + PV(i - 1, j, k)) * ihhr - 0.5f * (PV(i + 1, j, k) - PV(i - 1, j, k)) * ihr * ir;
-        } else if (COMP == 2) {
-            if (i == 1) rr = -(c53 * PV(i + 1, j, k) - 0.2f * PV(i + 2, j, k)) * ihhr - c43 * PV(i + 1, j, k) * ihr * ir;
-            else if (i == n1) rr = -(c53 * PV(i - 1, j, k) - 0.2f * PV(i - 2, j, k)) * ihhr + c43 * PV(i - 1, j, k) * ihr * ir;
-            else rr = -(PV(i + 1, j, k) + PV(i - 1, j, k)) * ihhr - 1.5f * (PV(i + 1, j, k) - PV(i - 1, j, k)) * ihr * ir;
-        } else {
-            rr = -(PV(i + 1, j, k) + PV(i - 1, j, k)) * ihhr - 1.5f * (PV(i + 1, j, k) - PV(i - 1, j, k)) * ihr * ir;
-        }
-        return rr - ph + RF(i, j, k);
-    } else {
-        const int i = p, j = q, k = e + 1;
-        const float ir = COMP == 3 ? L.irv[i] : L.irc[i];
-        float rr;
-        if (COMP == 1) {
-            if (i == 1) rr = -(c53 * PV(i + 1, j, k) - 0.2f * PV(i + 2, j, k)) * ihhr - 0.5f * PV(i + 1, j, k) * ihr * ir;
-            else if (i == n1) rr = -(c53 * PV(i - 1, j, k) - 0.2f * PV(i - 2, j, k)) * ihhr + 0.5f * PV(i - 1, j, k) * ihr * ir;
-            else rr = -(PV(i + 1, j, k) + PV(i - 1, j, k)) * ihhr - 0.5f * (PV(i + 1, j, k) - PV(i - 1, j, k)) * ihr * ir;
-        } else if (COMP == 2) {
-            if (i == 1) rr = -(c53 * PV(i + 1, j, k) - 0.2f * PV(i + 2, j, k)) * ihhr - c43 * PV(i + 1, j, k) * ihr * ir;
-            else if (i == n1) rr = -(c53 * PV(i - 1, j, k) - 0.2f * PV(i - 2, j, k)) * ihhr + c43 * PV(i - 1, j, k) * ihr * ir;
-            else rr = -(PV(i + 1, j, k) + PV(i - 1, j, k)) * ihhr - 1.5f * (PV(i + 1, j, k) - PV(i - 1, j, k)) * ihr * ir;
-        } else {
-            rr = -(PV(i + 1, j, k) + PV(i - 1, j, k)) * ihhr - 1.5f * (PV(i + 1, j, k) - PV(i - 1, j, k)) * ihr * ir;
-        }
-        float zz;
-        if (COMP == 1) zz = (PV(i, j + 1, k) + PV(i, j - 1, k)) * ihhz;
-        else if (j == 1) zz = (c53 * PV(i, j + 1, k) - 0.2f * PV(i, j + 2, k)) * ihhz;
-        else if (j == n2) zz = (c53 * PV(i, j - 1, k) - 0.2f * PV(i, j - 2, k)) * ihhz;
-        else zz = (PV(i, j - 1, k) + PV(i, j + 1, k)) * ihhz;
-        return rr - zz + RF(i, j, k);
-    }
-}
-
-// FP32 residual (only where a restriction follows).
-template <int COMP>
-__device__ __forceinline__ float r3_resid32(const R3Lev &L, const R3Work &W, int i, int j, int k)
-{
-    const int n1 = L.n1, n2 = L.n2, n3 = L.n3, L1 = L.L1, L2 = L.L2;
-    const float ihr = L.ihr, ihhr = L.ihhr, ihhz = L.ihhz, ihhp = L.ihhp;
-    const float c53 = 5.0f / 3.0f, c43 = 4.0f / 3.0f;
-    const float *v = W.v32, *f = W.f32;
-    const int ka = k == n3 ? 1 : k + 1, km = k - 1;
-    const float p0 = PV(i, j, k);
-    const float iq = COMP == 3 ? L.iqv[i] : L.iqc[i];
-    const float ir = COMP == 3 ? L.irv[i] : L.irc[i];
-    float t = (PV(i, j, ka) - 2.0f * p0 + PV(i, j, km)) * ihhp * iq;
-    if (COMP == 1) {
-        t += (PV(i, j + 1, k) - 2.0f * p0 + PV(i, j - 1, k)) * ihhz;
-        if (i == 1) t += (-2.0f * p0 + c53 * PV(i + 1, j, k) - 0.2f * PV(i + 2, j, k)) * ihhr + 0.5f * (PV(i + 1, j, k) - p0) * ihr * ir;
-        else if (i == n1) t += (-2.0f * p0 + c53 * PV(i - 1, j, k) - 0.2f * PV(i - 2, j, k)) * ihhr + 0.5f * (p0 - PV(i - 1, j, k)) * ihr * ir;
-        else t += (PV(i - 1, j, k) - 2.0f * p0 + PV(i + 1, j, k)) * ihhr + 0.5f * (PV(i + 1, j, k) - PV(i - 1, j, k)) * ihr * ir;
-    } else {
-        t += p0 * iq;
-        if (COMP == 2) {
-            if (i == 1) t += (-2.0f * p0 + c53 * PV(i + 1, j, k) - 0.2f * PV(i + 2, j, k)) * ihhr + c43 * PV(i + 1, j, k) * ihr * ir;
-            else if (i == n1) t += (-2.0f * p0 + c53 * PV(i - 1, j, k) - 0.2f * PV(i - 2, j, k)) * ihhr - c43 * PV(i - 1, j, k) * ihr * ir;
-            else t += (PV(i - 1, j, k) - 2.0f * p0 + PV(i + 1, j, k)) * ihhr + 1.5f * (PV(i + 1, j, k) - PV(i - 1, j, k)) * ihr * ir;
-        } else {
-            t += (PV(i - 1, j, k) - 2.0f * p0 + PV(i + 1, j, k)) * ihhr + 1.5f * (PV(i + 1, j, k) - PV(i - 1, j, k)) * ihr * ir;
-        }
-        if (j == 1) t += (-2.0f * p0 + c53 * PV(i, j + 1, k) - 0.2f * PV(i, j + 2, k)) * ihhz;
-        else if (j == n2) t += (-2.0f * p0 + c53 * PV(i, j - 1, k) - 0.2f * PV(i, j - 2, k)) * ihhz;
-        else t += (PV(i, j + 1, k) - 2.0f * p0 + PV(i, j - 1, k)) * ihhz;
-    }
-    return RF(i, j, k) - t;
-}
-
-#undef PV
-#undef RF
-
-template <int COMP>
-__device__ void r3_line32(const R3Lev &L, const R3Work &W, int dir, int p, int q, float *s)
-{
-    const int n1 = L.n1, n2 = L.n2, n3 = L.n3, L1 = L.L1, L2 = L.L2;
-    const int kind = r3_kind(COMP, dir);
-    const int n = r3_len(COMP, dir, n1, n2, n3);
-    float *v = W.v32;
-    size_t base;
-    long long step;
-    if (dir == 0) {
-        base = (size_t)1 + (size_t)L1 * ((size_t)p + (size_t)L2 * (size_t)q);
-        step = 1;
-    } else if (dir == 1) {
-        base = (size_t)p + (size_t)L1 * ((size_t)1 + (size_t)L2 * (size_t)q);
-        step = L1;
-    } else {
-        base = (size_t)p + (size_t)L1 * ((size_t)q + (size_t)L2);
-        step = (long long)L1 * L2;
-    }
-    const long long plane = (long long)L1 * L2 * n3;
-    const bool seam = dir != 2 && q == n3;
-    const float *T = L.fac32[COMP][dir];
-    if (dir != 0) T += (size_t)(p - 1) * r3_tabsize(kind, n);
-#define PUT(e, x)                                                                     \
-    do {                                                                              \
-        const float _x = (x);                                                         \
-        v[base + (size_t)((long long)(e) * step)] = _x;                               \
-        if (seam) v[base + (size_t)((long long)(e) * step) - plane] = _x;             \
-    } while (0)
+    float *o = L.fac32[J.comp][J.dir] + (size_t)(J.dir == 0 ? 0 : J.ti - 1) * r3_tabsize32(kind, n);
     if (kind == 0) {
-        const float *Ci = T, *Bb = T + n, *Aa = T + 2 * n, *Dd = T + 3 * n, *Ee = T + 4 * n;
-        float r0 = s[0], r1 = s[1];
-#pragma unroll 4
-        for (int k = 0; k <= n - 2; ++k) {
-            const float rk = r0 * Ci[k];
-            s[k] = rk;
-            const float rk1 = __fmaf_rn(-Bb[k + 1], rk, r1);
-            float rk2 = 0.f;
-            if (k != n - 2) rk2 = __fmaf_rn(-Aa[k + 2], rk, s[k + 2]);
-            r0 = rk1;
-            r1 = rk2;
-        }
-        float x1 = r0 * Ci[n - 1];
-        PUT(n - 1, x1);
-        float x0 = __fmaf_rn(-Dd[n - 2], x1, s[n - 2]);
-        PUT(n - 2, x0);
-        float x2 = x1;
-        x1 = x0;
-#pragma unroll 4
-        for (int j = n - 3; j >= 0; --j) {
-            const float x = __fmaf_rn(-Ee[j], x2, __fmaf_rn(-Dd[j], x1, s[j]));
-            PUT(j, x);
-            x2 = x1;
-            x1 = x;
-        }
+        pdma32_fold(J.tab, n, o);
     } else if (kind == 1) {
-        const float *F = T, *Bi = T + n, *Cc = T + 2 * n;
-        float rprev = s[0];
-#pragma unroll 4
-        for (int j = 1; j < n; ++j) {
-            const float rj = __fmaf_rn(-F[j], rprev, s[j]);
-            s[j] = rj;
-            rprev = rj;
-        }
-        float y = rprev * Bi[n - 1];
-        PUT(n - 1, y);
-#pragma unroll 4
-        for (int j = n - 2; j >= 0; --j) {
-            y = __fmaf_rn(-Cc[j], y, s[j]) * Bi[j];
-            PUT(j, y);
-        }
+        tdma32_fold(J.tab, n, o);
     } else {
-        const float *Aa = T, *Bi = T + n, *Cc = T + 2 * n, *F1 = T + 3 * n, *F2 = T + 4 * n, *F3 = T + 5 * n;
-        const int N = n - 1;
-        float rN = s[N];
-        float rprev = s[0];
-#pragma unroll 4
-        for (int j = 1; j <= n - 3; ++j) {
-            const float rj = __fmaf_rn(-F1[j], rprev, s[j]);
-            rN = __fmaf_rn(-F2[j], rprev, rN);
-            s[j] = rj;
-            rprev = rj;
+        double a, b, c, dd, ee;
+        r3_coef(L, J.comp, J.dir, J.ti, 0, a, b, c, dd, ee);
+        const double h = -b / (2.0 * a);
+        if (!(h > 1.0 + 1e-9)) {
+            *(R3Ring *)o = R3Ring{0.f, 0.f, 0.f, 0};
+            return;
         }
-        const float rn2 = __fmaf_rn(-F1[n - 2], rprev, s[n - 2]);
-        rN = __fmaf_rn(-F2[n - 2], rprev, rN);
-        rN = __fmaf_rn(-F3[0], rn2, rN);
-        const float yN = rN * Bi[N];
-        PUT(N, yN);
-        float y = __fmaf_rn(-Cc[n - 2], yN, rn2) * Bi[n - 2];
-        PUT(n - 2, y);
-#pragma unroll 4
-        for (int j = n - 3; j >= 0; --j) {
-            y = __fmaf_rn(-Aa[j], yN, __fmaf_rn(-Cc[j], y, s[j])) * Bi[j];
-            PUT(j, y);
-        }
-        v[base - (size_t)step] = yN;
+        const double rho = 1.0 / (h + sqrt(h * h - 1.0)), turn = pow(rho, (double)n);
+        int steps = 0;
+        const int lw = wl_log2w(n), M = 1 << wl_log2m(n);
+        while (steps < lw && pow(rho, (double)(M << steps)) > 9.313226e-10) ++steps;
+        *(R3Ring *)o = R3Ring{(float)rho, (float)(-rho / a), (float)(1.0 / (1.0 - turn)), steps};
     }
-#undef PUT
 }
 
-template <int COMP>
-__device__ void r3_phase32(const R3Lev &L, const R3Work &W, int dir, const int *lines, int a, int b, float *sm)
+// One scan-step count per level, component and direction (block x: level,
+// y: component, z: direction 1 or 2).
+__global__ void k_r3d_steps32(const __grid_constant__ R3Dev d)
 {
-    const int n = r3_len(COMP, dir, L.n1, L.n2, L.n3);
-    const int pitch = n | 1;
-    const int per = (b - a + (int)gridDim.x - 1) / (int)gridDim.x;
-    const int my0 = r3_group_start(lines, a, b, a + (int)blockIdx.x * per);
-    const int my1 = r3_group_start(lines, a, b, a + ((int)blockIdx.x + 1) * per);
-    const int chunk = max(1, min((int)blockDim.x, (2 * R3_SMEM_DOUBLES) / pitch));
-    for (int c0 = my0; c0 < my1;) {
-        const int c1 = r3_chunk_end(lines, c0, min(my1, c0 + chunk));
-        const int nl = c1 - c0;
-        for (int t = threadIdx.x; t < nl * n; t += blockDim.x) {
-            const int li = t / n, e = t - li * n;
-            const int pk = lines[c0 + li] & 0x7fffffff;
-            sm[li * pitch + e] = r3_rhs32<COMP>(L, W, dir, pk & 0xffff, pk >> 16, e);
-        }
+    const R3Lev &L = d.lev[1 + blockIdx.x];
+    const int comp = 1 + blockIdx.y, dir = 1 + blockIdx.z;
+    const int kind = r3_kind(comp, dir), n = r3_len(comp, dir, L.n1, L.n2, L.n3), inst = r3_imax(comp, L.n1);
+    float *tab = L.fac32[comp][dir];
+    if (kind != 2) {
+        wl_common_steps(tab, r3_tabsize32(kind, n), inst);
+    } else {   // the count is a ring's fourth word
+        wl_common_steps(tab + 3, 4, inst);
+        __shared__ int weak;
+        if (threadIdx.x == 0) weak = 0;
         __syncthreads();
-        if ((int)threadIdx.x < nl) {
-            const int pk = lines[c0 + threadIdx.x] & 0x7fffffff;
-            r3_line32<COMP>(L, W, dir, pk & 0xffff, pk >> 16, sm + threadIdx.x * pitch);
-        }
+        R3Ring *ring = (R3Ring *)tab;
+        for (int q = threadIdx.x; q < inst; q += blockDim.x)
+            if (ring[q].scale == 0.f) weak = 1;
         __syncthreads();
-        c0 = c1;
+        if (weak)
+            for (int q = threadIdx.x; q < inst; q += blockDim.x) ring[q].steps = -1;
     }
+}
+
+// Matrix weights of row i in r and of row j in z, from relax's operator: the
+// references are those of r3_coef and r3_resid.
+__global__ void k_r3d_weights32(const __grid_constant__ R3Dev d)
+{
+    const R3Lev &L = d.lev[1 + blockIdx.x];
+    const int comp = 1 + blockIdx.y;
+    const double ihr = 1.0 / L.hr, ihhr = 1.0 / L.hhr, ihhz = 1.0 / L.hhz, ihhp = 1.0 / L.hhp;
+    for (int i = 1 + threadIdx.x; i <= L.n1; i += blockDim.x) {
+        const double r = comp == 3 ? L.rvv[i] : L.rvc[i], ir = 1.0 / r, iq = 1.0 / (r * r);
+        const double g = comp == 1 ? 0.5 : 1.5;
+        double m = ihhr - g * ihr * ir, p = ihhr + g * ihr * ir, f = 0.0, c = -2.0 * ihhr;
+        if (comp != 3 && (i == 1 || i == L.n1)) {
+            const double e = (comp == 1 ? 0.5 : 4.0 / 3.0) * ihr * ir, s = i == 1 ? 1.0 : -1.0;
+            m = i == 1 ? 0.0 : 5.0 / 3.0 * ihhr - e;
+            p = i == 1 ? 5.0 / 3.0 * ihhr + e : 0.0;
+            f = -0.2 * ihhr;
+            if (comp == 1) c -= s * e;
+        }
+        c -= 2.0 * ihhp * iq;
+        if (comp != 1) c += iq;
+        L.wi[comp][i] = make_float4((float)m, (float)p, (float)f, (float)c);
+        L.wp[comp][i] = (float)(ihhp * iq);
+    }
+    for (int j = 1 + threadIdx.x; j <= L.n2; j += blockDim.x) {
+        double m = ihhz, p = ihhz, f = 0.0;
+        if (comp != 1 && (j == 1 || j == L.n2)) {
+            m = j == 1 ? 0.0 : 5.0 / 3.0 * ihhz;
+            p = j == 1 ? 5.0 / 3.0 * ihhz : 0.0;
+            f = -0.2 * ihhz;
+        }
+        L.wj[comp][j] = make_float4((float)m, (float)p, (float)f, (float)(-2.0 * ihhz));
+    }
+}
+
+// A point's neighbours in FP32: right-hand side of its line in direction dir,
+// or the residual (dir 3).  Loads first, arithmetic after, so that a thread
+// has several points' loads in flight (r3_rhs32_batch).
+template <int COMP> struct R3Point {
+    float f, im, ip, ifar, jm, jp, jfar, ka, km, c;
+    float4 wi, wj;
+    float wp;
+    __device__ __forceinline__ void load(const R3Lev &L, const R3Work &W, int dir, int i, int j, int k)
+    {
+        const int L1 = L.L1, P = L1 * L.L2, n1 = L.n1, n2 = L.n2, n3 = L.n3;
+        const int o = i + L1 * j + P * k;
+        const float *v = W.v32 + o;
+        f = W.f32[o];
+        if (dir != 0) {
+            im = v[-1];
+            ip = v[1];
+            ifar = COMP != 3 ? v[i == 1 ? 2 : i == n1 ? -2 : 0] : 0.f;
+        }
+        if (dir != 1) {
+            jm = v[-L1];
+            jp = v[L1];
+            jfar = COMP != 1 ? v[j == 1 ? 2 * L1 : j == n2 ? -2 * L1 : 0] : 0.f;
+        }
+        if (dir != 2) {
+            km = v[-P];
+            ka = v[k == n3 ? P * (1 - n3) : P];
+        }
+        if (dir == 3) c = v[0];
+        wi = L.wi[COMP][i];
+        wj = L.wj[COMP][j];
+        wp = L.wp[COMP][i];
+    }
+    __device__ __forceinline__ float value(int dir) const
+    {
+        float r = f;
+        if (dir != 0) {
+            r = __fmaf_rn(-wi.x, im, __fmaf_rn(-wi.y, ip, r));
+            if (COMP != 3) r = __fmaf_rn(-wi.z, ifar, r);
+        }
+        if (dir != 1) {
+            r = __fmaf_rn(-wj.x, jm, __fmaf_rn(-wj.y, jp, r));
+            if (COMP != 1) r = __fmaf_rn(-wj.z, jfar, r);
+        }
+        if (dir != 2) r = __fmaf_rn(-wp, ka + km, r);
+        if (dir == 3) r = __fmaf_rn(-(wi.w + wj.w), c, r);
+        return r;
+    }
+};
+
+
+// The right-hand sides of a chunk's lines, four points per thread in flight.
+template <int COMP>
+__device__ __forceinline__ void r3_rhs32_batch(const R3Lev &L, const R3Work &W, int dir, const int *s_line, int nl, int n,
+                                               const RowSplit &split, float *x, int lpitch, int lg)
+{
+    constexpr int U = 4;
+    auto run = [&](auto d) {
+        constexpr int DIR = decltype(d)::value;
+        for (int base = threadIdx.x; base < nl * n; base += U * R3_THREADS) {
+            R3Point<COMP> pt[U];
+            int slot[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int idx = min(base + u * R3_THREADS, nl * n - 1);   // a repeated point is not stored
+                int t, e;
+                if (DIR == 0) split(idx, t, e);
+                else split(idx, e, t);
+                const int p = s_line[t] & 0xffff, q = s_line[t] >> 16;
+                slot[u] = t * lpitch + wl_slot(lg, e);
+                pt[u].load(L, W, DIR, DIR == 0 ? e + 1 : p, DIR == 0 ? p : DIR == 1 ? e + 1 : q, DIR == 2 ? e + 1 : q);
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (base + u * R3_THREADS < nl * n) x[slot[u]] = pt[u].value(DIR);
+        }
+    };
+    if (dir == 0) run(std::integral_constant<int, 0>());
+    else if (dir == 1) run(std::integral_constant<int, 1>());
+    else run(std::integral_constant<int, 2>());
 }
 
 // relax in FP32; the residual only when a restriction follows.
 template <int COMP>
-__device__ bool r3_relax32(const R3Dev &d, int klev, bool residual, float *sm)
+__device__ bool r3_relax32(const R3Dev &d, int klev, bool residual)
 {
-    const R3Lev &L = d.lev[klev];
-    const R3Work &W = d.work[COMP][klev];
-    const GridSync &gs = d.gs[COMP];
-    const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long T = (long long)gridDim.x * blockDim.x;
-    const int im = r3_imax(COMP, L.n1), jm = r3_jmax(COMP, L.n2), n3 = L.n3;
-    for (int irel = 1; irel <= d.nrel; ++irel)
-        for (int dir = 0; dir < 3; ++dir) {
-            const int *lines = L.lines[COMP][dir];
-            const int *off = L.poff[COMP][dir];
-            for (int ph = 0; ph < L.nphase[COMP][dir]; ++ph) {
-                r3_phase32<COMP>(L, W, dir, lines, off[ph], off[ph + 1], sm);
-                if (!grid_sync(gs)) return false;
-            }
+    if (!r3_sweeps<COMP, float>(d, klev)) return false;
+    if (!residual) return true;
+    const R3Lev &L = r3_shared().lev[klev];
+    const R3Work &W = r3_shared().work[klev];
+    const int im = r3_imax(COMP, L.n1), jm = r3_jmax(COMP, L.n2), npts = im * jm * L.n3;
+    const RowSplit si(im), sj(jm);
+    const int T = gridDim.x * blockDim.x;
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < npts; t += 2 * T) {
+        R3Point<COMP> pt[2];
+        int o[2];
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            int i, j, k, rest;
+            si(min(t + u * T, npts - 1), rest, i);
+            sj(rest, k, j);
+            o[u] = i + 1 + L.L1 * (j + 1 + L.L2 * (k + 1));
+            pt[u].load(L, W, 3, i + 1, j + 1, k + 1);
         }
-    if (residual) {
-        const long long npts = (long long)im * jm * n3;
-        for (long long t = gt; t < npts; t += T) {
-            const int i = 1 + (int)(t % im);
-            const long long rest = t / im;
-            const int j = 1 + (int)(rest % jm);
-            const int k = 1 + (int)(rest / jm);
-            W.res32[(size_t)i + (size_t)L.L1 * ((size_t)j + (size_t)L.L2 * (size_t)k)] = r3_resid32<COMP>(L, W, i, j, k);
-        }
-        if (!grid_sync(gs)) return false;
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+            if (t + u * T < npts) W.res32[o[u]] = pt[u].value(3);
     }
-    return true;
+    return grid_sync(d.gs[COMP]);
 }
 
 __device__ void r3_corser32(const R3Dev &d, int comp, int klev)
 {
-    const R3Lev &F = d.lev[klev], &Cl = d.lev[klev + 1];
-    const R3Work &WF = d.work[comp][klev], &WC = d.work[comp][klev + 1];
+    const R3Lev &F = r3_shared().lev[klev], &Cl = r3_shared().lev[klev + 1];
+    const R3Work &WF = r3_shared().work[klev], &WC = r3_shared().work[klev + 1];
     const int n1c = Cl.n1, n2c = Cl.n2, n3c = Cl.n3;
-    const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long T = (long long)gridDim.x * blockDim.x;
-    const long long npts = (long long)Cl.L1 * Cl.L2 * (n3c + 1);
+    const int gt = blockIdx.x * blockDim.x + threadIdx.x;
+    const int T = gridDim.x * blockDim.x;
+    const int npts = Cl.L1 * Cl.L2 * (n3c + 1);
+    const RowSplit si(Cl.L1), sj(Cl.L2);
     const float *rf = WF.res32;
     const size_t F1 = (size_t)F.L1, F2 = (size_t)F.L2;
 #define R(i, j, k) rf[(size_t)(i) + F1 * ((size_t)(j) + F2 * (size_t)(k))]
-    for (long long t = gt; t < npts; t += T) {
-        const int i = (int)(t % Cl.L1);
-        const long long rest = t / Cl.L1;
-        const int j = (int)(rest % Cl.L2);
-        const int k = (int)(rest / Cl.L2);
+    for (int t = gt; t < npts; t += T) {
+        int i, j, k, rest;
+        si(t, rest, i);
+        sj(rest, k, j);
         float val;
         if (i == 0 || i == n1c || j == 0 || j == n2c) {
             val = 0.f;
@@ -1776,19 +2036,19 @@ __device__ void r3_corser32(const R3Dev &d, int comp, int klev)
 
 __device__ void r3_finer32(const R3Dev &d, int comp, int klev)
 {
-    const R3Lev &Cl = d.lev[klev], &F = d.lev[klev - 1];
-    const R3Work &WC = d.work[comp][klev], &WF = d.work[comp][klev - 1];
-    const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long T = (long long)gridDim.x * blockDim.x;
-    const long long npts = (long long)F.L1 * F.L2 * (F.n3 + 1);
+    const R3Lev &Cl = r3_shared().lev[klev], &F = r3_shared().lev[klev - 1];
+    const R3Work &WC = r3_shared().work[klev], &WF = r3_shared().work[klev - 1];
+    const int gt = blockIdx.x * blockDim.x + threadIdx.x;
+    const int T = gridDim.x * blockDim.x;
+    const int npts = F.L1 * F.L2 * (F.n3 + 1);
+    const RowSplit si(F.L1), sj(F.L2);
     const float *pc = WC.v32;
     const size_t C1 = (size_t)Cl.L1, C2 = (size_t)Cl.L2;
 #define PC(i, j, k) pc[(size_t)(i) + C1 * ((size_t)(j) + C2 * (size_t)(k))]
-    for (long long t = gt; t < npts; t += T) {
-        const int i = (int)(t % F.L1);
-        const long long rest = t / F.L1;
-        const int j = (int)(rest % F.L2);
-        const int k = (int)(rest / F.L2);
+    for (int t = gt; t < npts; t += T) {
+        int i, j, k, rest;
+        si(t, rest, i);
+        sj(rest, k, j);
         const int i1 = i >> 1, j1 = j >> 1, k1 = k >> 1;
         const int i2 = i1 + (i & 1), j2 = j1 + (j & 1), k2 = k1 + (k & 1);
         const float p = 0.125f * (PC(i1, j1, k1) + PC(i2, j1, k1) + PC(i1, j2, k1) + PC(i2, j2, k1) + PC(i1, j1, k2) +
@@ -1803,31 +2063,38 @@ __device__ void r3_finer32(const R3Dev &d, int comp, int klev)
 template <int COMP>
 __global__ void __launch_bounds__(R3_THREADS, 2) k_r3d_solve_mixed(const __grid_constant__ R3Dev d, int step)
 {
-    __shared__ float sm[2 * R3_SMEM_DOUBLES];
     if (*(volatile int *)d.abort) return;
     const int ni = d.ni, nj = d.nj;
-    const long long gt = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long T = (long long)gridDim.x * blockDim.x;
+    const int gt = blockIdx.x * blockDim.x + threadIdx.x, T = gridDim.x * blockDim.x;
+    r3_descriptors(d, COMP, true);
     double *psi = d.fld[COMP == 1 ? GB_R_wel : COMP == 2 ? GB_R_vel : GB_R_uel];
     double *psip = d.fld[COMP == 1 ? GB_R_welp : COMP == 2 ? GB_R_velp : GB_R_uelp];
     const double *rhs = d.fld[COMP == 1 ? GB_R_wrh : COMP == 2 ? GB_R_vrh : GB_R_urh];
-    const R3Lev &L = d.lev[1];
-    const R3Work &W = d.work[COMP][1];
-    const GridSync &gs = d.gs[COMP];
-    const long long n1p = L.L1, n2p = L.L2;
-    const long long nlvl = n1p * n2p * (L.n3 + 1);
-    for (long long t = gt; t < nlvl; t += T) {
-        const int i = (int)(t % n1p);
-        const long long rest = t / n1p;
-        const int j = (int)(rest % n2p);
-        const int k = (int)(rest / n2p);
+    const R3Lev &L = r3_shared().lev[1];
+    const R3Work W = r3_shared().work[1];
+    const GridSync gs = d.gs[COMP];
+    const int n1p = L.L1, n2p = L.L2;
+    const int nlvl = n1p * n2p * (L.n3 + 1);
+    const RowSplit si(n1p), sj(n2p);
+    // a barrier that prepares the first line phase of level l
+    auto sync_before = [&](int l) {
+        const bool ok = grid_sync(gs, [&] { r3_prepare<COMP, float>(l, 0, 0); });
+        if (!ok) async_copy_wait();   // no copy in flight outlives the block
+        return ok;
+    };
+    for (int t = gt; t < nlvl; t += T) {
+        int i, j, k, rest;
+        si(t, rest, i);
+        sj(rest, k, j);
         W.f[t] = FX(rhs, i, j, k);
         W.v[t] = 2.0 * FX(psi, i, j, k) - FX(psip, i, j, k);
         W.f32[t] = 0.f;
+        W.v32[t] = 0.f;
     }
     if (!grid_sync(gs)) return;
     const int im = r3_imax(COMP, L.n1), jm = r3_jmax(COMP, L.n2), n3 = L.n3;
-    const long long nunk = (long long)im * jm * n3;
+    const int nunk = im * jm * n3;
+    const RowSplit ui(im), uj(jm);
     int status = GB_MAXSWEEPS, cycles = d.maxsweeps, m = 0;
     const int nlev = d.nlev;
     for (int it = 0;; ++it) {
@@ -1837,29 +2104,32 @@ __global__ void __launch_bounds__(R3_THREADS, 2) k_r3d_solve_mixed(const __grid_
             d.resmax[2 * COMP + (slot ^ 1)] = 0ull;
             d.nanflag[2 * COMP + (slot ^ 1)] = 0;
         }
-        double lmax = 0.0;
+        unsigned long long lmax = 0;   // bit patterns of non-negative doubles are ordered as they are
         int lnan = 0;
-        for (long long t = gt; t < nunk; t += T) {
-            const int i = 1 + (int)(t % im);
-            const long long rest = t / im;
-            const int j = 1 + (int)(rest % jm);
-            const int k = 1 + (int)(rest / jm);
+        for (int t = gt; t < nunk; t += T) {
+            int i, j, k, rest;
+            ui(t, rest, i);
+            uj(rest, k, j);
+            ++i;
+            ++j;
+            ++k;
             const double r = r3_resid<COMP>(L, W, i, j, k);
-            W.f32[(size_t)i + (size_t)L.L1 * ((size_t)j + (size_t)L.L2 * (size_t)k)] = (float)r;
-            const double a = fabs(r);
-            if (a != a) lnan = 1;
-            if (a > lmax) lmax = a;
+            W.f32[(size_t)i + (size_t)L.L1 * ((size_t)j + (size_t)L.L2 * (size_t)k)] = d2f_rn(r);
+            const unsigned long long a = (unsigned long long)__double_as_longlong(r) & 0x7fffffffffffffffull;
+            if (a > 0x7ff0000000000000ull) lnan = 1;
+            else if (a > lmax) lmax = a;
         }
         for (int o = 16; o > 0; o >>= 1) {
-            lmax = fmax(lmax, __shfl_xor_sync(0xffffffffu, lmax, o));
+            const unsigned long long v = __shfl_xor_sync(0xffffffffu, lmax, o);
+            lmax = v > lmax ? v : lmax;
             lnan |= __shfl_xor_sync(0xffffffffu, lnan, o);
         }
         if ((threadIdx.x & 31) == 0) {
-            if (lmax > 0.0) atomicMax(&d.resmax[2 * COMP + slot], (unsigned long long)__double_as_longlong(lmax));
+            if (lmax) atomicMax(&d.resmax[2 * COMP + slot], lmax);
             if (lnan) atomicOr(&d.nanflag[2 * COMP + slot], 1);
         }
         ++m;
-        if (!grid_sync(gs)) return;
+        if (!sync_before(1)) return;
         const double res = __longlong_as_double((long long)*(volatile unsigned long long *)&d.resmax[2 * COMP + slot]);
         if (*(volatile int *)&d.nanflag[2 * COMP + slot]) {
             status = GB_NAN;
@@ -1872,35 +2142,37 @@ __global__ void __launch_bounds__(R3_THREADS, 2) k_r3d_solve_mixed(const __grid_
             break;
         }
         if (it == d.maxsweeps) break;
-        // e = 0, one FP32 cycle: relax on level 1, descent, ascent
-        for (long long t = gt; t < nlvl; t += T) W.v32[t] = 0.f;
-        if (!grid_sync(gs)) return;
-        if (!r3_relax32<COMP>(d, 1, nlev > 1, sm)) return;
+        // one FP32 cycle from e = 0: relax on level 1, descent, ascent
+        if (!r3_relax32<COMP>(d, 1, nlev > 1)) return;
         for (int l = 1; l <= nlev - 1; ++l) {
             r3_corser32(d, COMP, l);
-            if (!grid_sync(gs)) return;
-            if (!r3_relax32<COMP>(d, l + 1, l + 1 < nlev, sm)) return;
+            if (!sync_before(l + 1)) return;
+            if (!r3_relax32<COMP>(d, l + 1, l + 1 < nlev)) return;
         }
         for (int l = nlev; l >= 2; --l) {
             r3_finer32(d, COMP, l);
-            if (!grid_sync(gs)) return;
-            if (!r3_relax32<COMP>(d, l - 1, false, sm)) return;
+            if (!sync_before(l - 1)) return;
+            if (!r3_relax32<COMP>(d, l - 1, false)) return;
         }
         const double w = (it == 0 || d.horizontal) ? 1.0 : d.sor;
-        for (long long t = gt; t < nlvl; t += T) W.v[t] += w * (double)W.v32[t];
+        for (int t = gt; t < nlvl; t += T) {
+            W.v[t] += w * f2d(W.v32[t]);
+            W.v32[t] = 0.f;
+        }
         if (!grid_sync(gs)) return;
     }
+    async_copy_wait();   // the copies prepared for a cycle that is not run
     if (status == GB_OK) {
         const int imax = COMP == 3 ? d.nr : d.nr + 1;
         const int jmax = COMP == 1 ? d.nz : d.nz + 1;
         const int ii1 = COMP == 3 ? d.nr - 1 : d.nr;
         const int jj1 = COMP == 1 ? d.nz - 1 : d.nz;
-        const long long npts = (long long)(imax + 1) * (jmax + 1) * (d.np + 1);
-        for (long long t = gt; t < npts; t += T) {
-            const int i = (int)(t % (imax + 1));
-            const long long rest = t / (imax + 1);
-            const int j = (int)(rest % (jmax + 1));
-            const int k = (int)(rest / (jmax + 1));
+        const int npts = (imax + 1) * (jmax + 1) * (d.np + 1);
+        const RowSplit ti(imax + 1), tj(jmax + 1);
+        for (int t = gt; t < npts; t += T) {
+            int i, j, k, rest;
+            ti(t, rest, i);
+            tj(rest, k, j);
             const double old = FX(psi, i, j, k);
             FX(psip, i, j, k) = old;
             const bool inner = i >= 1 && i <= ii1 && j >= 1 && j <= jj1;
@@ -2012,9 +2284,17 @@ extern "C" int gb_r3d_destroy(gb_r3d *h)
 // the same order.
 #define R3_CONT 0x80000000u
 
-static int r3_chunk_lines(int n) { return std::max(1, std::min(R3_THREADS, R3_SMEM_DOUBLES / (n | 1))); }
+// Lines that any chunk of n-row lines holds (r3_phase's rule, the least of both
+// types).
+static int r3_chunk_lines(int comp, int dir, int n)
+{
+    int c = std::min(R3_THREADS, std::min(R3_CHUNK_BYTES / 8 / (n | 1), R3_CHUNK_BYTES / 4 / wl_pitch(n)));
+    if (dir == 1) c = std::min(c, R3_FAC_BYTES / 4 / r3_tabsize32(r3_kind(comp, dir), n));
+    return std::max(1, c);
+}
 
-static void r3_phases(int mode, int comp, int dir, int n1, int n2, int n3, std::vector<int> &lines, std::vector<int> &off)
+static void r3_phases(int mode, int pslow, int comp, int dir, int n1, int n2, int n3, std::vector<int> &lines,
+                      std::vector<int> &off)
 {
     const int im = r3_imax(comp, n1), jm = r3_jmax(comp, n2);
     int P, Q, p_os, q_os;
@@ -2044,7 +2324,7 @@ static void r3_phases(int mode, int comp, int dir, int n1, int n2, int n3, std::
         }
         return;
     }
-    const int chunk = r3_chunk_lines(r3_len(comp, dir, n1, n2, n3));
+    const int chunk = r3_chunk_lines(comp, dir, r3_len(comp, dir, n1, n2, n3));
     auto cls_of = [&](int p, int q) { return (p_os && (p == 1 || p == P)) + (q_os && (q == 1 || q == Q)); };
     auto id = [&](int p, int q) { return (q - 1) * P + (p - 1); };
     for (int colour = 0; colour < 2; ++colour) {
@@ -2067,6 +2347,17 @@ static void r3_phases(int mode, int comp, int dir, int n1, int n2, int n3, std::
             for (int q = 1; q <= Q; ++q)
                 for (int p = 1; p <= P; ++p)
                     if (((p + q) & 1) == colour && cls_of(p, q) == cls) groups[root(id(p, q))].push_back(p | (q << 16));
+        // FP64 lines share a radius's factors: its lines in a row (p slow); FP32
+        // ones take what runs with memory (p fast)
+        if (pslow)
+            std::stable_sort(groups.begin(), groups.end(), [](const std::vector<int> &x, const std::vector<int> &y) {
+                auto key = [](const std::vector<int> &g) {
+                    int m = 1 << 30;
+                    for (int e : g) m = std::min(m, e & 0xffff);
+                    return m;
+                };
+                return key(x) < key(y);
+            });
         size_t biggest = 0;
         for (const auto &g : groups) biggest = std::max(biggest, g.size());
         if ((int)biggest <= chunk) {
@@ -2190,14 +2481,14 @@ static int r3_create(const gb_r3d_params *p, const double *spacing, gb_r3d **out
         const int n1 = nr >> (l - 1), n2 = nz >> (l - 1), n3 = np >> (l - 1);
         const size_t sz = (size_t)(n1 + 1) * (n2 + 1) * (n3 + 1);
         wneed += 3 * (3 * sz + (3 * sz + 1) / 2 + 2);
-        need += 2 * (size_t)(n1 + 2);
-        size_t f32 = 4 * (size_t)(n1 + 2);
+        need += 6 * (size_t)(n1 + 2);
+        size_t f32 = 3 * (4 * (size_t)(n1 + 1) + 4 * (size_t)(n2 + 1) + (size_t)(n1 + 4)) + 4;
         for (int comp = 1; comp <= 3; ++comp)
             for (int dir = 0; dir < 3; ++dir) {
                 const int n = r3_len(comp, dir, n1, n2, n3);
                 const int inst = dir == 0 ? 1 : r3_imax(comp, n1);
                 need += (size_t)inst * r3_tabsize(r3_kind(comp, dir), n);
-                f32 += (size_t)inst * r3_tabsize(r3_kind(comp, dir), n);
+                f32 += (size_t)inst * r3_tabsize32(r3_kind(comp, dir), n) + 4;
             }
         need += (f32 + 1) / 2 + 2;
     }
@@ -2226,6 +2517,10 @@ static int r3_create(const gb_r3d_params *p, const double *spacing, gb_r3d **out
         L.hhr = L.hr * L.hr;
         L.hhz = L.hz * L.hz;
         L.hhp = L.hp * L.hp;
+        L.ihr = 1.0 / L.hr;
+        L.ihhr = 1.0 / L.hhr;
+        L.ihhz = 1.0 / L.hhz;
+        L.ihhp = 1.0 / L.hhp;
         const size_t sz = (size_t)L.L1 * L.L2 * (L.n3 + 1);
         for (int comp = 1; comp <= 3; ++comp) {
             R3Work &W = d.work[comp][l];
@@ -2240,10 +2535,20 @@ static int r3_create(const gb_r3d_params *p, const double *spacing, gb_r3d **out
         }
         L.rvc = b; b += L.n1 + 2;
         L.rvv = b; b += L.n1 + 2;
-        rv_host.assign(2 * (size_t)(L.n1 + 2), 0.0);
+        L.dirc = b; b += L.n1 + 2;
+        L.dirv = b; b += L.n1 + 2;
+        L.diqc = b; b += L.n1 + 2;
+        L.diqv = b; b += L.n1 + 2;
+        const size_t m = (size_t)L.n1 + 2;
+        rv_host.assign(6 * m, 0.0);
         for (int i = 0; i <= L.n1 + 1; ++i) {
-            rv_host[i] = d.r0 + ((double)i - 0.5) * L.hr;
-            rv_host[L.n1 + 2 + i] = (double)i * L.hr + d.r0;
+            const double rc = d.r0 + ((double)i - 0.5) * L.hr, rv = (double)i * L.hr + d.r0;
+            rv_host[i] = rc;
+            rv_host[m + i] = rv;
+            rv_host[2 * m + i] = 1.0 / rc;
+            rv_host[3 * m + i] = 1.0 / rv;
+            rv_host[4 * m + i] = 1.0 / (rc * rc);
+            rv_host[5 * m + i] = 1.0 / (rv * rv);
         }
         cudaMemcpy(L.rvc, rv_host.data(), sizeof(double) * rv_host.size(), cudaMemcpyHostToDevice);
         for (int comp = 1; comp <= 3; ++comp)
@@ -2255,7 +2560,7 @@ static int r3_create(const gb_r3d_params *p, const double *spacing, gb_r3d **out
                 for (int q = 0; q < inst; ++q) jobs.push_back({l, comp, dir, dir == 0 ? 0 : q + 1, b + (size_t)q * r3_tabsize(kind, n)});
                 b += (size_t)inst * r3_tabsize(kind, n);
                 std::vector<int> lines, off;
-                r3_phases(p->smoother, comp, dir, L.n1, L.n2, L.n3, lines, off);
+                r3_phases(p->smoother, p->precision == GB_PRB_FP64, comp, dir, L.n1, L.n2, L.n3, lines, off);
                 TabRef tr;
                 tr.l = l;
                 tr.comp = comp;
@@ -2270,29 +2575,19 @@ static int r3_create(const gb_r3d_params *p, const double *spacing, gb_r3d **out
         // FP32 storage of the level
         {
             float *fb = (float *)b;
-            L.irc = fb; fb += L.n1 + 2;
-            L.irv = fb; fb += L.n1 + 2;
-            L.iqc = fb; fb += L.n1 + 2;
-            L.iqv = fb; fb += L.n1 + 2;
-            std::vector<float> rr(4 * (size_t)(L.n1 + 2));
-            for (int i = 0; i <= L.n1 + 1; ++i) {
-                const double rc = rv_host[i], rv = rv_host[L.n1 + 2 + i];
-                rr[i] = (float)(1.0 / rc);
-                rr[L.n1 + 2 + i] = (float)(1.0 / rv);
-                rr[2 * (L.n1 + 2) + i] = (float)(1.0 / (rc * rc));
-                rr[3 * (L.n1 + 2) + i] = (float)(1.0 / (rv * rv));
+            fb = (float *)(((uintptr_t)fb + 15) & ~(uintptr_t)15);
+            for (int comp = 1; comp <= 3; ++comp) {
+                L.wi[comp] = (float4 *)fb; fb += 4 * (L.n1 + 1);
+                L.wj[comp] = (float4 *)fb; fb += 4 * (L.n2 + 1);
+                L.wp[comp] = fb; fb += (L.n1 + 4) & ~3;
             }
-            cudaMemcpy(L.irc, rr.data(), sizeof(float) * rr.size(), cudaMemcpyHostToDevice);
-            L.ihr = (float)(1.0 / L.hr);
-            L.ihhr = (float)(1.0 / L.hhr);
-            L.ihhz = (float)(1.0 / L.hhz);
-            L.ihhp = (float)(1.0 / L.hhp);
             for (int comp = 1; comp <= 3; ++comp)
                 for (int dir = 0; dir < 3; ++dir) {
                     const int n = r3_len(comp, dir, L.n1, L.n2, L.n3);
                     const int inst = dir == 0 ? 1 : r3_imax(comp, L.n1);
+                    fb = (float *)(((uintptr_t)fb + 15) & ~(uintptr_t)15);   // copied 16 bytes at a time
                     L.fac32[comp][dir] = fb;
-                    fb += (size_t)inst * r3_tabsize(r3_kind(comp, dir), n);
+                    fb += (size_t)inst * r3_tabsize32(r3_kind(comp, dir), n);
                 }
             b = (double *)(((uintptr_t)fb + 15) & ~(uintptr_t)15);
         }
@@ -2352,23 +2647,17 @@ static int r3_create(const gb_r3d_params *p, const double *spacing, gb_r3d **out
     e = cudaMalloc(&djobs, sizeof(FacJob) * jobs.size());
     if (e != cudaSuccess) { gb_r3d_destroy(h); gb_set_error("gb_r3d_create: factor jobs"); return GB_ERR_ALLOC; }
     cudaMemcpy(djobs, jobs.data(), sizeof(FacJob) * jobs.size(), cudaMemcpyHostToDevice);
-    k_r3d_factors<<<gb_ceil_div(jobs.size(), 64), 64>>>(d, djobs, (int)jobs.size());
     {
-        // FP32 tables: the same job list, destinations in the FP32 pool
-        std::vector<float *> dst(jobs.size());
-        for (size_t q = 0; q < jobs.size(); ++q) {
-            const FacJob &J = jobs[q];
-            const R3Lev &L = d.lev[J.lev];
-            dst[q] = L.fac32[J.comp][J.dir] + (J.tab - L.fac[J.comp][J.dir]);
-        }
-        float **ddst = nullptr;
-        e = cudaMalloc(&ddst, sizeof(float *) * dst.size());
-        if (e == cudaSuccess) {
-            cudaMemcpy(ddst, dst.data(), sizeof(float *) * dst.size(), cudaMemcpyHostToDevice);
-            k_r3d_factors32<<<gb_ceil_div(jobs.size(), 64), 64>>>(d, djobs, (int)jobs.size(), ddst);
-            cudaDeviceSynchronize();
-            cudaFree(ddst);
-        }
+        const int wstride = 7 * std::max(nr, std::max(nz, np));
+        double *work = nullptr;
+        e = cudaMalloc(&work, sizeof(double) * (size_t)wstride * jobs.size());
+        if (e != cudaSuccess) { cudaFree(djobs); gb_r3d_destroy(h); gb_set_error("gb_r3d_create: factor scratch"); return GB_ERR_ALLOC; }
+        k_r3d_factors<<<gb_ceil_div(jobs.size(), 64), 64>>>(d, djobs, (int)jobs.size(), work, wstride);
+        k_r3d_factors32<<<gb_ceil_div(jobs.size(), 64), 64>>>(d, djobs, (int)jobs.size());
+        k_r3d_steps32<<<dim3(nlev, 3, 2), 128>>>(d);
+        k_r3d_weights32<<<dim3(nlev, 3), 128>>>(d);
+        cudaDeviceSynchronize();
+        cudaFree(work);
     }
     e = cudaDeviceSynchronize();
     cudaFree(djobs);
@@ -2383,7 +2672,8 @@ static int r3_create(const gb_r3d_params *p, const double *spacing, gb_r3d **out
                             (const void *)k_r3d_solve_mixed<1>, (const void *)k_r3d_solve_mixed<2>,
                             (const void *)k_r3d_solve_mixed<3>};
     for (int q = 0; q < 6; ++q) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kerns[q], R3_THREADS, 0);
+        cudaFuncSetAttribute(kerns[q], cudaFuncAttributeMaxDynamicSharedMemorySize, R3_SMEM_BYTES);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kerns[q], R3_THREADS, R3_SMEM_BYTES);
         worst = std::min(worst, per_sm);
     }
     if (!coop || worst < 1) {
@@ -2494,7 +2784,7 @@ static int r3_launch_solve(gb_r3d *h, int comp, int step, cudaStream_t s, int gr
     const void *k = comp == 1   ? (mixed ? (const void *)k_r3d_solve_mixed<1> : (const void *)k_r3d_solve<1>)
                     : comp == 2 ? (mixed ? (const void *)k_r3d_solve_mixed<2> : (const void *)k_r3d_solve<2>)
                                 : (mixed ? (const void *)k_r3d_solve_mixed<3> : (const void *)k_r3d_solve<3>);
-    cudaError_t e = cudaLaunchCooperativeKernel(k, grid, R3_THREADS, args, 0, s);
+    cudaError_t e = cudaLaunchCooperativeKernel(k, grid, R3_THREADS, args, R3_SMEM_BYTES, s);
     if (e != cudaSuccess) {
         gb_set_error("gb_r3d: cooperative solve launch (%d blocks): %s", grid, cudaGetErrorString(e));
         return GB_ERR_CUDA;
