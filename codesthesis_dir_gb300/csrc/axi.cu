@@ -45,7 +45,7 @@ struct AxiLevel {
     double *v, *f;            // packed (n1+1)*(n2+1)
     double *fac_r;            // r-line factors, tdma_fac_len(n1-1)
     double *fac_z;            // z-line factors, tdma_fac_len(n2-1) for each i = 1..n1-1
-    // mixed precision: FP32 correction cycle (folded line tables)
+    // mixed precision: FP32 correction cycle (line tables, warpline.cuh)
     float *v32, *f32, *fac_r32, *fac_z32;
 };
 
@@ -478,9 +478,9 @@ __device__ __forceinline__ AxiView<float> axi_view(const AxiDev &d, int l, float
 #define V(i, j) L.v[(i) + L.ld * (j)]
 #define F(i, j) L.f[(i) + L.ld * (j)]
 
-// x / h: the IEEE quotient from the stored reciprocal, or a product with it
+// x / h: the IEEE quotient (FP64: from the stored reciprocal)
 __device__ __forceinline__ double axi_over(double x, double h, double ih) { return div_by_rcp(x, h, ih); }
-__device__ __forceinline__ float axi_over(float x, float, float ih) { return x * ih; }
+__device__ __forceinline__ float axi_over(float x, float h, float) { return x / h; }
 
 // Right-hand sides of r-line j at row i (rotann2.f:698-710) and of z-line i
 // at row j (rotann2.f:712-725).
@@ -668,12 +668,16 @@ template <class T> __device__ __noinline__ void axi_corser(const AxiDev &d, int 
         T temp = T(0);
         if (i >= 1 && i <= n1c - 1 && j >= 1 && j <= n2c - 1 && j != n1c) {
             const T *q = rc + (i + i) + ld * (j + j);
-            temp = q[0];
-            temp = temp * T(2) + q[1] + q[-1];
-            temp = temp + q[ld] + q[-ld];
-            temp = temp * T(2) + q[1 + ld] + q[-1 - ld];
-            temp = temp + q[1 - ld] + q[-1 + ld];
-            temp = temp * T(0.0625);   // / 16, exactly
+            if constexpr (sizeof(T) == 8) {
+                temp = q[0];
+                temp = temp * T(2) + q[1] + q[-1];
+                temp = temp + q[ld] + q[-ld];
+                temp = temp * T(2) + q[1 + ld] + q[-1 - ld];
+                temp = temp + q[1 - ld] + q[-1 + ld];
+                temp = temp * T(0.0625);   // / 16, exactly
+            } else {
+                temp = 0.25f * q[0] + 0.125f * (q[1] + q[-1] + q[ld] + q[-ld]) + 0.0625f * (q[1 + ld] + q[-1 - ld] + q[1 - ld] + q[-1 + ld]);
+            }
         }
         fc[idx] = temp;
         L.v[idx] = T(0);
@@ -834,7 +838,7 @@ __device__ __forceinline__ void k_axi_mg_solve_mixed_body(const AxiDev &d)
 
 __global__ void __maxnreg__(255) k_axi_mg_solve_mixed(const __grid_constant__ AxiDev d) { k_axi_mg_solve_mixed_body(d); }
 
-// FP32 copies of rval and the folded factors: block l - 1 takes level l, its
+// FP32 copies of rval and the line tables: block l - 1 takes level l, its
 // threads the level's lines (thread 0 also the r-line table).
 __global__ void k_axi_factors32(AxiDev d)
 {
@@ -847,7 +851,6 @@ __global__ void k_axi_factors32(AxiDev d)
         const int n = L.n2 - 1;
         for (int i = 1 + threadIdx.x; i <= L.n1 - 1; i += blockDim.x)
             tdma32_fold(L.fac_z + (size_t)(i - 1) * tdma_fac_len(n), n, L.fac_z32 + (size_t)(i - 1) * tdma32_len(n));
-        wl_common_steps(L.fac_z32, tdma32_len(n), L.n1 - 1);
     }
 }
 
@@ -856,15 +859,18 @@ __global__ void k_axi_weights(const __grid_constant__ AxiDev d, const __grid_con
 {
     const int l = 1 + blockIdx.y, t = blockIdx.x * blockDim.x + threadIdx.x;
     const AxiLevel &L = d.lev[l];
-    auto put = [&](const float4 *c4, const MerW *d4, int q, double cm, double cp, double cd) {
-        const_cast<float4 *>(c4)[q] = make_float4((float)cm, (float)cp, 0.f, (float)cd);
-        if (l == 1) const_cast<MerW *>(d4)[q] = MerW{cm, cp, 0.0, cd};
-    };
     if (t >= 1 && t < L.n1) {
-        const double rv = d.rval[t * L.lf];
-        put(m.lev[l].c4i, m.d4i, t, 1.0 / L.hhr - 0.5 / L.hr / rv, 1.0 / L.hhr + 0.5 / L.hr / rv, -2.0 / L.hhr - 1.0 / (rv * rv));
+        const float r = d.rval32[t * L.lf];
+        const_cast<float4 *>(m.lev[l].ci)[t] = make_float4(r, r * r, 0.f, 0.f);
+        if (l == 1) {
+            const double rv = d.rval[t];
+            MerRow &q = const_cast<MerRow *>(m.d_i)[t];
+            q.r = rv;
+            q.ir = d.irv[t];
+            q.rr = rv * rv;
+            q.irr = d.irq[t];
+        }
     }
-    if (t >= 1 && t < L.n2) put(m.lev[l].c4j, m.d4j, t, 1.0 / L.hhz, 1.0 / L.hhz, -2.0 / L.hhz);
 }
 
 __global__ void k_axi_rval(AxiDev d)
@@ -1032,8 +1038,17 @@ static cudaError_t axi_mer_create(gb_axi *h)
         L.fac_r = d.lev[l].fac_r32;
         L.fac_z = d.lev[l].fac_z32;
         L.fac_r_step = 0;
+        L.hr = (float)d.lev[l].hr;
+        L.hhr = (float)d.lev[l].hhr;
+        L.hhz = (float)d.lev[l].hhz;
+        L.drdz = 2.0f * (1.0f / L.hhr + 1.0f / L.hhz);
         L.fac_z_step = (int)tdma32_len(L.n2 - 1);
     }
+    const AxiLevel &L1 = d.lev[1];
+    m.hr = MerOver{L1.hr, L1.ihr};
+    m.hhr = MerOver{L1.hhr, L1.ihhr};
+    m.hhz = MerOver{L1.hhz, L1.ihhz};
+    m.drdz = 2.0 * (1.0 / L1.hhr + 1.0 / L1.hhz);
     m.v = d.lev[1].v;
     m.psi = d.f[GB_A_phi];
     m.rhs = d.f[GB_A_omegn];

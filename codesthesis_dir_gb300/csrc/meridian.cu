@@ -18,13 +18,12 @@
 // back: one value per unknown each way.
 //
 // The FP64 residual is the one part bound by arithmetic (the FP64 pipe issues
-// two lanes a cycle and SM): the r and z weights are combined per row in FP64
-// (nine fused multiply-adds a point), the conversions and the norm go to the
-// integer pipe.
+// two lanes a cycle and SM): its divisions are products with stored reciprocals
+// and a correction, the conversions and the norm go to the integer pipe.
 //
 // Measured (GB300, mixed solve, a step's whole time): 257 x 257 stretched, five
 // cycles, 22.3 ms on one SM and global memory, 4.5 ms on a cluster of 16 with
-// the levels in L2, 2.2 ms resident.
+// the levels in L2, 2.8 ms resident.
 #include "meridian.cuh"
 
 #include <algorithm>
@@ -161,7 +160,7 @@ template <int M, bool PENTA> __device__ __noinline__ int mer_r_sweep(const MerLe
     const int sub = (threadIdx.x & 31) >> lw, lane = threadIdx.x & ((1 << lw) - 1);
     const int slot = (threadIdx.x >> 5) * per + sub, nslots = (MER_THREADS / 32) * per;
     const MerOwn own(L, cl);
-    const float4 *c4j = (const float4 *)(s_mer + L.o4j);
+    const float4 *cj = (const float4 *)(s_mer + L.ocj);
     const unsigned *rows = (const unsigned *)(s_mer + L.rows);
     const int col = 2 + lane * (M + 1);
     for (int c = 1; c <= NC; ++c, ++k) {
@@ -172,15 +171,27 @@ template <int M, bool PENTA> __device__ __noinline__ int mer_r_sweep(const MerLe
             if (jc + NC * (tb + slot - sub) >= own.j1) continue;   // no line for this warp
             const bool live = jc + NC * (tb + slot) < own.j1;
             const int t0 = live ? tb + slot : tb + slot - sub, j = jc + NC * t0;   // idle groups repeat a line and store nothing
-            const float4 w = c4j[j];
             const int row = (j - own.j0 + 1) * L.pitch + col;
-            const int jf = j <= L.n2 / 2 ? j + 2 : j - 2;
-            const int near[3] = {j - 1, j + 1, jf};
-            const float weight[3] = {w.x, w.y, w.z};
+            // the neighbours in the order their terms are added
+            constexpr int NN = PENTA ? 3 : 2;
+            int near[NN];
+            float weight[NN];
+            if constexpr (PENTA) {
+                const float4 w = cj[j];
+                const bool low = j <= L.n2 / 2;
+                near[0] = low ? j - 1 : j - 2;
+                near[1] = low ? j + 1 : j - 1;
+                near[2] = low ? j + 2 : j + 1;
+                weight[0] = w.x;
+                weight[1] = low ? w.z : w.y;
+                weight[2] = w.w;
+            } else {
+                near[0] = j + 1;
+                near[1] = j - 1;
+            }
             float t[M];
 #pragma unroll
             for (int u = 0; u < M; ++u) t[u] = s_mer[L.f + row + u];
-            constexpr int NN = PENTA ? 3 : 2;
             const float *src[NN];
 #pragma unroll
             for (int q = 0; q < NN; ++q) {
@@ -199,9 +210,10 @@ template <int M, bool PENTA> __device__ __noinline__ int mer_r_sweep(const MerLe
             }
             __syncwarp();
 #pragma unroll
-            for (int q = 0; q < NN; ++q)
-#pragma unroll
-                for (int u = 0; u < M; ++u) t[u] = __fmaf_rn(-weight[q], src[q][u], t[u]);
+            for (int u = 0; u < M; ++u) {
+                if constexpr (PENTA) t[u] = -(weight[0] * src[0][u] + weight[1] * src[1][u] + weight[2] * src[2][u]) + t[u];
+                else t[u] = -(src[0][u] + src[1][u]) / L.hhz + t[u];
+            }
             if (!ready) {
                 mer_tables(pipe, k);
                 ready = true;
@@ -244,7 +256,7 @@ __device__ __noinline__ int mer_z_sweep(const MerLevel &lev, MerPipe &pipe, int 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = MER_THREADS / 32;
     const MerOwn own(L, cl);
     const int ni = L.n1 - 1;
-    const float4 *c4i = (const float4 *)(s_mer + L.o4i);
+    const float4 *ci = (const float4 *)(s_mer + L.oci);
     const unsigned *rows = (const unsigned *)(s_mer + L.rows), *xline = (const unsigned *)(s_mer + L.xline);
     const float *x = s_mer + xoff;
     const int share = mer_share<NC>(ni, cl.size), l0 = cl.rank * share;
@@ -258,11 +270,19 @@ __device__ __noinline__ int mer_z_sweep(const MerLevel &lev, MerPipe &pipe, int 
             const int xj = 4 * ((j - 1) * share + ((j - 1) >> LGM));
             for (int l = lane; l < nl; l += 32) {
                 const int i = c + NC * l;
-                const float4 w = c4i[i];
-                float r = fr[mer_col(lg, i)];
-                r = __fmaf_rn(-w.x, vr[mer_col(lg, i - 1)], r);
-                r = __fmaf_rn(-w.y, vr[mer_col(lg, i + 1)], r);
-                if (PENTA) r = __fmaf_rn(-w.z, vr[mer_col(lg, i <= L.n1 / 2 ? i + 2 : i - 2)], r);
+                const float f = fr[mer_col(lg, i)];
+                float r;
+                if constexpr (PENTA) {
+                    const float4 a = ci[2 * i], b = ci[2 * i + 1];
+                    const bool low = i <= L.n1 / 2;
+                    const float p0 = vr[mer_col(lg, low ? i - 1 : i - 2)], p1 = vr[mer_col(lg, low ? i + 1 : i - 1)];
+                    const float p2 = vr[mer_col(lg, low ? i + 2 : i + 1)];
+                    const float over = (b.x * (low ? p0 : p1) + b.z * (low ? p1 : p2)) * b.w;
+                    r = -(a.x * p0 + (low ? a.z : a.y) * p1 + a.w * p2 + over) + f;
+                } else {
+                    const float vp = vr[mer_col(lg, i + 1)], vm = vr[mer_col(lg, i - 1)];
+                    r = -(vp + vm) / L.hhr + f - (vp - vm) * 0.5f / ci[i].x / L.hr;
+                }
                 cst(xline[l] + xj, r);
             }
         }
@@ -305,28 +325,32 @@ template <bool PENTA> __device__ __noinline__ void mer_residual(const MerLevel &
     const Cluster cl = Cluster::self();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = MER_THREADS / 32;
     const MerOwn own(L, cl);
-    const float4 *c4i = (const float4 *)(s_mer + L.o4i), *c4j = (const float4 *)(s_mer + L.o4j);
+    const float4 *ci = (const float4 *)(s_mer + L.oci), *cj = (const float4 *)(s_mer + L.ocj);
     const unsigned *rows = (const unsigned *)(s_mer + L.rows);
     for (int j = own.j0 + warp; j < own.j1; j += nw) {
-        const float4 wj = c4j[j];
-        const unsigned vm = rows[j - 1], vp = rows[j + 1], vf = PENTA ? rows[j <= L.n2 / 2 ? j + 2 : j - 2] : vm;
+        const bool lowj = j <= L.n2 / 2;
+        const unsigned vm = rows[j - 1], vp = rows[j + 1], vf = PENTA ? rows[lowj ? j + 2 : j - 2] : vm;
         const int row = (j - own.j0 + 1) * L.pitch;
         const float *v = s_mer + L.v + row, *f = s_mer + L.f + row;
         float *out = s_mer + rc + row;
 #pragma unroll 2
         for (int i = 1 + lane; i < L.n1; i += 32) {
-            const float4 wi = c4i[i];
             const int c = mer_col(lg, i);
-            const float a = cld(vm + 4 * c), b = cld(vp + 4 * c), e = PENTA ? cld(vf + 4 * c) : 0.f;
-            float r = f[c];
-            r = __fmaf_rn(-wi.x, v[mer_col(lg, i - 1)], r);
-            r = __fmaf_rn(-wi.y, v[mer_col(lg, i + 1)], r);
-            if (PENTA) r = __fmaf_rn(-wi.z, v[mer_col(lg, i <= L.n1 / 2 ? i + 2 : i - 2)], r);
-            r = __fmaf_rn(-(wi.w + wj.w), v[c], r);
-            r = __fmaf_rn(-wj.x, a, r);
-            r = __fmaf_rn(-wj.y, b, r);
-            if (PENTA) r = __fmaf_rn(-wj.z, e, r);
-            out[c] = r;
+            const float d = cld(vm + 4 * c), u = cld(vp + 4 * c), e = PENTA ? cld(vf + 4 * c) : 0.f;
+            const float p = v[c], pm = v[mer_col(lg, i - 1)], pp = v[mer_col(lg, i + 1)];
+            float t;
+            if constexpr (PENTA) {
+                const float4 a = ci[2 * i], b = ci[2 * i + 1], w = cj[j];
+                const bool low = i <= L.n1 / 2;
+                const float far = v[mer_col(lg, low ? i + 2 : i - 2)];
+                const float over = (b.x * pm + b.y * p + b.z * pp) * b.w, overq = p * (b.w * b.w);
+                t = a.x * (low ? pm : far) + a.y * (low ? p : pm) + a.z * (low ? pp : p) + a.w * (low ? far : pp) + over - overq;
+                t = t + w.x * (lowj ? d : e) + w.y * (lowj ? p : d) + w.z * (lowj ? u : p) + w.w * (lowj ? e : u);
+            } else {
+                const float4 a = ci[i];
+                t = (pp + pm) / L.hhr + (pp - pm) * 0.5f / L.hr / a.x - p / a.y + (u + d) / L.hhz - p * L.drdz;
+            }
+            out[c] = f[c] - t;
         }
     }
     cl.sync();
@@ -335,7 +359,7 @@ template <bool PENTA> __device__ __noinline__ void mer_residual(const MerLevel &
 // corser (rotann2.f:755-801, rcsc.f:1343-1390): nine-point restriction; the
 // row j = n1c that both clear (n1 of the coarse level in both directions) is
 // zero, and the coarse correction is cleared.
-__device__ __noinline__ void mer_corser(const MerLevel &fine, const MerLevel &coarse, int rc)
+template <bool PENTA> __device__ __noinline__ void mer_corser(const MerLevel &fine, const MerLevel &coarse, int rc)
 {
     extern __shared__ __align__(16) float s_mer[];
     const MerLevel F = fine, L = coarse;
@@ -350,8 +374,17 @@ __device__ __noinline__ void mer_corser(const MerLevel &fine, const MerLevel &co
         const int row = (j - own.j0 + 1) * L.pitch;
         for (int i = 1 + lane; i < L.n1; i += 32) {
             const int a = 4 * mer_col(lgf, 2 * i - 1), b = 4 * mer_col(lgf, 2 * i), c = 4 * mer_col(lgf, 2 * i + 1);
-            const float t = 0.25f * cld(q0 + b) + 0.125f * (cld(q0 + c) + cld(q0 + a) + cld(qp + b) + cld(qm + b)) +
-                            0.0625f * (cld(qp + c) + cld(qm + a) + cld(qm + c) + cld(qp + a));
+            const float o0 = cld(q0 + b), e = cld(q0 + c), w = cld(q0 + a), n = cld(qp + b), s = cld(qm + b);
+            const float ne = cld(qp + c), sw = cld(qm + a), se = cld(qm + c), nw_ = cld(qp + a);
+            float t;
+            if (PENTA) {   // the sums as each of the two references orders them
+                t = o0 * 2.f + e + w;
+                t = t + n + s;
+                t = t * 2.f + ne + sw;
+                t = (t + se + nw_) * 0.0625f;
+            } else {
+                t = 0.25f * o0 + 0.125f * (e + w + n + s) + 0.0625f * (ne + sw + se + nw_);
+            }
             const int o = row + mer_col(lg, i);
             s_mer[L.f + o] = j == L.n1 ? 0.f : t;
             s_mer[L.v + o] = 0.f;
@@ -376,7 +409,8 @@ __device__ __noinline__ void mer_finer(const MerLevel &coarse, const MerLevel &f
 #pragma unroll 2
         for (int i = 1 + lane; i < L.n1; i += 32) {
             const int a = 4 * mer_col(lgc, i >> 1), b = 4 * mer_col(lgc, (i + 1) >> 1);
-            v[mer_col(lg, i)] += 0.25f * (cld(q0 + a) + cld(q1 + b) + cld(q1 + a) + cld(q0 + b));
+            const float u = cld(q0 + a) + cld(q1 + b);   // one point twice, two, or two of four
+            v[mer_col(lg, i)] += i & j & 1 ? (u + cld(q1 + a) + cld(q0 + b)) * 0.25f : u * 0.5f;
         }
     }
     cl.sync();
@@ -398,16 +432,29 @@ template <bool PENTA> __device__ __forceinline__ int mer_relax(const MerDev &d, 
     return k;
 }
 
+// x / h: the IEEE quotient up to the sign of a zero (divrn.cuh).
+__device__ __forceinline__ double mer_over(double x, double h, double ih)
+{
+    const double q = __dmul_rn(x, ih);
+    return __fma_rn(__fma_rn(-h, q, x), ih, q);
+}
+
 // FP64 residual of the iterate over this CTA's rows: its FP32 rounding is the
 // cycle's right-hand side.  Returns the largest magnitude's bit pattern (NaNs
 // excluded; the order of non-negative doubles is the order of their bits).
+// The terms stand in the reference's order: with the weights of a row combined
+// (9 operations instead of 32) the last bits of a small residual, and with them
+// the whole correction, round differently: 3e-9 of the streamfunction.
 template <bool PENTA> __device__ __noinline__ double mer_residual64(const MerDev &d, int *nan_out)
 {
     extern __shared__ __align__(16) float s_mer[];
     const Cluster cl = Cluster::self();
     const MerLevel L = d.lev[1];
     const double *dv = d.v, *drhs = d.rhs;
-    const MerW *d4i = d.d4i, *d4j = d.d4j;
+    const MerRow *di = d.d_i;
+    const MerCol *dj = d.d_j;
+    const MerOver hr = d.hr, hhr = d.hhr, hhz = d.hhz;
+    const double drdz = d.drdz;
     const int ld = L.n1 + 1, ni = L.n1 - 1, lg = wl_log2m(ni);
     const MerOwn own(L, cl);
     const int j0 = own.j0, j1 = own.j1;
@@ -420,17 +467,21 @@ template <bool PENTA> __device__ __noinline__ double mer_residual64(const MerDev
         ++i;
         const int j = j0 + jj;
         const double *v = dv + (size_t)j * ld + i;
-        const MerW a = d4i[i], b = d4j[j];
-        double r = drhs[(size_t)j * ld + i];
-        r = __fma_rn(-(a.w + b.w), v[0], r);
-        r = __fma_rn(-a.x, v[-1], r);
-        r = __fma_rn(-a.y, v[1], r);
-        r = __fma_rn(-b.x, v[-ld], r);
-        r = __fma_rn(-b.y, v[ld], r);
-        if (PENTA) {
-            r = __fma_rn(-a.z, v[i <= L.n1 / 2 ? 2 : -2], r);
-            r = __fma_rn(-b.z, v[j <= L.n2 / 2 ? 2 * ld : -2 * ld], r);
+        const MerRow &a = di[i];
+        const double p = v[0], pm = v[-1], pp = v[1], pd = v[-ld], pu = v[ld];
+        double t;
+        if constexpr (PENTA) {
+            const MerCol &w = dj[j];
+            const bool low = i <= L.n1 / 2, lowj = j <= L.n2 / 2;
+            const double far = v[low ? 2 : -2], farj = v[lowj ? 2 * ld : -2 * ld];
+            t = a.crr[0] * (low ? pm : far) + a.crr[1] * (low ? p : pm) + a.crr[2] * (low ? pp : p) + a.crr[3] * (low ? far : pp) +
+                mer_over(a.cr[0] * pm + a.cr[1] * p + a.cr[2] * pp, a.r, a.ir) - mer_over(p, a.rr, a.irr);
+            t = t + w.czz[0] * (lowj ? pd : farj) + w.czz[1] * (lowj ? p : pd) + w.czz[2] * (lowj ? pu : p) + w.czz[3] * (lowj ? farj : pu);
+        } else {
+            t = mer_over(pp + pm, hhr.h, hhr.ih) + mer_over(mer_over((pp - pm) * 0.5, hr.h, hr.ih), a.r, a.ir) - mer_over(p, a.rr, a.irr) +
+                mer_over(pu + pd, hhz.h, hhz.ih) - p * drdz;
         }
+        const double r = drhs[(size_t)j * ld + i] - t;
         const unsigned long long bits = (unsigned long long)__double_as_longlong(r) & 0x7fffffffffffffffull;
         if (bits > 0x7ff0000000000000ull) nan = 1;
         else if (bits > m) m = bits;
@@ -470,9 +521,9 @@ template <bool PENTA> __device__ __forceinline__ void mer_solve_body(const MerDe
     }
     for (int l = 1; l <= nlev; ++l) {
         const MerLevel &K = d.lev[l];
-        for (int i = threadIdx.x; i <= K.n1; i += MER_THREADS) ((float4 *)(s_mer + K.o4i))[i] = K.c4i[i];
+        for (int i = threadIdx.x; i < (PENTA ? 2 : 1) * (K.n1 + 1); i += MER_THREADS) ((float4 *)(s_mer + K.oci))[i] = K.ci[i];
         for (int j = threadIdx.x; j <= K.n2; j += MER_THREADS) {
-            ((float4 *)(s_mer + K.o4j))[j] = K.c4j[j];
+            if (PENTA) ((float4 *)(s_mer + K.ocj))[j] = K.cj[j];
             const int o = min((max(j, 1) - 1) / K.rp, cl.size - 1);
             const float *p = s_mer + K.v + (j - o * K.rp) * K.pitch;
             ((unsigned *)(s_mer + K.rows))[j] = o == cl.rank ? cta_addr(p) : peer_addr(p, o);
@@ -507,7 +558,7 @@ template <bool PENTA> __device__ __forceinline__ void mer_solve_body(const MerDe
         k = mer_relax<PENTA>(d, pipe, 1, nlev > 1, k);
         for (int l = 1; l < nlev; ++l) {
             fetch(l + 1);
-            mer_corser(d.lev[l], d.lev[l + 1], d.rc);
+            mer_corser<PENTA>(d.lev[l], d.lev[l + 1], d.rc);
             k = mer_relax<PENTA>(d, pipe, l + 1, l + 1 < nlev, k);
         }
         for (int l = nlev; l >= 2; --l) {
@@ -567,8 +618,8 @@ bool mer_plan(MerDev &d, int ctas)
         L.pitch = std::max(2 + wl_pitch(L.n1 - 1), mer_col(lg, L.n1 + 1) + 1);
         L.v = take((L.rp + 2) * L.pitch);
         L.f = take((L.rp + 2) * L.pitch);
-        L.o4i = take(4 * (L.n1 + 1));
-        L.o4j = take(4 * (L.n2 + 1));
+        L.oci = take((d.penta ? 8 : 4) * (L.n1 + 1));
+        L.ocj = take(d.penta ? 4 * (L.n2 + 1) : 0);
         const int lines = (L.n1 - 2) / nc + 1, share = (lines + ctas - 1) / ctas;
         L.rows = take(L.n2 + 1);
         L.xline = take(lines);
@@ -589,20 +640,21 @@ bool mer_plan(MerDev &d, int ctas)
 
 size_t mer_weight_bytes(const MerDev &d)
 {
-    size_t b = sizeof(MerW) * (size_t)(d.lev[1].n1 + 1 + d.lev[1].n2 + 1);
-    for (int l = 1; l <= d.nlev; ++l) b += sizeof(float4) * (size_t)(d.lev[l].n1 + 1 + d.lev[l].n2 + 1);
+    size_t b = sizeof(MerRow) * (size_t)(d.lev[1].n1 + 1) + sizeof(MerCol) * (size_t)(d.lev[1].n2 + 1);
+    for (int l = 1; l <= d.nlev; ++l) b += sizeof(float4) * (size_t)(2 * (d.lev[l].n1 + 1) + d.lev[l].n2 + 1);
     return b;
 }
 
 void mer_weight_layout(MerDev &d, void *mem)
 {
-    MerW *p = (MerW *)mem;
-    d.d4i = p; p += d.lev[1].n1 + 1;
-    d.d4j = p; p += d.lev[1].n2 + 1;
-    float4 *q = (float4 *)p;
+    MerRow *r = (MerRow *)mem;
+    d.d_i = r; r += d.lev[1].n1 + 1;
+    MerCol *c = (MerCol *)r;
+    d.d_j = c; c += d.lev[1].n2 + 1;
+    float4 *q = (float4 *)c;
     for (int l = 1; l <= d.nlev; ++l) {
-        d.lev[l].c4i = q; q += d.lev[l].n1 + 1;
-        d.lev[l].c4j = q; q += d.lev[l].n2 + 1;
+        d.lev[l].ci = q; q += 2 * (d.lev[l].n1 + 1);
+        d.lev[l].cj = q; q += d.lev[l].n2 + 1;
     }
 }
 

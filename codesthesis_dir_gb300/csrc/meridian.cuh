@@ -6,21 +6,35 @@
 
 #define MER_MAXLEV 8
 
-struct __align__(16) MerW {
-    double x, y, z, w;
+// Level 1's operator in FP64, row i in r and row j in z: the same weights as
+// MerLevel's, with the reciprocals of the divisors (the uniform grid uses r,
+// rr and theirs only).
+struct __align__(16) MerRow {
+    double crr[4], cr[3], r, ir, rr, irr, pad;
+};
+struct __align__(16) MerCol {
+    double czz[4];
+};
+// A divisor and its reciprocal.
+struct MerOver {
+    double h, ih;
 };
 
-// One level.  Off-diagonal weights of row i in r: c4i[i] = (i-1, i+1, far,
-// diagonal), far being i + 2 for i <= n1/2 and i - 2 beyond it (the stretched
-// grid's one-sided points; the uniform grid's far weight is zero), and of
-// row j in z: c4j[j] the same with n2.
+// One level.  The FP32 cycles apply the operators term by term, in the order
+// of the reference's statements.  Stretched grid (rcsc.f): row i's weights of
+// d2/dr2 and of d/dr and 1/r, (crr1 .. crr4), (cr1, cr2, cr3, 1/r), and row j's
+// of d2/dz2, (czz1 .. czz4); the points of row i are i-1 .. i+2 for i <= n1/2
+// and i-2 .. i+1 beyond it, in z likewise.  Uniform grid (rotann2.f): row i's
+// (r, r r, 0, 0) and the spacings h.
 struct MerLevel {
     int n1, n2;
-    const float4 *c4i, *c4j;        // i = 0..n1, j = 0..n2
-    const float *fac_r, *fac_z;     // folded line tables (warpline.cuh) of line 1
+    const float4 *ci;               // i = 0..n1, two a row (stretched) or one
+    const float4 *cj;               // j = 0..n2, stretched only
+    float hr, hhr, hhz, drdz;       // uniform: 1/h's denominators, 2 (1/hhr + 1/hhz)
+    const float *fac_r, *fac_z;     // line tables (warpline.cuh) of line 1
     int fac_r_step, fac_z_step;     // floats from one line's table to the next (0: one table for all)
     // shared-memory plan of one CTA (floats): rows per CTA, row pitch, offsets
-    int rp, pitch, v, f, o4i, o4j;
+    int rp, pitch, v, f, oci, ocj;
     int rows;                       // addresses of the rows of v, j = 0..n2
     int xline;                      // addresses of a colour's z-lines in their owners' line buffers
 };
@@ -29,7 +43,10 @@ struct MerDev {
     int nlev, maxcycles, nrel;
     double tolcon;
     MerLevel lev[MER_MAXLEV];
-    const MerW *d4i, *d4j;       // level 1's weights in FP64
+    const MerRow *d_i;              // level 1, i = 0..n1
+    const MerCol *d_j;              // j = 0..n2
+    MerOver hr, hhr, hhz;           // uniform grid
+    double drdz;
     double *psi;                    // in, and out on convergence; pitch n1 + 1
     const double *rhs;
     double *v;                      // the FP64 iterate, pitch n1 + 1
@@ -43,8 +60,8 @@ struct MerDev {
 // Lays out one CTA's shared memory for clusters of `ctas`; false when a level
 // has lines longer than a warp holds (512 rows) or the arrays do not fit.
 bool mer_plan(MerDev &d, int ctas);
-// The weights of every level and of level 1 in FP64, in one allocation sized
-// by mer_weight_bytes; the levels' n1, n2 must be set.
+// The weights of every level and level 1's in FP64, in one allocation sized
+// by mer_weight_bytes; penta and the levels' n1, n2 must be set.
 size_t mer_weight_bytes(const MerDev &d);
 void mer_weight_layout(MerDev &d, void *mem);
 // Clusters of this size that fit the device for d's plan (halved from want).

@@ -469,7 +469,7 @@ __global__ void __maxnreg__(128) k_mg_solve_mixed(const MgEq *eqs, int first_eq)
     cl.sync();
 }
 
-// FP32 copies of the radii and the folded factors, a block per level.
+// FP32 copies of the radii and the line tables, a block per level.
 __global__ void k_mg_factors32(MgEq eq)
 {
     const MgLevel &L = eq.lev[1 + blockIdx.x];

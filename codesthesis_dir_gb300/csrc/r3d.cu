@@ -65,7 +65,7 @@ struct R3Lev {
     // far is the one-sided rows' point two over
     float4 *wi[4], *wj[4];
     float *wp[4];
-    float *fac32[4][3];         // folded line tables (warpline.cuh); phi-lines: R3Ring per radius
+    float *fac32[4][3];         // fused line tables (warpline.cuh); phi-lines: R3Ring per radius
 };
 
 struct R3Dev {
@@ -1057,7 +1057,7 @@ template <int U = 2> __device__ __forceinline__ void ptdma_staged(const double *
 // 1 - rho^n, is the value it should have entered with.
 struct R3Ring {
     float rho, scale, turn;   // rho, 1/s, 1/(1 - rho^n)
-    int steps;                // scan steps (warpline.cuh); -1: a ring of the level is not diagonally dominant
+    int steps;                // scan steps; -1: a ring of the level is not diagonally dominant
 };
 
 // y(u) = t(u) + rho y(u-1) around the ring of n rows over W = 2^lw lanes (BACK:
@@ -1403,14 +1403,14 @@ template <int COMP, class T> __device__ __noinline__ void r3_phase(int lev, int 
         } else if (kind == 2) {
             r3_rings((const R3Ring *)fac, L.fac[COMP][2], s_line, n, x, lpitch, nl);
         } else if (staged) {
-            if (kind == 0) wl_lines<true>(sfac, dir == 0 ? 0 : len, n, x, lpitch, nl);
-            else wl_lines<false>(sfac, dir == 0 ? 0 : len, n, x, lpitch, nl);
+            if (kind == 0) wl_lines<true, true>(sfac, dir == 0 ? 0 : len, n, x, lpitch, nl);
+            else wl_lines<false, true>(sfac, dir == 0 ? 0 : len, n, x, lpitch, nl);
         } else {   // each line's table from global memory
             for (int t = 0; t < nl; ++t) {
                 const T *tab = fac + (dir == 0 ? 0 : (size_t)((s_line[t] & 0xffff) - 1) * len);
                 if (threadIdx.x < 32) {
-                    if (kind == 0) wl_lines_m<16, true>(tab, 0, n, x + t * lpitch, lpitch, 1, 0, 1);
-                    else wl_lines_m<16, false>(tab, 0, n, x + t * lpitch, lpitch, 1, 0, 1);
+                    if (kind == 0) wl_lines_m<16, true, true>(tab, 0, n, x + t * lpitch, lpitch, 1, 0, 1);
+                    else wl_lines_m<16, false, true>(tab, 0, n, x + t * lpitch, lpitch, 1, 0, 1);
                 }
             }
         }
@@ -1795,7 +1795,7 @@ __global__ void __launch_bounds__(R3_THREADS, 2) k_r3d_solve(const __grid_consta
 // stored as reciprocals.
 // ---------------------------------------------------------------------------
 
-// FP32 folded tables (one thread per line class).
+// FP32 fused tables (one thread per line class).
 __global__ void k_r3d_factors32(const __grid_constant__ R3Dev d, const FacJob *jobs, int njobs)
 {
     const int q = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1806,9 +1806,9 @@ __global__ void k_r3d_factors32(const __grid_constant__ R3Dev d, const FacJob *j
     const int n = r3_len(J.comp, J.dir, L.n1, L.n2, L.n3);
     float *o = L.fac32[J.comp][J.dir] + (size_t)(J.dir == 0 ? 0 : J.ti - 1) * r3_tabsize32(kind, n);
     if (kind == 0) {
-        pdma32_fold(J.tab, n, o);
+        pdma32_fold<true>(J.tab, n, o);
     } else if (kind == 1) {
-        tdma32_fold(J.tab, n, o);
+        tdma32_fold<true>(J.tab, n, o);
     } else {
         double a, b, c, dd, ee;
         r3_coef(L, J.comp, J.dir, J.ti, 0, a, b, c, dd, ee);
@@ -1825,28 +1825,25 @@ __global__ void k_r3d_factors32(const __grid_constant__ R3Dev d, const FacJob *j
     }
 }
 
-// One scan-step count per level, component and direction (block x: level,
-// y: component, z: direction 1 or 2).
+// One scan-step count per level, component and ring direction (block x:
+// level, y: component, z: direction 1 or 2): a warp's rings scan together, and
+// the result must not depend on which rings share a warp.
 __global__ void k_r3d_steps32(const __grid_constant__ R3Dev d)
 {
     const R3Lev &L = d.lev[1 + blockIdx.x];
     const int comp = 1 + blockIdx.y, dir = 1 + blockIdx.z;
-    const int kind = r3_kind(comp, dir), n = r3_len(comp, dir, L.n1, L.n2, L.n3), inst = r3_imax(comp, L.n1);
-    float *tab = L.fac32[comp][dir];
-    if (kind != 2) {
-        wl_common_steps(tab, r3_tabsize32(kind, n), inst);
-    } else {   // the count is a ring's fourth word
-        wl_common_steps(tab + 3, 4, inst);
-        __shared__ int weak;
-        if (threadIdx.x == 0) weak = 0;
-        __syncthreads();
-        R3Ring *ring = (R3Ring *)tab;
-        for (int q = threadIdx.x; q < inst; q += blockDim.x)
-            if (ring[q].scale == 0.f) weak = 1;
-        __syncthreads();
-        if (weak)
-            for (int q = threadIdx.x; q < inst; q += blockDim.x) ring[q].steps = -1;
+    if (r3_kind(comp, dir) != 2) return;
+    const int inst = r3_imax(comp, L.n1);
+    R3Ring *ring = (R3Ring *)L.fac32[comp][dir];
+    __shared__ int most, weak;
+    if (threadIdx.x == 0) most = weak = 0;
+    __syncthreads();
+    for (int q = threadIdx.x; q < inst; q += blockDim.x) {
+        atomicMax(&most, ring[q].steps);
+        if (ring[q].scale == 0.f) weak = 1;
     }
+    __syncthreads();
+    for (int q = threadIdx.x; q < inst; q += blockDim.x) ring[q].steps = weak ? -1 : most;
 }
 
 // Matrix weights of row i in r and of row j in z, from relax's operator: the

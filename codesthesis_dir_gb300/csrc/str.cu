@@ -516,7 +516,7 @@ __global__ void __maxnreg__(255) k_str_solve_mixed(const __grid_constant__ StrDe
 #undef V
 #undef F
 
-// FP32 copies of a level's tables and its folded factors: block row y takes
+// FP32 copies of a level's tables and its line tables: block row y takes
 // level y + 1, one thread per r-line, then per z-line.
 __global__ void k_str_factors32(const __grid_constant__ StrDev d)
 {
@@ -549,34 +549,30 @@ struct gb_str {
     void *mer_mem = nullptr;
 };
 
-// One scan-step count per level and direction (block x: direction).
-__global__ void k_str_steps32(const __grid_constant__ StrDev d)
-{
-    const StrLevel &L = d.lev[1 + blockIdx.y];
-    if (blockIdx.x == 0) wl_common_steps(L.fac_r32, pdma32_len(L.n1 - 1), L.n2 - 1);
-    else wl_common_steps(L.fac_z32, pdma32_len(L.n2 - 1), L.n1 - 1);
-}
-
-// The resident solve's weights: grid.f's first and second derivatives of a
-// row combined in FP64 (and rounded once for the correction cycles).
+// The resident solve's weights: grid.f's in FP32 for every level and in FP64
+// for level 1's residual.
 __global__ void k_str_weights(const __grid_constant__ StrDev d, const __grid_constant__ MerDev m)
 {
     const int l = 1 + blockIdx.y, t = blockIdx.x * blockDim.x + threadIdx.x;
     const StrLevel &L = d.lev[l];
-    auto put = [&](const float4 *c4, const MerW *d4, int q, double cm, double cp, double cf, double cd) {
-        const_cast<float4 *>(c4)[q] = make_float4((float)cm, (float)cp, (float)cf, (float)cd);
-        if (l == 1) const_cast<MerW *>(d4)[q] = MerW{cm, cp, cf, cd};
-    };
     if (t >= 1 && t < L.n1) {
         const int i = t;
-        const double r = L.r[i], cr1 = CR(i, 1) / r, cr2 = CR(i, 2) / r - 1.0 / (r * r), cr3 = CR(i, 3) / r;
-        if (i <= L.n1 / 2) put(m.lev[l].c4i, m.d4i, i, CRR(i, 1) + cr1, CRR(i, 3) + cr3, CRR(i, 4), CRR(i, 2) + cr2);
-        else put(m.lev[l].c4i, m.d4i, i, CRR(i, 2) + cr1, CRR(i, 4) + cr3, CRR(i, 1), CRR(i, 3) + cr2);
+        float4 *c = const_cast<float4 *>(m.lev[l].ci) + 2 * i;
+        const float *crr = L.crr32 + 4 * (i - 1), *cr = L.cr32 + 3 * (i - 1);
+        c[0] = make_float4(crr[0], crr[1], crr[2], crr[3]);
+        c[1] = make_float4(cr[0], cr[1], cr[2], 1.0f / L.r32[i]);
+        if (l == 1) {
+            const double r = L.r[i];
+            const_cast<MerRow *>(m.d_i)[i] = MerRow{{CRR(i, 1), CRR(i, 2), CRR(i, 3), CRR(i, 4)}, {CR(i, 1), CR(i, 2), CR(i, 3)},
+                                                    r, L.ir[i], r * r, L.irr[i], 0.0};
+        }
     }
     if (t >= 1 && t < L.n2) {
         const int j = t;
-        if (j <= L.n2 / 2) put(m.lev[l].c4j, m.d4j, j, CZZ(j, 1), CZZ(j, 3), CZZ(j, 4), CZZ(j, 2));
-        else put(m.lev[l].c4j, m.d4j, j, CZZ(j, 2), CZZ(j, 4), CZZ(j, 1), CZZ(j, 3));
+        const float *czz = L.czz32 + 4 * (j - 1);
+        const_cast<float4 *>(m.lev[l].cj)[j] = make_float4(czz[0], czz[1], czz[2], czz[3]);
+        if (l == 1)
+            const_cast<MerCol *>(m.d_j)[j] = MerCol{{CZZ(j, 1), CZZ(j, 2), CZZ(j, 3), CZZ(j, 4)}};
     }
 }
 
@@ -751,7 +747,6 @@ extern "C" int gb_str_create(int nlev, const gb_str_level *lv, double tolcon, in
     cudaFree(work);
     if (e == cudaSuccess) {
         k_str_factors32<<<dim3(gb_ceil_div((size_t)n1 + n2, 32), nlev), 32>>>(d);
-        k_str_steps32<<<dim3(2, nlev), 256>>>(d);
         e = cudaDeviceSynchronize();
     }
     if (e != cudaSuccess) { gb_set_error("gb_str_create: factors: %s", cudaGetErrorString(e)); gb_str_destroy(h); return GB_ERR_CUDA; }
