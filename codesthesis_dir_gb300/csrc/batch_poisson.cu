@@ -512,123 +512,293 @@ __device__ void op_prolong(const BatchDev &B, TileEntry e, int l, int src, int d
 // Coarse levels of one problem in shared memory (one block per problem):
 // the V-cycle below level dloc, solution and right-hand side of every level
 // resident, residuals formed inside the restriction.
+//
+// Everything is latency here (60 dependent phases, 63 x 63 points at most), in
+// FP64 also the FP64 pipe, so the phases are short: n = 2^LG + 1, so a colour of
+// a row is 2^(LG-1) slots, and with the level and the thread count known when
+// compiling all indexing is immediates (run-time: 400 to 450 cycles a phase of
+// the 17 and 33 levels); the two colours stand in separate halves (n is odd:
+// the parity of row + column is the parity of the linear index), so a phase
+// reads consecutive words; a restriction forms six residuals per coarse point,
+// its left fine columns, and gets the right one from the next lane (nine
+// before); the levels up to LOC_SOLO, one warp's worth of points a colour, are
+// one warp's, which needs no block barrier.  k_local, n = 65: 28.8 -> 15 us in
+// FP32; FP64 76 -> 68 us, of which the FP64 pipe's instructions are 50.
 // ---------------------------------------------------------------------------
-// One colour of a red-black sweep over the interior: the points of that
-// colour only, (m + 1) / 2 slots per row (row j starts at i = 1 or 2).
-template <class T>
-__device__ void loc_rb_half(T *x, const T *f, int n, T h2, int color)
+#define LOC_SOLO 3      // LG of the largest one-warp level (n = 9)
+#define LOC_MAX 7       // of the largest local level (n = 129)
+
+// One level's arrays: per colour half the even (odd) linear indices, a whole
+// number of 128-byte rows and half a row, so that accesses alternating between
+// the halves use different banks; the coarser levels' arrays come first.
+__host__ __device__ constexpr int loc_half(int n, int words) { return ((n * n + 1) / 2 + words - 1) / words * words + words / 2; }
+__host__ __device__ constexpr int loc_offset(int lg, int words)
 {
-    const int m = n - 2, w = (m + 1) >> 1;
-    for (int q = threadIdx.x; q < m * w; q += blockDim.x) {
-        const int jj = q / w, j = jj + 1;
-        const int i = 1 + ((1 + j + color) & 1) + 2 * (q - jj * w);
-        if (i > m) continue;
-        const int c = j * n + i;
-        const T s = (x[c - 1] + x[c + 1]) + (x[c - n] + x[c + n]);
-        x[c] = fmaT<T>(-h2, f[c], s) * (T)0.25;
+    int o = 0;
+    for (int k = 1; k < lg; ++k) o += 4 * loc_half((1 << k) + 1, words);
+    return o;
+}
+template <class T, int LG> struct Loc {
+    static constexpr int W = 128 / (int)sizeof(T);
+    static constexpr int n = (1 << LG) + 1, m = n - 2, half = loc_half(n, W), d = (n - 1) / 2;
+    T *X, *F;
+    __device__ __forceinline__ explicit Loc(T *mem) : X(mem + loc_offset(LG, W)), F(X + 2 * half) {}
+    __device__ __forceinline__ static int at(int c) { return (c & 1) * half + (c >> 1); }
+    __device__ __forceinline__ static T ih2() { return (T)(1 << LG) * (T)(1 << LG); }
+};
+
+// A thread's slots of a level: slot s of rows j, j + R, ... (NT threads are R
+// whole rows; R is even, so row j + R lies R n / 2 further on in either half).
+template <int LG, int NT> struct LocSlot {
+    static constexpr int lw = LG - 1, w = 1 << lw, R = NT >> lw;
+    int j, s;
+    __device__ __forceinline__ LocSlot() : j(((int)threadIdx.x >> lw) + 1), s(threadIdx.x & (w - 1)) {}
+};
+template <int NT> __device__ __forceinline__ void loc_sync()
+{
+    if constexpr (NT == 32) __syncwarp();
+    else __syncthreads();
+}
+
+// nu red-black sweeps over the interior: a colour's points only, w slots per
+// row (row j starts at i = 1 or 2).  With p = c >> 1 the place of c in its
+// half, its neighbours lie in the other half at p - 1, p (even c) or p, p + 1
+// (odd), and d + 1 - odd before and d + odd after.  All of a thread's loads of
+// a colour (up to four rows') go out together.
+template <class T, int LG, int NT, int COLOR> __device__ __forceinline__ void loc_color(const Loc<T, LG> &L, const LocSlot<LG, NT> &S)
+{
+    using V = Loc<T, LG>;
+    using Q = LocSlot<LG, NT>;
+    constexpr int rows = (V::m + Q::R - 1) / Q::R, U = rows < 4 ? rows : 4, step = (Q::R * V::n) / 2;
+    const T h2 = (T)1 / V::ih2();
+    const int i = 1 + ((1 + S.j + COLOR) & 1) + 2 * S.s;
+    const int p0 = (S.j * V::n + i) >> 1;
+    T *x = L.X + COLOR * V::half + p0;
+    const T *f = L.F + COLOR * V::half + p0, *o = L.X + (COLOR ^ 1) * V::half + COLOR + p0;
+#pragma unroll
+    for (int u0 = 0; u0 < rows; u0 += U) {
+        T v[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            if (i > V::m || S.j + (u0 + u) * Q::R > V::m) continue;
+            const T *q = o + (u0 + u) * step;
+            const T s = (q[-1] + q[0]) + (q[-V::d - 1] + q[V::d]);
+            v[u] = fmaT<T>(-h2, f[(u0 + u) * step], s) * (T)0.25;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (i <= V::m && S.j + (u0 + u) * Q::R <= V::m) x[(u0 + u) * step] = v[u];
     }
-    __syncthreads();
+    loc_sync<NT>();
 }
-
-template <class T>
-__device__ __forceinline__ T loc_residual(const T *x, const T *f, int n, int c, T ih2)
+template <class T, int LG, int NT> __device__ __forceinline__ void loc_smooth(const Loc<T, LG> &L, int nu)
 {
-    const T s = (x[c - 1] + x[c + 1]) + (x[c - n] + x[c + n]);
-    const T lap = fmaT<T>((T)-4, x[c], s);
-    return fmaT<T>(-ih2, lap, f[c]);
+    const LocSlot<LG, NT> S;
+#pragma unroll 1
+    for (int s = 0; s < nu; ++s) {
+        loc_color<T, LG, NT, 0>(L, S);
+        loc_color<T, LG, NT, 1>(L, S);
+    }
 }
 
-// zero0: the level-dloc solution starts at zero (a coarse correction, or the
-// first inner cycle of a mixed solve); corr0 (dloc == 0 only): add the
-// result to the solution instead of storing it, as float pairs or (f64) to
+// f - A x at place p of a colour.
+template <int COLOR, class T, int LG> __device__ __forceinline__ T loc_residual(const Loc<T, LG> &L, int p)
+{
+    using V = Loc<T, LG>;
+    const T *o = L.X + (COLOR ^ 1) * V::half + COLOR + p;
+    const T s = (o[-1] + o[0]) + (o[-V::d - 1] + o[V::d]);
+    const T lap = fmaT<T>((T)-4, L.X[COLOR * V::half + p], s);
+    return fmaT<T>(-V::ih2(), lap, L.F[COLOR * V::half + p]);
+}
+
+// The residual's full weighting (rotann2.f:773-785 summation order) into the
+// coarse right-hand side, and zeros into its solution; whole warps.  Slot s of
+// coarse row J takes column I = s + 1 and forms the residuals of fine columns
+// 2 I - 1 and 2 I; column 2 I + 1 is the next slot's.
+template <class T, int LG, int NT> __device__ __forceinline__ void loc_restrict(const Loc<T, LG> &L, const Loc<T, LG - 1> &C)
+{
+    using V = Loc<T, LG>;
+    using Q = LocSlot<LG, NT>;
+    constexpr int mc = Loc<T, LG - 1>::m, nc = Loc<T, LG - 1>::n, d = V::d, width = Q::w < 32 ? Q::w : 32;
+    const Q S;
+    const int I = S.s + 1, lane = threadIdx.x & 31;
+    const bool col = I <= mc;   // the last slot's column 2 I is the boundary
+#pragma unroll 1
+    for (int J0 = 1; J0 <= mc; J0 += Q::R) {
+        const int J = min(J0 + S.j - 1, mc);
+        const int p = J * V::n + I;   // place of (2 J, 2 I), an even point
+        T k0 = (T)0, k1 = (T)0, k2 = (T)0;
+        const T l0 = loc_residual<0>(L, p - d - 1), l1 = loc_residual<1>(L, p - 1), l2 = loc_residual<0>(L, p + d);
+        if (col) {
+            k0 = loc_residual<1>(L, p - d - 1);
+            k1 = loc_residual<0>(L, p);
+            k2 = loc_residual<1>(L, p + d);
+        }
+        T r0 = __shfl_down_sync(0xffffffffu, l0, 1, width), r1 = __shfl_down_sync(0xffffffffu, l1, 1, width);
+        T r2 = __shfl_down_sync(0xffffffffu, l2, 1, width);
+        if (Q::w > 32 && lane == 31 && col) {   // the next slot is another warp's
+            r0 = loc_residual<0>(L, p - d);
+            r1 = loc_residual<1>(L, p);
+            r2 = loc_residual<0>(L, p + d + 1);
+        }
+        T t = k1;
+        t = t * (T)2 + r1 + l1;
+        t = t + k2 + k0;
+        t = t * (T)2 + r2 + l0;
+        t = t + r0 + l2;
+        if (col && J0 + S.j - 1 <= mc) {
+            const int o = C.at(J * nc + I);
+            C.F[o] = t * (T)0.0625;
+            C.X[o] = (T)0;
+        }
+    }
+    loc_sync<NT>();
+}
+
+// Bilinear prolongation added (rotann2.f:821-858): slot s of fine row j takes
+// columns 2 s + 1 and 2 s + 2.
+template <class T, int LG, int NT> __device__ __forceinline__ void loc_prolong(const Loc<T, LG> &L, const Loc<T, LG - 1> &C)
+{
+    using V = Loc<T, LG>;
+    using Q = LocSlot<LG, NT>;
+    constexpr int nc = Loc<T, LG - 1>::n;
+    const Q S;
+#pragma unroll 1
+    for (int j = S.j; j <= V::m; j += Q::R) {
+        const int s = S.s, e = (j >> 1) * nc + s, c = j * V::n + 2 * s + 1;
+        const T e00 = C.X[C.at(e)], e01 = C.X[C.at(e + 1)];
+        T v1, v2;
+        if ((j & 1) == 0) {
+            v1 = (e00 + e01) * (T)0.5;
+            v2 = e01;
+        } else {
+            const T e10 = C.X[C.at(e + nc)], e11 = C.X[C.at(e + nc + 1)];
+            T t = e00 + e11;
+            t = t + e10 + e01;
+            v1 = t * (T)0.25;
+            v2 = (e01 + e11) * (T)0.5;
+        }
+        T *x1 = L.X + L.at(c), *x2 = L.X + L.at(c + 1);
+        *x1 = *x1 + v1;
+        if (2 * s + 2 <= V::m) *x2 = *x2 + v2;
+    }
+    loc_sync<NT>();
+}
+
+// One V-cycle on a level's X and F; the coarser levels start from zero (their
+// boundary values are kept zero by loc_clear).  The levels up to LOC_SOLO run
+// in the first warp.
+template <class T, int LG, int NT> __device__ __noinline__ void loc_cycle(T *mem, int nu1, int nu2)
+{
+    const Loc<T, LG> L(mem);
+    if constexpr (LG == 1) {
+        loc_color<T, 1, NT, 0>(L, LocSlot<1, NT>());
+    } else {
+        loc_smooth<T, LG, NT>(L, nu1);
+        const Loc<T, LG - 1> C(mem);
+        loc_restrict<T, LG, NT>(L, C);
+        if constexpr (NT > 32 && LG - 1 <= LOC_SOLO) {
+            if (threadIdx.x < 32) loc_cycle<T, LG - 1, 32>(mem, nu1, nu2);
+            __syncthreads();
+        } else {
+            loc_cycle<T, LG - 1, NT>(mem, nu1, nu2);
+        }
+        loc_prolong<T, LG, NT>(L, C);
+        loc_smooth<T, LG, NT>(L, nu2);
+    }
+}
+
+// Calls g with the block's level as a constant.
+template <int LG, class G> __device__ __forceinline__ void loc_with_level(int lg, const G &g)
+{
+    if constexpr (LG >= 1) {
+        if (lg == LG) g(std::integral_constant<int, LG>());
+        else loc_with_level<LG - 1>(lg, g);
+    }
+}
+template <class T, int NT> __device__ __forceinline__ void loc_vcycle(T *mem, int lg, int nu1, int nu2)
+{
+    constexpr int most = sizeof(T) == 8 ? LOC_MAX - 1 : LOC_MAX;
+    loc_with_level<most>(lg, [&](auto c) {
+        constexpr int LG = decltype(c)::value;
+        if constexpr (LG <= LOC_SOLO) {
+            if (threadIdx.x < 32) loc_cycle<T, LG, 32>(mem, nu1, nu2);
+            __syncthreads();
+        } else {
+            loc_cycle<T, LG, NT>(mem, nu1, nu2);
+        }
+    });
+}
+
+// Level lg's arrays where lg is not a constant.
+template <class T> struct LocTop {
+    int half;
+    T *X, *F;
+    __device__ __forceinline__ LocTop(T *mem, int lg)
+    {
+        constexpr int W = 128 / (int)sizeof(T);
+        half = loc_half((1 << lg) + 1, W);
+        X = mem + loc_offset(lg, W);
+        F = X + 2 * half;
+        // the boundary values of the coarser levels (the block synchronises)
+        for (T *q = mem + threadIdx.x; q < X; q += blockDim.x) *q = (T)0;
+    }
+    __device__ __forceinline__ int at(int c) const { return (c & 1) * half + (c >> 1); }
+};
+
+// zero_level0: the level-dloc solution starts at zero (a coarse correction, or
+// the first inner cycle of a mixed solve); correct_level0 (dloc == 0 only): add
+// the result to the solution instead of storing it, as float pairs or (f64) to
 // the FP64 solution.
-template <class T>
+template <class T, int NT>
 __device__ void op_local(const BatchDev &B, int p, int nu1, int nu2, int zero_level0, int correct_level0,
                          int f64, unsigned char *smem)
 {
-    T *sm = (T *)smem;
-    const int L = B.nlev[p], d0 = B.dloc[p];
-    int off[BP_MAXL];
-    int tot = 0;
-    for (int l = d0; l < L; ++l) {
-        off[l] = tot;
-        const int n = B.n_of[p * BP_MAXL + l];
-        tot += n * n;
-    }
-    T *X = sm, *F = sm + tot;
-    for (int q = threadIdx.x; q < tot; q += blockDim.x) { X[q] = (T)0; F[q] = (T)0; }
-    __syncthreads();
+    const int d0 = B.dloc[p], n0 = B.n_of[p * BP_MAXL + d0], lg = 31 - __clz(n0 - 1);
+    const int tid = threadIdx.x, nthr = NT;
+    const LocTop<T> v((T *)smem, lg);
     {
         const bool zero = d0 > 0 || zero_level0;
-        const int n = B.n_of[p * BP_MAXL + d0];
         const T *gx = XS<T>(B, p, d0, 0), *gf = FP<T>(B, p, d0);
-        for (int q = threadIdx.x; q < n * n; q += blockDim.x) {
-            if (!zero) X[q] = gx[q];
-            F[q] = gf[q];
+        constexpr int U = 5;   // loads in flight
+        for (int q0 = tid; q0 < n0 * n0; q0 += U * nthr) {
+            T x[U], f[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int q = min(q0 + u * nthr, n0 * n0 - 1);
+                x[u] = zero ? (T)0 : gx[q];
+                f[u] = gf[q];
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int q = min(q0 + u * nthr, n0 * n0 - 1);
+                v.X[v.at(q)] = x[u];
+                v.F[v.at(q)] = f[u];
+            }
         }
     }
     __syncthreads();
-    for (int l = d0; l < L - 1; ++l) {
-        const int n = B.n_of[p * BP_MAXL + l], nc = B.n_of[p * BP_MAXL + l + 1];
-        T *x = X + off[l], *f = F + off[l];
-        const T h2 = H2<T>(B, p, l), ih2 = IH2<T>(B, p, l);
-        for (int s = 0; s < nu1; ++s) { loc_rb_half(x, f, n, h2, 0); loc_rb_half(x, f, n, h2, 1); }
-        T *fc = F + off[l + 1];
-        const int mc = nc - 2;
-        for (int q = threadIdx.x; q < mc * mc; q += blockDim.x) {
-            const int j = q / mc + 1, i = q - (j - 1) * mc + 1;
-            const int c = (2 * j) * n + 2 * i;
-            T t = loc_residual(x, f, n, c, ih2);
-            t = t * (T)2 + loc_residual(x, f, n, c + 1, ih2) + loc_residual(x, f, n, c - 1, ih2);
-            t = t + loc_residual(x, f, n, c + n, ih2) + loc_residual(x, f, n, c - n, ih2);
-            t = t * (T)2 + loc_residual(x, f, n, c + 1 + n, ih2) + loc_residual(x, f, n, c - 1 - n, ih2);
-            t = t + loc_residual(x, f, n, c + 1 - n, ih2) + loc_residual(x, f, n, c - 1 + n, ih2);
-            fc[j * nc + i] = t * (T)0.0625;
-        }
-        __syncthreads();
-    }
-    {
-        const int n = B.n_of[p * BP_MAXL + L - 1];
-        loc_rb_half(X + off[L - 1], F + off[L - 1], n, H2<T>(B, p, L - 1), 0);
-    }
-    for (int l = L - 2; l >= d0; --l) {
-        const int n = B.n_of[p * BP_MAXL + l], nc = B.n_of[p * BP_MAXL + l + 1], m = n - 2;
-        T *x = X + off[l], *f = F + off[l];
-        const T *ec = X + off[l + 1];
-        for (int q = threadIdx.x; q < m * m; q += blockDim.x) {
-            const int j = q / m + 1, i = q - (j - 1) * m + 1;
-            const T *ep = ec + (j / 2) * nc + (i / 2);
-            T v;
-            if ((i & 1) == 0) {
-                if ((j & 1) == 0) v = ep[0];
-                else v = (ep[0] + ep[nc]) * (T)0.5;
-            } else {
-                if ((j & 1) == 0) v = (ep[0] + ep[1]) * (T)0.5;
-                else {
-                    T t = ep[0] + ep[nc + 1];
-                    t = t + ep[nc] + ep[1];
-                    v = t * (T)0.25;
-                }
+    loc_vcycle<T, NT>((T *)smem, lg, nu1, nu2);
+    auto correct = [&](auto *psi, auto add) {
+        constexpr int U = 5;
+        for (int q0 = tid; q0 < n0 * n0; q0 += U * nthr) {
+            decltype(add(*psi, v.X[0])) o[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) o[u] = psi[min(q0 + u * nthr, n0 * n0 - 1)];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const int q = q0 + u * nthr;
+                if (q < n0 * n0) psi[q] = add(o[u], v.X[v.at(q)]);
             }
-            const int c = j * n + i;
-            x[c] = x[c] + v;
         }
-        __syncthreads();
-        const T h2 = H2<T>(B, p, l);
-        for (int s = 0; s < nu2; ++s) { loc_rb_half(x, f, n, h2, 0); loc_rb_half(x, f, n, h2, 1); }
-    }
-    {
-        const int n = B.n_of[p * BP_MAXL + d0];
-        if (d0 == 0 && correct_level0 && f64) {
-            double *psi = (double *)B.psi[p];
-            for (int q = threadIdx.x; q < n * n; q += blockDim.x) psi[q] = psi[q] + f2d((float)X[q]);
-        } else if (d0 == 0 && correct_level0) {
-            float2 *psi = (float2 *)B.psi[p];
-            for (int q = threadIdx.x; q < n * n; q += blockDim.x) psi[q] = df_add_f(psi[q], (float)X[q]);
-        } else {
-            T *gx = XS<T>(B, p, d0, 0);
-            for (int q = threadIdx.x; q < n * n; q += blockDim.x) gx[q] = X[q];
-        }
+    };
+    if (d0 == 0 && correct_level0 && f64) {
+        correct((double *)B.psi[p], [](double a, T e) { return a + f2d((float)e); });
+    } else if (d0 == 0 && correct_level0) {
+        correct((float2 *)B.psi[p], [](float2 a, T e) { return df_add_f(a, (float)e); });
+    } else {
+        T *gx = XS<T>(B, p, d0, 0);
+        for (int q = tid; q < n0 * n0; q += nthr) gx[q] = v.X[v.at(q)];
     }
     __syncthreads();
 }
@@ -910,7 +1080,7 @@ __device__ __forceinline__ void run_item(const BatchDev &B, const TileEntry *til
     }
     case OP_LOCAL:
         if (!B.active[item]) return;
-        op_local<T>(B, item, nu1, nu2, op.aux & 1, (op.aux >> 1) & 1, (op.aux >> 2) & 1, smem);
+        op_local<T, TILE_THREADS>(B, item, nu1, nu2, op.aux & 1, (op.aux >> 1) & 1, (op.aux >> 2) & 1, smem);
         return;
     case OP_OUTER:
         if (op.nu) run_outer<T, true>(B, tiles[op.off + item], item, f_p, op, smem);
@@ -929,6 +1099,7 @@ __device__ __forceinline__ void run_item(const BatchDev &B, const TileEntry *til
 // The coarse levels of every problem below its tiled levels (graph path):
 // one block of LOCAL_THREADS per problem.
 #define LOCAL_THREADS 512
+#define LOCAL_SOLVE_SMEM (220 * 1024)
 // Programmatic dependent launch (the graph path's kernels are launched with
 // programmatic stream serialization): a kernel may be scheduled while its
 // predecessor's last blocks still run, and waits here until that
@@ -947,7 +1118,129 @@ __global__ void __launch_bounds__(LOCAL_THREADS) k_local(BatchDev B, Op op, int 
     extern __shared__ __align__(16) unsigned char smem_raw[];
     grid_dependency_wait();
     if (!B.active[blockIdx.x]) return;
-    op_local<T>(B, blockIdx.x, nu1, nu2, op.aux & 1, (op.aux >> 1) & 1, (op.aux >> 2) & 1, smem_raw);
+    op_local<T, LOCAL_THREADS>(B, blockIdx.x, nu1, nu2, op.aux & 1, (op.aux >> 1) & 1, (op.aux >> 2) & 1, smem_raw);
+}
+
+// Whole solves of problems that are local altogether (dloc 0), one block each:
+// the outer iteration of OP_OUTER, OP_FINALIZE and OP_LOCAL with the solution
+// and the right-hand side (V: FP64, or float pairs) in shared memory beside the
+// inner hierarchy; in plain FP64 the hierarchy's level 0 holds both.  The
+// operations are the same; the norm's sum runs in another order.
+//
+// As single launches an iteration of a small batch is launch and host latency
+// (eight problems of n = 17 .. 65, FP64 outer: 55 us an iteration, 550 us a
+// solve; here 20 us an iteration, most of it the FP64 residual, and 250 us a
+// solve).
+template <class T, int CM> struct LocOuter {
+    using V = typename CorrVal<CM>::type;
+};
+template <class T> struct LocOuter<T, CM_NONE> {
+    using V = double;
+};
+template <class T, int CM>
+__global__ void __launch_bounds__(LOCAL_THREADS) k_local_solve(BatchDev B, const double *const *f_p, int nu1, int nu2, int hierarchy)
+{
+    using V = typename LocOuter<T, CM>::V;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ double s_part[LOCAL_THREADS / 32];
+    __shared__ int s_go;
+    const int p = blockIdx.x, n = B.n_of[p * BP_MAXL], lg = 31 - __clz(n - 1), m = n - 2, tid = threadIdx.x, nthr = LOCAL_THREADS;
+    T *mem = (T *)smem_raw;
+    const LocTop<T> v(mem, lg);
+    V *psi = (V *)(smem_raw + hierarchy), *f = psi + n * n;
+    const V *gf = ((const V *const *)f_p)[p];
+    V *gpsi = (V *)B.psi[p];
+    V zero;
+    if constexpr (CM == CM_PAIR) zero = make_float2(0.f, 0.f);
+    else zero = 0.0;
+    for (int q = tid; q < n * n; q += nthr) {
+        if constexpr (CM == CM_NONE) {
+            v.X[v.at(q)] = (T)0;
+            v.F[v.at(q)] = gf[q];
+        } else {
+            psi[q] = zero;
+            f[q] = gf[q];
+        }
+    }
+    __syncthreads();
+    const int ls = lg;   // n - 1 slots a row, the first the boundary column
+    const T ih2 = (T)(n - 1) * (T)(n - 1);
+    double fnorm = 0.0;
+    int cycles = 0;
+    for (bool first = true;; first = false) {
+        double acc = 0.0;
+        for (int q = tid; q < m << ls; q += nthr) {
+            const int j = (q >> ls) + 1, i = q & ((1 << ls) - 1), c = j * n + i;
+            if (i == 0) continue;
+            double rw;
+            if constexpr (CM == CM_NONE) {
+                const T sum = (v.X[v.at(c - 1)] + v.X[v.at(c + 1)]) + (v.X[v.at(c - n)] + v.X[v.at(c + n)]);
+                rw = __fma_rn(-ih2, __fma_rn(-4.0, v.X[v.at(c)], sum), v.F[v.at(c)]);
+            } else if constexpr (CM == CM_PAIR) {
+                float2 r;
+                if (first) {
+                    r = df_add(f[c], make_float2(-0.0f, -0.0f));
+                } else {
+                    const float2 sum = df_add(df_add(psi[c - 1], psi[c + 1]), df_add(psi[c - n], psi[c + n]));
+                    const float2 lap = df_add(sum, df_scale(psi[c], -4.0f));
+                    r = df_add(f[c], df_scale(lap, -ih2));
+                }
+                rw = f2d(r.x);
+                v.F[v.at(c)] = r.x;
+            } else {
+                if (first) {
+                    rw = f[c];
+                } else {
+                    const double sum = (psi[c - 1] + psi[c + 1]) + (psi[c - n] + psi[c + n]);
+                    const double lap = __fma_rn(-4.0, psi[c], sum);
+                    rw = __fma_rn(-f2d(ih2), lap, f[c]);
+                }
+                v.F[v.at(c)] = d2f_rn(rw);
+            }
+            acc = __fma_rn(rw, rw, acc);
+        }
+        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if ((tid & 31) == 0) s_part[tid >> 5] = acc;
+        __syncthreads();
+        if (tid == 0) {   // op_finalize
+            double s = 0.0;
+            for (int w = 0; w < nthr / 32; ++w) s += s_part[w];
+            const double rn = sqrt(s);
+            if (first) fnorm = rn;
+            B.relres[p] = fnorm > 0.0 ? rn / fnorm : 0.0;
+            int failed = 0;
+            s_go = 0;
+            if (!(rn <= 1.79769313486231570815e308)) failed = 2;
+            else if (rn <= B.rtol * fnorm) failed = 0;
+            else if (cycles >= B.max_cycles) failed = 1;
+            else s_go = 1;
+            if (s_go) cycles += B.inner;
+            else B.failed[p] = failed;
+        }
+        __syncthreads();
+        if (!s_go) break;
+        if constexpr (CM == CM_NONE) {
+            loc_vcycle<T, LOCAL_THREADS>(mem, lg, nu1, nu2);
+        } else {
+            for (int q = tid; q < 2 * v.half; q += nthr) v.X[q] = (T)0;
+            __syncthreads();
+            for (int k = 0; k < B.inner; ++k) loc_vcycle<T, LOCAL_THREADS>(mem, lg, nu1, nu2);
+            for (int q = tid; q < n * n; q += nthr) {
+                if constexpr (CM == CM_PAIR) psi[q] = df_add_f(psi[q], v.X[v.at(q)]);
+                else psi[q] = psi[q] + f2d(v.X[v.at(q)]);
+            }
+            __syncthreads();
+        }
+    }
+    for (int q = tid; q < n * n; q += nthr) {
+        if constexpr (CM == CM_NONE) gpsi[q] = v.X[v.at(q)];
+        else gpsi[q] = psi[q];
+    }
+    if (tid == 0) {
+        B.cycles[p] = cycles;
+        B.fnorm[p] = fnorm;
+        B.active[p] = 0;
+    }
 }
 
 // One kernel launch per operation (graph path).
@@ -1419,8 +1712,8 @@ static int batch_create(int nprob, const int *n, int precision, int nu1, int nu2
     size_t smax = 0;
     for (int p = 0; p < nprob; ++p) {
         size_t sz = 0;
-        for (int l = b->dloc[p]; l < b->L[p]; ++l) sz += (size_t)nof[(size_t)p * BP_MAXL + l] * nof[(size_t)p * BP_MAXL + l];
-        smax = std::max(smax, 2 * sz * esz);
+        for (int l = b->dloc[p]; l < b->L[p]; ++l) sz += 4 * (size_t)loc_half(nof[(size_t)p * BP_MAXL + l], 128 / (int)esz);
+        smax = std::max(smax, sz * esz);
     }
     b->local_smem = smax;
     // tile tables
@@ -1895,6 +2188,24 @@ static int solve_graph(gb_batch *b, cudaStream_t s)
     return GB_OK;
 }
 
+// Whether every problem is local altogether and one block holds its solve.
+static size_t whole_local_smem(const gb_batch *b)
+{
+    const int n = *std::max_element(b->n.begin(), b->n.end());
+    if (b->maxdepth_global > 0) return 0;
+    const size_t sm = b->local_smem + (inner32(b) ? 2 * 8 * (size_t)n * n : 0);
+    return sm <= LOCAL_SOLVE_SMEM ? sm : 0;
+}
+
+template <class T, int CM> static int solve_local(gb_batch *b, size_t sm, cudaStream_t s)
+{
+    GB_CUDA_TRY(cudaFuncSetAttribute(k_local_solve<T, CM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    k_local_solve<T, CM><<<b->nprob, LOCAL_THREADS, sm, s>>>(b->dev, (const double *const *)b->d_f_tab, b->nu1, b->nu2, (int)b->local_smem);
+    GB_CUDA_TRY(cudaGetLastError());
+    b->launches += 1;
+    return GB_OK;
+}
+
 static int solve_persistent(gb_batch *b, cudaStream_t s)
 {
     const int n0 = (int)b->ops0.size(), n1 = (int)b->ops.size();
@@ -1974,7 +2285,11 @@ extern "C" int gb_batch_solve_device(gb_batch *b, const double *d_f, double *d_p
     GB_CUDA_TRY(cudaMemcpyAsync(D.active, ones.data(), sizeof(int) * b->nprob, cudaMemcpyHostToDevice, s));
     GB_CUDA_TRY(cudaMemsetAsync(D.cycles, 0, sizeof(int) * b->nprob, s));
     GB_CUDA_TRY(cudaMemsetAsync(D.failed, 0, sizeof(int) * b->nprob, s));
-    st = b->exec == GB_BATCH_EXEC_PERSISTENT ? solve_persistent(b, s) : solve_graph(b, s);
+    const size_t whole = b->exec == GB_BATCH_EXEC_GRAPH && !b->profile ? whole_local_smem(b) : 0;
+    if (whole && b->precision == GB_BATCH_FP64) st = solve_local<double, CM_NONE>(b, whole, s);
+    else if (whole && b->precision == GB_BATCH_MIXED) st = solve_local<float, CM_PAIR>(b, whole, s);
+    else if (whole) st = solve_local<float, CM_F64>(b, whole, s);
+    else st = b->exec == GB_BATCH_EXEC_PERSISTENT ? solve_persistent(b, s) : solve_graph(b, s);
     if (st != GB_OK) return st;
     if (b->precision == GB_BATCH_MIXED && b->total > 0) {
         // the mixed solve held psi as float pairs in place: back to FP64
