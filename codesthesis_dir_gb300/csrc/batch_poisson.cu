@@ -1312,6 +1312,7 @@ struct gb_batch {
     std::vector<int> n, L, dloc;
     long long total = 0;
     std::vector<long long> off0;        // level-0 offsets in the packed user arrays
+    long long *d_off0 = nullptr;
     int maxdepth_global = 0;            // levels 0..maxdepth_global-1 have tile work
     void *pool = nullptr;               // per-level x (two buffers), f (T = double or float)
     size_t pool_bytes = 0;
@@ -1365,6 +1366,7 @@ struct gb_batch {
     double kind_ms[8] = {0}, kind_bytes[8] = {0};
     long long kind_launches[8] = {0};
     int *h_active = nullptr;            // page-locked: the active flags after a profiled iteration
+    double *h_out = nullptr;            // page-locked: relres, cycles, failed of a solve
     int nsm = 0;                        // the device's SMs (grid-stride element-wise launches)
     std::vector<int> prof_prev;         // the flags before it: the problems its outer pass covered
 };
@@ -1783,6 +1785,9 @@ static int batch_create(int nprob, const int *n, int precision, int nu1, int nu2
     BTRY(cudaMemset(b->d_sync, 0, sizeof(unsigned) * 4));
     BTRY(cudaMallocHost(&b->h_pinned, sizeof(int) * 16));
     BTRY(cudaMallocHost(&b->h_active, sizeof(int) * (size_t)nprob));
+    BTRY(cudaMallocHost(&b->h_out, (sizeof(double) + 2 * sizeof(int)) * (size_t)nprob));
+    BTRY(cudaMalloc(&b->d_off0, sizeof(long long) * (size_t)nprob));
+    BTRY(cudaMemcpy(b->d_off0, b->off0.data(), sizeof(long long) * (size_t)nprob, cudaMemcpyHostToDevice));
     BTRY(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
     b->hx.assign(2 * (size_t)nprob * BP_MAXL, nullptr);
     b->hf.assign((size_t)nprob * BP_MAXL, nullptr);
@@ -1806,7 +1811,7 @@ static int batch_create(int nprob, const int *n, int precision, int nu1, int nu2
     int *d_nlev = di; di += nprob;
     int *d_dloc = di; di += nprob;
     int *d_active = di; di += nprob;
-    int *d_cycles = di; di += nprob;
+    int *d_cycles = di; di += nprob;   // read back with d_failed
     int *d_failed = di; di += nprob;
     int *d_pb0 = di; di += nprob;
     int *d_pnb0 = di; di += nprob;
@@ -1930,6 +1935,8 @@ extern "C" int gb_batch_destroy(gb_batch *b)
     cudaFree(b->pipe_buf);
     if (b->h_pinned) cudaFreeHost(b->h_pinned);
     if (b->h_active) cudaFreeHost(b->h_active);
+    if (b->h_out) cudaFreeHost(b->h_out);
+    cudaFree(b->d_off0);
     if (b->stream) cudaStreamDestroy(b->stream);
     delete b;
     return GB_OK;
@@ -2120,33 +2127,34 @@ extern "C" int gb_batch_profile_read_kind(gb_batch *b, int kind, double *ms, lon
     return GB_OK;
 }
 
-static int batch_bind_io(gb_batch *b, const double *d_f, double *d_psi, cudaStream_t s)
+// A solve's start: the tables of the caller's arrays (FP64: level 0 of the
+// cycles works on them in place) and the problems' state.
+__global__ void k_begin(BatchDev B, const long long *off0, const double *f, const float2 *fpairs, double *psi, const void **f_tab,
+                        double **psi_tab, int fp64, void **x_of, void **f_of)
 {
-    std::vector<const void *> pf(b->nprob), pp(b->nprob);
-    const bool mixed = b->precision == GB_BATCH_MIXED;   // float-pair right-hand side
-    for (int p = 0; p < b->nprob; ++p) {
-        pf[p] = mixed ? (const void *)(b->d_fpairs + b->off0[p]) : (const void *)(d_f + b->off0[p]);
-        pp[p] = d_psi + b->off0[p];
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= B.nprob) return;
+    const long long o = off0[p];
+    f_tab[p] = fpairs ? (const void *)(fpairs + o) : (const void *)(f + o);
+    psi_tab[p] = psi + o;
+    if (fp64) {
+        x_of[p * BP_MAXL] = psi + o;
+        f_of[p * BP_MAXL] = const_cast<double *>(f) + o;
     }
-    if (mixed && b->total > 0) {
+    B.active[p] = 1;
+    B.cycles[p] = B.failed[p] = 0;
+}
+
+static int batch_begin(gb_batch *b, const double *d_f, double *d_psi, cudaStream_t s)
+{
+    const bool pairs = b->precision == GB_BATCH_MIXED;   // float-pair right-hand side
+    if (pairs && b->total > 0) {
         k_split_pairs<<<b->nsm * 8, 256, 0, s>>>(d_f, b->d_fpairs, b->total);
         GB_CUDA_TRY(cudaGetLastError());
     }
-    GB_CUDA_TRY(cudaMemcpyAsync(b->d_f_tab, pf.data(), sizeof(void *) * b->nprob, cudaMemcpyHostToDevice, s));
-    GB_CUDA_TRY(cudaMemcpyAsync(b->d_psi_tab, pp.data(), sizeof(void *) * b->nprob, cudaMemcpyHostToDevice, s));
-    if (b->precision == GB_BATCH_FP64) {
-        // level-0 x (buffer 0) and f of the plain cycle are the caller's arrays
-        for (int p = 0; p < b->nprob; ++p) {
-            b->hx[(size_t)p * BP_MAXL] = d_psi + b->off0[p];
-            b->hf[(size_t)p * BP_MAXL] = (void *)(d_f + b->off0[p]);
-        }
-        GB_CUDA_TRY(cudaMemcpyAsync(b->d_ptrs, b->hx.data(), sizeof(void *) * b->hx.size(), cudaMemcpyHostToDevice, s));
-        GB_CUDA_TRY(cudaMemcpyAsync(b->d_ptrs + b->hx.size(), b->hf.data(), sizeof(void *) * b->hf.size(),
-                                    cudaMemcpyHostToDevice, s));
-    }
-    // the pointer tables live in pageable host vectors: complete the copies
-    // before those vectors can change
-    GB_CUDA_TRY(cudaStreamSynchronize(s));
+    k_begin<<<gb_ceil_div((size_t)b->nprob, 128), 128, 0, s>>>(b->dev, b->d_off0, d_f, pairs ? b->d_fpairs : nullptr, d_psi, (const void **)b->d_f_tab,
+                                                              b->d_psi_tab, b->precision == GB_BATCH_FP64, b->d_ptrs, b->d_ptrs + b->hx.size());
+    GB_CUDA_TRY(cudaGetLastError());
     return GB_OK;
 }
 
@@ -2278,13 +2286,9 @@ extern "C" int gb_batch_solve_device(gb_batch *b, const double *d_f, double *d_p
     BatchDev &D = b->dev;
     b->launches = 0;
     if (b->plan_inner != b->inner) build_plans(b);
-    int st = batch_bind_io(b, d_f, d_psi, s);
+    int st = batch_begin(b, d_f, d_psi, s);
     if (st != GB_OK) return st;
     GB_CUDA_TRY(cudaMemsetAsync(d_psi, 0, sizeof(double) * (size_t)b->total, s));
-    std::vector<int> ones(b->nprob, 1);
-    GB_CUDA_TRY(cudaMemcpyAsync(D.active, ones.data(), sizeof(int) * b->nprob, cudaMemcpyHostToDevice, s));
-    GB_CUDA_TRY(cudaMemsetAsync(D.cycles, 0, sizeof(int) * b->nprob, s));
-    GB_CUDA_TRY(cudaMemsetAsync(D.failed, 0, sizeof(int) * b->nprob, s));
     const size_t whole = b->exec == GB_BATCH_EXEC_GRAPH && !b->profile ? whole_local_smem(b) : 0;
     if (whole && b->precision == GB_BATCH_FP64) st = solve_local<double, CM_NONE>(b, whole, s);
     else if (whole && b->precision == GB_BATCH_MIXED) st = solve_local<float, CM_PAIR>(b, whole, s);
@@ -2296,12 +2300,16 @@ extern "C" int gb_batch_solve_device(gb_batch *b, const double *d_f, double *d_p
         k_join_pairs<<<b->nsm * 8, 256, 0, s>>>(d_psi, b->total);
         GB_CUDA_TRY(cudaGetLastError());
     }
-    std::vector<int> fl(b->nprob);
-    GB_CUDA_TRY(cudaMemcpyAsync(fl.data(), D.failed, sizeof(int) * b->nprob, cudaMemcpyDeviceToHost, s));
-    if (cycles) GB_CUDA_TRY(cudaMemcpyAsync(cycles, D.cycles, sizeof(int) * b->nprob, cudaMemcpyDeviceToHost, s));
-    if (relres) GB_CUDA_TRY(cudaMemcpyAsync(relres, D.relres, sizeof(double) * b->nprob, cudaMemcpyDeviceToHost, s));
+    // through page-locked memory: a copy into pageable memory is a
+    // synchronisation of its own (ten microseconds each)
+    double *h_relres = b->h_out;
+    int *h_cycles = (int *)(h_relres + b->nprob), *fl = h_cycles + b->nprob;
+    GB_CUDA_TRY(cudaMemcpyAsync(h_relres, D.relres, sizeof(double) * b->nprob, cudaMemcpyDeviceToHost, s));
+    GB_CUDA_TRY(cudaMemcpyAsync(h_cycles, D.cycles, sizeof(int) * 2 * b->nprob, cudaMemcpyDeviceToHost, s));   // and failed
     GB_CUDA_TRY(cudaStreamSynchronize(s));
     GB_CUDA_TRY(cudaGetLastError());
+    if (relres) std::copy(h_relres, h_relres + b->nprob, relres);
+    if (cycles) std::copy(h_cycles, h_cycles + b->nprob, cycles);
     int st_out = GB_OK;
     for (int p = 0; p < b->nprob; ++p) {
         if (fl[p] == 2) {
