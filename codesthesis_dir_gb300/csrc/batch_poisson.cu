@@ -26,9 +26,11 @@
 #include <type_traits>
 #include <vector>
 
+#include "cluster.cuh"
 #include "convert.cuh"
 #include "gbcommon.cuh"
 #include "gridsync.cuh"
+#include "warpline.cuh"
 
 #define BP_MAXL 16
 #define LOCAL_N 65        // default: levels with n <= 65 run in one block per problem
@@ -116,6 +118,9 @@ template <class T> __device__ __forceinline__ T *XS(const BatchDev &B, int p, in
 }
 template <class T> __device__ __forceinline__ T *FP(const BatchDev &B, int p, int l) { return (T *)B.f[p * BP_MAXL + l]; }
 template <class T> __device__ __forceinline__ T *RP(const BatchDev &B, int p, int l) { return (T *)B.r[p * BP_MAXL + l]; }
+// Points from one row of a level's arrays to the next: FP64 packed (level 0 is
+// the caller's), FP32 whole float4s.
+template <class T> __host__ __device__ __forceinline__ int pitch_of(int n) { return sizeof(T) == 4 ? (n + 3) & ~3 : n; }
 template <class T> __device__ __forceinline__ T H2(const BatchDev &B, int p, int l);
 template <> __device__ __forceinline__ double H2<double>(const BatchDev &B, int p, int l) { return B.h2d[p * BP_MAXL + l]; }
 template <> __device__ __forceinline__ float H2<float>(const BatchDev &B, int p, int l) { return B.h2f[p * BP_MAXL + l]; }
@@ -136,11 +141,7 @@ template <> __device__ __forceinline__ float IH2<float>(const BatchDev &B, int p
 // halo while they run.  Each operation ends with a block barrier so that a
 // block may run the next operation in the same shared memory.
 // ---------------------------------------------------------------------------
-// 128 x 32 tiles of 256 threads.  128 x 64 tiles of 512 threads (halo
-// rings adding 17% instead of 29% to a down operation's sweeps, the same
-// warps per SM) measured 5% slower per solve of the 256-problem workload
-// (5.96 against 5.67 ms); updating two points per lane with paired shared
-// loads measured no faster (5.63 ms either way).
+// 128 x 32 tiles of 256 threads.
 #define TX 128
 #define TY 32
 #define TILE_THREADS (8 * TY)   // 256
@@ -247,44 +248,7 @@ __device__ __forceinline__ void tile_sweeps(T *sx, const T *sf, int ox, int oy, 
     }
 }
 
-// Correction modes of the last level-0 operation of an inner cycle:
-// CM_NONE stores the tile into x; CM_PAIR adds it to psi held as float
-// pairs (GB_BATCH_MIXED); CM_F64 adds it, widened exactly, to the FP64 psi
-// (GB_BATCH_MIXED_F64OUTER).
-#define CM_NONE 0
-#define CM_PAIR 1
-#define CM_F64 2
-
-// psi values of the points this thread stores (fixed assignment: row
-// warp + 8*rr, column lane + 32*cc of the tile), fetched together after the
-// sweeps so that the defect correction's reads of psi overlap one another.
-// Both correction modes hold 8 bytes per point (a float pair or a double).
-template <class V>
-__device__ __forceinline__ void psi_prefetch(const V *psi, int x0, int y0, int n, V (&pv)[ST_R * ST_C])
-{
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int rr = 0; rr < ST_R; ++rr)
-#pragma unroll
-        for (int cc = 0; cc < ST_C; ++cc) {
-            const int gy = y0 + warp + (TILE_THREADS / 32) * rr, gx = x0 + lane + 32 * cc;
-            const bool in = gx >= 1 && gx <= n - 2 && gy >= 1 && gy <= n - 2;
-            V z;
-            if constexpr (std::is_same<V, float2>::value) z = make_float2(0.f, 0.f);
-            else z = (V)0;
-            pv[rr * ST_C + cc] = in ? psi[(size_t)gy * n + gx] : z;
-        }
-}
-
-template <int CM> struct CorrVal { typedef float2 type; };
-template <> struct CorrVal<CM_F64> { typedef double type; };
-
-// Stores the tile's interior points into x, or (CM != CM_NONE) adds them to
-// the solution: the last level-0 operation of an inner cycle applies the
-// defect correction psi += e point by point.
-template <class T, int H, int CM>
-__device__ __forceinline__ void tile_store(const T *sx, int ox, int oy, int x0, int y0, int n, T *x, void *psi,
-                                           const typename CorrVal<CM>::type (&pv)[ST_R * ST_C])
+template <class T, int H> __device__ __forceinline__ void tile_store(const T *sx, int ox, int oy, int x0, int y0, int n, T *x)
 {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
@@ -293,11 +257,7 @@ __device__ __forceinline__ void tile_store(const T *sx, int ox, int oy, int x0, 
         for (int cc = 0; cc < ST_C; ++cc) {
             const int gy = y0 + warp + (TILE_THREADS / 32) * rr, gx = x0 + lane + 32 * cc;
             if (gx < 1 || gx > n - 2 || gy < 1 || gy > n - 2) continue;
-            const size_t g = (size_t)gy * n + gx;
-            const T v = sx[TileLayout<T, H>::at(gy - oy, gx - ox)];
-            if constexpr (CM == CM_PAIR) ((float2 *)psi)[g] = df_add_f(pv[rr * ST_C + cc], (float)v);
-            else if constexpr (CM == CM_F64) ((double *)psi)[g] = pv[rr * ST_C + cc] + f2d((float)v);
-            else x[g] = v;
+            x[(size_t)gy * n + gx] = sx[TileLayout<T, H>::at(gy - oy, gx - ox)];
         }
 }
 
@@ -355,11 +315,10 @@ __device__ __forceinline__ void tile_load(T *sx, T *sf, const T *x, const T *f, 
 
 // NU smoothing sweeps of level l from buffer src into buffer dst.
 // zero_init: the level's current solution is zero (a coarse-level
-// correction, or the FP32 correction of the defect-correction loop) and is
-// not read.  RESTRICT: also form the residual on the tile plus one ring and
+// correction) and is not read.  RESTRICT: also form the residual on the tile plus one ring and
 // its full weighting (rotann2.f:773-785 summation order) onto the coarse
 // points of the tile, which the halo of 2*NU + 2 makes exact.
-template <class T, int NU, int CM, bool RESTRICT>
+template <class T, int NU, bool RESTRICT>
 __device__ void op_smooth(const BatchDev &B, TileEntry e, int l, int zero_init, int src, int dst,
                           unsigned char *smem)
 {
@@ -371,9 +330,7 @@ __device__ void op_smooth(const BatchDev &B, TileEntry e, int l, int zero_init, 
     tile_load<T, H>(sx, sf, XS<T>(B, e.p, l, src), FP<T>(B, e.p, l), ox, oy, n, zero_init != 0, true);
     __syncthreads();
     tile_sweeps<T, H>(sx, sf, ox, oy, x0, y0, n, H2<T>(B, e.p, l), NU);
-    typename CorrVal<CM>::type pv[ST_R * ST_C];
-    if (CM != CM_NONE) psi_prefetch((const typename CorrVal<CM>::type *)B.psi[e.p], x0, y0, n, pv);
-    tile_store<T, H, CM>(sx, ox, oy, x0, y0, n, XS<T>(B, e.p, l, dst), CM != CM_NONE ? (void *)B.psi[e.p] : nullptr, pv);
+    tile_store<T, H>(sx, ox, oy, x0, y0, n, XS<T>(B, e.p, l, dst));
     if (RESTRICT) {
         // residual on the tile plus one ring, in place of f (each point
         // reads f only at itself and x, which stays put, so both colours of
@@ -438,8 +395,8 @@ __device__ void op_smooth(const BatchDev &B, TileEntry e, int l, int zero_init, 
 
 // Bilinear prolongation of level l+1 (buffer 0) added into level l (buffer
 // src) over the tile and its halo (rotann2.f:821-858), then NU
-// post-smoothing sweeps, stored into buffer dst (or added to psi: CM).
-template <class T, int NU, int CM>
+// post-smoothing sweeps, stored into buffer dst.
+template <class T, int NU>
 __device__ void op_prolong(const BatchDev &B, TileEntry e, int l, int src, int dst, unsigned char *smem)
 {
     constexpr int H = 2 * NU, SX = TX + 2 * H, SY = TY + 2 * H;
@@ -502,10 +459,256 @@ __device__ void op_prolong(const BatchDev &B, TileEntry e, int l, int src, int d
     }
     __syncthreads();
     if (NU > 0) tile_sweeps<T, H>(sx, sf, ox, oy, x0, y0, n, H2<T>(B, e.p, l), NU);
-    typename CorrVal<CM>::type pv[ST_R * ST_C];
-    if (CM != CM_NONE) psi_prefetch((const typename CorrVal<CM>::type *)B.psi[e.p], x0, y0, n, pv);
-    tile_store<T, H, CM>(sx, ox, oy, x0, y0, n, XS<T>(B, e.p, l, dst), CM != CM_NONE ? (void *)B.psi[e.p] : nullptr, pv);
+    tile_store<T, H>(sx, ox, oy, x0, y0, n, XS<T>(B, e.p, l, dst));
     __syncthreads();
+}
+
+// ---------------------------------------------------------------------------
+// Register tiles: the FP32 tile operations.
+//
+// In shared memory a point's update is five loads, a store and their
+// addresses, and the operations were bound by exactly that (issue slots 75 %
+// and the shared pipe 71 % busy, DRAM 15 %).  Here a warp holds RT_R whole rows
+// of 128 points, four neighbouring ones per lane: a point's row neighbours are
+// the lane's own but for one shuffle a row and phase, its column neighbours the
+// lane's own but for the band's first and last row, which the warps exchange
+// through shared memory, double buffered, with one block barrier a phase.  No
+// phase keeps to the rings that are still exact (TileLayout): the points that
+// are not lie outside what the tile owns, so they may hold anything.
+//
+// Rows have a pitch of a whole number of float4s (pitch_of; the padding stays
+// zero) and a tile's first column is a multiple of four, so that a band is read
+// with one 16-byte load per lane and row.  A tile owns its points but for H at
+// the sides where another tile follows; the domain's own edge needs no halo,
+// so n = 129 takes one tile across.
+//
+// The right-hand side, read twice a sweep, stays in shared memory (copied there
+// asynchronously, each lane its own float4s): with it in registers, 116 a
+// thread, two blocks fit an SM and every second issue slot waited for a tile's
+// loads (88 and 110 us); at 64 registers four blocks do.
+//
+// Finest level of 256 problems of 65 .. 513, two sweeps a pass: down 122 -> 75
+// us, up 120 -> 88 (135 M -> 64 M warp instructions, down); the solve 5.15 ->
+// 3.94 ms.
+//
+// The order of every sum is that of the FP64 tiles and the oracle.
+// ---------------------------------------------------------------------------
+#define RT_W 128
+#define RT_R 8
+#define RT_H (RT_R * (TILE_THREADS / 32))   // rows of a tile
+#define RT_HALOS 4                          // halos 0, 2, 4, 6
+#define RT_SMEM ((5 + RT_R) * (TILE_THREADS / 32) * 32 * sizeof(float4))
+
+// Tiles of size len whose owned parts, halo h, cover n points.
+static int rt_count(int n, int len, int h) { return n <= len ? 1 : gb_ceil_div((size_t)(n - len), (size_t)(len - 2 * h)) + 1; }
+
+// Correction modes of the last level-0 operation of an inner cycle:
+// CM_NONE stores the tile into x; CM_PAIR adds it to psi held as float
+// pairs (GB_BATCH_MIXED); CM_F64 adds it, widened exactly, to the FP64 psi
+// (GB_BATCH_MIXED_F64OUTER).
+#define CM_NONE 0
+#define CM_PAIR 1
+#define CM_F64 2
+template <int CM> struct CorrVal { typedef float2 type; };
+template <> struct CorrVal<CM_F64> { typedef double type; };
+
+// NU smoothing sweeps of level l from buffer src (zero: from zero) into buffer
+// dst.  PROLONG: first level l + 1's bilinear prolongation (rotann2.f:821-858)
+// is added.  RESTRICT: the residual's full weighting (rotann2.f:773-785) goes
+// to level l + 1's right-hand side.
+template <int NU, int CM, bool RESTRICT, bool PROLONG>
+__device__ __forceinline__ void op_tile32_body(const BatchDev &B, TileEntry e, int l, int zero, int src, int dst, unsigned char *smem)
+{
+    constexpr int H = 2 * NU + (RESTRICT ? 2 : 0), NW = TILE_THREADS / 32;
+    const unsigned full = 0xffffffffu;
+    float4 *edge = (float4 *)smem;                 // [buffer][first, last row][warp][lane]
+    float4 *stage = edge + 2 * 2 * NW * 32;        // [warp][lane]
+    float4 *f = stage + NW * 32 + (threadIdx.x >> 5) * RT_R * 32 + (threadIdx.x & 31);   // own: [row], 32 apart
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int n = B.n_of[e.p * BP_MAXL + l], P = pitch_of<float>(n);
+    const int ox = e.tx * (RT_W - 2 * H), oy = e.ty * (RT_H - 2 * H);
+    const int gx = ox + 4 * lane, gy = oy + RT_R * warp;
+    const int xlo = e.tx ? ox + H : 0, xhi = ox + RT_W >= n ? P : ox + RT_W - H;   // owned columns, pairs of them
+    const int ylo = e.ty ? oy + H : 1, yhi = oy + RT_H >= n ? n - 1 : oy + RT_H - H;
+    const float h2 = H2<float>(B, e.p, l), ih2 = IH2<float>(B, e.p, l);
+    const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 x[RT_R];
+    {
+        const float *xs = XS<float>(B, e.p, l, src) + (size_t)gy * P + gx, *fs = FP<float>(B, e.p, l) + (size_t)gy * P + gx;
+#pragma unroll
+        for (int r = 0; r < RT_R; ++r) {
+            const bool in = gx < n && gy + r < n;
+            x[r] = in && !zero ? *(const float4 *)(xs + r * P) : z4;
+            if (NU == 0 && !RESTRICT) continue;
+            if (in) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(f + r * 32)), "l"(fs + r * P) : "memory");
+            else f[r * 32] = z4;
+        }
+    }
+    // interior columns of the lane
+    const bool c0 = gx >= 1 && gx <= n - 2, c1 = gx + 1 <= n - 2, c2 = gx + 2 <= n - 2, c3 = gx + 3 <= n - 2;
+    if (PROLONG) {
+        const int nc = B.n_of[e.p * BP_MAXL + l + 1], Pc = pitch_of<float>(nc);
+        const float *ec = XS<float>(B, e.p, l + 1, 0) + (gx >> 1);
+        const bool in = gx < n;
+        float2 a[RT_R / 2 + 1];
+        float b[RT_R / 2 + 1];
+#pragma unroll
+        for (int r = 0; r <= RT_R / 2; ++r) {
+            const int J = (gy >> 1) + r;
+            const bool ok = in && J < nc;
+            a[r] = ok ? *(const float2 *)(ec + (size_t)J * Pc) : make_float2(0.f, 0.f);
+            b[r] = ok && (gx >> 1) + 2 < nc ? ec[(size_t)J * Pc + 2] : 0.f;
+        }
+#pragma unroll
+        for (int r = 0; r < RT_R; ++r) {
+            if (gy + r < 1 || gy + r > n - 2) continue;
+            const float e00 = a[r / 2].x, e01 = a[r / 2].y, e02 = b[r / 2];
+            float4 v;
+            if (r % 2 == 0) {
+                v = make_float4(e00, (e00 + e01) * 0.5f, e01, (e01 + e02) * 0.5f);
+            } else {
+                const float e10 = a[r / 2 + 1].x, e11 = a[r / 2 + 1].y, e12 = b[r / 2 + 1];
+                float t = e00 + e11;
+                t = t + e10 + e01;
+                float u = e01 + e12;
+                u = u + e11 + e02;
+                v = make_float4((e00 + e10) * 0.5f, t * 0.25f, (e01 + e11) * 0.5f, u * 0.25f);
+            }
+            if (c0) x[r].x = x[r].x + v.x;
+            if (c1) x[r].y = x[r].y + v.y;
+            if (c2) x[r].z = x[r].z + v.z;
+            if (c3) x[r].w = x[r].w + v.w;
+        }
+    }
+    // the band's neighbour rows of exchange number k
+    auto give = [&](int k) {
+        float4 *q = edge + ((k & 1) * 2 * NW + warp) * 32 + lane;
+        q[0] = x[0];
+        q[NW * 32] = x[RT_R - 1];
+        __syncthreads();
+    };
+    auto above = [&](int k) { return warp > 0 ? edge[((k & 1) * 2 * NW + NW + warp - 1) * 32 + lane] : z4; };
+    auto below = [&](int k) { return warp < NW - 1 ? edge[((k & 1) * 2 * NW + warp + 1) * 32 + lane] : z4; };
+    async_copy_wait();   // a lane reads only what it copied
+#pragma unroll
+    for (int k = 0; k < 2 * NU; ++k) {
+        give(k);
+        const float4 top = above(k), bot = below(k);
+#pragma unroll
+        for (int r = 0; r < RT_R; ++r) {
+            if (gy + r < 1 || gy + r > n - 2) continue;
+            const float4 u = r > 0 ? x[r - 1] : top, d = r < RT_R - 1 ? x[r + 1] : bot, g = f[r * 32];
+            if (((r + k) & 1) == 0) {
+                const float lf = __shfl_up_sync(full, x[r].w, 1);
+                const float s0 = (lf + x[r].y) + (u.x + d.x), s2 = (x[r].y + x[r].w) + (u.z + d.z);
+                const float v0 = __fmaf_rn(-h2, g.x, s0) * 0.25f, v2 = __fmaf_rn(-h2, g.z, s2) * 0.25f;
+                if (c0) x[r].x = v0;
+                if (c2) x[r].z = v2;
+            } else {
+                const float rt = __shfl_down_sync(full, x[r].x, 1);
+                const float s1 = (x[r].x + x[r].z) + (u.y + d.y), s3 = (x[r].z + rt) + (u.w + d.w);
+                const float v1 = __fmaf_rn(-h2, g.y, s1) * 0.25f, v3 = __fmaf_rn(-h2, g.w, s3) * 0.25f;
+                if (c1) x[r].y = v1;
+                if (c3) x[r].w = v3;
+            }
+        }
+    }
+    if constexpr (CM == CM_NONE) {
+        float *xd = XS<float>(B, e.p, l, dst) + (size_t)gy * P + gx;
+        const bool p0 = gx >= xlo && gx < xhi, p1 = gx + 2 >= xlo && gx + 2 < xhi;
+#pragma unroll
+        for (int r = 0; r < RT_R; ++r) {
+            if (gy + r < ylo || gy + r >= yhi) continue;
+            if (p0) *(float2 *)(xd + r * P) = make_float2(x[r].x, x[r].y);
+            if (p1) *(float2 *)(xd + r * P + 2) = make_float2(x[r].z, x[r].w);
+        }
+    } else {
+        // psi lies packed with pitch n: through shared memory, so that a warp
+        // reads and writes consecutive points
+        using V = typename CorrVal<CM>::type;
+        V *psi = (V *)B.psi[e.p];
+        float *st = (float *)(stage + warp * 32);
+        const int a = max(xlo, 1), b = min(xhi, n - 1);
+#pragma unroll
+        for (int r = 0; r < RT_R; ++r) {
+            if (gy + r < ylo || gy + r >= yhi) continue;
+            __syncwarp();
+            ((float4 *)st)[lane] = x[r];
+            __syncwarp();
+            V *q = psi + (size_t)(gy + r) * n + ox + lane;
+            V v[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+                if (ox + lane + 32 * c >= a && ox + lane + 32 * c < b) v[c] = q[32 * c];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                if (ox + lane + 32 * c < a || ox + lane + 32 * c >= b) continue;
+                if constexpr (CM == CM_PAIR) q[32 * c] = df_add_f(v[c], st[lane + 32 * c]);
+                else q[32 * c] = v[c] + f2d(st[lane + 32 * c]);
+            }
+        }
+    }
+    if (RESTRICT) {
+        give(2 * NU);
+        const float4 top = above(2 * NU), bot = below(2 * NU);
+        auto residual = [&](int r) {
+            const float4 u = r > 0 ? x[r > 0 ? r - 1 : 0] : top, d = r < RT_R - 1 ? x[r < RT_R - 1 ? r + 1 : 0] : bot, v = x[r], g = f[r * 32];
+            const float lf = __shfl_up_sync(full, v.w, 1), rt = __shfl_down_sync(full, v.x, 1);
+            const bool in = gy + r >= 1 && gy + r <= n - 2;
+            const float s0 = (lf + v.y) + (u.x + d.x), s1 = (v.x + v.z) + (u.y + d.y);
+            const float s2 = (v.y + v.w) + (u.z + d.z), s3 = (v.z + rt) + (u.w + d.w);
+            return make_float4(in && c0 ? __fmaf_rn(-ih2, __fmaf_rn(-4.f, v.x, s0), g.x) : 0.f,
+                               in && c1 ? __fmaf_rn(-ih2, __fmaf_rn(-4.f, v.y, s1), g.y) : 0.f,
+                               in && c2 ? __fmaf_rn(-ih2, __fmaf_rn(-4.f, v.z, s2), g.z) : 0.f,
+                               in && c3 ? __fmaf_rn(-ih2, __fmaf_rn(-4.f, v.w, s3), g.w) : 0.f);
+        };
+        const float4 last = residual(RT_R - 1);
+        stage[warp * 32 + lane] = last;
+        __syncthreads();
+        float4 up = warp > 0 ? stage[(warp - 1) * 32 + lane] : z4;
+        float lu = __shfl_up_sync(full, up.w, 1);
+        const int nc = B.n_of[e.p * BP_MAXL + l + 1], Pc = pitch_of<float>(nc);
+        float *fc = FP<float>(B, e.p, l + 1) + (gx >> 1);
+        const int I = gx >> 1;
+        const bool o0 = gx >= xlo && gx < xhi && I >= 1 && I <= nc - 2, o1 = gx + 2 >= xlo && gx + 2 < xhi && I + 1 <= nc - 2;
+#pragma unroll
+        for (int r = 0; r < RT_R; r += 2) {
+            const float4 m = residual(r), d = r + 1 < RT_R - 1 ? residual(r + 1) : last;
+            const float lm = __shfl_up_sync(full, m.w, 1), ld = __shfl_up_sync(full, d.w, 1);
+            const int J = (gy + r) >> 1;
+            if (gy + r >= ylo && gy + r < yhi && J <= nc - 2) {
+                float t = m.x;
+                t = t * 2.f + m.y + lm;
+                t = t + d.x + up.x;
+                t = t * 2.f + d.y + lu;
+                t = t + up.y + ld;
+                if (o0) fc[(size_t)J * Pc] = t * 0.0625f;
+                t = m.z;
+                t = t * 2.f + m.w + m.y;
+                t = t + d.z + up.z;
+                t = t * 2.f + d.w + up.y;
+                t = t + up.w + d.y;
+                if (o1) fc[(size_t)J * Pc + 1] = t * 0.0625f;
+            }
+            up = d;
+            lu = ld;
+        }
+    }
+    __syncthreads();
+}
+
+// Called by the persistent kernel, which holds all of the variants, expanded
+// in the kernels of one operation.
+template <int NU, int CM, bool RESTRICT, bool PROLONG>
+__device__ __noinline__ void op_tile32_call(const BatchDev &B, TileEntry e, int l, int zero, int src, int dst, unsigned char *smem)
+{
+    op_tile32_body<NU, CM, RESTRICT, PROLONG>(B, e, l, zero, src, dst, smem);
+}
+template <bool CALL, int NU, int CM, bool RESTRICT, bool PROLONG>
+__device__ __forceinline__ void op_tile32(const BatchDev &B, TileEntry e, int l, int zero, int src, int dst, unsigned char *smem)
+{
+    if constexpr (CALL) op_tile32_call<NU, CM, RESTRICT, PROLONG>(B, e, l, zero, src, dst, smem);
+    else op_tile32_body<NU, CM, RESTRICT, PROLONG>(B, e, l, zero, src, dst, smem);
 }
 
 // ---------------------------------------------------------------------------
@@ -761,19 +964,23 @@ __device__ void op_local(const BatchDev &B, int p, int nu1, int nu2, int zero_le
         const bool zero = d0 > 0 || zero_level0;
         const T *gx = XS<T>(B, p, d0, 0), *gf = FP<T>(B, p, d0);
         constexpr int U = 5;   // loads in flight
-        for (int q0 = tid; q0 < n0 * n0; q0 += U * nthr) {
+        const int P = pitch_of<T>(n0);
+        const RowSplit row(P);
+        for (int q0 = tid; q0 < n0 * P; q0 += U * nthr) {
             T x[U], f[U];
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                const int q = min(q0 + u * nthr, n0 * n0 - 1);
+                const int q = min(q0 + u * nthr, n0 * P - 1);
                 x[u] = zero ? (T)0 : gx[q];
                 f[u] = gf[q];
             }
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                const int q = min(q0 + u * nthr, n0 * n0 - 1);
-                v.X[v.at(q)] = x[u];
-                v.F[v.at(q)] = f[u];
+                int j, i;
+                row(min(q0 + u * nthr, n0 * P - 1), j, i);
+                if (i >= n0) continue;
+                v.X[v.at(j * n0 + i)] = x[u];
+                v.F[v.at(j * n0 + i)] = f[u];
             }
         }
     }
@@ -798,7 +1005,13 @@ __device__ void op_local(const BatchDev &B, int p, int nu1, int nu2, int zero_le
         correct((float2 *)B.psi[p], [](float2 a, T e) { return df_add_f(a, (float)e); });
     } else {
         T *gx = XS<T>(B, p, d0, 0);
-        for (int q = tid; q < n0 * n0; q += nthr) gx[q] = v.X[v.at(q)];
+        const int P = pitch_of<T>(n0);
+        const RowSplit row(P);
+        for (int q = tid; q < n0 * P; q += nthr) {
+            int j, i;
+            row(q, j, i);
+            if (i < n0) gx[q] = v.X[v.at(j * n0 + i)];
+        }
     }
     __syncthreads();
 }
@@ -867,6 +1080,7 @@ __device__ void op_outer(const BatchDev &B, TileEntry e, int item, const void *c
         __syncthreads();
     }
     float *f32 = store_r ? FP<float>(B, e.p, 0) : nullptr;
+    const int P = pitch_of<float>(n);
     // one accumulator per column group: the sum of squares is a dependent
     // FP64 chain, and TX / 32 independent chains let the points overlap
     double accs[TX / 32];
@@ -891,7 +1105,7 @@ __device__ void op_outer(const BatchDev &B, TileEntry e, int item, const void *c
             const int gy = gy0 + h * nw, gx = x0 + lane + 32 * a;
             if (gy >= gyb || gx < gxa || gx >= gxb) continue;
             const int q = (gy - oy) * SX + gx - ox;
-            const size_t g = (size_t)gy * n + gx;
+            const size_t g = (size_t)gy * P + gx;
             double rw;
             if constexpr (FIRST) {
                 if constexpr (PAIR) {
@@ -1023,21 +1237,21 @@ struct Op {
 // Runs work item `item` of op on this block.  op.corr is the correction
 // mode (CM_*) of the operation that applies the defect correction, and of
 // the outer pass.
-template <class T, int NU, bool RESTRICT>
+template <class T, bool CALL, int NU, bool RESTRICT>
 __device__ __forceinline__ void run_smooth(const BatchDev &B, TileEntry e, const Op &op, unsigned char *smem)
 {
-    if constexpr (sizeof(T) == 8) op_smooth<T, NU, CM_NONE, RESTRICT>(B, e, op.l, op.zero, op.src, op.dst, smem);
-    else if (op.corr == CM_PAIR) op_smooth<T, NU, CM_PAIR, RESTRICT>(B, e, op.l, op.zero, op.src, op.dst, smem);
-    else if (op.corr == CM_F64) op_smooth<T, NU, CM_F64, RESTRICT>(B, e, op.l, op.zero, op.src, op.dst, smem);
-    else op_smooth<T, NU, CM_NONE, RESTRICT>(B, e, op.l, op.zero, op.src, op.dst, smem);
+    if constexpr (sizeof(T) == 8) op_smooth<T, NU, RESTRICT>(B, e, op.l, op.zero, op.src, op.dst, smem);
+    else if (!RESTRICT && op.corr == CM_PAIR) op_tile32<CALL, NU, CM_PAIR, false, false>(B, e, op.l, op.zero, op.src, op.dst, smem);
+    else if (!RESTRICT && op.corr == CM_F64) op_tile32<CALL, NU, CM_F64, false, false>(B, e, op.l, op.zero, op.src, op.dst, smem);
+    else op_tile32<CALL, NU, CM_NONE, RESTRICT, false>(B, e, op.l, op.zero, op.src, op.dst, smem);
 }
-template <class T, int NU>
+template <class T, bool CALL, int NU>
 __device__ __forceinline__ void run_prolong(const BatchDev &B, TileEntry e, const Op &op, unsigned char *smem)
 {
-    if constexpr (sizeof(T) == 8) op_prolong<T, NU, CM_NONE>(B, e, op.l, op.src, op.dst, smem);
-    else if (op.corr == CM_PAIR) op_prolong<T, NU, CM_PAIR>(B, e, op.l, op.src, op.dst, smem);
-    else if (op.corr == CM_F64) op_prolong<T, NU, CM_F64>(B, e, op.l, op.src, op.dst, smem);
-    else op_prolong<T, NU, CM_NONE>(B, e, op.l, op.src, op.dst, smem);
+    if constexpr (sizeof(T) == 8) op_prolong<T, NU>(B, e, op.l, op.src, op.dst, smem);
+    else if (op.corr == CM_PAIR) op_tile32<CALL, NU, CM_PAIR, false, true>(B, e, op.l, 0, op.src, op.dst, smem);
+    else if (op.corr == CM_F64) op_tile32<CALL, NU, CM_F64, false, true>(B, e, op.l, 0, op.src, op.dst, smem);
+    else op_tile32<CALL, NU, CM_NONE, false, true>(B, e, op.l, 0, op.src, op.dst, smem);
 }
 
 template <class T, bool FIRST>
@@ -1051,7 +1265,7 @@ __device__ __forceinline__ void run_outer(const BatchDev &B, TileEntry e, int it
     else op_outer<T, CM_NONE, FIRST>(B, e, item, fp, op.aux, smem);
 }
 
-template <class T>
+template <class T, bool CALL>
 __device__ __forceinline__ void run_item(const BatchDev &B, const TileEntry *tiles, const double *const *f_p,
                                          const Op &op, int item, int nu1, int nu2, unsigned char *smem)
 {
@@ -1059,23 +1273,23 @@ __device__ __forceinline__ void run_item(const BatchDev &B, const TileEntry *til
     case OP_SMOOTH: {
         const TileEntry e = tiles[op.off + item];
         if (!B.active[e.p]) return;
-        if (op.nu == 2) run_smooth<T, 2, false>(B, e, op, smem);
-        else run_smooth<T, 1, false>(B, e, op, smem);
+        if (op.nu == 2) run_smooth<T, CALL, 2, false>(B, e, op, smem);
+        else run_smooth<T, CALL, 1, false>(B, e, op, smem);
         return;
     }
     case OP_SMOOTH_R: {
         const TileEntry e = tiles[op.off + item];
         if (!B.active[e.p]) return;
-        if (op.nu == 2) op_smooth<T, 2, CM_NONE, true>(B, e, op.l, op.zero, op.src, op.dst, smem);
-        else op_smooth<T, 1, CM_NONE, true>(B, e, op.l, op.zero, op.src, op.dst, smem);
+        if (op.nu == 2) run_smooth<T, CALL, 2, true>(B, e, op, smem);
+        else run_smooth<T, CALL, 1, true>(B, e, op, smem);
         return;
     }
     case OP_PROLONG: {
         const TileEntry e = tiles[op.off + item];
         if (!B.active[e.p]) return;
-        if (op.nu == 2) run_prolong<T, 2>(B, e, op, smem);
-        else if (op.nu == 1) run_prolong<T, 1>(B, e, op, smem);
-        else run_prolong<T, 0>(B, e, op, smem);
+        if (op.nu == 2) run_prolong<T, CALL, 2>(B, e, op, smem);
+        else if (op.nu == 1) run_prolong<T, CALL, 1>(B, e, op, smem);
+        else run_prolong<T, CALL, 0>(B, e, op, smem);
         return;
     }
     case OP_LOCAL:
@@ -1244,15 +1458,14 @@ __global__ void __launch_bounds__(LOCAL_THREADS) k_local_solve(BatchDev B, const
 }
 
 // One kernel launch per operation (graph path).
-// The prolongation variants fit five blocks' shared tiles per SM and are
-// held to the registers of five, except those that also apply the defect
-// correction (eight more values per thread: held to four, where they need no
-// spills); the outer pass is held to four.
-template <int KIND, int CM> struct OpMinBlocks {
-    static constexpr int value = KIND == OP_PROLONG ? (CM == CM_NONE ? 5 : 4) : (KIND == OP_OUTER ? 4 : 1);
+// The FP64 prolongation's shared tiles fit five blocks per SM and it is held to
+// the registers of five; the FP32 tiles live in registers, four blocks' worth;
+// the outer pass is held to four.
+template <class T, int KIND> struct OpMinBlocks {
+    static constexpr int value = KIND == OP_OUTER ? 4 : sizeof(T) == 4 ? 4 : KIND == OP_PROLONG ? 5 : 1;
 };
 template <class T, int KIND, int NU, int CM>
-__global__ void __launch_bounds__(TILE_THREADS, (OpMinBlocks<KIND, CM>::value)) k_op(BatchDev B, const TileEntry *tiles, const double *const *f_p,
+__global__ void __launch_bounds__(TILE_THREADS, (OpMinBlocks<T, KIND>::value)) k_op(BatchDev B, const TileEntry *tiles, const double *const *f_p,
                                                      Op op, int nu1, int nu2)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -1266,14 +1479,14 @@ __global__ void __launch_bounds__(TILE_THREADS, (OpMinBlocks<KIND, CM>::value)) 
     o.kind = KIND;
     o.nu = NU;
     o.corr = CM;
-    run_item<T>(B, tiles, f_p, o, blockIdx.x, nu1, nu2, smem_raw);
+    run_item<T, false>(B, tiles, f_p, o, blockIdx.x, nu1, nu2, smem_raw);
 }
 
 // The whole solve in one launch: the first iteration's operations, then
 // further iterations until every problem has converged (or hit the cycle
 // limit).  Must be launched cooperatively (all blocks resident).
 template <class T>
-__global__ void __launch_bounds__(TILE_THREADS, 3) k_persistent(BatchDev B, const TileEntry *tiles,
+__global__ void __launch_bounds__(TILE_THREADS, 3) k_persistent(const __grid_constant__ BatchDev B, const TileEntry *tiles,
                                                              const double *const *f_p, const Op *ops0, int n0,
                                                              const Op *ops, int nops, int nu1, int nu2,
                                                              int max_iter, GridSync gs)
@@ -1291,7 +1504,7 @@ __global__ void __launch_bounds__(TILE_THREADS, 3) k_persistent(BatchDev B, cons
                 for (int p = gwarp; p < B.nprob; p += warps_total) op_finalize(B, p, op.aux);
             } else {
                 for (int item = blockIdx.x; item < op.cnt; item += gridDim.x)
-                    run_item<T>(B, tiles, f_p, op, item, nu1, nu2, smem_raw);
+                    run_item<T, true>(B, tiles, f_p, op, item, nu1, nu2, smem_raw);
             }
             if (!grid_sync(gs)) return;
             if (op.kind == OP_FINALIZE && *(volatile int *)B.num_active == 0) return;
@@ -1322,7 +1535,7 @@ struct gb_batch {
     float2 *d_fpairs = nullptr;         // mixed: the right-hand side as float pairs (total)
     void **d_ptrs = nullptr;
     TileEntry *d_tiles = nullptr;
-    std::vector<int> ft_off, ft_cnt;    // per level: tiles of problems with l < dloc
+    std::vector<int> ft_off, ft_cnt;    // per level (and half halo, FP32): tiles of problems with l < dloc
     int ot_off = 0, ot_cnt = 0;         // level-0 tiles of every problem (outer pass)
     BatchDev dev;
     double **d_psi_tab = nullptr, **d_f_tab = nullptr;
@@ -1390,9 +1603,11 @@ static int corr_mode(const gb_batch *b)
     return b->precision == GB_BATCH_MIXED ? CM_PAIR : b->precision == GB_BATCH_MIXED_F64OUTER ? CM_F64 : CM_NONE;
 }
 
-// Two colour-split arrays (x and f) of a tile with halo H (TileLayout).
+// Shared memory of a tile operation of halo H: two colour-split arrays (x and
+// f, TileLayout), or the register tiles' exchange.
 template <class T> static size_t smem_tile(int H)
 {
+    if (sizeof(T) == 4) return RT_SMEM;
     const int SXH = (TX + 2 * H) / 2, SY = TY + 2 * H, W = 128 / (int)sizeof(T);
     const size_t half = (size_t)((SY * SXH + W - 1) / W) * W + W / 2;
     return 2 * sizeof(T) * 2 * half;
@@ -1445,8 +1660,14 @@ static void plan_vcycle(gb_batch *b, std::vector<Op> &v, bool zero0, bool corr0,
     const int k1 = ops_for(b, b->nu1);
     const int pro = std::min(b->nu2, b->fuse);  // sweeps fused into the prolongation
     const int k2 = ops_for(b, b->nu2 - pro);
+    // an operation's tiles: FP32 ones by their halo
+    auto tiles = [&](Op &o) {
+        const int k = mixed ? o.nu + (o.kind == OP_SMOOTH_R ? 1 : 0) : 0;
+        o.off = b->ft_off[o.l * RT_HALOS + k];
+        o.cnt = b->ft_cnt[o.l * RT_HALOS + k];
+    };
     for (int l = 0; l < b->maxdepth_global; ++l) {
-        if (b->ft_cnt[l] == 0) continue;
+        if (b->ft_cnt[l * RT_HALOS] == 0) continue;
         const bool zero = l > 0 || (mixed && zero0);
         const int writes = k1 + 1 + k2;
         int src, dst;
@@ -1459,7 +1680,7 @@ static void plan_vcycle(gb_batch *b, std::vector<Op> &v, bool zero0, bool corr0,
             Op o{};
             o.kind = (i == k1 - 1) ? OP_SMOOTH_R : OP_SMOOTH;
             o.l = l; o.nu = k; o.zero = (zero && i == 0) ? 1 : 0; o.src = src; o.dst = dst; o.corr = 0;
-            o.off = b->ft_off[l]; o.cnt = b->ft_cnt[l];
+            tiles(o);
             v.push_back(o);
             nu -= k;
             src = dst;
@@ -1475,13 +1696,13 @@ static void plan_vcycle(gb_batch *b, std::vector<Op> &v, bool zero0, bool corr0,
         v.push_back(o);
     }
     for (int l = b->maxdepth_global - 1; l >= 0; --l) {
-        if (b->ft_cnt[l] == 0) continue;
+        if (b->ft_cnt[l * RT_HALOS] == 0) continue;
         const int correct_last = (mixed && l == 0 && corr0) ? cm : CM_NONE;
         int src = cur[l], dst = 1 - cur[l];
         Op o{};
         o.kind = OP_PROLONG; o.l = l; o.nu = pro; o.src = src; o.dst = dst;
         o.corr = k2 == 0 ? correct_last : CM_NONE;
-        o.off = b->ft_off[l]; o.cnt = b->ft_cnt[l];
+        tiles(o);
         v.push_back(o);
         src = dst;
         dst = 1 - dst;
@@ -1491,7 +1712,7 @@ static void plan_vcycle(gb_batch *b, std::vector<Op> &v, bool zero0, bool corr0,
             Op q{};
             q.kind = OP_SMOOTH; q.l = l; q.nu = k; q.zero = 0; q.src = src; q.dst = dst;
             q.corr = (i == k2 - 1) ? correct_last : CM_NONE;
-            q.off = b->ft_off[l]; q.cnt = b->ft_cnt[l];
+            tiles(q);
             v.push_back(q);
             nu -= k;
             src = dst;
@@ -1500,7 +1721,7 @@ static void plan_vcycle(gb_batch *b, std::vector<Op> &v, bool zero0, bool corr0,
         cur[l] = src;
         if (!mixed && l == 0 && cur[0] != 0) {
             Op c{};
-            c.kind = OP_COPYBACK; c.off = b->ft_off[0]; c.cnt = b->ft_cnt[0];
+            c.kind = OP_COPYBACK; tiles(c);
             v.push_back(c);
         }
     }
@@ -1702,7 +1923,7 @@ static int batch_create(int nprob, const int *n, int precision, int nu1, int nu2
             nof[(size_t)p * BP_MAXL + l] = nl[l];
             // x buffers 0 and 1 plus f; the plain solve's level 0 uses the
             // caller's psi and f, with one internal FP64 buffer beside psi
-            const size_t sz = (size_t)nl[l] * nl[l];
+            const size_t sz = (size_t)nl[l] * (precision == GB_BATCH_FP64 ? pitch_of<double>(nl[l]) : pitch_of<float>(nl[l]));
             if (precision == GB_BATCH_FP64 && l == 0) pool_elems += sz;
             else pool_elems += 3 * sz;
         }
@@ -1720,19 +1941,29 @@ static int batch_create(int nprob, const int *n, int precision, int nu1, int nu2
     b->local_smem = smax;
     // tile tables
     std::vector<TileEntry> tiles;
-    b->ft_off.assign(BP_MAXL + 1, 0);
-    b->ft_cnt.assign(BP_MAXL + 1, 0);
+    b->ft_off.assign(BP_MAXL * RT_HALOS, 0);
+    b->ft_cnt.assign(BP_MAXL * RT_HALOS, 0);
     std::vector<int> pb0(nprob), pnb0(nprob);
     auto add_tiles = [&](int p, int nn) {
         for (int ty = 0; ty * TY < nn - 1; ++ty)
             for (int tx = 0; tx * TX < nn - 1; ++tx) tiles.push_back({p, (short)tx, (short)ty});
     };
-    for (int l = 0; l < BP_MAXL; ++l) {
-        b->ft_off[l] = (int)tiles.size();
-        for (int p = 0; p < nprob; ++p)
-            if (l < b->dloc[p]) add_tiles(p, nof[(size_t)p * BP_MAXL + l]);
-        b->ft_cnt[l] = (int)tiles.size() - b->ft_off[l];
-    }
+    for (int l = 0; l < BP_MAXL; ++l)
+        for (int k = 0; k < (precision == GB_BATCH_FP64 ? 1 : RT_HALOS); ++k) {
+            const int at = l * RT_HALOS + k;
+            b->ft_off[at] = (int)tiles.size();
+            for (int p = 0; p < nprob; ++p) {
+                if (l >= b->dloc[p]) continue;
+                const int nn = nof[(size_t)p * BP_MAXL + l];
+                if (precision == GB_BATCH_FP64) {
+                    add_tiles(p, nn);
+                    continue;
+                }
+                for (int ty = 0; ty < rt_count(nn, RT_H, 2 * k); ++ty)
+                    for (int tx = 0; tx < rt_count(nn, RT_W, 2 * k); ++tx) tiles.push_back({p, (short)tx, (short)ty});
+            }
+            b->ft_cnt[at] = (int)tiles.size() - b->ft_off[at];
+        }
     b->ot_off = (int)tiles.size();
     for (int p = 0; p < nprob; ++p) {
         pb0[p] = (int)tiles.size() - b->ot_off;
@@ -1794,7 +2025,8 @@ static int batch_create(int nprob, const int *n, int precision, int nu1, int nu2
     char *base = (char *)b->pool;
     for (int p = 0; p < nprob; ++p) {
         for (int l = 0; l < b->L[p]; ++l) {
-            const size_t sz = (size_t)nof[(size_t)p * BP_MAXL + l] * nof[(size_t)p * BP_MAXL + l] * esz;
+            const int m = nof[(size_t)p * BP_MAXL + l];
+            const size_t sz = (size_t)m * (precision == GB_BATCH_FP64 ? pitch_of<double>(m) : pitch_of<float>(m)) * esz;
             const size_t k = (size_t)p * BP_MAXL + l;
             const size_t k1 = ((size_t)nprob + p) * BP_MAXL + l;
             if (precision == GB_BATCH_FP64 && l == 0) {
