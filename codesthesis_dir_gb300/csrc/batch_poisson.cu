@@ -2454,7 +2454,6 @@ static int solve_persistent(gb_batch *b, cudaStream_t s)
     GB_CUDA_TRY(cudaMemsetAsync(b->d_sync, 0, sizeof(unsigned) * 4, s));
     GridSync gs;
     gs.count = b->d_sync;
-    gs.gen = b->d_sync + 1;
     gs.err = (int *)(b->d_sync + 2);
     gs.limit = b->wait_limit;
     gs.tally = nullptr;

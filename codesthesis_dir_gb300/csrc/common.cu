@@ -120,7 +120,6 @@ extern "C" int gb_measure_grid_barrier(int blocks, int threads, int nbarriers, d
         e = cudaMemset(sync, 0, 4 * sizeof(unsigned));
         GridSync gs;
         gs.count = sync;
-        gs.gen = sync + 1;
         gs.err = (int *)(sync + 2);
         gs.limit = GB_GRID_WAIT_LIMIT_DEFAULT;
         gs.tally = nullptr;

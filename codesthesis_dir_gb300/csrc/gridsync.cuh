@@ -10,8 +10,7 @@
 // and handed to the whole block through shared memory, so all threads of a
 // block leave together even when another block raises the flag meanwhile.
 struct GridSync {
-    unsigned *count;
-    unsigned *gen;
+    unsigned *count;   // zero when the kernel starts
     int *err;
     long long limit;
     unsigned long long *tally;   // optional (may be null): barriers passed, counted once per barrier by block 0
@@ -20,27 +19,24 @@ struct GridSync {
 // Default wait limit: some seconds of polling at an L2 round trip per poll.
 #define GB_GRID_WAIT_LIMIT_DEFAULT (1LL << 24)
 
-// Arrival and wait of one thread per block.  The arrival count grows from one
-// barrier to the next (gen counts the barriers passed), so that nothing is
-// reset: the last arriver publishes the next generation, and the release and
-// acquire are those of the counter and the generation themselves instead of
-// fences around relaxed accesses.
+// Arrival and wait of one thread per block.  The count grows from one barrier
+// to the next (it is zero at the launch), so that nothing is reset and nobody
+// has to announce the last arrival: the blocks poll the count itself, a release
+// and its trip through L2 less than with a generation that the last one
+// publishes.
 __device__ __forceinline__ void grid_barrier(const GridSync &gs)
 {
-    unsigned g, arrived;
-    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(g) : "l"(gs.gen) : "memory");
+    unsigned arrived;
     asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(arrived) : "l"(gs.count) : "memory");
-    if (arrived + 1u == (g + 1u) * gridDim.x) {
-        asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(gs.gen), "r"(g + 1u) : "memory");
-    } else {
-        unsigned now = g;
-        for (long long it = 0; now == g;) {
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(gs.gen) : "memory");
-            if (now != g) break;
-            if (++it > gs.limit || ((it & 15) == 0 && *(volatile int *)gs.err)) {
-                atomicExch(gs.err, 1);
-                break;
-            }
+    const unsigned all = arrived - arrived % gridDim.x + gridDim.x;
+    if (arrived + 1u == all) return;
+    for (long long it = 0;;) {
+        unsigned now;
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(gs.count) : "memory");
+        if ((int)(now - all) >= 0) break;
+        if (++it > gs.limit || ((it & 15) == 0 && *(volatile int *)gs.err)) {
+            atomicExch(gs.err, 1);
+            break;
         }
     }
 }
