@@ -58,6 +58,8 @@ struct RowSplit {
     {
         if (n_ == 1) magic = 0;
     }
+    // of a divisor whose magic was formed before
+    __device__ __forceinline__ RowSplit(int n_, unsigned magic_) : n(n_), magic(magic_) {}
     __device__ __forceinline__ void operator()(int idx, int &q, int &r) const
     {
         if (n == 1) {

@@ -1184,6 +1184,10 @@ struct R3Shared {
     R3Work work[R3_LEVS];
     int my0, my1;           // the block's share of the phase at hand
     int p0, staged;         // its first chunk's factors: first radius, whether staged
+    int n, len, chunk;      // rows of a line, elements of a table, lines of a chunk
+    int lpitch, lg;         // FP32 lines' layout (warpline.cuh)
+    int nl;                 // lines of the first chunk
+    unsigned by_line, by_row;   // RowSplit of n and of nl
     int line[R3_THREADS];   // its first chunk's lines
     float4 weights[R3_WEIGHTS];   // the FP32 operator's, where they fit
 };
@@ -1295,7 +1299,8 @@ __device__ __forceinline__ bool r3_fetch(const R3Lev &L, int dir, int n, int len
 }
 
 // What phase ph of direction dir on level lev reads besides the solution: the
-// block's share of the lines, the first chunk's lines and factors.  None of it
+// block's share of the lines, the first chunk's lines and factors, and what
+// takes divisions to know (a thousand cycles of a phase of eight).  None of it
 // changes during a solve, so it is fetched while the block waits at the
 // barrier before the phase (threads 32 .. of the block).
 template <int COMP, class T> __device__ __noinline__ void r3_prepare(int lev, int dir, int ph)
@@ -1313,9 +1318,12 @@ template <int COMP, class T> __device__ __noinline__ void r3_prepare(int lev, in
     const int my1 = r3_group_start(lines, a, b, a + ((int)blockIdx.x + 1) * per);
     int p0 = 1;
     bool staged = false;
+    int nl = 0, chunk = 1;
     if (my0 < my1) {
-        const int c1 = r3_chunk_end(lines, my0, min(my1, my0 + r3_chunk<COMP, T>(dir, n, len)));
-        for (int t = tid; t < c1 - my0; t += nthr) S.line[t] = lines[my0 + t] & 0x7fffffff;
+        chunk = r3_chunk<COMP, T>(dir, n, len);
+        const int c1 = r3_chunk_end(lines, my0, min(my1, my0 + chunk));
+        nl = c1 - my0;
+        for (int t = tid; t < nl; t += nthr) S.line[t] = lines[my0 + t] & 0x7fffffff;
         staged = r3_fetch<COMP, T>(L, dir, n, len, c1 - my0, [&](int t) { return lines[my0 + t] & 0x7fffffff; }, tid, nthr, p0);
     }
     if (tid == 0) {
@@ -1323,6 +1331,14 @@ template <int COMP, class T> __device__ __noinline__ void r3_prepare(int lev, in
         S.my1 = my1;
         S.p0 = p0;
         S.staged = staged;
+        S.n = n;
+        S.len = len;
+        S.chunk = chunk;
+        S.lpitch = F64 ? 0 : wl_pitch(n);
+        S.lg = F64 ? 0 : wl_log2m(n);
+        S.nl = nl;
+        S.by_line = RowSplit(n).magic;
+        S.by_row = RowSplit(max(nl, 1)).magic;
     }
 }
 
@@ -1342,21 +1358,22 @@ template <int COMP, class T> __device__ __noinline__ void r3_phase(int lev, int 
     constexpr bool F64 = sizeof(T) == 8;
     const int my0 = S.my0, my1 = S.my1;
     if (my0 >= my1) return;
-    const int n1 = L.n1, n2 = L.n2, n3 = L.n3;
-    const size_t L1 = L.L1, L2 = L.L2;
-    const int kind = r3_kind(COMP, dir), n = r3_len(COMP, dir, n1, n2, n3);
-    const int len = F64 ? r3_tabsize(kind, n) : r3_tabsize32(kind, n);
-    const int lpitch = F64 ? 0 : wl_pitch(n), lg = F64 ? 0 : wl_log2m(n);
-    const int chunk = r3_chunk<COMP, T>(dir, n, len);
+    const int n3 = L.n3, L1 = L.L1, L2 = L.L2;
+    const int kind = r3_kind(COMP, dir), n = S.n, len = S.len, lpitch = S.lpitch, lg = S.lg, chunk = S.chunk;
     const int *lines = L.lines[COMP][dir];
     int *s_line = S.line;
     T *v = F64 ? (T *)W.v : (T *)W.v32;
     const T *fac = F64 ? (const T *)L.fac[COMP][dir] : (const T *)L.fac32[COMP][dir];
     T *x = (T *)(s_r3 + sizeof(R3Shared)), *sfac = (T *)(s_r3 + sizeof(R3Shared) + R3_CHUNK_BYTES);
-    const RowSplit by_line(n);
+    const RowSplit by_line(n, S.by_line);
+    RowSplit by_row(S.nl, S.by_row);
     for (int c0 = my0; c0 < my1;) {
-        const int c1 = r3_chunk_end(lines, c0, min(my1, c0 + chunk));
-        const int nl = c1 - c0, pitch = nl | 1;
+        int nl = S.nl;
+        if (c0 != my0) {
+            nl = r3_chunk_end(lines, c0, min(my1, c0 + chunk)) - c0;
+            if (nl != by_row.n) by_row = RowSplit(nl);
+        }
+        const int c1 = c0 + nl, pitch = nl | 1;
         auto at = [&](int t, int e) -> T & { return F64 ? x[e * pitch + t] : x[t * lpitch + wl_slot(lg, e)]; };
         int p0 = S.p0;
         bool staged = S.staged;
@@ -1367,7 +1384,7 @@ template <int COMP, class T> __device__ __noinline__ void r3_phase(int lev, int 
             staged = r3_fetch<COMP, T>(L, dir, n, len, nl, [&](int t) { return s_line[t]; }, threadIdx.x, R3_THREADS, p0);
         }
         if constexpr (!F64) {
-            r3_rhs32_batch<COMP>(L, W, dir, s_line, nl, n, dir == 0 ? by_line : RowSplit(nl), x, lpitch, lg);
+            r3_rhs32_batch<COMP>(L, W, dir, s_line, nl, n, dir == 0 ? by_line : by_row, x, lpitch, lg);
         } else if (dir == 0) {
             for (int idx = threadIdx.x; idx < nl * n; idx += R3_THREADS) {
                 int t, e;
@@ -1375,7 +1392,6 @@ template <int COMP, class T> __device__ __noinline__ void r3_phase(int lev, int 
                 at(t, e) = r3_rhs<COMP>(L, W, 0, s_line[t] & 0xffff, s_line[t] >> 16, e);
             }
         } else {
-            const RowSplit by_row(nl);
             for (int idx = threadIdx.x; idx < nl * n; idx += R3_THREADS) {
                 int e, t;
                 by_row(idx, e, t);
@@ -1383,8 +1399,9 @@ template <int COMP, class T> __device__ __noinline__ void r3_phase(int lev, int 
             }
         }
         if constexpr (!F64) {   // rows past the line's end
-            const int pad = wl_rows(n) - n;
-            for (int idx = threadIdx.x; idx < nl * pad; idx += R3_THREADS) at(idx / pad, n + idx % pad) = T(0);
+            const int pad = wl_rows(n) - n, warp = threadIdx.x >> 5;
+            for (int t = warp; t < nl; t += R3_THREADS / 32)
+                for (int q = threadIdx.x & 31; q < pad; q += 32) at(t, n + q) = T(0);
         }
         async_copy_wait();
         __syncthreads();
@@ -1421,21 +1438,20 @@ template <int COMP, class T> __device__ __noinline__ void r3_phase(int lev, int 
                 by_line(idx, t, e);
                 const int j = s_line[t] & 0xffff, k = s_line[t] >> 16;
                 const T val = at(t, e);
-                const size_t o = (size_t)(e + 1) + L1 * ((size_t)j + L2 * (size_t)k);
+                const int o = e + 1 + L1 * (j + L2 * k);
                 v[o] = val;
-                if (k == n3) v[o - L1 * L2 * (size_t)n3] = val;
+                if (k == n3) v[o - L1 * L2 * n3] = val;
             }
         } else {
-            const RowSplit by_row(nl);
             for (int idx = threadIdx.x; idx < nl * n; idx += R3_THREADS) {
                 int e, t;
                 by_row(idx, e, t);
                 const int i = s_line[t] & 0xffff, q = s_line[t] >> 16;
                 const int j = dir == 1 ? e + 1 : q, k = dir == 1 ? q : e + 1;
                 const T val = at(t, e);
-                const size_t o = (size_t)i + L1 * ((size_t)j + L2 * (size_t)k);
+                const int o = i + L1 * (j + L2 * k);
                 v[o] = val;
-                if (k == n3) v[o - L1 * L2 * (size_t)n3] = val;
+                if (k == n3) v[o - L1 * L2 * n3] = val;
             }
         }
         c0 = c1;
