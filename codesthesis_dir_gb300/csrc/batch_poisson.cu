@@ -1314,6 +1314,7 @@ __device__ __forceinline__ void run_item(const BatchDev &B, const TileEntry *til
 // one block of LOCAL_THREADS per problem.
 #define LOCAL_THREADS 512
 #define LOCAL_SOLVE_SMEM (220 * 1024)
+#define LOC_CTAS 8   // CTAs per problem, at most
 // Programmatic dependent launch (the graph path's kernels are launched with
 // programmatic stream serialization): a kernel may be scheduled while its
 // predecessor's last blocks still run, and waits here until that
@@ -1341,10 +1342,15 @@ __global__ void __launch_bounds__(LOCAL_THREADS) k_local(BatchDev B, Op op, int 
 // inner hierarchy; in plain FP64 the hierarchy's level 0 holds both.  The
 // operations are the same; the norm's sum runs in another order.
 //
+// With FP32 cycles a problem may have several CTAs, a cluster: the residual,
+// 12 k cycles of one SM's FP64 pipe at n = 65 where a cycle takes 13 k, is
+// shared by rows, each CTA storing its rows into every CTA's right-hand side,
+// and the cycle is run by all of them alike, which needs no exchange at all.
+//
 // As single launches an iteration of a small batch is launch and host latency
 // (eight problems of n = 17 .. 65, FP64 outer: 55 us an iteration, 550 us a
-// solve; here 20 us an iteration, most of it the FP64 residual, and 250 us a
-// solve).
+// solve; here 20 us an iteration with one CTA per problem, 12 with eight, and
+// 159 us a solve).
 template <class T, int CM> struct LocOuter {
     using V = typename CorrVal<CM>::type;
 };
@@ -1356,18 +1362,26 @@ __global__ void __launch_bounds__(LOCAL_THREADS) k_local_solve(BatchDev B, const
 {
     using V = typename LocOuter<T, CM>::V;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    __shared__ double s_part[LOCAL_THREADS / 32];
+    __shared__ double s_part[LOCAL_THREADS / 32], s_norm[LOC_CTAS];
     __shared__ int s_go;
-    const int p = blockIdx.x, n = B.n_of[p * BP_MAXL], lg = 31 - __clz(n - 1), m = n - 2, tid = threadIdx.x, nthr = LOCAL_THREADS;
+    const Cluster cl = Cluster::self();
+    const int p = blockIdx.x / cl.size, n = B.n_of[p * BP_MAXL], lg = 31 - __clz(n - 1), m = n - 2, tid = threadIdx.x, nthr = LOCAL_THREADS;
     T *mem = (T *)smem_raw;
     const LocTop<T> v(mem, lg);
     V *psi = (V *)(smem_raw + hierarchy), *f = psi + n * n;
     const V *gf = ((const V *const *)f_p)[p];
     V *gpsi = (V *)B.psi[p];
+    // own rows of the residual and of psi (psi also holds their neighbours)
+    const int share = (m + cl.size - 1) / cl.size, j0 = min(1 + cl.rank * share, m + 1), j1 = min(j0 + share, m + 1);
+    const int q0 = max(j0 - 1, 0) * n, q1 = min(j1 + 1, n) * n;
+    T *peer[LOC_CTAS];
+#pragma unroll
+    for (int r = 0; r < LOC_CTAS; ++r)
+        peer[r] = cl.size > 1 && r < cl.size ? cooperative_groups::this_cluster().map_shared_rank(v.F, r) : v.F;
     V zero;
     if constexpr (CM == CM_PAIR) zero = make_float2(0.f, 0.f);
     else zero = 0.0;
-    for (int q = tid; q < n * n; q += nthr) {
+    for (int q = q0 + tid; q < q1; q += nthr) {
         if constexpr (CM == CM_NONE) {
             v.X[v.at(q)] = (T)0;
             v.F[v.at(q)] = gf[q];
@@ -1376,60 +1390,85 @@ __global__ void __launch_bounds__(LOCAL_THREADS) k_local_solve(BatchDev B, const
             f[q] = gf[q];
         }
     }
-    __syncthreads();
+    cl.arrive();
     const int ls = lg;   // n - 1 slots a row, the first the boundary column
     const T ih2 = (T)(n - 1) * (T)(n - 1);
     double fnorm = 0.0;
     int cycles = 0;
     for (bool first = true;; first = false) {
+        if (cl.size == 1) __syncthreads();
+        else cl.wait();   // every CTA has finished the cycle that read F
         double acc = 0.0;
-        for (int q = tid; q < m << ls; q += nthr) {
-            const int j = (q >> ls) + 1, i = q & ((1 << ls) - 1), c = j * n + i;
+        for (int q = tid; q < (j1 - j0) << ls; q += nthr) {
+            const int j = (q >> ls) + j0, i = q & ((1 << ls) - 1), c = j * n + i;
             if (i == 0) continue;
             double rw;
             if constexpr (CM == CM_NONE) {
                 const T sum = (v.X[v.at(c - 1)] + v.X[v.at(c + 1)]) + (v.X[v.at(c - n)] + v.X[v.at(c + n)]);
                 rw = __fma_rn(-ih2, __fma_rn(-4.0, v.X[v.at(c)], sum), v.F[v.at(c)]);
-            } else if constexpr (CM == CM_PAIR) {
-                float2 r;
-                if (first) {
-                    r = df_add(f[c], make_float2(-0.0f, -0.0f));
-                } else {
-                    const float2 sum = df_add(df_add(psi[c - 1], psi[c + 1]), df_add(psi[c - n], psi[c + n]));
-                    const float2 lap = df_add(sum, df_scale(psi[c], -4.0f));
-                    r = df_add(f[c], df_scale(lap, -ih2));
-                }
-                rw = f2d(r.x);
-                v.F[v.at(c)] = r.x;
             } else {
-                if (first) {
-                    rw = f[c];
+                float r32;
+                if constexpr (CM == CM_PAIR) {
+                    float2 r;
+                    if (first) {
+                        r = df_add(f[c], make_float2(-0.0f, -0.0f));
+                    } else {
+                        const float2 sum = df_add(df_add(psi[c - 1], psi[c + 1]), df_add(psi[c - n], psi[c + n]));
+                        const float2 lap = df_add(sum, df_scale(psi[c], -4.0f));
+                        r = df_add(f[c], df_scale(lap, -ih2));
+                    }
+                    r32 = r.x;
+                    rw = f2d(r32);
                 } else {
-                    const double sum = (psi[c - 1] + psi[c + 1]) + (psi[c - n] + psi[c + n]);
-                    const double lap = __fma_rn(-4.0, psi[c], sum);
-                    rw = __fma_rn(-f2d(ih2), lap, f[c]);
+                    if (first) {
+                        rw = f[c];
+                    } else {
+                        const double sum = (psi[c - 1] + psi[c + 1]) + (psi[c - n] + psi[c + n]);
+                        const double lap = __fma_rn(-4.0, psi[c], sum);
+                        rw = __fma_rn(-f2d(ih2), lap, f[c]);
+                    }
+                    r32 = d2f_rn(rw);
                 }
-                v.F[v.at(c)] = d2f_rn(rw);
+                const int o = v.at(c);
+#pragma unroll
+                for (int r = 0; r < LOC_CTAS; ++r)
+                    if (r < cl.size) peer[r][o] = r32;
             }
             acc = __fma_rn(rw, rw, acc);
         }
         for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
         if ((tid & 31) == 0) s_part[tid >> 5] = acc;
         __syncthreads();
-        if (tid == 0) {   // op_finalize
-            double s = 0.0;
-            for (int w = 0; w < nthr / 32; ++w) s += s_part[w];
+        if (tid < 32) {
+            double s = tid < nthr / 32 ? s_part[tid] : 0.0;
+            for (int o = nthr / 64; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (cl.size == 1) {
+                if (tid == 0) s_norm[0] = s;
+            } else if (tid < cl.size) {
+                cooperative_groups::this_cluster().map_shared_rank(s_norm, tid)[cl.rank] = s;
+            }
+        }
+        cl.sync();
+        if (tid == 0) {   // op_finalize; every CTA decides alike
+            double s = s_norm[0];
+            for (int r = 1; r < cl.size; ++r) s += s_norm[r];
             const double rn = sqrt(s);
             if (first) fnorm = rn;
-            B.relres[p] = fnorm > 0.0 ? rn / fnorm : 0.0;
             int failed = 0;
             s_go = 0;
             if (!(rn <= 1.79769313486231570815e308)) failed = 2;
             else if (rn <= B.rtol * fnorm) failed = 0;
             else if (cycles >= B.max_cycles) failed = 1;
             else s_go = 1;
-            if (s_go) cycles += B.inner;
-            else B.failed[p] = failed;
+            if (s_go) {
+                cycles += B.inner;
+            } else if (cl.rank == 0) {
+                B.failed[p] = failed;
+                B.relres[p] = fnorm > 0.0 ? rn / fnorm : 0.0;
+                B.cycles[p] = cycles;
+                B.fnorm[p] = fnorm;
+                B.active[p] = 0;
+            }
         }
         __syncthreads();
         if (!s_go) break;
@@ -1439,21 +1478,20 @@ __global__ void __launch_bounds__(LOCAL_THREADS) k_local_solve(BatchDev B, const
             for (int q = tid; q < 2 * v.half; q += nthr) v.X[q] = (T)0;
             __syncthreads();
             for (int k = 0; k < B.inner; ++k) loc_vcycle<T, LOCAL_THREADS>(mem, lg, nu1, nu2);
-            for (int q = tid; q < n * n; q += nthr) {
+            cl.arrive();
+            for (int q = q0 + tid; q < q1; q += nthr) {
                 if constexpr (CM == CM_PAIR) psi[q] = df_add_f(psi[q], v.X[v.at(q)]);
                 else psi[q] = psi[q] + f2d(v.X[v.at(q)]);
             }
             __syncthreads();
         }
     }
-    for (int q = tid; q < n * n; q += nthr) {
-        if constexpr (CM == CM_NONE) gpsi[q] = v.X[v.at(q)];
+    // own rows; the first and the last CTA also the boundary's
+    const int a = cl.rank == 0 ? 0 : j0 * n, b = cl.rank == cl.size - 1 ? n * n : j1 * n;
+    for (int q = a + tid; q < b; q += nthr) {
+        if (q < q0 || q >= q1) gpsi[q] = zero;   // a CTA without rows
+        else if constexpr (CM == CM_NONE) gpsi[q] = v.X[v.at(q)];
         else gpsi[q] = psi[q];
-    }
-    if (tid == 0) {
-        B.cycles[p] = cycles;
-        B.fnorm[p] = fnorm;
-        B.active[p] = 0;
     }
 }
 
@@ -2440,8 +2478,13 @@ static size_t whole_local_smem(const gb_batch *b)
 template <class T, int CM> static int solve_local(gb_batch *b, size_t sm, cudaStream_t s)
 {
     GB_CUDA_TRY(cudaFuncSetAttribute(k_local_solve<T, CM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    k_local_solve<T, CM><<<b->nprob, LOCAL_THREADS, sm, s>>>(b->dev, (const double *const *)b->d_f_tab, b->nu1, b->nu2, (int)b->local_smem);
-    GB_CUDA_TRY(cudaGetLastError());
+    // as many as share the SMs evenly; where the FP64 pipe does the cycles as
+    // well, or there are no SMs to spare, one
+    int ctas = 1;
+    while (CM != CM_NONE && ctas < LOC_CTAS && b->nprob * ctas * 2 <= b->nsm) ctas *= 2;
+    ctas = cl_fit(k_local_solve<T, CM>, ctas, LOCAL_THREADS, sm);
+    GB_CUDA_TRY(cl_launch(k_local_solve<T, CM>, b->nprob, ctas, LOCAL_THREADS, sm, s, b->dev, (const double *const *)b->d_f_tab, b->nu1, b->nu2,
+                          (int)b->local_smem));
     b->launches += 1;
     return GB_OK;
 }

@@ -1,5 +1,5 @@
-"""Batches whose problems are all small enough for one block each are solved
-whole in one launch (k_local_solve): bit for bit the oracle's solutions and
+"""Batches whose problems are all small enough for one block each (or a cluster
+that repeats one block's cycles) are solved whole in one launch (k_local_solve): bit for bit the oracle's solutions and
 cycle counts at every size from one interior point to the largest such problem,
 in each precision, and the same endings as the level-by-level solve (cycle
 limit, right-hand sides of zero and with a NaN)."""
@@ -14,7 +14,8 @@ MODES = [(0, 1), (1, 1), (1, 3), (2, 1), (2, 4)]
 
 
 @pytest.mark.parametrize("precision,inner", MODES)
-@pytest.mark.parametrize("sizes", [[3], [5, 3], [9], [17, 9, 17], [33], [65, 3, 33, 5, 17, 9, 65]])
+@pytest.mark.parametrize("sizes", [[3], [5, 3], [9], [17, 9, 17], [33], [65, 3, 33, 5, 17, 9, 65], [65, 5, 33] * 8, [17, 3, 65] * 16,
+                                   [9, 33, 17] * 32])   # eight, four, two and one CTA per problem
 def test_matches_oracle(oracle, gblib, precision, inner, sizes):
     from codesthesis_dir_gb300.batch import BatchPoisson
     f = make_batch(sizes, 31)
