@@ -165,76 +165,32 @@ template <class T, int H> struct TileLayout {
     __device__ static __forceinline__ int at(int r, int c) { return ((r + c) & 1) * HALF + r * SXH + (c >> 1); }
 };
 
-// One row of a red-black phase: the points of one colour between the
-// bounds, as consecutive words of one half (c = 2k + odd; the row neighbours
-// c -+ 1 are k - 1 + odd and k + odd of the other half).
-template <class T> struct PhaseRow {
-    T *X;
-    const T *F, *N;
-    int odd, k0, kend;
-};
-
-template <class T, int H>
-__device__ __forceinline__ PhaseRow<T> phase_row(T *sx, const T *sf, int gy, int oy, int ox, int gxa, int gxb,
-                                                 int color)
-{
-    using LY = TileLayout<T, H>;
-    const int row = (gy - oy) * LY::SXH;
-    const int first = gxa + ((gxa + gy + color) & 1);
-    const int c0 = first - ox, odd = c0 & 1;
-    PhaseRow<T> R;
-    R.X = sx + color * LY::HALF + row;
-    R.F = sf + color * LY::HALF + row;
-    R.N = sx + (color ^ 1) * LY::HALF + row;
-    R.odd = odd;
-    R.k0 = c0 >> 1;
-    R.kend = (gxb - ox - odd + 1) >> 1;
-    return R;
-}
-
-template <class T, int H>
-__device__ __forceinline__ void phase_point(const PhaseRow<T> &R, int k, T h2)
-{
-    using LY = TileLayout<T, H>;
-    const T s = (R.N[k - 1 + R.odd] + R.N[k + R.odd]) + (R.N[k - LY::SXH] + R.N[k + LY::SXH]);
-    R.X[k] = fmaT<T>(-h2, R.F[k], s) * (T)0.25;
-}
-
 // One red (color 0) or black (color 1) phase on ring rho around the tile.
-// The smem tile has origin (ox, oy) in grid coordinates, colour-split.  A
-// row holds at most SXH = 64 + H points of a colour, so a warp covers the
-// first 64 of each of two rows in two passes per row and the rest of both
-// (at most H each) in one shared pass: half the lanes per row.
+// The smem tile has origin (ox, oy) in grid coordinates, colour-split.  The
+// FP64 pipe takes a warp instruction's 64 cycles whatever its lanes do, so the
+// phase's points are dealt to the threads one after the other, whole warps of
+// them (a row's 64 + rho points by two and a half passes of 32 lanes left a
+// sixth of the lanes idle, and 42 rows a sixth of the eight warps); the index
+// arithmetic costs a tenth of the five FP64 instructions.
 template <class T, int H>
 __device__ __forceinline__ void tile_phase(T *sx, const T *sf, int ox, int oy, int x0, int y0, int n, T h2,
                                            int rho, int color)
 {
-    static_assert(TileLayout<T, H>::SXH <= 64 + 16, "row remainder must fit in half a warp");
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    using LY = TileLayout<T, H>;
     const int gxa = max(x0 - rho, 1), gxb = min(x0 + TX + rho, n - 1);
     const int gya = max(y0 - rho, 1), gyb = min(y0 + TY + rho, n - 1);
-    for (int gy = gya + warp; gy < gyb; gy += 2 * nw) {
-        const PhaseRow<T> A = phase_row<T, H>(sx, sf, gy, oy, ox, gxa, gxb, color);
-        const bool two = gy + nw < gyb;
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const int k = A.k0 + lane + 32 * j;
-            if (k < A.kend) phase_point<T, H>(A, k, h2);
-        }
-        if (two) {
-            const PhaseRow<T> B = phase_row<T, H>(sx, sf, gy + nw, oy, ox, gxa, gxb, color);
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                const int k = B.k0 + lane + 32 * j;
-                if (k < B.kend) phase_point<T, H>(B, k, h2);
-            }
-            const PhaseRow<T> &R = lane < 16 ? A : B;
-            const int k = R.k0 + 64 + (lane & 15);
-            if (k < R.kend) phase_point<T, H>(R, k, h2);
-        } else if (lane < 16) {
-            const int k = A.k0 + 64 + lane;
-            if (k < A.kend) phase_point<T, H>(A, k, h2);
-        }
+    const RowSplit row((gxb - gxa + 1) >> 1);
+    const int total = (gyb - gya) * row.n;
+#pragma unroll 2
+    for (int q = threadIdx.x; q < total; q += TILE_THREADS) {
+        int r, k;
+        row(q, r, k);
+        const int gy = gya + r, gx = gxa + ((gxa + gy + color) & 1) + 2 * k;
+        if (gx >= gxb) continue;
+        const int c = gx - ox, odd = c & 1, at = (gy - oy) * LY::SXH + (c >> 1);
+        const T *N = sx + (color ^ 1) * LY::HALF + at;
+        const T s = (N[odd - 1] + N[odd]) + (N[-LY::SXH] + N[LY::SXH]);
+        sx[color * LY::HALF + at] = fmaT<T>(-h2, sf[color * LY::HALF + at], s) * (T)0.25;
     }
     __syncthreads();
 }
@@ -333,39 +289,23 @@ __device__ void op_smooth(const BatchDev &B, TileEntry e, int l, int zero_init, 
     tile_store<T, H>(sx, ox, oy, x0, y0, n, XS<T>(B, e.p, l, dst));
     if (RESTRICT) {
         // residual on the tile plus one ring, in place of f (each point
-        // reads f only at itself and x, which stays put, so both colours of
-        // a row go in one pass: 65 points each, two full passes per colour
-        // and one shared pass for the last point of each)
+        // reads f only at itself and x, which stays put), dealt to the threads
+        // as a phase's points are
         const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
         const T ih2 = IH2<T>(B, e.p, l);
-        const int gxa = x0 - 1, gxb = x0 + TX + 1;
-        for (int gy = y0 - 1 + warp; gy <= y0 + TY; gy += nw) {
-            const bool rin = gy >= 1 && gy <= n - 2;
-            const PhaseRow<T> R0 = phase_row<T, H>(sx, sf, gy, oy, ox, gxa, gxb, 0);
-            const PhaseRow<T> R1 = phase_row<T, H>(sx, sf, gy, oy, ox, gxa, gxb, 1);
-            auto res_point = [&](const PhaseRow<T> &R, int k) {
-                const int gx = 2 * k + R.odd + ox;
-                T rv = (T)0;
-                if (rin && gx >= 1 && gx <= n - 2) {
-                    const T s = (R.N[k - 1 + R.odd] + R.N[k + R.odd]) + (R.N[k - LY::SXH] + R.N[k + LY::SXH]);
-                    const T lap = fmaT<T>((T)-4, R.X[k], s);
-                    rv = fmaT<T>(-ih2, lap, R.F[k]);
-                }
-                const_cast<T *>(R.F)[k] = rv;
-            };
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                const int k = R0.k0 + lane + 32 * j;
-                if (k < R0.kend) res_point(R0, k);
+        constexpr int RX = TX + 2, RY = TY + 2;
+#pragma unroll 2
+        for (int q = threadIdx.x; q < RX * RY; q += TILE_THREADS) {
+            const int r = q / RX, gy = y0 - 1 + r, gx = x0 - 1 + q - r * RX;
+            const int c = gx - ox, odd = c & 1, color = (gx + gy) & 1, at = (gy - oy) * LY::SXH + (c >> 1);
+            T rv = (T)0;
+            if (gx >= 1 && gx <= n - 2 && gy >= 1 && gy <= n - 2) {
+                const T *N = sx + (color ^ 1) * LY::HALF + at;
+                const T s = (N[odd - 1] + N[odd]) + (N[-LY::SXH] + N[LY::SXH]);
+                const T lap = fmaT<T>((T)-4, sx[color * LY::HALF + at], s);
+                rv = fmaT<T>(-ih2, lap, sf[color * LY::HALF + at]);
             }
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                const int k = R1.k0 + lane + 32 * j;
-                if (k < R1.kend) res_point(R1, k);
-            }
-            const PhaseRow<T> &R = lane < 16 ? R0 : R1;
-            const int k = R.k0 + 64 + (lane & 15);
-            if (k < R.kend) res_point(R, k);
+            sf[color * LY::HALF + at] = rv;
         }
         __syncthreads();
         const int nc = B.n_of[e.p * BP_MAXL + l + 1];
