@@ -387,7 +387,8 @@ int gb_axi_run_end(gb_axi *h, int nsteps, double *nu, int *sweeps, int *steps_do
  * (monashubuntudir_velvor2dhorconvtankdir/sleeprun.s:1-8).  Every phase of
  * a step (each transport routine, the heat flux, the right-hand sides, the
  * update, the bookkeeping) is one launch over the blocks of all members; the
- * multigrid solves of all members are one launch of one block per equation.
+ * multigrid solves of all members are one launch, a cluster (or one CTA) per
+ * equation.
  * Each member runs exactly its own routines, so its fields, Nusselt history
  * and sweep counts are bit-identical to stepping it alone.
  *
