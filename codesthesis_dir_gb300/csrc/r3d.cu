@@ -2665,9 +2665,11 @@ static int r3_create(const gb_r3d_params *p, const double *spacing, gb_r3d **out
         e = cudaMalloc(&work, sizeof(double) * (size_t)wstride * jobs.size());
         if (e != cudaSuccess) { cudaFree(djobs); gb_r3d_destroy(h); gb_set_error("gb_r3d_create: factor scratch"); return GB_ERR_ALLOC; }
         k_r3d_factors<<<gb_ceil_div(jobs.size(), 64), 64>>>(d, djobs, (int)jobs.size(), work, wstride);
-        k_r3d_factors32<<<gb_ceil_div(jobs.size(), 64), 64>>>(d, djobs, (int)jobs.size());
-        k_r3d_steps32<<<dim3(nlev, 3, 2), 128>>>(d);
-        k_r3d_weights32<<<dim3(nlev, 3), 128>>>(d);
+        if (p->precision == GB_PRB_MIXED) {
+            k_r3d_factors32<<<gb_ceil_div(jobs.size(), 64), 64>>>(d, djobs, (int)jobs.size());
+            k_r3d_steps32<<<dim3(nlev, 3, 2), 128>>>(d);
+            k_r3d_weights32<<<dim3(nlev, 3), 128>>>(d);
+        }
         cudaDeviceSynchronize();
         cudaFree(work);
     }
