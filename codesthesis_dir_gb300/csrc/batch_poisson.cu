@@ -1519,6 +1519,7 @@ struct gb_batch {
     double **d_psi_tab = nullptr, **d_f_tab = nullptr;
     std::vector<void *> hx, hf;
     size_t local_smem = 0;
+    int local_ctas = 0;                 // CTAs per problem of whole solves (k_local_solve), once known
     int *h_pinned = nullptr;
     double *host_stage = nullptr;       // f and psi of gb_batch_solve_host, allocated on first use
     // pipelined host-buffer solves (gb_batch_submit_host): two slots of f and
@@ -2417,13 +2418,15 @@ static size_t whole_local_smem(const gb_batch *b)
 
 template <class T, int CM> static int solve_local(gb_batch *b, size_t sm, cudaStream_t s)
 {
-    GB_CUDA_TRY(cudaFuncSetAttribute(k_local_solve<T, CM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    // as many as share the SMs evenly; where the FP64 pipe does the cycles as
-    // well, or there are no SMs to spare, one
-    int ctas = 1;
-    while (CM != CM_NONE && ctas < LOC_CTAS && b->nprob * ctas * 2 <= b->nsm) ctas *= 2;
-    ctas = cl_fit(k_local_solve<T, CM>, ctas, LOCAL_THREADS, sm);
-    GB_CUDA_TRY(cl_launch(k_local_solve<T, CM>, b->nprob, ctas, LOCAL_THREADS, sm, s, b->dev, (const double *const *)b->d_f_tab, b->nu1, b->nu2,
+    if (!b->local_ctas) {
+        GB_CUDA_TRY(cudaFuncSetAttribute(k_local_solve<T, CM>, cudaFuncAttributeMaxDynamicSharedMemorySize, LOCAL_SOLVE_SMEM));
+        // as many as share the SMs evenly; where the FP64 pipe does the cycles
+        // as well, or there are no SMs to spare, one
+        int ctas = 1;
+        while (CM != CM_NONE && ctas < LOC_CTAS && b->nprob * ctas * 2 <= b->nsm) ctas *= 2;
+        b->local_ctas = cl_fit(k_local_solve<T, CM>, ctas, LOCAL_THREADS, sm);
+    }
+    GB_CUDA_TRY(cl_launch(k_local_solve<T, CM>, b->nprob, b->local_ctas, LOCAL_THREADS, sm, s, b->dev, (const double *const *)b->d_f_tab, b->nu1, b->nu2,
                           (int)b->local_smem));
     b->launches += 1;
     return GB_OK;
