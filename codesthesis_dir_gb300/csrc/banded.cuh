@@ -41,26 +41,6 @@ __device__ inline void factor_tdma(const double *a, const double *b, const doubl
     for (int j = 0; j < n; ++j) ibp[j] = 1.0 / bp[j];
 }
 
-// Solve in place: x[j*stride] holds r on entry, the solution on exit.
-// rhs(j) supplies r lazily when x == nullptr-like use is not wanted; the
-// generic form below reads r from x.
-__device__ inline void apply_tdma(const double *fac, int n, double *x, int stride)
-{
-    const double *fact = fac, *bp = fac + n, *c = fac + 2 * n, *ibp = fac + 3 * n;
-    double prev = x[0];
-    for (int j = 1; j < n; ++j) {
-        double rj = x[(size_t)j * stride] - fact[j] * prev;
-        x[(size_t)j * stride] = rj;
-        prev = rj;
-    }
-    double y = div_by_rcp(x[(size_t)(n - 1) * stride], bp[n - 1], ibp[n - 1]);
-    x[(size_t)(n - 1) * stride] = y;
-    for (int j = n - 2; j >= 0; --j) {
-        y = div_by_rcp(x[(size_t)j * stride] - c[j] * y, bp[j], ibp[j]);
-        x[(size_t)j * stride] = y;
-    }
-}
-
 // ---------------------------------------------------------------------------
 // Periodic tridiagonal (ptdma, velvor2dperiodicrbconv.f:3066-3116), n >= 4.
 // Factor layout (6n + 3 doubles): f1[n), f2[n), a'[n), b'[n), c'[n), 1/b'[n),
@@ -178,39 +158,6 @@ __device__ inline void factor_pdma(const double *a0, const double *b0, const dou
     fac[6 * n + 3] = (double)je;
 }
 
-// Solve with the right-hand side produced by rhs(j) (0-based row j), writing
-// the normalised eliminated rows and then the solution to x[j*stride].
-template <class Rhs>
-__device__ inline void apply_pdma_rhs(const double *fac, int n, double *x, int stride, Rhs rhs)
-{
-    const double *cdiv = fac, *bk1 = fac + n, *aa = fac + 2 * n, *dn = fac + 3 * n, *en = fac + 4 * n;
-    const double *icdiv = fac + 5 * n + 1;
-    const double cN = fac[5 * n], icN = fac[6 * n + 1];
-    double rk = rhs(0);
-    double rk1 = rhs(1);
-#pragma unroll 4
-    for (int k = 0; k <= n - 2; ++k) {
-        rk = div_by_rcp(rk, cdiv[k], icdiv[k]);
-        x[(size_t)k * stride] = rk;
-        rk1 = rk1 - bk1[k] * rk;
-        double rk2 = 0.0;
-        if (k != n - 2) rk2 = rhs(k + 2) - aa[k + 2] * rk;
-        rk = rk1;
-        rk1 = rk2;
-    }
-    double x1 = div_by_rcp(rk, cN, icN);
-    x[(size_t)(n - 1) * stride] = x1;
-    double x0 = x[(size_t)(n - 2) * stride] - dn[n - 2] * x1;
-    x[(size_t)(n - 2) * stride] = x0;
-#pragma unroll 4
-    for (int j = n - 3; j >= 0; --j) {
-        double xj = x[(size_t)j * stride] - dn[j] * x0 - en[j] * x1;
-        x[(size_t)j * stride] = xj;
-        x1 = x0;
-        x0 = xj;
-    }
-}
-
 // Tridiagonal solve with a lazily produced right-hand side.
 template <class Rhs>
 __device__ inline void apply_tdma_rhs(const double *fac, int n, double *x, int stride, Rhs rhs)
@@ -238,57 +185,6 @@ __device__ inline void apply_ptdma_rhs(const double *fac, int n, double *x, int 
 {
     for (int j = 0; j < n; ++j) x[(size_t)j * stride] = rhs(j);
     apply_ptdma(fac, n, x, stride);
-}
-
-// ---------------------------------------------------------------------------
-// FP32 eliminations in place on a line held in shared memory at x[k * pitch]
-// (the mixed-precision correction cycles).  Factor layouts: pentadiagonal
-// 1/cdiv[n), bk1[n), a[n), dn[n), en[n), 1/cN; tridiagonal fact[n), 1/bp[n),
-// c[n).  Pivots are multiplied by their stored reciprocals.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ void pdma32_smem(const float *fac, int n, float *x, int pitch)
-{
-    const float *icdiv = fac, *bk1 = fac + n, *aa = fac + 2 * n, *dn = fac + 3 * n, *en = fac + 4 * n;
-    float rk = x[0], rk1 = x[pitch];
-#pragma unroll 4
-    for (int k = 0; k <= n - 2; ++k) {
-        const float xr = (k + 2 < n) ? x[(k + 2) * pitch] : 0.f;
-        rk = rk * icdiv[k];
-        x[k * pitch] = rk;
-        rk1 = rk1 - bk1[k] * rk;
-        const float rk2 = (k != n - 2) ? xr - aa[k + 2] * rk : 0.f;
-        rk = rk1;
-        rk1 = rk2;
-    }
-    float x1 = rk * fac[5 * n];
-    x[(n - 1) * pitch] = x1;
-    float x0 = x[(n - 2) * pitch] - dn[n - 2] * x1;
-    x[(n - 2) * pitch] = x0;
-#pragma unroll 4
-    for (int j = n - 3; j >= 0; --j) {
-        const float xj = x[j * pitch] - dn[j] * x0 - en[j] * x1;
-        x[j * pitch] = xj;
-        x1 = x0;
-        x0 = xj;
-    }
-}
-
-__device__ __forceinline__ void tdma32_smem(const float *fac, int n, float *x, int pitch)
-{
-    const float *fact = fac, *ibp = fac + n, *c = fac + 2 * n;
-    float prev = x[0];
-#pragma unroll 4
-    for (int j = 1; j < n; ++j) {
-        prev = x[j * pitch] - fact[j] * prev;
-        x[j * pitch] = prev;
-    }
-    float y = prev * ibp[n - 1];
-    x[(n - 1) * pitch] = y;
-#pragma unroll 4
-    for (int j = n - 2; j >= 0; --j) {
-        y = (x[j * pitch] - c[j] * y) * ibp[j];
-        x[j * pitch] = y;
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -392,7 +288,7 @@ __device__ __forceinline__ void pdma_up(const double *fac, int n, double *x, int
         }
     }
 }
-// Pentadiagonal, factor_pdma's layout: apply_pdma_rhs's operations in its order.
+// Pentadiagonal, factor_pdma's layout: pdma's right-hand-side operations in its order.
 template <int U = 2> __device__ __forceinline__ void pdma_staged(const double *fac, int n, double *x, int pitch)
 {
     const int ka = (int)fac[6 * n + 2], je = (int)fac[6 * n + 3];
