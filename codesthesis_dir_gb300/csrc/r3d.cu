@@ -2360,27 +2360,29 @@ static void r3_phases(int mode, int pslow, int comp, int dir, int n1, int n2, in
             for (int q = 1; q <= Q; ++q)
                 for (int p = 1; p <= P; ++p)
                     if (((p + q) & 1) == colour && cls_of(p, q) == cls) groups[root(id(p, q))].push_back(p | (q << 16));
-        // FP64 lines share a radius's factors: its lines in a row (p slow); FP32
-        // ones take what runs with memory (p fast)
-        if (pslow)
-            std::stable_sort(groups.begin(), groups.end(), [](const std::vector<int> &x, const std::vector<int> &y) {
-                auto key = [](const std::vector<int> &g) {
-                    int m = 1 << 30;
-                    for (int e : g) m = std::min(m, e & 0xffff);
-                    return m;
-                };
-                return key(x) < key(y);
-            });
+        // FP64 lines share a radius's factors: its lines in a row (p slow, a
+        // group where its least p belongs); FP32 ones take what runs with memory
+        // (p fast)
+        std::vector<std::vector<int>> at(pslow ? (size_t)P + 1 : 1);
+        for (int g = 0; g < (int)groups.size(); ++g) {
+            if (groups[g].empty()) continue;
+            int least = pslow ? P : 0;
+            if (pslow)
+                for (int e : groups[g]) least = std::min(least, e & 0xffff);
+            at[least].push_back(g);
+        }
         size_t biggest = 0;
         for (const auto &g : groups) biggest = std::max(biggest, g.size());
         if ((int)biggest <= chunk) {
             const size_t before = lines.size();
             for (int multi = 1; multi >= 0; --multi)   // groups of several lines first, then single lines
-                for (const auto &g : groups) {
-                    if (g.empty() || (g.size() > 1) != (multi == 1)) continue;
-                    for (size_t t = 0; t < g.size(); ++t)
-                        lines.push_back((int)((unsigned)g[t] | (t + 1 < g.size() ? R3_CONT : 0u)));
-                }
+                for (const auto &some : at)
+                    for (int which : some) {
+                        const auto &g = groups[which];
+                        if ((g.size() > 1) != (multi == 1)) continue;
+                        for (size_t t = 0; t < g.size(); ++t)
+                            lines.push_back((int)((unsigned)g[t] | (t + 1 < g.size() ? R3_CONT : 0u)));
+                    }
             if (lines.size() != before) off.push_back((int)lines.size());
         } else {
             for (int cls = 2; cls >= 0; --cls) {
