@@ -94,44 +94,64 @@ template <class T> struct PlView {
     __device__ __forceinline__ T at(int k, int i) const { return pl_load(rows[k] + (unsigned)sizeof(T) * col(i), T(0)); }
 };
 
-// One colour (lines first, first + 2, ...) of a sweep on level l.
-template <class T> __device__ __noinline__ void pl_colour(const MgEq &E, int l, int first)
+// One colour (lines first, first + 2, ...) of a sweep on level l in FP64.
+__device__ __noinline__ void pl_colour64(const MgEq &E, int l, int first)
 {
     const Cluster cl = Cluster::self();
-    const PlView<T> L(E, l, cl);
+    const PlView<double> L(E, l, cl);
     const int n = L.which == 2 ? L.n1 : L.n1 - 1;
     const int kb = L.k0 + ((first - L.k0) & 1), ke = min(L.k1, L.klast + 1);   // own lines kb, kb + 2, ... < ke
     const int nl = kb < ke ? (ke - 1 - kb) / 2 + 1 : 0;
-    auto seam = [&](int i, T x) { pl_store(L.rows[0] + (unsigned)sizeof(T) * L.col(i), L.xwall ? T(0) : x); };
-    if constexpr (sizeof(T) == 8) {
-        // right-hand sides in place (nothing reads this colour's lines now)
-        const RowSplit split(n);
-        for (int idx = threadIdx.x; idx < nl * n; idx += PL_THREADS) {
-            int t, q;
-            split(idx, t, q);
-            const int k = kb + 2 * t, i = q + 1;
-            T r = -(L.at(L.after(k), i) + L.at(k - 1, i)) * L.hhpi;
-            if (L.polar) r = r * L.rvq[i];
-            L.own(L.v, k)[i] = r + L.own(L.f, k)[i];
-        }
+    // right-hand sides in place (nothing reads this colour's lines now)
+    const RowSplit split(n);
+    for (int idx = threadIdx.x; idx < nl * n; idx += PL_THREADS) {
+        int t, q;
+        split(idx, t, q);
+        const int k = kb + 2 * t, i = q + 1;
+        double r = -(L.at(L.after(k), i) + L.at(k - 1, i)) * L.hhpi;
+        if (L.polar) r = r * L.rvq[i];
+        L.own(L.v, k)[i] = r + L.own(L.f, k)[i];
+    }
+    __syncthreads();
+    if ((int)threadIdx.x < nl) {
+        const int k = kb + 2 * threadIdx.x;
+        double *x = L.own(L.v, k) + 1;
+        if (L.which == 2) pdma_staged<2>(L.fac, n, x, 1);
+        else tdma_staged<2>(L.fac, n, x, 1);
+    }
+    if (ke - 1 == L.n3 && nl > 0 && ((L.n3 - kb) & 1) == 0) {   // line n3 was solved: k = 0 repeats it
         __syncthreads();
-        if ((int)threadIdx.x < nl) {
-            const int k = kb + 2 * threadIdx.x;
-            T *x = L.own(L.v, k) + 1;
-            if (L.which == 2) pdma_staged<2>(L.fac, n, x, 1);
-            else tdma_staged<2>(L.fac, n, x, 1);
-        }
-        if (ke - 1 == L.n3 && nl > 0 && ((L.n3 - kb) & 1) == 0) {   // line n3 was solved: k = 0 repeats it
-            __syncthreads();
-            for (int i = 1 + threadIdx.x; i <= n; i += PL_THREADS) seam(i, L.own(L.v, L.n3)[i]);
-        }
-    } else {
-        auto lines = [&](auto m, auto penta) {
-            constexpr int M = decltype(m)::value;
-            constexpr bool PENTA = decltype(penta)::value;
-            const int lw = wl_log2w(n), per = 32 >> lw;
-            const int sub = (threadIdx.x & 31) >> lw, lane = threadIdx.x & ((1 << lw) - 1);
-            const int slot = (threadIdx.x >> 5) * per + sub, nslots = (PL_THREADS / 32) * per;
+        for (int i = 1 + threadIdx.x; i <= n; i += PL_THREADS) pl_store(L.rows[0] + 8u * L.col(i), L.xwall ? 0.0 : L.own(L.v, L.n3)[i]);
+    }
+    cl.sync();
+}
+
+// The relaxations' sweeps on level l, colour by colour (lines 1, 3, ... and 2,
+// 4, ...).  One table serves all lines of a level: in FP32 the lanes load their
+// rows of it once for all the sweeps of a visit (layer 129 x 65 mixed, four
+// steps: 13.5 -> 12.4 ms); the FP64 chains gain nothing from it.
+__device__ __noinline__ void pl_sweeps32(const MgEq &E, int l)
+{
+    using T = float;
+    const Cluster cl = Cluster::self();
+    const PlView<T> L(E, l, cl);
+    const int n = L.which == 2 ? L.n1 : L.n1 - 1, phases = 2 * E.nrelax;
+    const int ke = min(L.k1, L.klast + 1);
+    auto seam = [&](int i, T x) { pl_store(L.rows[0] + (unsigned)sizeof(T) * L.col(i), L.xwall ? T(0) : x); };
+    // own lines of phase ph: kb, kb + 2, ... < ke, nl of them
+    auto begin = [&](int ph) { return L.k0 + ((1 + ph - L.k0) & 1); };
+    auto count = [&](int kb) { return kb < ke ? (ke - 1 - kb) / 2 + 1 : 0; };
+    auto lines = [&](auto m, auto penta) {
+        constexpr int M = decltype(m)::value;
+        constexpr bool PENTA = decltype(penta)::value;
+        const int lw = wl_log2w(n), per = 32 >> lw;
+        const int sub = (threadIdx.x & 31) >> lw, lane = threadIdx.x & ((1 << lw) - 1);
+        const int slot = (threadIdx.x >> 5) * per + sub, nslots = (PL_THREADS / 32) * per;
+        WlTab<M, PENTA> tab;
+        tab.load((const float *)L.fac, lw);
+#pragma unroll 1
+        for (int ph = 0; ph < phases; ++ph) {
+            const int kb = begin(ph), nl = count(kb);
             for (int tb = 0; tb < nl; tb += nslots) {
                 if (tb + slot - sub >= nl) continue;   // no line for this warp
                 const bool live = tb + slot < nl;
@@ -151,8 +171,6 @@ template <class T> __device__ __noinline__ void pl_colour(const MgEq &E, int l, 
                     if (L.polar) r = r * L.rvq[min(lane * M + u + 1, L.n1 + 1)];
                     t[u] = lane * M + u < n ? r + fr[u] : T(0);
                 }
-                WlTab<M, PENTA> tab;
-                tab.load((const float *)L.fac, lw);
                 tab.solve(lw, (float(&)[M])t);
                 if (live) {
                     T *vr = L.own(L.v, k) + c0;
@@ -164,16 +182,25 @@ template <class T> __device__ __noinline__ void pl_colour(const MgEq &E, int l, 
                         }
                 }
             }
-        };
-        if (L.lg == 3) {
-            if (L.which == 2) lines(std::integral_constant<int, 8>(), std::true_type());
-            else lines(std::integral_constant<int, 8>(), std::false_type());
-        } else {
-            if (L.which == 2) lines(std::integral_constant<int, 16>(), std::true_type());
-            else lines(std::integral_constant<int, 16>(), std::false_type());
+            cl.sync();
         }
+    };
+    if (L.lg == 3) {
+        if (L.which == 2) lines(std::integral_constant<int, 8>(), std::true_type());
+        else lines(std::integral_constant<int, 8>(), std::false_type());
+    } else {
+        if (L.which == 2) lines(std::integral_constant<int, 16>(), std::true_type());
+        else lines(std::integral_constant<int, 16>(), std::false_type());
     }
-    cl.sync();
+}
+template <class T> __device__ __forceinline__ void pl_sweeps(const MgEq &E, int l)
+{
+    if constexpr (sizeof(T) == 4) {
+        pl_sweeps32(E, l);
+    } else {
+        for (int irel = 0; irel < E.nrelax; ++irel)
+            for (int c = 1; c <= 2; ++c) pl_colour64(E, l, c);
+    }
 }
 
 // The residual of level l into rc (own lines; not followed by a barrier): its
@@ -258,12 +285,6 @@ template <class T> __device__ __noinline__ void pl_finer(const MgEq &E, int l)
         *v = p + *v;
     }
     cl.sync();
-}
-
-template <class T> __device__ __forceinline__ void pl_sweeps(const MgEq &E, int l)
-{
-    for (int irel = 0; irel < E.nrelax; ++irel)
-        for (int c = 1; c <= 2; ++c) pl_colour<T>(E, l, c);
 }
 
 // mg_legs of prb_mg.cu
