@@ -15,7 +15,7 @@
 // lanes (warpline.cuh); the FP64 iterate stays in global memory.
 //
 // Measured on the 129 x 65 layer (GB300, a step of about 26 sweeps): FP64
-// 20.7 ms on one CTA and global memory, 10.7 on a cluster of 16, 9.5 resident
+// 20.7 ms on one CTA and global memory, 10.7 on a cluster of 16, 9.1 resident
 // (6.6 of them eliminations); mixed 6.9, 4.7, 3.2.
 #include <string.h>
 
