@@ -28,6 +28,7 @@
 #include "cluster.cuh"
 #include "convert.cuh"
 #include "gridsync.cuh"
+#include "r3d_stage.cuh"
 #include "warpline.cuh"
 
 #include <math.h>
@@ -39,7 +40,6 @@
 #include <vector>
 
 #define R3_MAXLEV 8
-#define R3_THREADS 256
 #define R3_SYNC_STRIDE 32           // unsigneds between the components' barriers
 
 // Work arrays of one level of one component's solve (the w and v solves
@@ -1192,8 +1192,6 @@ struct R3Shared {
     float4 weights[R3_WEIGHTS];   // the FP32 operator's, where they fit
 };
 #define R3_SMEM_BYTES (110 * 1024)
-#define R3_CHUNK_BYTES (44 * 1024)
-#define R3_FAC_BYTES (52 * 1024)
 static_assert(sizeof(R3Shared) + R3_CHUNK_BYTES + R3_FAC_BYTES <= R3_SMEM_BYTES, "shared memory of a solve block");
 __device__ __forceinline__ R3Shared &r3_shared()
 {
@@ -1255,15 +1253,6 @@ template <int COMP>
 __device__ __forceinline__ void r3_rhs32_batch(const R3Lev &L, const R3Work &W, int dir, const int *s_line, int nl, int n, const RowSplit &split,
                                float *x, int lpitch, int lg);
 
-// Lines a chunk holds, and floats or doubles of factors beside them.
-template <int COMP, class T> __device__ __forceinline__ int r3_chunk(int dir, int n, int len)
-{
-    constexpr bool F64 = sizeof(T) == 8;
-    int chunk = min(R3_THREADS, (int)(R3_CHUNK_BYTES / sizeof(T)) / (F64 ? n | 1 : wl_pitch(n)));
-    if (!F64 && dir == 1) chunk = min(chunk, (int)(R3_FAC_BYTES / sizeof(T)) / len);   // a table per line
-    return max(1, chunk);
-}
-
 // Starts the copy of the factors of nl lines: one table in direction 0, else
 // one per radius p.  FP64 lists keep a radius's lines together, so the tables
 // of a chunk's radii are few and lie in a row (p0 gets the first); FP32 ones
@@ -1320,7 +1309,7 @@ template <int COMP, class T> __device__ __noinline__ void r3_prepare(int lev, in
     bool staged = false;
     int nl = 0, chunk = 1;
     if (my0 < my1) {
-        chunk = r3_chunk<COMP, T>(dir, n, len);
+        chunk = r3_chunk(F64, dir, n, len);
         const int c1 = r3_chunk_end(lines, my0, min(my1, my0 + chunk));
         nl = c1 - my0;
         for (int t = tid; t < nl; t += nthr) S.line[t] = lines[my0 + t] & 0x7fffffff;
@@ -2297,13 +2286,11 @@ extern "C" int gb_r3d_destroy(gb_r3d *h)
 // the same order.
 #define R3_CONT 0x80000000u
 
-// Lines that any chunk of n-row lines holds (r3_phase's rule, the least of both
-// types).
+// Lines that any chunk of n-row lines holds: the least of both types.
 static int r3_chunk_lines(int comp, int dir, int n)
 {
-    int c = std::min(R3_THREADS, std::min(R3_CHUNK_BYTES / 8 / (n | 1), R3_CHUNK_BYTES / 4 / wl_pitch(n)));
-    if (dir == 1) c = std::min(c, R3_FAC_BYTES / 4 / r3_tabsize32(r3_kind(comp, dir), n));
-    return std::max(1, c);
+    const int kind = r3_kind(comp, dir);
+    return std::min(r3_chunk(true, dir, n, r3_tabsize(kind, n)), r3_chunk(false, dir, n, r3_tabsize32(kind, n)));
 }
 
 static void r3_phases(int mode, int pslow, int comp, int dir, int n1, int n2, int n3, std::vector<int> &lines,
