@@ -113,9 +113,8 @@ __device__ __noinline__ void pl_colour64(const MgEq &E, int l, int first)
         L.own(L.v, k)[i] = r + L.own(L.f, k)[i];
     }
     __syncthreads();
-    if ((int)threadIdx.x < nl) {
-        const int k = kb + 2 * threadIdx.x;
-        double *x = L.own(L.v, k) + 1;
+    for (int t = threadIdx.x; t < nl; t += PL_THREADS) {
+        double *x = L.own(L.v, kb + 2 * t) + 1;
         if (L.which == 2) pdma_staged<2>(L.fac, n, x, 1);
         else tdma_staged<2>(L.fac, n, x, 1);
     }
