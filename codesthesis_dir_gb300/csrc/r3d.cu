@@ -2429,6 +2429,10 @@ static int r3_create(const gb_r3d_params *p, const double *spacing, gb_r3d **out
         gb_set_error("gb_r3d_create: unknown variant %d", p->variant);
         return GB_ERR_INVALID;
     }
+    if (p->precision == GB_PRB_FP64 && np > R3_MAX_ROWS) {
+        gb_set_error("gb_r3d_create: np=%d: an FP64 phi-line of more than %d rows does not fit a block's shared memory", np, R3_MAX_ROWS);
+        return GB_ERR_INVALID;
+    }
     if (p->variant == GB_R3D_HORIZONTAL && nz < 6) {
         gb_set_error("gb_r3d_create: the horizontal annulus's heat band j = nz/2-3..nz/2+3 needs nz >= 6 (nz=%d)", nz);
         return GB_ERR_INVALID;

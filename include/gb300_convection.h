@@ -443,7 +443,7 @@ enum gb_r3d_field {
 };
 
 typedef struct gb_r3d_params {
-    int nr, nz, np;           /* intervals in r, z and phi */
+    int nr, nz, np;           /* intervals in r, z and phi (np at most 16384, in FP64 12288) */
     double dt, r0, rmax, zmax;
     double Ra, Re, Gr, Pr;    /* COMMON /val/ Ra, Re, Ptl, Gr (rot3dmg.f:38) */
     double tolcon;            /* max-norm residual tolerance (1e-5, rot3dmg.f:1562) */

@@ -47,3 +47,25 @@ def test_chunks_fit_their_area(tmp_path):
     subprocess.run([_build.nvcc(), *_build.ARCH, "-std=c++17", "--expt-relaxed-constexpr", "-I", CSRC, "-o", str(exe), str(src)], check=True)
     r = subprocess.run([str(exe)], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout
+
+
+def test_lines_longer_than_the_buffer_are_refused(gblib):
+    """An FP64 ring one step too long is refused before anything is allocated;
+    mixed ones (FP32 lines) of the same length fit, as does the longest FP64 one."""
+    import ctypes as C
+
+    from codesthesis_dir_gb300 import lib
+    def create(np_, precision):
+        p, h = lib.R3dParams(), C.c_void_p()
+        gblib.gb_r3d_default_params(C.byref(p), 4, 4, np_)
+        p.precision = precision
+        st = gblib.gb_r3d_create(C.byref(p), C.byref(h), None)
+        if st == 0:
+            gblib.gb_r3d_destroy(h)
+        return st
+
+    longest = 96 * 1024 // 8
+    assert create(longest + 8, lib.PRB_FP64) == lib.GB_ERR_INVALID
+    assert create(16384, lib.PRB_FP64) == lib.GB_ERR_INVALID
+    assert create(longest, lib.PRB_FP64) != lib.GB_ERR_INVALID
+    assert create(16384, lib.PRB_MIXED) != lib.GB_ERR_INVALID
