@@ -1540,7 +1540,7 @@ struct gb_batch {
     size_t nops_max = 0;
     int plan_inner = -1;
     // persistent launch
-    unsigned *d_sync = nullptr;         // count, gen, err
+    unsigned *d_sync = nullptr;         // count (two words), err
     long long wait_limit = GB_GRID_WAIT_LIMIT_DEFAULT;   // polls a barrier wait may take
     int pgrid = 0;
     size_t psmem = 0;
@@ -2439,7 +2439,7 @@ static int solve_persistent(gb_batch *b, cudaStream_t s)
     GB_CUDA_TRY(cudaMemcpyAsync(b->d_ops + n0, b->ops.data(), sizeof(Op) * n1, cudaMemcpyHostToDevice, s));
     GB_CUDA_TRY(cudaMemsetAsync(b->d_sync, 0, sizeof(unsigned) * 4, s));
     GridSync gs;
-    gs.count = b->d_sync;
+    gs.count = (unsigned long long *)b->d_sync;
     gs.err = (int *)(b->d_sync + 2);
     gs.limit = b->wait_limit;
     gs.tally = nullptr;

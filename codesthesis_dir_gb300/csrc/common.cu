@@ -119,7 +119,7 @@ extern "C" int gb_measure_grid_barrier(int blocks, int threads, int nbarriers, d
     for (int rep = 0; rep < 2 && e == cudaSuccess && hs[2] == 0; ++rep) {   // the first launch warms up
         e = cudaMemset(sync, 0, 4 * sizeof(unsigned));
         GridSync gs;
-        gs.count = sync;
+        gs.count = (unsigned long long *)sync;
         gs.err = (int *)(sync + 2);
         gs.limit = GB_GRID_WAIT_LIMIT_DEFAULT;
         gs.tally = nullptr;

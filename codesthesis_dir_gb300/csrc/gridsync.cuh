@@ -10,7 +10,7 @@
 // and handed to the whole block through shared memory, so all threads of a
 // block leave together even when another block raises the flag meanwhile.
 struct GridSync {
-    unsigned *count;   // zero when the kernel starts
+    unsigned long long *count;   // zero when the kernel starts
     int *err;
     long long limit;
     unsigned long long *tally;   // optional (may be null): barriers passed, counted once per barrier by block 0
@@ -19,6 +19,18 @@ struct GridSync {
 // Default wait limit: some seconds of polling at an L2 round trip per poll.
 #define GB_GRID_WAIT_LIMIT_DEFAULT (1LL << 24)
 
+// The count at which the barrier of an arrival that found it at `arrived` is
+// complete; `last`: at which the block's barrier before was (the first finds
+// less than the blocks).  64 bits: a 32-bit count wraps after 2^32 / blocks
+// barriers (14 million with 304, some 20 seconds of a solve that does not
+// converge), and beyond the wrap blocks would leave early.  From the barrier
+// before, because the remainder by the blocks is a 64-bit division on the last
+// arrival's way (1.29 -> 1.33 us with 152 blocks).
+__host__ __device__ __forceinline__ unsigned long long grid_barrier_end(unsigned long long arrived, unsigned blocks, unsigned long long last)
+{
+    return arrived < blocks ? blocks : last + blocks;
+}
+
 // Arrival and wait of one thread per block.  The count grows from one barrier
 // to the next (it is zero at the launch), so that nothing is reset and nobody
 // has to announce the last arrival: the blocks poll the count itself, a release
@@ -26,14 +38,16 @@ struct GridSync {
 // publishes.
 __device__ __forceinline__ void grid_barrier(const GridSync &gs)
 {
-    unsigned arrived;
-    asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(arrived) : "l"(gs.count) : "memory");
-    const unsigned all = arrived - arrived % gridDim.x + gridDim.x;
-    if (arrived + 1u == all) return;
+    __shared__ unsigned long long s_grid_end;   // of the arriving thread alone
+    unsigned long long arrived;
+    asm volatile("atom.add.acq_rel.gpu.global.u64 %0, [%1], 1;" : "=l"(arrived) : "l"(gs.count) : "memory");
+    const unsigned long long all = grid_barrier_end(arrived, gridDim.x, s_grid_end);
+    s_grid_end = all;
+    if (arrived + 1 == all) return;
     for (long long it = 0;;) {
-        unsigned now;
-        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(now) : "l"(gs.count) : "memory");
-        if ((int)(now - all) >= 0) break;
+        unsigned long long now;
+        asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(now) : "l"(gs.count) : "memory");
+        if (now >= all) break;
         if (++it > gs.limit || ((it & 15) == 0 && *(volatile int *)gs.err)) {
             atomicExch(gs.err, 1);
             break;

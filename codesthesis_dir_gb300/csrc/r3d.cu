@@ -2642,7 +2642,7 @@ static int r3_create(const gb_r3d_params *p, const double *spacing, gb_r3d **out
     d.trans = (double *)(sm + 4096);
     d.trans2 = d.trans + (np + 2);
     for (int c = 0; c < 4; ++c) {
-        d.gs[c].count = h->sync + R3_SYNC_STRIDE * c;
+        d.gs[c].count = (unsigned long long *)(h->sync + R3_SYNC_STRIDE * c);
         d.gs[c].err = (int *)(h->sync + R3_SYNC_STRIDE * c + 2);
         d.gs[c].limit = GB_GRID_WAIT_LIMIT_DEFAULT;
         d.gs[c].tally = (unsigned long long *)(sm + 448) + c;   // 4 counters, one per component
