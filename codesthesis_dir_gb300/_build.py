@@ -33,7 +33,7 @@ DROPINS = [(DROPIN_SRC, R3D_LIB), (AXI_DROPIN_SRC, AXI_LIB)]
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-COMMON = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-ffp-contract=off",
+COMMON = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-ffp-contract=off", "-Xcompiler", "-Werror=unused-result",
           "--expt-relaxed-constexpr", "-fmad=false", "-I", INCLUDE, "-I", CSRC]
 
 

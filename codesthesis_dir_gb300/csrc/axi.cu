@@ -1327,23 +1327,17 @@ static MerDev axi_mer(const gb_axi *h)
     return m;
 }
 
-static void axi_launch_mg(gb_axi *h, cudaStream_t s)
+[[nodiscard]] static cudaError_t axi_launch_mg(gb_axi *h, cudaStream_t s)
 {
     const AxiDev &d = h->dev;
-    if (d.stretched) {
-        gb_str_launch_device(h->str, d.f[GB_A_phi], d.f[GB_A_omegn], d.status, d.abort,
-                             h->p.precision == GB_PRB_MIXED, d.tolcon, d.maxsweeps, d.nrel, d.mode, s);
-        return;
-    }
+    if (d.stretched)
+        return gb_str_launch_device(h->str, d.f[GB_A_phi], d.f[GB_A_omegn], d.status, d.abort,
+                                    h->p.precision == GB_PRB_MIXED, d.tolcon, d.maxsweeps, d.nrel, d.mode, s);
     // the reference's line order is one chain of lines: one CTA
     const int ctas = d.mode == GB_SMOOTHER_LEX ? 1 : h->ctas;
-    if (h->p.precision != GB_PRB_MIXED) {
-        cl_launch(k_axi_mg_solve, 1, ctas, AXI_THREADS, AXI_SMEM_BYTES, s, d);
-    } else if (d.mode == GB_SMOOTHER_ZEBRA && h->mer_ctas) {
-        mer_launch(axi_mer(h), h->mer_ctas, s);
-    } else {
-        cl_launch(k_axi_mg_solve_mixed, 1, ctas, AXI_THREADS, AXI_SMEM_BYTES, s, d);
-    }
+    if (h->p.precision != GB_PRB_MIXED) return cl_launch(k_axi_mg_solve, 1, ctas, AXI_THREADS, AXI_SMEM_BYTES, s, d);
+    if (d.mode == GB_SMOOTHER_ZEBRA && h->mer_ctas) return mer_launch(axi_mer(h), h->mer_ctas, s);
+    return cl_launch(k_axi_mg_solve_mixed, 1, ctas, AXI_THREADS, AXI_SMEM_BYTES, s, d);
 }
 
 static int axi_sync(gb_axi *h, const char *what)
@@ -1388,7 +1382,7 @@ extern "C" int gb_axi_poisson(gb_axi *h, int *sweeps)
 {
     if (!h) return GB_ERR_INVALID;
     axi_begin(h);
-    axi_launch_mg(h, h->stream);
+    GB_CUDA_TRY(axi_launch_mg(h, h->stream));
     int st[2] = {0, 0};
     GB_CUDA_TRY(cudaMemcpyAsync(st, h->dev.status, sizeof(st), cudaMemcpyDeviceToHost, h->stream));
     int r = axi_sync(h, "gb_axi_poisson");
@@ -1424,11 +1418,14 @@ static int axi_build_graph(gb_axi *h)
     GB_CUDA_TRY(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
     axi_launch_vort_vel(h, 3, h->stream);
     axi_launch_temperature(h, h->stream);
-    axi_launch_mg(h, h->stream);
+    const cudaError_t e = axi_launch_mg(h, h->stream);
     axi_launch_update(h, h->stream);
     axi_launch_heat(h, h->stream);
     k_axi_record<<<1, 32, 0, h->stream>>>(h->dev);
-    GB_CUDA_TRY(cudaStreamEndCapture(h->stream, &g));
+    const cudaError_t ended = cudaStreamEndCapture(h->stream, &g);   // also ends one that failed
+    if (e != cudaSuccess && ended == cudaSuccess) cudaGraphDestroy(g);
+    GB_CUDA_TRY(e);
+    GB_CUDA_TRY(ended);
     GB_CUDA_TRY(cudaGraphInstantiate(&h->graph, g, 0));
     cudaGraphDestroy(g);
     return GB_OK;
@@ -1729,18 +1726,22 @@ extern "C" int gb_axi_gang_enqueue(gb_axi_gang *g, int nsteps, void *stream)
         GB_CUDA_TRY(cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal));
         k_axi_gang<AG_VV><<<g->blocks[AG_VV], g->threads[AG_VV], 0, cs>>>(t);
         k_axi_gang<AG_T><<<g->blocks[AG_T], g->threads[AG_T], 0, cs>>>(t);
-        if (g->nmer) mer_launch_many(g->d_mer, g->nmer, 0, g->mer_ctas, g->mer_smem, cs);
+        cudaError_t e = cudaSuccess;
+        if (g->nmer) e = mer_launch_many(g->d_mer, g->nmer, 0, g->mer_ctas, g->mer_smem, cs);
         auto solves = [&](int count, int ctas, const int *who) {
-            if (!count) return;
-            if (g->mixed) cl_launch(k_axi_gang_mg<true>, count, ctas, AXI_THREADS, AXI_SMEM_BYTES, cs, t, who);
-            else cl_launch(k_axi_gang_mg<false>, count, ctas, AXI_THREADS, AXI_SMEM_BYTES, cs, t, who);
+            if (!count || e != cudaSuccess) return;
+            e = g->mixed ? cl_launch(k_axi_gang_mg<true>, count, ctas, AXI_THREADS, AXI_SMEM_BYTES, cs, t, who)
+                         : cl_launch(k_axi_gang_mg<false>, count, ctas, AXI_THREADS, AXI_SMEM_BYTES, cs, t, who);
         };
         solves(g->nz, g->z_ctas, g->d_who);
         solves(g->nlex, 1, g->d_who + g->nz);
         k_axi_gang<AG_UPD><<<g->blocks[AG_UPD], g->threads[AG_UPD], 0, cs>>>(t);
         k_axi_gang<AG_HEAT><<<g->blocks[AG_HEAT], g->threads[AG_HEAT], g->heat_smem, cs>>>(t);
         k_axi_gang<AG_REC><<<g->blocks[AG_REC], g->threads[AG_REC], 0, cs>>>(t);
-        GB_CUDA_TRY(cudaStreamEndCapture(cs, &gr));
+        const cudaError_t ended = cudaStreamEndCapture(cs, &gr);
+        if (e != cudaSuccess && ended == cudaSuccess) cudaGraphDestroy(gr);
+        GB_CUDA_TRY(e);
+        GB_CUDA_TRY(ended);
         GB_CUDA_TRY(cudaGraphInstantiate(&g->graph, gr, 0));
         cudaGraphDestroy(gr);
     }

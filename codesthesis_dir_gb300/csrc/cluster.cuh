@@ -130,9 +130,12 @@ __device__ __forceinline__ double cl_max(const Cluster &cl, ClMaxState &s, int &
 
 // Launches kernel on clusters of `ctas` CTAs, nclusters of them (ctas = 1: an
 // ordinary launch).  Sizes above 8 need the kernel's
-// cudaFuncAttributeNonPortableClusterSizeAllowed (cl_prepare).
+// cudaFuncAttributeNonPortableClusterSizeAllowed (cl_prepare).  A cluster can be
+// refused where an ordinary launch is not, and while a stream is captured the
+// step would just lack its solve, so no caller may drop the result (the build
+// treats that as an error).
 template <class... P, class... A>
-static inline cudaError_t cl_launch(void (*kernel)(P...), int nclusters, int ctas, int threads, size_t smem, cudaStream_t s,
+[[nodiscard]] static inline cudaError_t cl_launch(void (*kernel)(P...), int nclusters, int ctas, int threads, size_t smem, cudaStream_t s,
                                     A... args)
 {
     cudaLaunchConfig_t cfg = {};
@@ -147,7 +150,9 @@ static inline cudaError_t cl_launch(void (*kernel)(P...), int nclusters, int cta
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+    if (e != cudaSuccess) cudaGetLastError();   // it is the caller's now, not a later call's
+    return e;
 }
 
 // Allows clusters of up to CL_MAX_CTAS and smem bytes of dynamic shared

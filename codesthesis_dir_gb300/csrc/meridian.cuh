@@ -66,6 +66,6 @@ size_t mer_weight_bytes(const MerDev &d);
 void mer_weight_layout(MerDev &d, void *mem);
 // Clusters of this size that fit the device for d's plan (halved from want).
 int mer_fit(MerDev &d, int want);
-cudaError_t mer_launch(const MerDev &d, int ctas, cudaStream_t s);
+[[nodiscard]] cudaError_t mer_launch(const MerDev &d, int ctas, cudaStream_t s);
 // n solves in one launch: d_devs on the device, all planned for `ctas`.
-cudaError_t mer_launch_many(const MerDev *d_devs, int n, int penta, int ctas, size_t smem, cudaStream_t s);
+[[nodiscard]] cudaError_t mer_launch_many(const MerDev *d_devs, int n, int penta, int ctas, size_t smem, cudaStream_t s);

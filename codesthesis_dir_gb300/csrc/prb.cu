@@ -960,10 +960,11 @@ extern "C" int gb_prb_poisson(gb_prb *h, int which, int *sweeps)
 {
     if (!h || (which != 2 && which != 3)) { gb_set_error("gb_prb_poisson: which must be 2 or 3"); return GB_ERR_INVALID; }
     prb_begin(h);
-    prb_launch_mg(h, which == 2 ? 1 : 0, which == 3 ? 1 : 0, h->stream);
+    int st = prb_launch_mg(h, which == 2 ? 1 : 0, which == 3 ? 1 : 0, h->stream);
+    if (st != GB_OK) return st;
     int stat[4];
     GB_CUDA_TRY(cudaMemcpyAsync(stat, h->dev.mg_status, sizeof(stat), cudaMemcpyDeviceToHost, h->stream));
-    int st = prb_sync(h, "gb_prb_poisson");
+    st = prb_sync(h, "gb_prb_poisson");
     if (st != GB_OK) return st;
     const int o = (which == 2) ? 0 : 2;
     if (sweeps) *sweeps = stat[o + 1];
@@ -971,15 +972,16 @@ extern "C" int gb_prb_poisson(gb_prb *h, int which, int *sweeps)
 }
 
 // One step's launches on stream s (v and u solves in one multigrid launch).
-static void prb_enqueue_step(gb_prb *h, int first, cudaStream_t s)
+static int prb_enqueue_step(gb_prb *h, int first, cudaStream_t s)
 {
     prb_launch_cvorticity(h, first, s);
     prb_launch_temperature(h, first, s);
     prb_launch_heat(h, s);
     prb_launch_rhs(h, 1, 1, s);
-    prb_launch_mg(h, 1, 1, s);
+    const int st = prb_launch_mg(h, 1, 1, s);
     prb_launch_update(h, s, true);
     prb_launch_record(h, s, first);
+    return st;
 }
 
 static int prb_build_graph(gb_prb *h, int first, cudaGraphExec_t *exec)
@@ -987,10 +989,15 @@ static int prb_build_graph(gb_prb *h, int first, cudaGraphExec_t *exec)
     cudaGraph_t g;
     GB_CUDA_TRY(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
     const long long l0 = h->launches;
-    prb_enqueue_step(h, first, h->stream);
+    const int st = prb_enqueue_step(h, first, h->stream);
     h->launches_per_step = h->launches - l0;
     h->launches = l0;
-    GB_CUDA_TRY(cudaStreamEndCapture(h->stream, &g));
+    const cudaError_t e = cudaStreamEndCapture(h->stream, &g);   // also ends one that failed
+    if (st != GB_OK) {
+        if (e == cudaSuccess) cudaGraphDestroy(g);
+        return st;
+    }
+    GB_CUDA_TRY(e);
     GB_CUDA_TRY(cudaGraphInstantiate(exec, g, 0));
     cudaGraphDestroy(g);
     return GB_OK;
@@ -1400,7 +1407,7 @@ extern "C" int gb_prb_gang_create(gb_prb *const *members, const int *nsteps_tota
     return GB_OK;
 }
 
-static void prb_gang_enqueue_step(gb_prb_gang *g, cudaStream_t s)
+static cudaError_t prb_gang_enqueue_step(gb_prb_gang *g, cudaStream_t s)
 {
     GangTab t{g->d_dev, g->d_off, g->d_rec, g->d_limit, g->n};
 #define GL(PH) k_prb_gang<PH><<<g->blocks[PH], g->threads[PH], PH == GP_HEAT ? g->heat_smem : 0, s>>>(t)
@@ -1414,13 +1421,14 @@ static void prb_gang_enqueue_step(gb_prb_gang *g, cudaStream_t s)
     GL(GP_TROB);
     GL(GP_HEAT);
     GL(GP_RHS);
-    prb_mg_launch_eqs(g->d_eqs, 0, g->nres, g->mixed, g->ctas, g->smem, s);
-    prb_mg_launch_eqs(g->d_eqs, g->nres, g->nzebra - g->nres, g->mixed, g->ctas, 0, s);
-    prb_mg_launch_eqs(g->d_eqs, g->nzebra, 2 * g->n - g->nzebra, g->mixed, 1, 0, s);
+    cudaError_t e = prb_mg_launch_eqs(g->d_eqs, 0, g->nres, g->mixed, g->ctas, g->smem, s);
+    if (e == cudaSuccess) e = prb_mg_launch_eqs(g->d_eqs, g->nres, g->nzebra - g->nres, g->mixed, g->ctas, 0, s);
+    if (e == cudaSuccess) e = prb_mg_launch_eqs(g->d_eqs, g->nzebra, 2 * g->n - g->nzebra, g->mixed, 1, 0, s);
     GL(GP_UPD);
     GL(GP_REC);
 #undef GL
     g->launches_per_step = GP_COUNT + (g->nres > 0) + (g->nzebra > g->nres) + (2 * g->n > g->nzebra);
+    return e;
 }
 
 // Plans the gang's solves.  A cluster takes as many CTAs as leave every
@@ -1461,8 +1469,10 @@ extern "C" int gb_prb_gang_enqueue(gb_prb_gang *g, int nsteps, void *stream)
     if (!g->graph) {
         cudaGraph_t gr;
         GB_CUDA_TRY(cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeThreadLocal));
-        prb_gang_enqueue_step(g, g->stream);
-        GB_CUDA_TRY(cudaStreamEndCapture(g->stream, &gr));
+        const cudaError_t e = prb_gang_enqueue_step(g, g->stream), ended = cudaStreamEndCapture(g->stream, &gr);
+        if (e != cudaSuccess && ended == cudaSuccess) cudaGraphDestroy(gr);
+        GB_CUDA_TRY(e);
+        GB_CUDA_TRY(ended);
         GB_CUDA_TRY(cudaGraphInstantiate(&g->graph, gr, 0));
         cudaGraphDestroy(gr);
     }

@@ -114,9 +114,9 @@ struct gb_prb {
 int prb_mg_levels(int nr, int variant);
 int prb_mg_create(gb_prb *h);
 void prb_mg_destroy(gb_prb *h);
-int prb_launch_mg(gb_prb *h, int do_v, int do_u, cudaStream_t s);
+[[nodiscard]] int prb_launch_mg(gb_prb *h, int do_v, int do_u, cudaStream_t s);
 bool prb_mg_plan(MgEq *eqs, int n, int mixed, int ctas);
-void prb_mg_launch_eqs(const MgEq *d_eqs, int first, int neq, int mixed, int ctas, int smem, cudaStream_t s);
+[[nodiscard]] cudaError_t prb_mg_launch_eqs(const MgEq *d_eqs, int first, int neq, int mixed, int ctas, int smem, cudaStream_t s);
 int prb_mg_cluster_ctas();
 // The solve in a cluster's shared memory (prb_resident.cu): plans E for
 // clusters of ctas CTAs (E.smem = 0 when it does not fit), prepares the
@@ -124,7 +124,7 @@ int prb_mg_cluster_ctas();
 void prb_resident_plan(MgEq &E, int mixed, int ctas);
 cudaError_t prb_resident_prepare();
 int prb_resident_fit(int mixed, int ctas, int smem);
-void prb_resident_launch(const MgEq *d_eqs, int first, int neq, int mixed, int ctas, int smem, cudaStream_t s);
+[[nodiscard]] cudaError_t prb_resident_launch(const MgEq *d_eqs, int first, int neq, int mixed, int ctas, int smem, cudaStream_t s);
 int prb_refresh_scalars(gb_prb *h);
 // the tank's transport (tank.cu)
 int tank_launch_cvorticity(gb_prb *h, int first, cudaStream_t s);

@@ -679,15 +679,12 @@ bool prb_mg_plan(MgEq *eqs, int n, int mixed, int ctas)
 // The solves of neq equation descriptors (any instances') in one launch, one
 // cluster of ctas CTAs each; smem: the most any of them takes in shared
 // memory, 0: on global memory.
-void prb_mg_launch_eqs(const MgEq *d_eqs, int first, int neq, int mixed, int ctas, int smem, cudaStream_t s)
+cudaError_t prb_mg_launch_eqs(const MgEq *d_eqs, int first, int neq, int mixed, int ctas, int smem, cudaStream_t s)
 {
-    if (neq <= 0) return;
-    if (smem) {
-        prb_resident_launch(d_eqs, first, neq, mixed, ctas, smem, s);
-        return;
-    }
-    if (mixed) cl_launch(k_mg_solve_mixed, neq, ctas, MG_THREADS_MIXED, MG_SMEM_BYTES, s, d_eqs, first);
-    else cl_launch(k_mg_solve, neq, ctas, MG_THREADS, MG_SMEM_BYTES, s, d_eqs, first);
+    if (neq <= 0) return cudaSuccess;
+    if (smem) return prb_resident_launch(d_eqs, first, neq, mixed, ctas, smem, s);
+    if (mixed) return cl_launch(k_mg_solve_mixed, neq, ctas, MG_THREADS_MIXED, MG_SMEM_BYTES, s, d_eqs, first);
+    return cl_launch(k_mg_solve, neq, ctas, MG_THREADS, MG_SMEM_BYTES, s, d_eqs, first);
 }
 
 int prb_mg_cluster_ctas() { return MG_SPREAD; }
@@ -710,11 +707,12 @@ int prb_launch_mg(gb_prb *h, int do_v, int do_u, cudaStream_t s)
     if (n == 0) return GB_OK;
     const int mixed = h->p.precision == GB_PRB_MIXED;
     if (h->p.smoother == GB_SMOOTHER_LEX) {
-        prb_mg_launch_eqs(h->eq_dev, first, n, mixed, 1, 0, s);
+        GB_CUDA_TRY(prb_mg_launch_eqs(h->eq_dev, first, n, mixed, 1, 0, s));
     } else {
         // v and u in one launch: in shared memory when both fit
         const int smem = h->eq_host[0].smem && h->eq_host[1].smem ? std::max(h->eq_host[0].smem, h->eq_host[1].smem) : 0;
-        prb_mg_launch_eqs(h->eq_dev, first, n, mixed, h->mg_spread ? std::min(h->mg_spread, h->mg_ctas) : h->mg_ctas, smem, s);
+        const int ctas = h->mg_spread ? std::min(h->mg_spread, h->mg_ctas) : h->mg_ctas;
+        GB_CUDA_TRY(prb_mg_launch_eqs(h->eq_dev, first, n, mixed, ctas, smem, s));
     }
     h->launches += 1;
     return GB_OK;

@@ -583,7 +583,7 @@ int prb_resident_fit(int mixed, int ctas, int smem)
     return cl_fit(mixed ? k_pl_solve_mixed : k_pl_solve, ctas, PL_THREADS, smem);
 }
 
-void prb_resident_launch(const MgEq *d_eqs, int first, int neq, int mixed, int ctas, int smem, cudaStream_t s)
+cudaError_t prb_resident_launch(const MgEq *d_eqs, int first, int neq, int mixed, int ctas, int smem, cudaStream_t s)
 {
-    cl_launch(mixed ? k_pl_solve_mixed : k_pl_solve, neq, ctas, PL_THREADS, (size_t)smem, s, d_eqs, first);
+    return cl_launch(mixed ? k_pl_solve_mixed : k_pl_solve, neq, ctas, PL_THREADS, (size_t)smem, s, d_eqs, first);
 }
