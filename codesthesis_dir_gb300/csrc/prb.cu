@@ -1283,31 +1283,37 @@ struct gb_prb_gang {
     int spread = 1;                // the batched multigrid's equations on one CTA (1) or a cluster each
     std::vector<MgEq> eqs;         // the members' equations, those in the reference's line order last
     int nzebra = 0;                // the others
-    int nres = 0, ctas = 1, smem = 0;   // resident ones (first), CTAs per cluster, shared memory
     int most = 1;                  // the largest cluster the device holds
+    // the plans of both spreads, each made when steps are first queued with it and
+    // kept: steps queued on any stream go on with the one they were captured with
+    struct Plan {
+        MgEq *d_eqs = nullptr;
+        int nres = 0, ctas = 1, smem = 0;   // resident equations (first), CTAs per cluster, shared memory
+        long long launches = 0;
+        cudaGraphExec_t graph = nullptr;
+    } plan[2];
+    Plan &now() { return plan[spread != 1]; }
     PrbDev *d_dev = nullptr;
     int *d_off = nullptr, *d_limit = nullptr;
     GangRec *d_rec = nullptr;
-    MgEq *d_eqs = nullptr;
     std::vector<int> blocks;       // [GP_COUNT] total blocks of each phase
     int threads[GP_COUNT];
     size_t heat_smem = 0;
     cudaStream_t stream = nullptr;
-    cudaGraphExec_t graph = nullptr;
     long long launches_per_step = 0;
 };
-
-static cudaError_t prb_gang_plan(gb_prb_gang *g, gb_prb *const *members);
 
 extern "C" int gb_prb_gang_destroy(gb_prb_gang *g)
 {
     if (!g) return GB_OK;
-    if (g->graph) cudaGraphExecDestroy(g->graph);
+    for (auto &p : g->plan) {
+        if (p.graph) cudaGraphExecDestroy(p.graph);
+        cudaFree(p.d_eqs);
+    }
     cudaFree(g->d_dev);
     cudaFree(g->d_off);
     cudaFree(g->d_limit);
     cudaFree(g->d_rec);
-    cudaFree(g->d_eqs);
     if (g->stream) cudaStreamDestroy(g->stream);
     delete g;
     return GB_OK;
@@ -1391,12 +1397,11 @@ extern "C" int gb_prb_gang_create(gb_prb *const *members, const int *nsteps_tota
     GTRY(cudaMalloc(&g->d_off, sizeof(int) * off.size()));
     GTRY(cudaMalloc(&g->d_limit, sizeof(int) * n));
     GTRY(cudaMalloc(&g->d_rec, sizeof(GangRec) * n));
-    GTRY(cudaMalloc(&g->d_eqs, sizeof(MgEq) * g->eqs.size()));
     GTRY(cudaMemcpy(g->d_dev, devs.data(), sizeof(PrbDev) * n, cudaMemcpyHostToDevice));
     GTRY(cudaMemcpy(g->d_off, off.data(), sizeof(int) * off.size(), cudaMemcpyHostToDevice));
     GTRY(cudaMemcpy(g->d_limit, nsteps_total, sizeof(int) * n, cudaMemcpyHostToDevice));
     GTRY(cudaMemcpy(g->d_rec, rec.data(), sizeof(GangRec) * n, cudaMemcpyHostToDevice));
-    GTRY(prb_gang_plan(g, members));
+    g->most = members[0]->mg_ctas;
     // the members' own queued work (their first steps) finishes before the gang's
     for (int q = 0; q < n; ++q) GTRY(cudaStreamSynchronize(members[q]->stream));
     GTRY(cudaStreamCreateWithFlags(&g->stream, cudaStreamNonBlocking));
@@ -1421,43 +1426,52 @@ static cudaError_t prb_gang_enqueue_step(gb_prb_gang *g, cudaStream_t s)
     GL(GP_TROB);
     GL(GP_HEAT);
     GL(GP_RHS);
-    cudaError_t e = prb_mg_launch_eqs(g->d_eqs, 0, g->nres, g->mixed, g->ctas, g->smem, s);
-    if (e == cudaSuccess) e = prb_mg_launch_eqs(g->d_eqs, g->nres, g->nzebra - g->nres, g->mixed, g->ctas, 0, s);
-    if (e == cudaSuccess) e = prb_mg_launch_eqs(g->d_eqs, g->nzebra, 2 * g->n - g->nzebra, g->mixed, 1, 0, s);
+    gb_prb_gang::Plan &p = g->now();
+    cudaError_t e = prb_mg_launch_eqs(p.d_eqs, 0, p.nres, g->mixed, p.ctas, p.smem, s);
+    if (e == cudaSuccess) e = prb_mg_launch_eqs(p.d_eqs, p.nres, g->nzebra - p.nres, g->mixed, p.ctas, 0, s);
+    if (e == cudaSuccess) e = prb_mg_launch_eqs(p.d_eqs, g->nzebra, 2 * g->n - g->nzebra, g->mixed, 1, 0, s);
     GL(GP_UPD);
     GL(GP_REC);
 #undef GL
-    g->launches_per_step = GP_COUNT + (g->nres > 0) + (g->nzebra > g->nres) + (2 * g->n > g->nzebra);
+    p.launches = GP_COUNT + (p.nres > 0) + (g->nzebra > p.nres) + (2 * g->n > g->nzebra);
     return e;
 }
 
-// Plans the gang's solves.  A cluster takes as many CTAs as leave every
+// Plans the gang's solves of its present spread.  A cluster takes as many CTAs as leave every
 // equation its own SMs (a CTA fills one), at least what keeps every member
 // that fits a cluster's shared memory there: a gang step waits for its
 // slowest solve.  The results do not depend on it.
-static cudaError_t prb_gang_plan(gb_prb_gang *g, gb_prb *const *members)
+static cudaError_t prb_gang_plan(gb_prb_gang *g)
 {
+    gb_prb_gang::Plan &p = g->now();
+    if (p.d_eqs) return cudaSuccess;
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
-    if (members) g->most = members[0]->mg_ctas;
-    MgEq *e = g->eqs.data();
+    std::vector<MgEq> eqs = g->eqs;
+    MgEq *e = eqs.data();
     auto resident = [](const MgEq &q) { return q.smem > 0; };
     if (g->spread == 1) {
-        g->ctas = 1;
+        p.ctas = 1;
         prb_mg_plan(e, g->nzebra, g->mixed, 1);
     } else {
         prb_mg_plan(e, g->nzebra, g->mixed, g->most);
         const long can = std::count_if(e, e + g->nzebra, resident);
-        for (g->ctas = 1; 2 * g->ctas <= g->most && 2 * g->ctas * g->nzebra <= sms;) g->ctas *= 2;
-        for (;; g->ctas *= 2) {
-            prb_mg_plan(e, g->nzebra, g->mixed, g->ctas);
-            if (std::count_if(e, e + g->nzebra, resident) == can || 2 * g->ctas > g->most) break;
+        for (p.ctas = 1; 2 * p.ctas <= g->most && 2 * p.ctas * g->nzebra <= sms;) p.ctas *= 2;
+        for (;; p.ctas *= 2) {
+            prb_mg_plan(e, g->nzebra, g->mixed, p.ctas);
+            if (std::count_if(e, e + g->nzebra, resident) == can || 2 * p.ctas > g->most) break;
         }
     }
-    g->nres = (int)(std::stable_partition(e, e + g->nzebra, resident) - e);
-    g->smem = 0;
-    for (int q = 0; q < g->nres; ++q) g->smem = std::max(g->smem, e[q].smem);
-    return cudaMemcpy(g->d_eqs, e, sizeof(MgEq) * g->eqs.size(), cudaMemcpyHostToDevice);
+    p.nres = (int)(std::stable_partition(e, e + g->nzebra, resident) - e);
+    p.smem = 0;
+    for (int q = 0; q < p.nres; ++q) p.smem = std::max(p.smem, e[q].smem);
+    cudaError_t err = cudaMalloc(&p.d_eqs, sizeof(MgEq) * eqs.size());
+    if (err == cudaSuccess) err = cudaMemcpy(p.d_eqs, e, sizeof(MgEq) * eqs.size(), cudaMemcpyHostToDevice);
+    if (err != cudaSuccess) {
+        cudaFree(p.d_eqs);
+        p.d_eqs = nullptr;
+    }
+    return err;
 }
 
 // Queues nsteps leapfrog steps (not the first step of a run) of every
@@ -1466,17 +1480,20 @@ extern "C" int gb_prb_gang_enqueue(gb_prb_gang *g, int nsteps, void *stream)
 {
     if (!g || nsteps < 0) { gb_set_error("gb_prb_gang_enqueue: invalid argument"); return GB_ERR_INVALID; }
     cudaStream_t s = stream ? (cudaStream_t)stream : g->stream;
-    if (!g->graph) {
+    gb_prb_gang::Plan &p = g->now();
+    if (!p.graph) {
+        GB_CUDA_TRY(prb_gang_plan(g));
         cudaGraph_t gr;
         GB_CUDA_TRY(cudaStreamBeginCapture(g->stream, cudaStreamCaptureModeThreadLocal));
         const cudaError_t e = prb_gang_enqueue_step(g, g->stream), ended = cudaStreamEndCapture(g->stream, &gr);
         if (e != cudaSuccess && ended == cudaSuccess) cudaGraphDestroy(gr);
         GB_CUDA_TRY(e);
         GB_CUDA_TRY(ended);
-        GB_CUDA_TRY(cudaGraphInstantiate(&g->graph, gr, 0));
+        GB_CUDA_TRY(cudaGraphInstantiate(&p.graph, gr, 0));
         cudaGraphDestroy(gr);
     }
-    for (int k = 0; k < nsteps; ++k) GB_CUDA_TRY(cudaGraphLaunch(g->graph, s));
+    g->launches_per_step = p.launches;
+    for (int k = 0; k < nsteps; ++k) GB_CUDA_TRY(cudaGraphLaunch(p.graph, s));
     return GB_OK;
 }
 
@@ -1486,12 +1503,7 @@ extern "C" int gb_prb_gang_set_solve_spread(gb_prb_gang *g, int ctas)
         gb_set_error("gb_prb_gang_set_solve_spread: ctas must be 1 or %d", prb_mg_cluster_ctas());
         return GB_ERR_INVALID;
     }
-    if (g->spread != ctas) {
-        GB_CUDA_TRY(cudaStreamSynchronize(g->stream));   // queued steps use the present plan
-        g->spread = ctas;
-        GB_CUDA_TRY(prb_gang_plan(g, nullptr));
-        if (g->graph) { cudaGraphExecDestroy(g->graph); g->graph = nullptr; }
-    }
+    g->spread = ctas;
     return GB_OK;
 }
 
