@@ -1649,7 +1649,7 @@ extern "C" int gb_axi_gang_create(gb_axi *const *members, const int *nsteps_tota
     for (int ph = 0; ph < AG_COUNT; ++ph) off[(size_t)ph * (n + 1) + n] = g->blocks[ph];
     std::vector<MerDev> mers;
     std::vector<int> who, lex;
-    int sms = 0;
+    const int sms = gb_sm_count();
     for (int q = 0; q < n; ++q) {
         if (mixed && members[q]->p.smoother == GB_SMOOTHER_ZEBRA && members[q]->mer_ctas) mers.push_back(axi_mer(members[q]));
         else if (members[q]->p.smoother == GB_SMOOTHER_LEX) lex.push_back(q);
@@ -1659,7 +1659,6 @@ extern "C" int gb_axi_gang_create(gb_axi *const *members, const int *nsteps_tota
     g->nlex = (int)lex.size();
     g->nmer = (int)mers.size();
     who.insert(who.end(), lex.begin(), lex.end());
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
     auto per_member = [&](int members_) {
         int c = CL_MAX_CTAS;
         while (c > 1 && c * members_ > sms) c >>= 1;

@@ -28,4 +28,12 @@ void gb_set_error(const char *fmt, ...);
 // Column-major (i fastest) addressing of a (0:ld-1, 0:np) field.
 #define GIX(i, k, ld) ((size_t)(i) + (size_t)(ld) * (size_t)(k))
 
+// SMs of the current device (0 if that cannot be told).
+static inline int gb_sm_count()
+{
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return 0;
+    return sms;
+}
+
 static inline unsigned gb_ceil_div(size_t a, size_t b) { return (unsigned)((a + b - 1) / b); }

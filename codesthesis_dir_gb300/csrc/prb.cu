@@ -1445,8 +1445,7 @@ static cudaError_t prb_gang_plan(gb_prb_gang *g)
 {
     gb_prb_gang::Plan &p = g->now();
     if (p.d_eqs) return cudaSuccess;
-    int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, 0);
+    const int sms = gb_sm_count();
     std::vector<MgEq> eqs = g->eqs;
     MgEq *e = eqs.data();
     auto resident = [](const MgEq &q) { return q.smem > 0; };
