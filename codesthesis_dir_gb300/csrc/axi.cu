@@ -1648,36 +1648,37 @@ extern "C" int gb_axi_gang_create(gb_axi *const *members, const int *nsteps_tota
     }
     for (int ph = 0; ph < AG_COUNT; ++ph) off[(size_t)ph * (n + 1) + n] = g->blocks[ph];
     std::vector<MerDev> mers;
-    std::vector<int> who, lex;
+    std::vector<int> who, lex, res;
+    int most = CL_MAX_CTAS;
     const int sms = gb_sm_count();
     for (int q = 0; q < n; ++q) {
-        if (mixed && members[q]->p.smoother == GB_SMOOTHER_ZEBRA && members[q]->mer_ctas) mers.push_back(axi_mer(members[q]));
-        else if (members[q]->p.smoother == GB_SMOOTHER_LEX) lex.push_back(q);
-        else who.push_back(q);
+        if (mixed && members[q]->p.smoother == GB_SMOOTHER_ZEBRA && members[q]->mer_ctas) {
+            res.push_back(q);
+            mers.push_back(axi_mer(members[q]));
+            most = std::min(most, members[q]->mer_ctas);
+        } else if (members[q]->p.smoother == GB_SMOOTHER_LEX) {
+            lex.push_back(q);
+        } else {
+            who.push_back(q);
+        }
     }
-    g->nz = (int)who.size();
-    g->nlex = (int)lex.size();
-    g->nmer = (int)mers.size();
-    who.insert(who.end(), lex.begin(), lex.end());
     auto per_member = [&](int members_) {
         int c = CL_MAX_CTAS;
         while (c > 1 && c * members_ > sms) c >>= 1;
         return c;
     };
-    if (g->nmer) {
-        int most = CL_MAX_CTAS;
-        for (int q = 0; q < n; ++q)
-            if (members[q]->mer_ctas) most = std::min(most, members[q]->mer_ctas);
-        for (g->mer_ctas = std::min(most, per_member(g->nmer));; g->mer_ctas <<= 1) {
-            bool fits = true;
-            g->mer_smem = 0;
-            for (MerDev &m : mers) {
-                fits = mer_plan(m, g->mer_ctas) && fits;
-                g->mer_smem = std::max(g->mer_smem, sizeof(float) * (size_t)m.smem_floats);
-            }
-            if (fits || g->mer_ctas >= most) break;
+    if (!mers.empty()) {
+        std::vector<char> fits(mers.size());
+        g->mer_ctas = mer_plan_many(mers.data(), (int)mers.size(), std::min(most, per_member((int)mers.size())), most, &g->mer_smem, fits.data());
+        for (size_t q = 0; q < mers.size(); ++q) {
+            if (fits[q]) mers[g->nmer++] = mers[q];
+            else who.push_back(res[q]);
         }
+        mers.resize(g->nmer);
     }
+    g->nz = (int)who.size();
+    g->nlex = (int)lex.size();
+    who.insert(who.end(), lex.begin(), lex.end());
     if (g->nz) g->z_ctas = std::min(members[who[0]]->ctas, per_member(g->nz));
 #define GTRY(x)                                                                   \
     do {                                                                          \

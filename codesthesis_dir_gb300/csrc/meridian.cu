@@ -675,6 +675,20 @@ int mer_fit(MerDev &d, int want)
     return 0;
 }
 
+int mer_plan_many(MerDev *d, int n, int want, int most, size_t *smem, char *fits)
+{
+    for (int c = want;; c <<= 1) {
+        bool all = true;
+        *smem = 0;
+        for (int q = 0; q < n; ++q) {
+            fits[q] = mer_plan(d[q], c);
+            all = all && fits[q];
+            if (fits[q]) *smem = std::max(*smem, sizeof(float) * (size_t)d[q].smem_floats);
+        }
+        if (all || 2 * c > most) return c;
+    }
+}
+
 cudaError_t mer_launch(const MerDev &d, int ctas, cudaStream_t s)
 {
     const size_t smem = sizeof(float) * (size_t)d.smem_floats;

@@ -66,6 +66,10 @@ size_t mer_weight_bytes(const MerDev &d);
 void mer_weight_layout(MerDev &d, void *mem);
 // Clusters of this size that fit the device for d's plan (halved from want).
 int mer_fit(MerDev &d, int want);
+// One cluster size for n solves of a launch: the power of two `want` or, up to
+// `most`, as many more CTAs as the largest needs.  Plans the solves for it;
+// fits[q]: solve q does fit.  *smem: the most any of those takes.
+int mer_plan_many(MerDev *d, int n, int want, int most, size_t *smem, char *fits);
 [[nodiscard]] cudaError_t mer_launch(const MerDev &d, int ctas, cudaStream_t s);
 // n solves in one launch: d_devs on the device, all planned for `ctas`.
 [[nodiscard]] cudaError_t mer_launch_many(const MerDev *d_devs, int n, int penta, int ctas, size_t smem, cudaStream_t s);
