@@ -689,6 +689,9 @@ cudaError_t prb_mg_launch_eqs(const MgEq *d_eqs, int first, int neq, int mixed, 
 
 int prb_mg_cluster_ctas() { return MG_SPREAD; }
 
+// CTAs of a zebra solve: those asked for, or the largest cluster.
+static int prb_mg_ctas(const gb_prb *h) { return h->mg_spread ? std::min(h->mg_spread, h->mg_ctas) : h->mg_ctas; }
+
 // Refreshes the solve parameters that a caller may change between calls
 // (tolerance, sweep limit, smoother, SOR factor) and launches the solves.
 int prb_launch_mg(gb_prb *h, int do_v, int do_u, cudaStream_t s)
@@ -711,8 +714,7 @@ int prb_launch_mg(gb_prb *h, int do_v, int do_u, cudaStream_t s)
     } else {
         // v and u in one launch: in shared memory when both fit
         const int smem = h->eq_host[0].smem && h->eq_host[1].smem ? std::max(h->eq_host[0].smem, h->eq_host[1].smem) : 0;
-        const int ctas = h->mg_spread ? std::min(h->mg_spread, h->mg_ctas) : h->mg_ctas;
-        GB_CUDA_TRY(prb_mg_launch_eqs(h->eq_dev, first, n, mixed, ctas, smem, s));
+        GB_CUDA_TRY(prb_mg_launch_eqs(h->eq_dev, first, n, mixed, prb_mg_ctas(h), smem, s));
     }
     h->launches += 1;
     return GB_OK;
@@ -720,14 +722,14 @@ int prb_launch_mg(gb_prb *h, int do_v, int do_u, cudaStream_t s)
 
 extern "C" int gb_prb_set_solve_spread(gb_prb *h, int ctas)
 {
-    if (!h || (ctas != 1 && ctas != MG_SPREAD)) {
-        gb_set_error("gb_prb_set_solve_spread: ctas must be 1 or %d", MG_SPREAD);
+    if (!h || (ctas != 0 && ctas != 1 && ctas != MG_SPREAD)) {
+        gb_set_error("gb_prb_set_solve_spread: ctas must be 1 or %d, or 0 for the default", MG_SPREAD);
         return GB_ERR_INVALID;
     }
     if (h->mg_spread != ctas) {
         GB_CUDA_TRY(cudaStreamSynchronize(h->stream));   // queued steps use the present plan
         h->mg_spread = ctas;
-        prb_mg_plan(h->eq_host, 2, h->p.precision == GB_PRB_MIXED, std::min(ctas, h->mg_ctas));
+        prb_mg_plan(h->eq_host, 2, h->p.precision == GB_PRB_MIXED, prb_mg_ctas(h));
         GB_CUDA_TRY(cudaMemcpy(h->eq_dev, h->eq_host, sizeof(MgEq) * 2, cudaMemcpyHostToDevice));
         if (h->graph_exec) { cudaGraphExecDestroy(h->graph_exec); h->graph_exec = nullptr; }
         if (h->graph_exec1) { cudaGraphExecDestroy(h->graph_exec1); h->graph_exec1 = nullptr; }
