@@ -39,8 +39,12 @@
 // The thread that starts the table copies: the last warp has lines only when
 // every other has.
 #define MER_FETCHER (MER_THREADS - 32)
-// Polls of a table copy's barrier before a solve gives up (about a second).
+// Polls of a table copy's barrier before a solve gives up (about a second), and
+// before it ends without a copy that is still on its way.
+#ifndef MER_POLLS
 #define MER_POLLS (1 << 22)
+#endif
+#define MER_DRAIN_POLLS (1 << 22)
 
 // Column i of a row: two leading pads (the far point of i = 1 is never read
 // with a nonzero weight, but is read), then a lane's rows padded to an odd
@@ -90,7 +94,7 @@ template <int NC> __device__ __forceinline__ int mer_share(int ni, int ctas) { r
 // half-sweeps: stage k & 1 holds the tables of half-sweep k.
 struct MerPipe {
     unsigned long long bar[2];
-    int timeout;
+    int timeout;   // 0, or 1 + the half-sweep whose wait gave up: no copy is started any more
 };
 
 // One thread of the CTA: starts the copy of the CTA's tables of colour c of
@@ -99,6 +103,7 @@ struct MerPipe {
 template <bool PENTA> __device__ __forceinline__ void mer_fetch(const MerLevel &L, MerPipe &pipe, int tab, int tab_floats, int dir, int c, int k)
 {
     extern __shared__ __align__(16) float s_mer[];
+    const int timeout = *(volatile int *)&pipe.timeout;   // on its way while the rest is formed
     const Cluster cl = Cluster::self();
     constexpr int NC = PENTA ? 4 : 2;
     const int n = dir == 0 ? L.n1 - 1 : L.n2 - 1;
@@ -120,6 +125,7 @@ template <bool PENTA> __device__ __forceinline__ void mer_fetch(const MerLevel &
         step = L.fac_z_step;
         src = L.fac_z;
     }
+    if (timeout) return;   // the stage may still be waiting for the copy before
     const unsigned bar = cta_addr(&pipe.bar[k & 1]);
     const unsigned dst = cta_addr(s_mer + tab + (k & 1) * tab_floats);
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(count * len * 4) : "memory");
@@ -128,19 +134,35 @@ template <bool PENTA> __device__ __forceinline__ void mer_fetch(const MerLevel &
                      "l"(src + (size_t)(line - 1 + NC * t) * step), "r"(len * 4), "r"(bar)
                      : "memory");
 }
-// Waits for half-sweep k's tables; gives up after MER_POLLS polls, once.
+// Whether half-sweep k's tables have landed.
+__device__ __forceinline__ bool mer_landed(MerPipe &pipe, int k)
+{
+    unsigned ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok)
+                 : "r"(cta_addr(&pipe.bar[k & 1])), "r"((k >> 1) & 1)
+                 : "memory");
+    return ok;
+}
+// Waits for them; gives up after MER_POLLS polls, once.
 __device__ __forceinline__ void mer_tables(MerPipe &pipe, int k)
 {
-    const unsigned bar = cta_addr(&pipe.bar[k & 1]);
-    unsigned ok = 0;
+    bool ok = false;
     for (int q = 0; !ok && q < MER_POLLS; ++q) {
         if ((q & 1023) == 1023 && *(volatile int *)&pipe.timeout) return;
-        asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                     : "=r"(ok)
-                     : "r"(bar), "r"((k >> 1) & 1)
-                     : "memory");
+        ok = mer_landed(pipe, k);
     }
-    if (!ok) pipe.timeout = 1;
+    if (!ok && !*(volatile int *)&pipe.timeout) pipe.timeout = k + 1;
+}
+// The end of a solve: the copies still on their way (the one prepared for a cycle
+// that is not run, k's, or the one that a wait gave up on and the one after it)
+// land before the block leaves.
+__device__ __forceinline__ void mer_drain(MerPipe &pipe, int k)
+{
+    const int timeout = *(volatile int *)&pipe.timeout;
+    for (int c = timeout ? timeout - 1 : k; c <= (timeout ? timeout : k); ++c)
+        for (int q = 0; !mer_landed(pipe, c) && q < MER_DRAIN_POLLS; ++q) {
+        }
 }
 
 // The r-lines of one sweep, colour by colour: the CTA's lines of the colour go
@@ -585,8 +607,8 @@ template <bool PENTA> __device__ __forceinline__ void mer_solve_body(const MerDe
         d.status[1] = cycles;
         if ((status == GB_NAN || status == GB_TIMEOUT) && d.abort) *d.abort = 1;
     }
-    mer_tables(pipe, k);   // the copy in flight
-    cl.sync();             // no CTA leaves while another may still read its shared memory
+    mer_drain(pipe, k);
+    cl.sync();   // no CTA leaves while another may still read its shared memory
 }
 
 template <bool PENTA> __global__ void __maxnreg__(255) k_mer_solve(const __grid_constant__ MerDev d) { mer_solve_body<PENTA>(d); }
