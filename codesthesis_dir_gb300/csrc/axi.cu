@@ -861,7 +861,7 @@ __global__ void k_axi_weights(const __grid_constant__ AxiDev d, const __grid_con
     const AxiLevel &L = d.lev[l];
     if (t >= 1 && t < L.n1) {
         const float r = d.rval32[t * L.lf];
-        const_cast<float4 *>(m.lev[l].ci)[t] = make_float4(r, r * r, 0.f, 0.f);
+        const_cast<float4 *>(m.lev[l].ci)[t] = make_float4(r, r * r, 1.0f / r, 1.0f / (r * r));
         if (l == 1) {
             const double rv = d.rval[t];
             MerRow &q = const_cast<MerRow *>(m.d_i)[t];
@@ -1042,6 +1042,13 @@ static cudaError_t axi_mer_create(gb_axi *h)
         L.hhr = (float)d.lev[l].hhr;
         L.hhz = (float)d.lev[l].hhz;
         L.drdz = 2.0f * (1.0f / L.hhr + 1.0f / L.hhz);
+        L.ihr = 1.0f / L.hr;
+        L.ihhr = 1.0f / L.hhr;
+        L.ihhz = 1.0f / L.hhz;
+        const float r0 = (float)(d.r0 * d.r0 < 1.0 ? d.r0 * d.r0 : 1.0), r1 = (float)std::max(1.0, h->p.rmax * h->p.rmax);
+        L.quick = 1;
+        for (float v : {L.hr, L.hhr, L.hhz, r0, r1})
+            if (!(v >= 0x1p-24f && v <= 0x1p24f)) L.quick = 0;
         L.fac_z_step = (int)tdma32_len(L.n2 - 1);
     }
     const AxiLevel &L1 = d.lev[1];

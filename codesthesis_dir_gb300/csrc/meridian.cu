@@ -69,6 +69,23 @@ __device__ __forceinline__ unsigned peer_addr(const void *p, int rank)
     return a;
 }
 
+// x / h for h > 0 from ih, the rounded 1 / h: a product and two corrections.  The
+// first leaves a faithful quotient, the second the correctly rounded one (the
+// remainder is exact then; Markstein, IBM J. Res. Dev. 34(1), 1990).  Divided by
+// itself, a lane's rows go one after the other through the division's branch, 290
+// cycles each (16 x 16, a cycle's r half-sweep 4.0 k cycles).  Both corrections
+// need x away from the ends of the exponent's range, MerLevel::quick the same of
+// the divisors; else `bad` is set and the caller divides.
+__device__ __forceinline__ float mer_quot(float x, float h, float ih, bool &bad)
+{
+    const unsigned e = (__float_as_uint(x) >> 23) & 0xffu;
+    if (e - (127u - 95u) > 2u * 95u && x != 0.f) bad = true;
+    float q = x * ih;
+    q = __fmaf_rn(__fmaf_rn(-h, q, x), ih, q);
+    q = __fmaf_rn(__fmaf_rn(-h, q, x), ih, q);
+    return x == 0.f ? x : q;
+}
+
 // Own rows of a level: j0 .. j1 - 1 at local indices 1, 2, ...
 struct MerOwn {
     int j0, j1;
@@ -231,10 +248,22 @@ template <int M, bool PENTA> __device__ __noinline__ int mer_r_sweep(const MerLe
                 }
             }
             __syncwarp();
+            if constexpr (PENTA) {
 #pragma unroll
-            for (int u = 0; u < M; ++u) {
-                if constexpr (PENTA) t[u] = -(weight[0] * src[0][u] + weight[1] * src[1][u] + weight[2] * src[2][u]) + t[u];
-                else t[u] = -(src[0][u] + src[1][u]) / L.hhz + t[u];
+                for (int u = 0; u < M; ++u) t[u] = -(weight[0] * src[0][u] + weight[1] * src[1][u] + weight[2] * src[2][u]) + t[u];
+            } else {
+                float s[M], q[M];
+                bool bad = !L.quick;
+#pragma unroll
+                for (int u = 0; u < M; ++u) s[u] = -(src[0][u] + src[1][u]);
+#pragma unroll
+                for (int u = 0; u < M; ++u) q[u] = mer_quot(s[u], L.hhz, L.ihhz, bad);
+                if (bad) {
+#pragma unroll
+                    for (int u = 0; u < M; ++u) q[u] = s[u] / L.hhz;
+                }
+#pragma unroll
+                for (int u = 0; u < M; ++u) t[u] = q[u] + t[u];
             }
             if (!ready) {
                 mer_tables(pipe, k);
@@ -242,7 +271,7 @@ template <int M, bool PENTA> __device__ __noinline__ int mer_r_sweep(const MerLe
             }
             WlTab<M, PENTA> T;
             T.load(s_mer + tab + (k & 1) * tab_floats + (size_t)t0 * len, lw);
-            T.solve(lw, t);
+            T.solve(n, t);
             if (live) {
 #pragma unroll
                 for (int u = 0; u < M; ++u)
@@ -303,7 +332,11 @@ __device__ __noinline__ int mer_z_sweep(const MerLevel &lev, MerPipe &pipe, int 
                     r = -(a.x * p0 + (low ? a.z : a.y) * p1 + a.w * p2 + over) + f;
                 } else {
                     const float vp = vr[mer_col(lg, i + 1)], vm = vr[mer_col(lg, i - 1)];
-                    r = -(vp + vm) / L.hhr + f - (vp - vm) * 0.5f / ci[i].x / L.hr;
+                    const float4 a = ci[i];
+                    const float s = -(vp + vm), e = (vp - vm) * 0.5f;
+                    bool bad = !L.quick;
+                    r = mer_quot(s, L.hhr, L.ihhr, bad) + f - mer_quot(mer_quot(e, a.x, a.z, bad), L.hr, L.ihr, bad);
+                    if (bad) r = s / L.hhr + f - e / a.x / L.hr;
                 }
                 cst(xline[l] + xj, r);
             }
@@ -325,7 +358,7 @@ __device__ __noinline__ int mer_z_sweep(const MerLevel &lev, MerPipe &pipe, int 
             }
             WlTab<M, PENTA> T;
             T.load(s_mer + tab + (k & 1) * tab_floats + (size_t)t * len, lw);
-            T.solve(lw, r);
+            T.solve(n, r);
             if (live) {
                 const unsigned col = 4 * mer_col(lg, c + NC * (l0 + t));
                 const int j = zl * M + 1;
@@ -370,7 +403,11 @@ template <bool PENTA> __device__ __noinline__ void mer_residual(const MerLevel &
                 t = t + w.x * (lowj ? d : e) + w.y * (lowj ? p : d) + w.z * (lowj ? u : p) + w.w * (lowj ? e : u);
             } else {
                 const float4 a = ci[i];
-                t = (pp + pm) / L.hhr + (pp - pm) * 0.5f / L.hr / a.x - p / a.y + (u + d) / L.hhz - p * L.drdz;
+                const float s = pp + pm, g = (pp - pm) * 0.5f, y = u + d;
+                bool bad = !L.quick;
+                t = mer_quot(s, L.hhr, L.ihhr, bad) + mer_quot(mer_quot(g, L.hr, L.ihr, bad), a.x, a.z, bad) - mer_quot(p, a.y, a.w, bad) +
+                    mer_quot(y, L.hhz, L.ihhz, bad) - p * L.drdz;
+                if (bad) t = s / L.hhr + g / L.hr / a.x - p / a.y + y / L.hhz - p * L.drdz;
             }
             out[c] = f[c] - t;
         }

@@ -25,12 +25,14 @@ struct MerOver {
 // d2/dr2 and of d/dr and 1/r, (crr1 .. crr4), (cr1, cr2, cr3, 1/r), and row j's
 // of d2/dz2, (czz1 .. czz4); the points of row i are i-1 .. i+2 for i <= n1/2
 // and i-2 .. i+1 beyond it, in z likewise.  Uniform grid (rotann2.f): row i's
-// (r, r r, 0, 0) and the spacings h.
+// (r, r r, 1/r, 1/(r r)) and the spacings h with 1/h.
 struct MerLevel {
     int n1, n2;
     const float4 *ci;               // i = 0..n1, two a row (stretched) or one
     const float4 *cj;               // j = 0..n2, stretched only
     float hr, hhr, hhz, drdz;       // uniform: 1/h's denominators, 2 (1/hhr + 1/hhz)
+    float ihr, ihhr, ihhz;          // 1/h (IEEE)
+    int quick;                      // every divisor lies in 2^-24 .. 2^24 (mer_quot)
     const float *fac_r, *fac_z;     // line tables (warpline.cuh) of line 1
     int fac_r_step, fac_z_step;     // floats from one line's table to the next (0: one table for all)
     // shared-memory plan of one CTA (floats): rows per CTA, row pitch, offsets

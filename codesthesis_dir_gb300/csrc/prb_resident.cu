@@ -170,7 +170,7 @@ __device__ __noinline__ void pl_sweeps32(const MgEq &E, int l)
                     if (L.polar) r = r * L.rvq[min(lane * M + u + 1, L.n1 + 1)];
                     t[u] = lane * M + u < n ? r + fr[u] : T(0);
                 }
-                tab.solve(lw, (float(&)[M])t);
+                tab.solve(n, t);
                 if (live) {
                     T *vr = L.own(L.v, k) + c0;
 #pragma unroll

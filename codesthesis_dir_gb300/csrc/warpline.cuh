@@ -48,6 +48,9 @@
 // 32 WL_MAXM rows take several segments of that many, one after the other.
 __host__ __device__ __forceinline__ int wl_log2m(int n) { return n <= 256 ? 3 : 4; }
 __host__ __device__ __forceinline__ int wl_log2w(int n) { return n <= 32 ? 2 : n <= 64 ? 3 : n <= 128 ? 4 : 5; }
+// log2 of the lanes that hold a line's rows: the passes of a line go over no more
+// (a line of up to 8 rows is one lane's and takes one pass).
+__host__ __device__ __forceinline__ int wl_log2p(int n) { return n <= 8 ? 0 : n <= 16 ? 1 : wl_log2w(n); }
 __host__ __device__ __forceinline__ int wl_segments(int n) { return n <= 256 ? 1 : (n + 511) / 512; }
 // Padded rows of a line, the floats of its table (5 or 3 coefficients a row
 // as [segment][coefficient][row in lane][lane]; a multiple of 16 bytes) and the
@@ -89,7 +92,7 @@ template <bool FUSED = false> __device__ inline void tdma32_fold(const double *f
     }
 }
 
-// A recurrence of up to second order over the W = 2^lw lanes' W M rows:
+// A recurrence of up to second order over the rows of W = 2^lw lanes, M each:
 // y(u) = row(u, y(u-1), y(u-2)), into y; (c1, c2) carries the two states
 // before the first row in and the last two out.  BACK runs it from the last
 // row to the first.  All 32 lanes of the warp take part.
@@ -190,9 +193,10 @@ template <int M, bool PENTA, bool FUSED = false> struct WlTab {
         else
             wl_chain<M, true, false>(lw, x, c1, c2, [&](int u, float y1, float) { return (z[u] - d[u] * y1) * s[u]; });
     }
-    // a line of one segment, in place
-    __device__ __forceinline__ void solve(int lw, float (&t)[M]) const
+    // a line of one segment and n rows, in place
+    __device__ __forceinline__ void solve(int n, float (&t)[M]) const
     {
+        const int lw = wl_log2p(n);
         float c1 = 0.f, c2 = 0.f, z[M];
         down(lw, t, z, c1, c2);
         c1 = c2 = 0.f;
