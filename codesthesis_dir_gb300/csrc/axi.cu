@@ -941,7 +941,8 @@ struct gb_axi {
     double dr_set = 0.0, dz_set = 0.0;   // a Fortran caller's /num/ spacings, 0 = derived
     int ctas = 1;                        // CTAs per ZEBRA solve on global memory
     MerDev mer;                          // the resident mixed solve, where its plan fits
-    int mer_ctas = 0;                    // its CTAs; 0: k_axi_mg_solve_mixed
+    int mer_most = 0;                    // the largest cluster it can have; 0: k_axi_mg_solve_mixed
+    int mer_ctas = 0;                    // its CTAs
     void *mer_mem = nullptr;
 };
 
@@ -1024,7 +1025,7 @@ extern "C" int gb_axi_destroy(gb_axi *h)
     return GB_OK;
 }
 
-// Prepares the resident mixed solve; a grid it cannot hold leaves mer_ctas 0.
+// Prepares the resident mixed solve; a grid it cannot hold leaves mer_most 0.
 static cudaError_t axi_mer_create(gb_axi *h)
 {
     const AxiDev &d = h->dev;
@@ -1061,8 +1062,9 @@ static cudaError_t axi_mer_create(gb_axi *h)
     m.rhs = d.f[GB_A_omegn];
     m.status = d.status;
     m.abort = d.abort;
-    h->mer_ctas = mer_fit(m, CL_MAX_CTAS);
-    if (!h->mer_ctas) return cudaSuccess;
+    h->mer_most = mer_fit(m, CL_MAX_CTAS);
+    if (!h->mer_most) return cudaSuccess;
+    h->mer_ctas = mer_alone(m, h->mer_most);
     cudaError_t e = cudaMalloc(&h->mer_mem, mer_weight_bytes(m));
     if (e != cudaSuccess) return e;
     mer_weight_layout(m, h->mer_mem);
@@ -1343,7 +1345,7 @@ static MerDev axi_mer(const gb_axi *h)
     // the reference's line order is one chain of lines: one CTA
     const int ctas = d.mode == GB_SMOOTHER_LEX ? 1 : h->ctas;
     if (h->p.precision != GB_PRB_MIXED) return cl_launch(k_axi_mg_solve, 1, ctas, AXI_THREADS, AXI_SMEM_BYTES, s, d);
-    if (d.mode == GB_SMOOTHER_ZEBRA && h->mer_ctas) return mer_launch(axi_mer(h), h->mer_ctas, s);
+    if (d.mode == GB_SMOOTHER_ZEBRA && h->mer_most) return mer_launch(axi_mer(h), h->mer_ctas, s);
     return cl_launch(k_axi_mg_solve_mixed, 1, ctas, AXI_THREADS, AXI_SMEM_BYTES, s, d);
 }
 
@@ -1659,10 +1661,10 @@ extern "C" int gb_axi_gang_create(gb_axi *const *members, const int *nsteps_tota
     int most = CL_MAX_CTAS;
     const int sms = gb_sm_count();
     for (int q = 0; q < n; ++q) {
-        if (mixed && members[q]->p.smoother == GB_SMOOTHER_ZEBRA && members[q]->mer_ctas) {
+        if (mixed && members[q]->p.smoother == GB_SMOOTHER_ZEBRA && members[q]->mer_most) {
             res.push_back(q);
             mers.push_back(axi_mer(members[q]));
-            most = std::min(most, members[q]->mer_ctas);
+            most = std::min(most, members[q]->mer_most);
         } else if (members[q]->p.smoother == GB_SMOOTHER_LEX) {
             lex.push_back(q);
         } else {

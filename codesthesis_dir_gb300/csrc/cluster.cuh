@@ -164,6 +164,12 @@ template <class F> static inline cudaError_t cl_prepare(F kernel, size_t smem)
     return e;
 }
 
+// Grids of so few points have no work to spread: their phases are latency, and a
+// cluster's barriers and remote accesses only add to it.  Mixed streamfunction
+// solves, four steps, on 16 CTAs and on one: 8 x 8 0.64 and 0.54 ms, 16 x 16 1.05
+// and 0.87, 32 x 32 1.24 and 1.14, 40 x 40 1.52 and 1.64.
+static inline bool cl_small_grid(int n1, int n2) { return (long long)n1 * n2 <= 1024; }
+
 // CTAs per cluster for a solve: `want`, halved until the device can hold one
 // such cluster with this shared memory.
 template <class F> static inline int cl_fit(F kernel, int want, int threads, size_t smem)

@@ -734,6 +734,13 @@ int mer_fit(MerDev &d, int want)
     return 0;
 }
 
+int mer_alone(MerDev &d, int most)
+{
+    if (cl_small_grid(d.lev[1].n1, d.lev[1].n2) && mer_plan(d, 1)) return 1;
+    mer_plan(d, most);
+    return most;
+}
+
 int mer_plan_many(MerDev *d, int n, int want, int most, size_t *smem, char *fits)
 {
     for (int c = want;; c <<= 1) {

@@ -66,8 +66,10 @@ bool mer_plan(MerDev &d, int ctas);
 // by mer_weight_bytes; penta and the levels' n1, n2 must be set.
 size_t mer_weight_bytes(const MerDev &d);
 void mer_weight_layout(MerDev &d, void *mem);
-// Clusters of this size that fit the device for d's plan (halved from want).
+// The largest cluster, up to `want`, that the device holds and d fits (0: none).
 int mer_fit(MerDev &d, int want);
+// CTAs of a solve of its own, planned for: `most`, or one for a small grid.
+int mer_alone(MerDev &d, int most);
 // One cluster size for n solves of a launch: the power of two `want` or, up to
 // `most`, as many more CTAs as the largest needs.  Plans the solves for it;
 // fits[q]: solve q does fit.  *smem: the most any of those takes.

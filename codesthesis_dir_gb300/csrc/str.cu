@@ -596,6 +596,7 @@ static cudaError_t str_mer_create(gb_str *h)
     m.v = d.lev[1].v;
     h->mer_ctas = mer_fit(m, CL_MAX_CTAS);
     if (!h->mer_ctas) return cudaSuccess;
+    h->mer_ctas = mer_alone(m, h->mer_ctas);
     cudaError_t e = cudaMalloc(&h->mer_mem, mer_weight_bytes(m));
     if (e != cudaSuccess) return e;
     mer_weight_layout(m, h->mer_mem);
@@ -758,7 +759,7 @@ extern "C" int gb_str_create(int nlev, const gb_str_level *lv, double tolcon, in
     e = cl_prepare(k_str_solve, STR_SMEM_BYTES);
     if (e == cudaSuccess) e = cl_prepare(k_str_solve_mixed, STR_SMEM_BYTES);
     if (e != cudaSuccess) { gb_str_destroy(h); gb_set_error("gb_str_create: shared memory: %s", cudaGetErrorString(e)); return GB_ERR_CUDA; }
-    h->ctas = cl_fit(k_str_solve, CL_MAX_CTAS, STR_THREADS, STR_SMEM_BYTES);
+    h->ctas = cl_fit(k_str_solve, cl_small_grid(n1, n2) ? 1 : CL_MAX_CTAS, STR_THREADS, STR_SMEM_BYTES);
     e = str_mer_create(h);
     if (e != cudaSuccess) { gb_set_error("gb_str_create: %s", cudaGetErrorString(e)); gb_str_destroy(h); return GB_ERR_CUDA; }
     *out = h;

@@ -129,7 +129,8 @@ class PRB:
     def set_solve_spread(self, ctas):
         """CTAs sharing one two-colour solve (FP64 or mixed): 1 (one CTA per
         equation) or 8 (a cluster); without a call, or again with 0, the
-        largest cluster the device holds.  All give the same bits."""
+        largest cluster the device holds (small grids: one CTA).  All give
+        the same bits."""
         _L.check(_L.load().gb_prb_set_solve_spread(self._h, ctas), "set_solve_spread")
 
     def update(self):

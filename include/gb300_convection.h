@@ -212,8 +212,9 @@ int gb_prb_poisson(gb_prb *h, int which, int *sweeps);
  * (one CTA per equation) or 8 (the lines of a colour, the residuals and the
  * transfers of each level are spread over a cluster of 8 CTAs that meet at
  * the hardware cluster barrier and reduce through distributed shared memory).
- * Without a call, or again with 0: the largest cluster the device holds (16).
- * All give the same bits; the reference's line order always uses one CTA.  No counterpart
+ * Without a call, or again with 0: the largest cluster the device holds (16),
+ * on small grids (at most 1024 points and 32 lines) one CTA.  All give the same
+ * bits; the reference's line order always uses one CTA.  No counterpart
  * in the reference (its solves are serial). */
 int gb_prb_set_solve_spread(gb_prb *h, int ctas);
 /* update (PRB:1557-1626); *clamps (may be NULL) gets the number of
