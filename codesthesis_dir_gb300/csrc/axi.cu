@@ -523,9 +523,10 @@ template <class T> __device__ __forceinline__ T axi_resid(const AxiView<T> &L, T
 // fit its shared memory: the lines' factors are copied there while all
 // threads form the right-hand sides, the lines are eliminated (FP64: one
 // thread per line in the reference's order; FP32: up to 32 lanes per line),
-// the solutions go back.
+// the solutions go back.  fresh: the r-lines' table is not staged yet (the
+// reference's order comes here line by line).
 template <class T, int DIR>
-__device__ __noinline__ void axi_lines(const AxiDev &d, int l, int first, int step, int nl)
+__device__ __noinline__ void axi_lines(const AxiDev &d, int l, int first, int step, int nl, bool fresh = true)
 {
     extern __shared__ __align__(16) unsigned char s_axi[];
     constexpr bool F64 = sizeof(T) == 8;
@@ -549,7 +550,7 @@ __device__ __noinline__ void axi_lines(const AxiDev &d, int l, int first, int st
         const int nb = min(B, t1 - b0), pitch = nb | 1;
         // FP64: [row][line], odd pitch; FP32: [line][row], padded per lane
         auto at = [&](int t, int q) -> T & { return F64 ? x[q * pitch + t] : x[t * lpitch + wl_slot(lg, q)]; };
-        if (staged)
+        if (staged && fresh)
             for (int t = 0; t < (DIR == 0 ? 1 : nb); ++t)
                 async_copy(sfac + t * fpitch, table(first + step * (b0 + t)), flen, threadIdx.x, blockDim.x);
         if (DIR == 0) {
@@ -580,8 +581,8 @@ __device__ __noinline__ void axi_lines(const AxiDev &d, int l, int first, int st
                 else tdma_staged(table(first + step * (b0 + t)), n, x + t, pitch);
             }
         } else {
-            if (staged) wl_lines<false>(sfac, fpitch, n, x, lpitch, nb);
-            else wl_lines<false>(table(first + step * b0), DIR == 0 ? 0 : (size_t)step * flen, n, x, lpitch, nb);
+            if (staged) wl_lines<false, false, true>(sfac, fpitch, n, x, lpitch, nb);
+            else wl_lines<false, false, true>(table(first + step * b0), DIR == 0 ? 0 : (size_t)step * flen, n, x, lpitch, nb);
         }
         __syncthreads();
         if (DIR == 0) {
@@ -612,7 +613,7 @@ template <class T> __device__ __forceinline__ void axi_sweeps(const AxiDev &d, i
     const int nj = d.lev[l].n2 - 1, ni = d.lev[l].n1 - 1;
     for (int irel = 0; irel < d.nrel; ++irel) {
         if (d.mode == GB_SMOOTHER_LEX) {
-            for (int j = 1; j <= nj; ++j) axi_lines<T, 0>(d, l, j, 1, 1);
+            for (int j = 1; j <= nj; ++j) axi_lines<T, 0>(d, l, j, 1, 1, j == 1);
             for (int i = 1; i <= ni; ++i) axi_lines<T, 1>(d, l, i, 1, 1);
         } else {
             for (int c = 1; c <= 2; ++c)

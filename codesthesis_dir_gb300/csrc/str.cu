@@ -264,8 +264,8 @@ __device__ __noinline__ void str_lines(const StrLevel &lev, int first, int step,
                 else pdma_staged(L.fac[DIR] + (size_t)(first + step * (b0 + t) - 1) * flen, n, x + t, pitch);
             }
         } else {
-            if (staged) wl_lines<true>(sfac, fpitch, n, x, lpitch, nb);
-            else wl_lines<true>(L.fac[DIR] + (size_t)(first + step * b0 - 1) * flen, (size_t)step * flen, n, x, lpitch, nb);
+            if (staged) wl_lines<true, false, true>(sfac, fpitch, n, x, lpitch, nb);
+            else wl_lines<true, false, true>(L.fac[DIR] + (size_t)(first + step * b0 - 1) * flen, (size_t)step * flen, n, x, lpitch, nb);
         }
         __syncthreads();
         if (DIR == 0) {

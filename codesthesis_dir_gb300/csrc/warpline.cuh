@@ -207,10 +207,12 @@ template <int M, bool PENTA, bool FUSED = false> struct WlTab {
 // Lines t0, t0 + tstep, ... < nl of n rows, in place in shared memory: line t
 // at x + t * xpitch (its slots) with its table at tab + t * tpitch (shared or
 // global).  One warp; all its lanes call.
-template <int M, bool PENTA, bool FUSED = false>
+// BRIEF: passes over the lanes that hold rows only (wl_log2p), where the kernel has
+// the registers for a second width (64 x 64 x 128 mixed, two steps: 217 -> 298 ms).
+template <int M, bool PENTA, bool FUSED = false, bool BRIEF = false>
 __device__ __forceinline__ void wl_lines_m(const float *tab, size_t tpitch, int n, float *x, int xpitch, int nl, int warp, int nwarps)
 {
-    const int lw = wl_log2w(n), nseg = wl_segments(n), per = 32 >> lw;
+    const int lw = wl_log2w(n), lp = BRIEF ? wl_log2p(n) : lw, nseg = wl_segments(n), per = 32 >> lw;
     const int sub = (threadIdx.x & 31) >> lw, lane = threadIdx.x & ((1 << lw) - 1);
     for (int t0 = warp * per; t0 < nl; t0 += nwarps * per) {
         const bool live = t0 + sub < nl;
@@ -222,7 +224,7 @@ __device__ __forceinline__ void wl_lines_m(const float *tab, size_t tpitch, int 
             T.load_down(tab + t * tpitch, lw, g);
 #pragma unroll
             for (int u = 0; u < M; ++u) r[u] = xs[u];
-            T.down(lw, r, z, c1, c2);
+            T.down(lp, r, z, c1, c2);
             if (g < nseg - 1) {
 #pragma unroll
                 for (int u = 0; u < M; ++u) xs[u] = z[u];
@@ -236,7 +238,7 @@ __device__ __forceinline__ void wl_lines_m(const float *tab, size_t tpitch, int 
 #pragma unroll
                 for (int u = 0; u < M; ++u) z[u] = xs[u];
             }
-            T.up(lw, z, r, c1, c2);
+            T.up(lp, z, r, c1, c2);
             if (live) {
 #pragma unroll
                 for (int u = 0; u < M; ++u) xs[u] = r[u];
@@ -244,12 +246,12 @@ __device__ __forceinline__ void wl_lines_m(const float *tab, size_t tpitch, int 
         }
     }
 }
-template <bool PENTA, bool FUSED = false>
+template <bool PENTA, bool FUSED = false, bool BRIEF = false>
 __device__ __forceinline__ void wl_lines(const float *tab, size_t tpitch, int n, float *x, int xpitch, int nl)
 {
     const int warp = threadIdx.x >> 5, nwarps = (int)blockDim.x >> 5;
-    if (wl_log2m(n) == 3) wl_lines_m<8, PENTA, FUSED>(tab, tpitch, n, x, xpitch, nl, warp, nwarps);
-    else wl_lines_m<16, PENTA, FUSED>(tab, tpitch, n, x, xpitch, nl, warp, nwarps);
+    if (wl_log2m(n) == 3) wl_lines_m<8, PENTA, FUSED, BRIEF>(tab, tpitch, n, x, xpitch, nl, warp, nwarps);
+    else wl_lines_m<16, PENTA, FUSED, BRIEF>(tab, tpitch, n, x, xpitch, nl, warp, nwarps);
 }
 
 // Asynchronous copy of n elements into shared memory by the block (16 bytes
