@@ -29,14 +29,16 @@ struct Cluster {
     __device__ __forceinline__ int nthr() const { return size * (int)blockDim.x; }
     // The two halves of sync: what is issued between them (fetches of the next
     // phase's constants) overlaps the barrier, where a fetch issued before the
-    // release would be waited for.
+    // release would be waited for.  The unaligned forms: a warp may come here
+    // diverged, from a loop that its lanes left at different times, and an aligned
+    // barrier is defined for converged warps only.
     __device__ __forceinline__ void arrive() const
     {
-        if (size > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        if (size > 1) asm volatile("barrier.cluster.arrive.release;" ::: "memory");
     }
     __device__ __forceinline__ void wait() const
     {
-        if (size > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        if (size > 1) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
         else __syncthreads();
     }
     // Orders global and distributed shared memory between all threads of the
