@@ -766,8 +766,11 @@ template <class T, int LG, int NT> __device__ __forceinline__ void loc_restrict(
     const Q S;
     const int I = S.s + 1, lane = threadIdx.x & 31;
     const bool col = I <= mc;   // the last slot's column 2 I is the boundary
+    // whole warps without a coarse row leave the residuals, which the FP64 pipe
+    // would take all the same (n = 17: 14 of 16 warps)
+    const int first = (int)(threadIdx.x & ~31u) >> Q::lw;
 #pragma unroll 1
-    for (int J0 = 1; J0 <= mc; J0 += Q::R) {
+    for (int J0 = 1; J0 + first <= mc; J0 += Q::R) {
         const int J = min(J0 + S.j - 1, mc);
         const int p = J * V::n + I;   // place of (2 J, 2 I), an even point
         T k0 = (T)0, k1 = (T)0, k2 = (T)0;
@@ -1376,7 +1379,8 @@ __global__ void __launch_bounds__(LOCAL_THREADS) k_local_solve(BatchDev B, const
             }
             acc = __fma_rn(rw, rw, acc);
         }
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if ((tid & ~31) < (j1 - j0) << ls)   // else the warp has no points
+            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
         if ((tid & 31) == 0) s_part[tid >> 5] = acc;
         __syncthreads();
         if (tid < 32) {
@@ -2407,11 +2411,17 @@ static int solve_graph(gb_batch *b, cudaStream_t s)
     return GB_OK;
 }
 
+// Whole solves take an SM's registers, one problem at a time; with many more
+// problems than SMs the level-by-level kernels, two to four blocks an SM, end
+// sooner (8000 problems: n = 17 FP64 5.85 and 5.37 ms, n = 9 pairs 1.86 and 1.77;
+// 4000: 3.00 and 2.90, 0.97 and 1.07; 20000 of n = 3 pairs 1.13 and 1.00).
+#define LOCAL_SOLVE_PER_SM 40
+
 // Whether every problem is local altogether and one block holds its solve.
 static size_t whole_local_smem(const gb_batch *b)
 {
     const int n = *std::max_element(b->n.begin(), b->n.end());
-    if (b->maxdepth_global > 0) return 0;
+    if (b->maxdepth_global > 0 || b->nprob > LOCAL_SOLVE_PER_SM * b->nsm) return 0;
     const size_t sm = b->local_smem + (inner32(b) ? 2 * 8 * (size_t)n * n : 0);
     return sm <= LOCAL_SOLVE_SMEM ? sm : 0;
 }
