@@ -40,8 +40,6 @@ template <class T> __device__ __forceinline__ T fmaT(T a, T b, T c);
 template <> __device__ __forceinline__ double fmaT<double>(double a, double b, double c) { return __fma_rn(a, b, c); }
 template <> __device__ __forceinline__ float fmaT<float>(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 
-__device__ __forceinline__ double to_double(float v) { return f2d(v); }
-
 // Float pairs (hi, lo), |lo| <= ulp(hi)/2: about 48 significand bits with
 // FP32 arithmetic only.  two_sum finds the rounding error of a float sum
 // exactly (Knuth, TAOCP vol. 2, 4.2.2); df_add is the accurate pair sum of
@@ -79,7 +77,6 @@ __device__ __forceinline__ float2 df_add_f(float2 a, float b)
     return make_float2(s, e);
 }
 __device__ __forceinline__ float2 df_scale(float2 a, float p) { return make_float2(a.x * p, a.y * p); }
-__device__ __forceinline__ double to_double(double v) { return v; }
 
 struct TileEntry {
     int p;            // problem
@@ -93,7 +90,6 @@ struct BatchDev {
     const int *dloc;          // [p] first level solved locally
     void *const *x;           // [(slot*nprob + p)*BP_MAXL + l] the two buffers of level l's solution (T*)
     void *const *f;           // right-hand side of level l (T*)
-    void *const *r;           // unused
     int *active;              // [p]
     int *cycles;              // [p]
     int *failed;              // [p]
@@ -117,7 +113,6 @@ template <class T> __device__ __forceinline__ T *XS(const BatchDev &B, int p, in
     return (T *)B.x[((size_t)slot * B.nprob + p) * BP_MAXL + l];
 }
 template <class T> __device__ __forceinline__ T *FP(const BatchDev &B, int p, int l) { return (T *)B.f[p * BP_MAXL + l]; }
-template <class T> __device__ __forceinline__ T *RP(const BatchDev &B, int p, int l) { return (T *)B.r[p * BP_MAXL + l]; }
 // Points from one row of a level's arrays to the next: FP64 packed (level 0 is
 // the caller's), FP32 whole float4s.
 template <class T> __host__ __device__ __forceinline__ int pitch_of(int n) { return sizeof(T) == 4 ? (n + 3) & ~3 : n; }
@@ -2054,7 +2049,6 @@ static int batch_create(int nprob, const int *n, int precision, int nu1, int nu2
     D.dloc = d_dloc;
     D.x = dp;
     D.f = dp + b->hx.size();
-    D.r = nullptr;
     D.psi = b->d_psi_tab;
     D.h2d = (const double *)b->d_spacing;
     D.ih2d = D.h2d + nsp;

@@ -42,7 +42,7 @@ struct MgEq {
     double r0;
     double tolcon, sor;
     MgLevel lev[PRB_MAXLEV];
-    double *psic, *psif, *rc, *rf, *tempa;   // COMMON /arrays/ (per equation)
+    double *psif, *rc;                       // the iterate and the residual (COMMON /arrays/, per equation)
     float *psif32, *rc32;                    // mixed precision: FP32 correction and residual
     double *psi, *psip;                      // solution and previous level (in/out)
     const double *rhs;

@@ -684,7 +684,6 @@ int prb_mg_create(gb_prb *h)
         double *base = h->mg_pool + q * per_eq;
         E.psif = base; base += (size_t)ld * (np + 1);
         E.rc = base; base += (size_t)ld * (np + 1);
-        E.psic = E.rf = E.tempa = nullptr;
         float *fbase = (float *)base;
         E.psif32 = fbase; fbase += (size_t)ld * (np + 1);
         E.rc32 = fbase; fbase += (size_t)ld * (np + 1);
