@@ -523,10 +523,10 @@ template <class T> __device__ __forceinline__ T axi_resid(const AxiView<T> &L, T
 // fit its shared memory: the lines' factors are copied there while all
 // threads form the right-hand sides, the lines are eliminated (FP64: one
 // thread per line in the reference's order; FP32: up to 32 lanes per line),
-// the solutions go back.  fresh: the r-lines' table is not staged yet (the
+// the solutions go back.  FRESH: the r-lines' table is not staged yet (the
 // reference's order comes here line by line).
-template <class T, int DIR>
-__device__ __noinline__ void axi_lines(const AxiDev &d, int l, int first, int step, int nl, bool fresh = true)
+template <class T, int DIR, bool FRESH = true>
+__device__ __noinline__ void axi_lines(const AxiDev &d, int l, int first, int step, int nl)
 {
     extern __shared__ __align__(16) unsigned char s_axi[];
     constexpr bool F64 = sizeof(T) == 8;
@@ -550,7 +550,7 @@ __device__ __noinline__ void axi_lines(const AxiDev &d, int l, int first, int st
         const int nb = min(B, t1 - b0), pitch = nb | 1;
         // FP64: [row][line], odd pitch; FP32: [line][row], padded per lane
         auto at = [&](int t, int q) -> T & { return F64 ? x[q * pitch + t] : x[t * lpitch + wl_slot(lg, q)]; };
-        if (staged && fresh)
+        if (staged && FRESH)
             for (int t = 0; t < (DIR == 0 ? 1 : nb); ++t)
                 async_copy(sfac + t * fpitch, table(first + step * (b0 + t)), flen, threadIdx.x, blockDim.x);
         if (DIR == 0) {
@@ -613,7 +613,10 @@ template <class T> __device__ __forceinline__ void axi_sweeps(const AxiDev &d, i
     const int nj = d.lev[l].n2 - 1, ni = d.lev[l].n1 - 1;
     for (int irel = 0; irel < d.nrel; ++irel) {
         if (d.mode == GB_SMOOTHER_LEX) {
-            for (int j = 1; j <= nj; ++j) axi_lines<T, 0>(d, l, j, 1, 1, j == 1);
+            for (int j = 1; j <= nj; ++j) {
+                if (j == 1) axi_lines<T, 0>(d, l, j, 1, 1);
+                else axi_lines<T, 0, false>(d, l, j, 1, 1);
+            }
             for (int i = 1; i <= ni; ++i) axi_lines<T, 1>(d, l, i, 1, 1);
         } else {
             for (int c = 1; c <= 2; ++c)
