@@ -55,8 +55,11 @@ def test_lines_longer_than_the_buffer_are_refused(gblib):
     import ctypes as C
 
     from codesthesis_dir_gb300 import lib
+
+    params = gblib.gb_r3d_default_params.argtypes[0]._type_   # the binding's, also after a reload of lib
+
     def create(np_, precision):
-        p, h = lib.R3dParams(), C.c_void_p()
+        p, h = params(), C.c_void_p()
         gblib.gb_r3d_default_params(C.byref(p), 4, 4, np_)
         p.precision = precision
         st = gblib.gb_r3d_create(C.byref(p), C.byref(h), None)
