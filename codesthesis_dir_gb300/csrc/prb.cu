@@ -1466,6 +1466,8 @@ static cudaError_t prb_gang_plan(gb_prb_gang *g)
     for (int q = 0; q < p.nres; ++q) p.smem = std::max(p.smem, e[q].smem);
     cudaError_t err = cudaMalloc(&p.d_eqs, sizeof(MgEq) * eqs.size());
     if (err == cudaSuccess) err = cudaMemcpy(p.d_eqs, e, sizeof(MgEq) * eqs.size(), cudaMemcpyHostToDevice);
+    // from pageable memory it may still be on its way, and the gang's stream does not wait for it
+    if (err == cudaSuccess) err = cudaStreamSynchronize(0);
     if (err != cudaSuccess) {
         cudaFree(p.d_eqs);
         p.d_eqs = nullptr;
