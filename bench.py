@@ -588,7 +588,7 @@ def run_axi_workload(args):
                    "l2": "working set (~6 MB) fits in L2; the step is latency and FP64-pipe bound"},
         "roofline": {"bound": "hbm", "achieved": None, "peak": peak, "unit": "GB/s", "frac": None, "traffic": None,
                      "peak_kind": peak_kind,
-                     "note": "one-block multigrid on a 257 x 257 grid: chain-latency bound, see detail"},
+                     "note": "multigrid of one 257 x 257 grid on a thread-block cluster: chain-latency bound, see detail"},
         "detail": summ, "clocks": clk.summary(),
     }
     if "cpu_baseline" in summ:

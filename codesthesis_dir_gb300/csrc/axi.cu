@@ -1530,8 +1530,8 @@ extern "C" int gb_axi_step(gb_axi *h, int nsteps, double *nu, int *sweeps, int *
 // ---------------------------------------------------------------------------
 // Gangs of annulus instances of different grid sizes stepped together (as
 // the PRB gangs in prb.cu): each phase of a step is one launch over all
-// members' blocks, the streamfunction solves one launch of one block per
-// member; every member runs its own kernel bodies, so its results are
+// members' blocks, the streamfunction solves up to three (gb_axi_gang), a
+// cluster per member; every member runs its own kernel bodies, so its results are
 // bit-identical to stepping it alone.  A member whose step index reaches
 // its step count sets its abort flag to GB_RUN_DONE.
 // ---------------------------------------------------------------------------
@@ -1575,9 +1575,8 @@ __global__ void k_axi_gang(AxiGangTab g)
     }
 }
 
-// The solves of the members listed in `who`, a cluster each.  128 registers
-// keep the solve free of spills (a launch bound of 512 threads left it at
-// 40-64 with spills).
+// The solves of the members listed in `who`, a cluster each; registers as the
+// single instance's kernels, free of spills.
 template <bool MIXED>
 __global__ void __maxnreg__(255) k_axi_gang_mg(AxiGangTab g, const int *who)
 {

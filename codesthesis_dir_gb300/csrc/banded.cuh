@@ -203,7 +203,7 @@ __device__ inline void apply_ptdma_rhs(const double *fac, int n, double *x, int 
 //     while a row is eliminated (the compiler cannot move those loads above
 //     the stores to x).
 // A row of the layer's pentadiagonal lines: 902 cycles with all products and
-// selections, 470 now (7 FP64 instructions).
+// selections, 560 now (7 FP64 instructions).
 // ---------------------------------------------------------------------------
 
 // Rows k0 .. k1 - 1 of the pentadiagonal forward elimination; A: with the

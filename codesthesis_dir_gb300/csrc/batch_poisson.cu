@@ -661,7 +661,7 @@ __device__ __forceinline__ void op_tile32(const BatchDev &B, TileEntry e, int l,
 // its left fine columns, and gets the right one from the next lane (nine
 // before); the levels up to LOC_SOLO, one warp's worth of points a colour, are
 // one warp's, which needs no block barrier.  k_local, n = 65: 28.8 -> 15 us in
-// FP32; FP64 76 -> 68 us, of which the FP64 pipe's instructions are 50.
+// FP32; FP64 76 -> 62 us, most of it the FP64 pipe's instructions.
 // ---------------------------------------------------------------------------
 #define LOC_SOLO 3      // LG of the largest one-warp level (n = 9)
 #define LOC_MAX 7       // of the largest local level (n = 129)
@@ -1288,7 +1288,7 @@ __global__ void __launch_bounds__(LOCAL_THREADS) k_local(BatchDev B, Op op, int 
 // As single launches an iteration of a small batch is launch and host latency
 // (eight problems of n = 17 .. 65, FP64 outer: 55 us an iteration, 550 us a
 // solve; here 20 us an iteration with one CTA per problem, 12 with eight, and
-// 159 us a solve).
+// 140 us a solve).
 template <class T, int CM> struct LocOuter {
     using V = typename CorrVal<CM>::type;
 };

@@ -5,8 +5,8 @@
 // lanes a cycle, so on one SM the phases around the eliminations cost more
 // than the eliminations; a cluster spreads them over up to 16 SMs and meets
 // at the hardware cluster barrier, 0.2 us where a grid-wide barrier takes
-// 1.3 us (129 x 129 uniform annulus, FP64, a step: one CTA 13.5 ms, 16 CTAs
-// with staged factors 4.1 ms, of which the eliminations' chains are 2.6).
+// 1.3 us (129 x 129 uniform annulus, FP64, four steps: one CTA 23.1 ms, 16 CTAs
+// 12.7, of which the eliminations' chains are 9).
 // Every CTA runs the same control flow: what decides it (residual
 // norms, NaN flags) comes from cl_max, which gives every CTA the same bits.
 #pragma once

@@ -22,8 +22,7 @@
 // and a correction, the conversions and the norm go to the integer pipe.
 //
 // Measured (GB300, mixed solve, a step's whole time): 257 x 257 stretched, five
-// cycles, 22.3 ms on one SM and global memory, 4.5 ms on a cluster of 16 with
-// the levels in L2, 2.8 ms resident.
+// cycles, 22.3 ms on one SM and global memory, 2.6 ms resident on a cluster of 16.
 #include "meridian.cuh"
 
 #include <algorithm>
@@ -73,7 +72,7 @@ __device__ __forceinline__ unsigned peer_addr(const void *p, int rank)
 // first leaves a faithful quotient, the second the correctly rounded one (the
 // remainder is exact then; Markstein, IBM J. Res. Dev. 34(1), 1990).  Divided by
 // itself, a lane's rows go one after the other through the division's branch, 290
-// cycles each (16 x 16, a cycle's r half-sweep 4.0 k cycles).  Both corrections
+// cycles each (16 x 16, an r half-sweep: 4.0 k cycles, 2.1 k this way).  Both corrections
 // need x away from the ends of the exponent's range, MerLevel::quick the same of
 // the divisors; else `bad` is set and the caller divides.
 __device__ __forceinline__ float mer_quot(float x, float h, float ih, bool &bad)

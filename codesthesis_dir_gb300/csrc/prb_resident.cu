@@ -14,9 +14,9 @@
 // reference's order.  FP32 (the mixed solve's correction cycles): by up to 32
 // lanes (warpline.cuh); the FP64 iterate stays in global memory.
 //
-// Measured on the 129 x 65 layer (GB300, a step of about 26 sweeps): FP64
-// 20.7 ms on one CTA and global memory, 10.7 on a cluster of 16, 9.1 resident
-// (6.6 of them eliminations); mixed 6.9, 4.7, 3.2.
+// Measured on the 129 x 65 layer (GB300, three steps at tolerance 2e-6): FP64 25.6
+// ms on one CTA (from global memory), 14.9 on a cluster of 16, most of it
+// eliminations; mixed 8.7 and 5.9.
 #include <string.h>
 
 #include <algorithm>

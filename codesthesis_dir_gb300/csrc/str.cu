@@ -5,13 +5,13 @@
 // nine-point restriction, bilinear prolongation, plain V-cycle (rcsc.f:
 // 1118-1444).
 //
-// One persistent block per solve (the AXI solver's structure).  Every
+// One cluster of CTAs per solve (cluster.cuh; the AXI solver's structure).  Every
 // r-line has its own matrix (the z weights of its row shift the diagonal)
 // and every z-line its own (the r weights and -1/r^2 of its column), so the
 // matrix halves of all line eliminations are done once at creation
 // (factor_pdma, one thread per line) and a sweep only carries right-hand
 // sides through them.  Line orders: the reference's (r-lines j = 1..n2-1 in
-// order, then z-lines i = 1..n1-1, on one thread: each line needs the one
+// order, then z-lines i = 1..n1-1, on one CTA: each line needs the one
 // before it) or four colours (index mod 4 = 1, 2, 3, 0: a line reads the
 // lines one and two away, never one of its colour), each colour's lines in
 // parallel.
@@ -36,8 +36,8 @@ struct StrLevel {
     double *r, *cr, *crr, *czz;
     double *ir, *irr;         // 1/r and 1/(r*r) per row (IEEE, host): the divisors' reciprocals
     double *v, *f;            // packed (n1+1)*(n2+1)
-    double *fac_r, *fac_z;    // per r-line j (5(n1-1)+1 each), per z-line i (5(n2-1)+1 each)
-    // mixed precision: FP32 copies (pivots of the factors as reciprocals)
+    double *fac_r, *fac_z;    // per r-line j (pdma_fac_len(n1-1) each), per z-line i (pdma_fac_len(n2-1))
+    // mixed precision: FP32 copies (the factors as warpline.cuh's tables)
     float *r32, *cr32, *crr32, *czz32, *v32, *f32, *fac_r32, *fac_z32;
 };
 
@@ -205,8 +205,8 @@ template <class T> __device__ __forceinline__ T str_resid(const StrView<T> &L, i
 // there asynchronously (read once, coalesced: fetched from L2 inside an
 // elimination they cost each row more than its arithmetic) while all threads
 // form the right-hand sides, the lines are eliminated (FP64: one thread per
-// line in the reference's order; FP32: one warp per line), the solutions go
-// back.  (Not inlined: one copy per type and direction keeps the
+// line in the reference's order; FP32: up to 32 lanes per line), the solutions
+// go back.  (Not inlined: one copy per type and direction keeps the
 // eliminations' register blocks free of spills.)
 template <class T, int DIR>
 __device__ __noinline__ void str_lines(const StrLevel &lev, int first, int step, int nl)

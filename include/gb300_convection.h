@@ -388,8 +388,9 @@ int gb_axi_run_end(gb_axi *h, int nsteps, double *nu, int *sweeps, int *steps_do
  * (monashubuntudir_velvor2dhorconvtankdir/sleeprun.s:1-8).  Every phase of
  * a step (each transport routine, the heat flux, the right-hand sides, the
  * update, the bookkeeping) is one launch over the blocks of all members; the
- * multigrid solves of all members are one launch, a cluster (or one CTA) per
- * equation.
+ * multigrid solves of all members are up to three launches, a cluster (or one
+ * CTA) per equation: those whose levels fit a cluster's shared memory, those
+ * on global memory, those in the reference's line order.
  * Each member runs exactly its own routines, so its fields, Nusselt history
  * and sweep counts are bit-identical to stepping it alone.
  *
@@ -521,7 +522,7 @@ int gb_r3d_nu2(gb_r3d *h, int nsteps, double *nu2);
 void *gb_r3d_stream(gb_r3d *h);
 /* Polls a grid-wide barrier wait of the cooperative multigrid launches may
  * take before the solve gives up with GB_TIMEOUT (default 2^24, about
- * 1-2 s); 0 gives up at the first wait that is not already released.  The
+ * 3 s); 0 gives up at the first wait that is not already released.  The
  * reference has no counterpart (its solves run on host threads); the
  * context stays usable after a timeout, its fields hold whatever the
  * interrupted step left. */
@@ -713,7 +714,7 @@ int gb_batch_set_exec(gb_batch *b, int mode);
 /* Total doubles of the packed f / psi arrays. */
 long long gb_batch_total_points(const gb_batch *b);
 /* Polls a grid-wide barrier wait of the persistent execution mode may take
- * before the solve gives up with GB_TIMEOUT (default 2^24, about 1-2 s);
+ * before the solve gives up with GB_TIMEOUT (default 2^24, about 3 s);
  * 0 gives up at the first wait that is not already released.  The handle
  * stays usable after a timeout. */
 int gb_batch_set_wait_limit(gb_batch *b, long long polls);
